@@ -38,11 +38,72 @@ __device__ __forceinline__ A sop(A a, A b) {
     } else if constexpr (OP == OP_MIN) return (a < b) ? a : b;
     else return (a > b) ? a : b;
 }
+// The values of a 256-lane tile's 8 warps at once, x[v] = this lane's value of
+// warp v, folded as one xor butterfly (offsets 16, 8, 4, 2, 1) per warp and
+// then ((w0, w1), (w2, w3)), ((w4, w5), (w6, w7)); the result is valid in lane
+// 0.  A butterfly adds in all 32 lanes though half of them hold a copy after
+// each step; here the first three steps give the freed half another warp's
+// values instead (lane bit 16 picks warps 0-3 or 4-7, bit 8 then bit 4 halve
+// again), so 8 warps cost 4 + 2 + 1 + 1 + 1 operations and 3 for the tile
+// instead of 40 and 7.  GB300 issues an FP64 instruction every 16 cycles per
+// SM, which is what bounds these folds.  Every operand pair, and its order in
+// lane 0's tree, is that of the separate butterflies.
 template <typename A, int OP>
-__device__ __forceinline__ A swarp(A v) {
+__device__ __forceinline__ A sop_lane(A own, A other, bool upper) {
+    if constexpr (OP == OP_SUM) return sop<A, OP>(own, other);  // commutes bit for bit
+    else return upper ? sop<A, OP>(other, own) : sop<A, OP>(own, other);
+}
+template <typename A, int OP>
+__device__ __forceinline__ A stile8(const A (&x)[8]) {
+    const unsigned lane = lane_id();
+    const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+    A a[4], b[2], c;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = sop<A, OP>(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    for (int i = 0; i < 4; i++)
+        a[i] = sop_lane<A, OP>(u16 ? x[i + 4] : x[i], __shfl_xor_sync(0xffffffffu, u16 ? x[i] : x[i + 4], 16), u16);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        b[i] = sop_lane<A, OP>(u8 ? a[i + 2] : a[i], __shfl_xor_sync(0xffffffffu, u8 ? a[i] : a[i + 2], 8), u8);
+    c = sop_lane<A, OP>(u4 ? b[1] : b[0], __shfl_xor_sync(0xffffffffu, u4 ? b[0] : b[1], 4), u4);
+    c = sop_lane<A, OP>(c, __shfl_xor_sync(0xffffffffu, c, 2), lane & 2);
+    c = sop_lane<A, OP>(c, __shfl_xor_sync(0xffffffffu, c, 1), lane & 1);
+    // lanes 4v .. 4v+3 hold warp v's value
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) c = sop<A, OP>(c, __shfl_down_sync(0xffffffffu, c, o));
+    return c;
+}
+// ... when warps 4 to 7 hold nothing but the identity
+template <typename A, int OP>
+__device__ __forceinline__ A stile4(const A (&x)[8], A ident) {
+    const unsigned lane = lane_id();
+    const bool u16 = lane & 16, u8 = lane & 8;
+    A a[2], b;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        a[i] = sop_lane<A, OP>(u16 ? x[i + 2] : x[i], __shfl_xor_sync(0xffffffffu, u16 ? x[i] : x[i + 2], 16), u16);
+    b = sop_lane<A, OP>(u8 ? a[1] : a[0], __shfl_xor_sync(0xffffffffu, u8 ? a[0] : a[1], 8), u8);
+    b = sop_lane<A, OP>(b, __shfl_xor_sync(0xffffffffu, b, 4), lane & 4);
+    b = sop_lane<A, OP>(b, __shfl_xor_sync(0xffffffffu, b, 2), lane & 2);
+    b = sop_lane<A, OP>(b, __shfl_xor_sync(0xffffffffu, b, 1), lane & 1);
+    // lanes 8v .. 8v+7 hold warp v's value
+    b = sop<A, OP>(b, __shfl_down_sync(0xffffffffu, b, 8));
+    b = sop<A, OP>(b, __shfl_down_sync(0xffffffffu, b, 16));
+    return sop<A, OP>(b, ident);
+}
+// the same for a block of 256 threads, thread t holding lane t & 31 of warp
+// t >> 5: valid in thread 0 (sh is free again after the caller's next barrier)
+template <typename A, int OP>
+__device__ __forceinline__ A sblock8(A acc, A* sh) {
+    sh[threadIdx.x] = acc;
+    __syncthreads();
+    A r = acc;
+    if (threadIdx.x < 32) {
+        A x[8];
+#pragma unroll
+        for (int v = 0; v < 8; v++) x[v] = sh[v * 32 + threadIdx.x];
+        r = stile8<A, OP>(x);
+    }
+    return r;
 }
 
 // element j of segment [s, e): x[rows[s+j]] (gather) or vals[s+j]
@@ -58,22 +119,22 @@ __device__ __forceinline__ T seg_elem(const T* __restrict__ src, const long long
     }
 }
 
-// The 16 elements k * 256 + (first - k * 256 ...) of one lane of a 256-lane
-// tile: positions first + k * 256, k = 0..15, those below `end` loaded (row
-// numbers first, then the values, so all 16 gathers are in flight together).
-template <typename T, bool GATHER>
-__device__ __forceinline__ void seg_load16(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
-                                           long long first, long long end, T v[16], bool& bad) {
+// 16 elements of one lane, STRIDE apart: positions first + k * STRIDE, k =
+// 0..15, those below `end` loaded (row numbers first, then the values, so all
+// 16 gathers are in flight together).
+template <typename T, bool GATHER, int STRIDE>
+__device__ __forceinline__ void seg_load16s(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
+                                            long long first, long long end, T v[16], bool& bad) {
     if constexpr (GATHER) {
         long long r[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-            const long long j = first + (long long)k * 256;
+            const long long j = first + (long long)k * STRIDE;
             r[k] = j < end ? rows[j] : 0;
         }
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-            const bool in = first + (long long)k * 256 < end;
+            const bool in = first + (long long)k * STRIDE < end;
             const bool ok = r[k] >= 0 && r[k] < nx;
             bad |= in && !ok;
             v[k] = (in && ok) ? src[r[k]] : T(0);
@@ -81,10 +142,16 @@ __device__ __forceinline__ void seg_load16(const T* __restrict__ src, const long
     } else {
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-            const long long j = first + (long long)k * 256;
+            const long long j = first + (long long)k * STRIDE;
             v[k] = j < end ? src[j] : T(0);
         }
     }
+}
+// the 16 elements of one lane of a 256-lane tile
+template <typename T, bool GATHER>
+__device__ __forceinline__ void seg_load16(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
+                                           long long first, long long end, T v[16], bool& bad) {
+    seg_load16s<T, GATHER, 256>(src, rows, nx, first, end, v, bad);
 }
 
 // Segments by size class, so that each is reduced by the narrowest unit that
@@ -183,15 +250,22 @@ __global__ void __launch_bounds__(256) k_seg_warps(const T* __restrict__ src, co
     if (bad) flag_error(derr, DERR_INDEX);
 }
 
-// Class 6 (33 to 4096 elements): one warp per segment walks the tile's 8
-// virtual warps, each lane's 16 elements loaded before they are added in order.
+// Class 6 (33 to 4096 elements).  What bounds it is the latency of the row
+// and value loads, so each lane has up to 16 of each in flight: a warp takes a
+// segment of up to 512 elements (two per lane of the 256-lane tile) and loads
+// all 8 virtual warps at once; the block's longer segments are taken one after
+// another by all 8 warps, warp v as virtual warp v.  (One warp walking the 8
+// virtual warps in turn, for every size: 0.98 ms against 0.50 ms for the
+// 157K mid-size groups of a 150M-row Zipf grouping.)
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256) k_seg_mid(const T* __restrict__ src, const long long* __restrict__ rows,
+__global__ void __launch_bounds__(256, 4) k_seg_mid(const T* __restrict__ src, const long long* __restrict__ rows,
                                                  long long nx, const long long* __restrict__ starts, long long ng,
                                                  long long total, const unsigned* __restrict__ ids,
                                                  const unsigned* __restrict__ cnt, A ident, A* __restrict__ out,
                                                  unsigned* derr) {
     __shared__ unsigned first;
+    __shared__ long long sbig[8];  // per warp: its segment when that is longer than 512, else -1
+    __shared__ A ws[256];
     if (threadIdx.x == 0) {
         unsigned o = 0;
         for (int c = 0; c < 6; c++) o += cnt[c];
@@ -199,29 +273,55 @@ __global__ void __launch_bounds__(256) k_seg_mid(const T* __restrict__ src, cons
     }
     __syncthreads();
     const long long n6 = cnt[6];
-    const unsigned lane = lane_id();
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     bool bad = false;
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n6; w += warps) {
-        const long long g = ids[first + w];
-        const long long s = starts[g], e = (g + 1 < ng) ? starts[g + 1] : total, m = e - s;
-        A ws[8];
+    // neighbouring segments go to different blocks: a Zipf grouping's long
+    // groups are neighbours, and a block takes its long segments in turn
+    for (long long w0 = blockIdx.x; w0 < n6; w0 += (long long)gridDim.x * 8) {
+        const long long w = w0 + (long long)gridDim.x * warp;
+        long long g = -1, s = 0, e = 0;
+        if (w < n6) {
+            g = ids[first + w];
+            s = starts[g];
+            e = (g + 1 < ng) ? starts[g + 1] : total;
+        }
+        const long long m = e - s;
+        if (lane == 0) sbig[warp] = m > 512 ? g : -1;
+        if (g >= 0 && m <= 512) {
+            T x[16];  // x[v + 8 k]: element k of lane `lane` of virtual warp v
+            seg_load16s<T, GATHER, 32>(src, rows, nx, s + lane, e, x, bad);
+            A acc[8], r;
 #pragma unroll
-        for (int v = 0; v < 8; v++) ws[v] = ident;
-        for (int v = 0; v < 8 && v * 32 < m; v++) {  // virtual warp v of the 256-lane tile
+            for (int v = 0; v < 8; v++) {
+                acc[v] = ident;
+                if (v * 32 >= m) continue;  // the whole warp: no FP64 issue for absent elements
+                if (v * 32 + (int)lane < m) acc[v] = sop<A, OP>(acc[v], (A)x[v]);
+            }
+            if (m > 256) {
+#pragma unroll
+                for (int v = 0; v < 8; v++)
+                    if (256 + v * 32 + (int)lane < m) acc[v] = sop<A, OP>(acc[v], (A)x[v + 8]);
+            }
+            if (m <= 128) r = stile4<A, OP>(acc, ident);
+            else r = stile8<A, OP>(acc);
+            if (lane == 0) out[g] = r;
+        }
+        __syncthreads();
+        for (int q = 0; q < 8; q++) {
+            const long long gb = sbig[q];  // the same in every warp
+            if (gb < 0) continue;
+            const long long sb = starts[gb], eb = (gb + 1 < ng) ? starts[gb + 1] : total;
             T x[16];
-            seg_load16<T, GATHER>(src, rows, nx, s + v * 32 + lane, e, x, bad);
+            seg_load16<T, GATHER>(src, rows, nx, sb + threadIdx.x, eb, x, bad);
             A acc = ident;
 #pragma unroll
             for (int k = 0; k < 16; k++)
-                if ((long long)k * 256 + v * 32 + lane < m) acc = sop<A, OP>(acc, (A)x[k]);
-            ws[v] = swarp<A, OP>(acc);
+                if (sb + (long long)k * 256 + threadIdx.x < eb) acc = sop<A, OP>(acc, (A)x[k]);
+            acc = sblock8<A, OP>(acc, ws);
+            if (threadIdx.x == 0) out[gb] = acc;
+            __syncthreads();
         }
-        if (lane == 0) {
-            A w01 = sop<A, OP>(ws[0], ws[1]), w23 = sop<A, OP>(ws[2], ws[3]);
-            A w45 = sop<A, OP>(ws[4], ws[5]), w67 = sop<A, OP>(ws[6], ws[7]);
-            out[g] = sop<A, OP>(sop<A, OP>(w01, w23), sop<A, OP>(w45, w67));
-        }
+        __syncthreads();  // sbig is rewritten by the next round
     }
     if (bad) flag_error(derr, DERR_INDEX);
 }
@@ -235,7 +335,7 @@ template <typename A, int OP>
 __global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ part, const long long* __restrict__ pstarts,
                                                       const long long* __restrict__ big, long long nbig,
                                                       long long nchunks, A ident, A* __restrict__ out) {
-    __shared__ A ws[8];
+    __shared__ A ws[256];
     const long long g = blockIdx.x;
     const long long s = pstarts[g], e = (g + 1 < nbig) ? pstarts[g + 1] : nchunks;
     bool bad = false;
@@ -245,14 +345,8 @@ __global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ part
 #pragma unroll
     for (int k = 0; k < 16; k++)
         if (s + k * 256 + threadIdx.x < e) acc = sop<A, OP>(acc, v[k]);
-    acc = swarp<A, OP>(acc);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        A w01 = sop<A, OP>(ws[0], ws[1]), w23 = sop<A, OP>(ws[2], ws[3]);
-        A w45 = sop<A, OP>(ws[4], ws[5]), w67 = sop<A, OP>(ws[6], ws[7]);
-        out[big[g]] = sop<A, OP>(sop<A, OP>(w01, w23), sop<A, OP>(w45, w67));
-    }
+    acc = sblock8<A, OP>(acc, ws);
+    if (threadIdx.x == 0) out[big[g]] = acc;
 }
 
 // The chunk a reduction CTA takes: from its descriptor (one 16-byte load)
@@ -285,13 +379,13 @@ __device__ __forceinline__ void chunk_of_block(const ChunkDesc* __restrict__ ord
 
 // one CTA per 4096-element chunk of the long segments
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256) k_seg_chunk(const T* __restrict__ src, const long long* __restrict__ rows,
+__global__ void __launch_bounds__(256, 4) k_seg_chunk(const T* __restrict__ src, const long long* __restrict__ rows,
                                                    long long nx, const long long* __restrict__ starts, long long ng,
                                                    long long total, const long long* __restrict__ big,
                                                    const unsigned long long* __restrict__ chunk0, long long nbig,
                                                    const ChunkDesc* __restrict__ order, A ident, A* __restrict__ part,
                                                    unsigned* derr) {
-    __shared__ A ws[8];
+    __shared__ A ws[256];
     long long c, base, e;
     chunk_of_block(order, starts, ng, total, big, chunk0, nbig, c, base, e);
     bool bad = false;
@@ -301,14 +395,8 @@ __global__ void __launch_bounds__(256) k_seg_chunk(const T* __restrict__ src, co
 #pragma unroll
     for (int k = 0; k < 16; k++)
         if (base + k * 256 + threadIdx.x < e) acc = sop<A, OP>(acc, (A)v[k]);
-    acc = swarp<A, OP>(acc);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        A w01 = sop<A, OP>(ws[0], ws[1]), w23 = sop<A, OP>(ws[2], ws[3]);
-        A w45 = sop<A, OP>(ws[4], ws[5]), w67 = sop<A, OP>(ws[6], ws[7]);
-        part[c] = sop<A, OP>(sop<A, OP>(w01, w23), sop<A, OP>(w45, w67));
-    }
+    acc = sblock8<A, OP>(acc, ws);
+    if (threadIdx.x == 0) part[c] = acc;
     if (bad) flag_error(derr, DERR_INDEX);
 }
 
@@ -658,18 +746,24 @@ static I seg_reduce(const T* src, const long long* rows, long long nx, const lon
     const unsigned *ids, *ccnt;
     HG_CHECK(seg_classes(starts, ng, total, li, &ids, &ccnt));
     const bool known = li && li->cls_known;
-    bool small = true, mid = true;
+    // warps for the small segments (32 >> c of class c each) and for the
+    // mid-size ones (one each): from the class counts when the host has
+    // them, else as many as ng segments could need.  The kernels stride over
+    // the segments, so the grid decides only how many run at once: with one
+    // thread per segment (8 warps per 256 segments) 64 plans' ~200 mid-size
+    // segments ran on 16 warps, 0.34 ms a launch against 0.01 ms now.
+    long long small_w = ng, mid_w = ng;
     if (known) {
-        small = false;
-        for (int c = 0; c < 6; c++) small = small || li->cls_host[c] != 0;
-        mid = li->cls_host[6] != 0;
+        small_w = 0;
+        for (int c = 0; c < 6; c++) small_w += (li->cls_host[c] + (32u >> c) - 1) / (32u >> c);
+        mid_w = li->cls_host[6];
     }
-    if (small)
-        HG_LAUNCH("seg_warps", gcap(ng * 4), 256, 0, (k_seg_warps<T, A, OP, GATHER>), src, rows, nx, starts, ng, total,
+    if (small_w)
+        HG_LAUNCH("seg_warps", gcap(small_w * 32), 256, 0, (k_seg_warps<T, A, OP, GATHER>), src, rows, nx, starts, ng,
+                  total, ids, ccnt, ident, out, g_derr);
+    if (mid_w)
+        HG_LAUNCH("seg_mid", gcap(mid_w * 32), 256, 0, (k_seg_mid<T, A, OP, GATHER>), src, rows, nx, starts, ng, total,
                   ids, ccnt, ident, out, g_derr);
-    if (mid)
-        HG_LAUNCH("seg_mid", gcap(ng), 256, 0, (k_seg_mid<T, A, OP, GATHER>), src, rows, nx, starts, ng, total, ids,
-                  ccnt, ident, out, g_derr);
     if (known && li->cls_host[7] == 0) return last_launch_error();
     LongPlan pl;
     HG_CHECK(seg_plan_long(starts, ng, total, li, &pl));
@@ -703,13 +797,13 @@ static I seg_reduce(const T* src, const long long* rows, long long nx, const lon
 constexpr int SEG_MANY = 4;
 struct SegCols { const double* src[SEG_MANY]; };
 template <int NCOL>
-__global__ void __launch_bounds__(256) k_seg_chunk_many(SegCols cols, int ncol, const long long* __restrict__ rows,
+__global__ void __launch_bounds__(256, 4) k_seg_chunk_many(SegCols cols, int ncol, const long long* __restrict__ rows,
                                                         long long nx, const long long* __restrict__ starts, long long ng,
                                                         long long total, const long long* __restrict__ big,
                                                         const unsigned long long* __restrict__ chunk0, long long nbig,
                                                         unsigned long long nchunks, const ChunkDesc* __restrict__ order,
                                                         double* __restrict__ part, unsigned* derr) {
-    __shared__ double ws[SEG_MANY][8];
+    __shared__ double ws[NCOL][256];
     long long c, base, e;
     chunk_of_block(order, starts, ng, total, big, chunk0, nbig, c, base, e);
     const long long first = base + threadIdx.x;
@@ -730,15 +824,16 @@ __global__ void __launch_bounds__(256) k_seg_chunk_many(SegCols cols, int ncol, 
 #pragma unroll
         for (int k = 0; k < 16; k++)
             if (first + (long long)k * 256 < e) acc = __dadd_rn(acc, v[k]);
-        acc = swarp<double, OP_SUM>(acc);
-        if ((threadIdx.x & 31) == 0) ws[q][threadIdx.x >> 5] = acc;
+        ws[q][threadIdx.x] = acc;
     }
     __syncthreads();
-    if (threadIdx.x < (unsigned)NCOL) {
-        const double* w = ws[threadIdx.x];
-        const double w01 = __dadd_rn(w[0], w[1]), w23 = __dadd_rn(w[2], w[3]);
-        const double w45 = __dadd_rn(w[4], w[5]), w67 = __dadd_rn(w[6], w[7]);
-        part[(unsigned long long)threadIdx.x * nchunks + c] = __dadd_rn(__dadd_rn(w01, w23), __dadd_rn(w45, w67));
+    const unsigned q = threadIdx.x >> 5;
+    if (q < (unsigned)NCOL) {  // warp q folds column q
+        double x[8];
+#pragma unroll
+        for (int v = 0; v < 8; v++) x[v] = ws[q][v * 32 + lane_id()];
+        const double r = stile8<double, OP_SUM>(x);
+        if (lane_id() == 0) part[(unsigned long long)q * nchunks + c] = r;
     }
     if (bad) flag_error(derr, DERR_INDEX);
 }
@@ -749,7 +844,7 @@ __global__ void __launch_bounds__(256) k_seg_partials_many(const double* __restr
                                                            const long long* __restrict__ pstarts,
                                                            const long long* __restrict__ big, long long nbig,
                                                            long long nchunks, SegOut so) {
-    __shared__ double ws[8];
+    __shared__ double ws[256];
     const long long g = blockIdx.x;
     const double* p = part + (size_t)blockIdx.y * (size_t)nchunks;
     const long long s = pstarts[g], e = (g + 1 < nbig) ? pstarts[g + 1] : nchunks;
@@ -760,14 +855,8 @@ __global__ void __launch_bounds__(256) k_seg_partials_many(const double* __restr
 #pragma unroll
     for (int k = 0; k < 16; k++)
         if (s + k * 256 + threadIdx.x < e) acc = __dadd_rn(acc, v[k]);
-    acc = swarp<double, OP_SUM>(acc);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double w01 = __dadd_rn(ws[0], ws[1]), w23 = __dadd_rn(ws[2], ws[3]);
-        const double w45 = __dadd_rn(ws[4], ws[5]), w67 = __dadd_rn(ws[6], ws[7]);
-        so.dst[blockIdx.y][big[g]] = __dadd_rn(__dadd_rn(w01, w23), __dadd_rn(w45, w67));
-    }
+    acc = sblock8<double, OP_SUM>(acc, ws);
+    if (threadIdx.x == 0) so.dst[blockIdx.y][big[g]] = acc;
 }
 
 // f64 sums of several columns over the segments of one grouping whose
