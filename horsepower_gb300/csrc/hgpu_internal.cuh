@@ -170,13 +170,15 @@ struct ListInfo {
     const long long* big;
     const unsigned long long* chunk0;
     const long long* pstarts;
-    const struct ChunkDesc* corder;  // chunk launch order (nullptr: in segment order)
+    const struct ChunkDesc* corder;  // the chunks in launch order
     // cached segment ids by size class and the class counts (output arena)
     const unsigned* cls_ids;
     const unsigned* cls_cnt;
     // host copy of the 8 class counts (cls_known), so empty classes launch nothing
     int cls_known;
     unsigned cls_host[8];
+    // 1: the plan's arrays live in scratch (a list known for one call only)
+    int scratch;
 };
 void register_list(const ListInfo& g);
 // The size classes and the long-segment plan of a list of at most

@@ -32,8 +32,8 @@ namespace hg {
 
 I scan_exclusive(const unsigned* in, long long n, unsigned long long* out, unsigned long long* total_h);
 I scan_counts(const unsigned* counts, long long n, unsigned long long* offs);
-I seg_sum_f64(const double* src, const long long* rows, long long nx, const long long* starts, long long ng,
-              long long total, double* out);
+I seg_sum_f64(const double* const* srcs, int ncol, const long long* rows, long long nx, const long long* starts,
+              long long ng, long long total, double* const* sums);
 
 constexpr int BT = 4096;  // rows per tile
 
@@ -847,7 +847,8 @@ done:
     return rc;
 }
 
-I seg_sum_f64_direct(const double* src, const long long* starts, long long ng, long long total, double* out);
+I seg_sum_f64_direct(const double* const* srcs, int ncol, const long long* starts, long long ng, long long total,
+                     double* const* sums);
 
 // The grouped path for the plans `ps` over one table set (date offsets dd
 // already computed).  Returns 1 when it ran (results in out[p], done[p] set),
@@ -922,9 +923,9 @@ static I shared_grouped(const hgpuJoinGroupPlan* plans, const std::vector<int>& 
                       (const int*)wins, npl, G, (const unsigned long long*)offs, (const unsigned long long*)base,
                       ntiles, vq, vp, vd);
             HG_CU(cudaMemcpyAsync(st, seg_start.data(), (size_t)nseg * 8, cudaMemcpyHostToDevice, g_stream));
-            HG_CHECK(seg_sum_f64_direct(vq, st, nseg, (long long)tot, res));
-            HG_CHECK(seg_sum_f64_direct(vp, st, nseg, (long long)tot, res + nseg));
-            HG_CHECK(seg_sum_f64_direct(vd, st, nseg, (long long)tot, res + 2 * nseg));
+            const double* cols[3] = {vq, vp, vd};
+            double* sums[3] = {res, res + nseg, res + 2 * nseg};
+            HG_CHECK(seg_sum_f64_direct(cols, 3, st, nseg, (long long)tot, sums));
             HG_LAUNCH("b_avg", (unsigned)((nseg + 255) / 256), 256, 0, k_b_avg, (const double*)(res + nseg),
                       (const long long*)st, nseg, (long long)tot, res + nseg);
         }
@@ -1293,9 +1294,9 @@ extern "C" I hgpuBatchJoinGroup(const hgpuJoinGroupPlan* plans, L nplans, hgpuJo
         HG_CU(cudaMemcpyAsync(dseg, segoff.data(), (np + 1) * 8, cudaMemcpyHostToDevice, g_stream));
         HG_CU(cudaMemcpyAsync(ng_dev, hg.data(), np * 4, cudaMemcpyHostToDevice, g_stream));
         HG_LAUNCH("b_starts", np, 256, 0, k_b_starts, moff, bucket, ng_dev, dseg, np, starts);
-        HG_CHECK(seg_sum_f64(vq, rows, mtot, starts, nseg, mtot, sq));
-        HG_CHECK(seg_sum_f64(vp, rows, mtot, starts, nseg, mtot, sp));
-        HG_CHECK(seg_sum_f64(vd, rows, mtot, starts, nseg, mtot, sd));
+        const double* cols[3] = {vq, vp, vd};
+        double* sums[3] = {sq, sp, sd};
+        HG_CHECK(seg_sum_f64(cols, 3, rows, mtot, starts, nseg, mtot, sums));
         HG_LAUNCH("b_avg", cap_grid(nseg), 256, 0, k_b_avg, sp, starts, nseg, mtot, sp);
     }
     std::vector<long long> hst(nseg > 0 ? nseg : 1);

@@ -154,6 +154,15 @@ __device__ __forceinline__ void seg_load16(const T* __restrict__ src, const long
     seg_load16s<T, GATHER, 256>(src, rows, nx, first, end, v, bad);
 }
 
+// The columns one launch reduces over the same segments: block row blockIdx.y
+// takes column blockIdx.y.
+constexpr int SEG_MANY = 4;
+template <typename T, typename A>
+struct SegIO {
+    const T* src[SEG_MANY];
+    A* out[SEG_MANY];
+};
+
 // Segments by size class, so that each is reduced by the narrowest unit that
 // reproduces the tile tree exactly: sizes 0-1, 2, 3-4, 5-8, 9-16, 17-32
 // (classes 0-5), 33-4096 (6) and longer (7).
@@ -165,16 +174,24 @@ __device__ __forceinline__ int seg_class(long long m) {
     if (m > 32) return 6;
     return 32 - __clz((int)(m - 1));  // ceil(log2 m): 2 -> 1, 3-4 -> 2, ..., 17-32 -> 5
 }
-// pass 1: segments per class (cnt[c])
+// pass 1: segments per class (cnt[c]) and the 4096-element chunks of the long
+// ones, in all (*nch)
 __global__ void k_seg_class_count(const long long* __restrict__ starts, long long ng, long long total,
-                                  unsigned* __restrict__ cnt) {
+                                  unsigned* __restrict__ cnt, unsigned long long* __restrict__ nch) {
     __shared__ unsigned sc[SEG_CLASSES];
+    __shared__ unsigned long long snch;
     if (threadIdx.x < SEG_CLASSES) sc[threadIdx.x] = 0;
+    if (threadIdx.x == 0) snch = 0;
     __syncthreads();
     const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (g < ng) atomicAdd(&sc[seg_class(((g + 1 < ng) ? starts[g + 1] : total) - starts[g])], 1u);
+    if (g < ng) {
+        const long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
+        atomicAdd(&sc[seg_class(m)], 1u);
+        if (m > TILE_SUM) atomicAdd(&snch, (unsigned long long)((m + TILE_SUM - 1) / TILE_SUM));
+    }
     __syncthreads();
     if (threadIdx.x < SEG_CLASSES && sc[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], sc[threadIdx.x]);
+    if (threadIdx.x == 0 && snch) atomicAdd(nch, snch);
 }
 // pass 2: the segment ids of class c at ids[off_c ...] (off_c = segments of
 // lower classes; order inside a class is immaterial); cur[c] counts the
@@ -208,11 +225,13 @@ __global__ void k_seg_class_ids(const long long* __restrict__ starts, long long 
 // tile tree reduces to the xor butterfly over the first P lanes; a warp
 // reduces 32 / P such segments in sub-warps of P lanes.
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256) k_seg_warps(const T* __restrict__ src, const long long* __restrict__ rows,
+__global__ void __launch_bounds__(256) k_seg_warps(SegIO<T, A> io, const long long* __restrict__ rows,
                                                    long long nx, const long long* __restrict__ starts, long long ng,
                                                    long long total, const unsigned* __restrict__ ids,
-                                                   const unsigned* __restrict__ cnt, A ident, A* __restrict__ out,
+                                                   const unsigned* __restrict__ cnt, A ident,
                                                    unsigned* derr) {
+    const T* __restrict__ src = io.src[blockIdx.y];
+    A* __restrict__ out = io.out[blockIdx.y];
     __shared__ long long wfirst[7];  // first warp of each class 0-5; wfirst[6] = warps in all
     __shared__ unsigned cfirst[6];   // first id of each class
     if (threadIdx.x == 0) {
@@ -255,14 +274,16 @@ __global__ void __launch_bounds__(256) k_seg_warps(const T* __restrict__ src, co
 // segment of up to 512 elements (two per lane of the 256-lane tile) and loads
 // all 8 virtual warps at once; the block's longer segments are taken one after
 // another by all 8 warps, warp v as virtual warp v.  (One warp walking the 8
-// virtual warps in turn, for every size: 0.98 ms against 0.50 ms for the
+// virtual warps in turn, for every size: 0.98 ms against 0.61 ms for the
 // 157K mid-size groups of a 150M-row Zipf grouping.)
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256, 4) k_seg_mid(const T* __restrict__ src, const long long* __restrict__ rows,
+__global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long long* __restrict__ rows,
                                                  long long nx, const long long* __restrict__ starts, long long ng,
                                                  long long total, const unsigned* __restrict__ ids,
-                                                 const unsigned* __restrict__ cnt, A ident, A* __restrict__ out,
+                                                 const unsigned* __restrict__ cnt, A ident,
                                                  unsigned* derr) {
+    const T* __restrict__ src = io.src[blockIdx.y];
+    A* __restrict__ out = io.out[blockIdx.y];
     __shared__ unsigned first;
     __shared__ long long sbig[8];  // per warp: its segment when that is longer than 512, else -1
     __shared__ A ws[256];
@@ -332,11 +353,13 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(const T* __restrict__ src, c
 // follow, whatever size class would have scheduled the segment); the result
 // goes straight to the segment's slot of out.
 template <typename A, int OP>
-__global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ part, const long long* __restrict__ pstarts,
+__global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ parts, const long long* __restrict__ pstarts,
                                                       const long long* __restrict__ big, long long nbig,
-                                                      long long nchunks, A ident, A* __restrict__ out) {
+                                                      long long nchunks, A ident, SegIO<A, A> io) {
     __shared__ A ws[256];
     const long long g = blockIdx.x;
+    const A* __restrict__ part = parts + (size_t)blockIdx.y * (size_t)nchunks;
+    A* __restrict__ out = io.out[blockIdx.y];
     const long long s = pstarts[g], e = (g + 1 < nbig) ? pstarts[g + 1] : nchunks;
     bool bad = false;
     A v[16];
@@ -349,45 +372,18 @@ __global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ part
     if (threadIdx.x == 0) out[big[g]] = acc;
 }
 
-// The chunk a reduction CTA takes: from its descriptor (one 16-byte load)
-// when the chunks run in a planned order, else chunk blockIdx.x, found
-// among the long segments by a binary search over their first chunks.
-// base = its first element, e = one past its last (at most base + 4096).
-__device__ __forceinline__ void chunk_of_block(const ChunkDesc* __restrict__ order, const long long* __restrict__ starts,
-                                               long long ng, long long total, const long long* __restrict__ big,
-                                               const unsigned long long* __restrict__ chunk0, long long nbig,
-                                               long long& c, long long& base, long long& e) {
-    if (order) {
-        const ChunkDesc d = order[blockIdx.x];
-        c = d.chunk;
-        base = d.first;
-        e = d.first + d.len;
-        return;
-    }
-    c = blockIdx.x;
-    long long lo = 0, hi = nbig - 1;  // the long segment owning chunk c
-    while (lo < hi) {
-        long long mid = (lo + hi + 1) >> 1;
-        if ((long long)chunk0[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    const long long g = big[lo];
-    const long long s = starts[g];
-    const long long se = (g + 1 < ng) ? starts[g + 1] : total;
-    base = s + (c - (long long)chunk0[lo]) * TILE_SUM;
-    e = se < base + TILE_SUM ? se : base + TILE_SUM;
-}
-
-// one CTA per 4096-element chunk of the long segments
+// one CTA per 4096-element chunk of the long segments, each from its
+// descriptor (one 16-byte load; finding the chunk by a binary search over the
+// segments instead put seven dependent loads before its first row)
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256, 4) k_seg_chunk(const T* __restrict__ src, const long long* __restrict__ rows,
-                                                   long long nx, const long long* __restrict__ starts, long long ng,
-                                                   long long total, const long long* __restrict__ big,
-                                                   const unsigned long long* __restrict__ chunk0, long long nbig,
-                                                   const ChunkDesc* __restrict__ order, A ident, A* __restrict__ part,
-                                                   unsigned* derr) {
+__global__ void __launch_bounds__(256, 4) k_seg_chunk(SegIO<T, A> io, const long long* __restrict__ rows,
+                                                      long long nx, const ChunkDesc* __restrict__ order, A ident,
+                                                      A* __restrict__ part, unsigned* derr) {
+    const T* __restrict__ src = io.src[blockIdx.y];
+    part += (size_t)blockIdx.y * gridDim.x;
     __shared__ A ws[256];
-    long long c, base, e;
-    chunk_of_block(order, starts, ng, total, big, chunk0, nbig, c, base, e);
+    const ChunkDesc d = order[blockIdx.x];
+    const long long base = d.first, e = d.first + d.len;
     bool bad = false;
     T v[16];
     seg_load16<T, GATHER>(src, rows, nx, base + threadIdx.x, e, v, bad);
@@ -396,47 +392,121 @@ __global__ void __launch_bounds__(256, 4) k_seg_chunk(const T* __restrict__ src,
     for (int k = 0; k < 16; k++)
         if (base + k * 256 + threadIdx.x < e) acc = sop<A, OP>(acc, (A)v[k]);
     acc = sblock8<A, OP>(acc, ws);
-    if (threadIdx.x == 0) part[c] = acc;
+    if (threadIdx.x == 0) part[d.chunk] = acc;
     if (bad) flag_error(derr, DERR_INDEX);
 }
 
-__global__ void k_big_flags(const long long* __restrict__ starts, long long ng, long long total, uint8_t* __restrict__ f,
-                            unsigned* __restrict__ nch) {
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
-        long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
-        f[g] = m > TILE_SUM;
-        if (nch) nch[g] = 0;
+// The long segments of a list from the ids of their class: big[k], the first
+// chunk of each (c0, and as i64 in ps), in one block (a list of 2^31 rows has
+// fewer than 2^19 of them).
+__global__ void __launch_bounds__(1024) k_big_plan(const long long* __restrict__ starts, long long ng, long long total,
+                                                   const unsigned* __restrict__ ids, long long nbig,
+                                                   long long* __restrict__ big, unsigned long long* __restrict__ c0,
+                                                   long long* __restrict__ ps) {
+    __shared__ unsigned long long wsum[32];
+    __shared__ unsigned long long carry;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (long long b = 0; b < nbig; b += 1024) {
+        const long long k = b + threadIdx.x;
+        long long g = 0;
+        unsigned long long n = 0;
+        if (k < nbig) {
+            g = ids[k];
+            const long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
+            n = (unsigned long long)((m + TILE_SUM - 1) / TILE_SUM);
+        }
+        const unsigned long long incl = warp_incl_scan64(n);
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned long long x = wsum[lane];
+            wsum[lane] = warp_incl_scan64(x) - x;
+        }
+        __syncthreads();
+        const unsigned long long first = carry + wsum[warp] + incl - n;
+        if (k < nbig) {
+            big[k] = g;
+            c0[k] = first;
+            ps[k] = (long long)first;
+        }
+        __syncthreads();
+        if (threadIdx.x == 1023) carry = first + n;
+        __syncthreads();
     }
 }
-__global__ void k_big_chunks(const long long* __restrict__ starts, long long ng, long long total,
-                             const long long* __restrict__ big, long long nbig, unsigned* __restrict__ nch) {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nbig; k += (long long)gridDim.x * blockDim.x) {
-        long long g = big[k];
-        long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
-        nch[k] = (unsigned)((m + TILE_SUM - 1) / TILE_SUM);
+// The descriptors of a general list's chunks, one thread each, and for a
+// gather the order in which they run: by the region of the source column that
+// their middle row lies in (nx >> shift < CHUNK_BUCKETS regions), so that the
+// CTAs resident together gather from one region in every segment and a sector
+// fetched for one is still in L2 for the others.  A counting sort: the
+// descriptors and the regions' counts, the regions' first places, the
+// descriptors placed.  Only the schedule depends on the order, so chunks of
+// one region may come in any order, and a row outside the column only puts
+// its chunk into the first or last region.  (150M Zipf rows, 25K chunks of
+// 1640 segments: ranking every chunk against every segment took 0.12 ms.)
+// Without `region` the descriptors stay in segment order.
+constexpr int CHUNK_BUCKETS = 4096;
+__global__ void k_chunk_desc(const long long* __restrict__ rows, const long long* __restrict__ starts, long long ng,
+                             long long total, const long long* __restrict__ big,
+                             const unsigned long long* __restrict__ c0, long long nbig, long long nchunks, int shift,
+                             ChunkDesc* __restrict__ desc, unsigned short* __restrict__ region,
+                             unsigned* __restrict__ hist) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= nchunks) return;
+    long long lo = 0, hi = nbig - 1;  // the long segment owning chunk t
+    while (lo < hi) {
+        const long long mid = (lo + hi + 1) >> 1;
+        if ((long long)c0[mid] <= t) lo = mid; else hi = mid - 1;
     }
+    const long long g = big[lo], s = starts[g], e = (g + 1 < ng) ? starts[g + 1] : total;
+    const long long first = s + (t - (long long)c0[lo]) * TILE_SUM;
+    const long long len = e - first < TILE_SUM ? e - first : TILE_SUM;
+    desc[t] = ChunkDesc{first, (unsigned)len, (unsigned)t};
+    if (region) {
+        const long long r = rows[first + len / 2] >> shift;
+        const unsigned b = r < 0 ? 0u : (r >= CHUNK_BUCKETS ? CHUNK_BUCKETS - 1u : (unsigned)r);
+        region[t] = (unsigned short)b;
+        atomicAdd(&hist[b], 1u);
+    }
+}
+__global__ void __launch_bounds__(1024) k_chunk_regions(unsigned* __restrict__ hist) {
+    __shared__ unsigned wsum[32];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    uint4* h4 = reinterpret_cast<uint4*>(hist);  // CHUNK_BUCKETS = 4 per thread
+    const uint4 v = h4[threadIdx.x];
+    const unsigned n = v.x + v.y + v.z + v.w, incl = warp_incl_scan(n);
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned x = wsum[lane];
+        wsum[lane] = warp_incl_scan(x) - x;
+    }
+    __syncthreads();
+    const unsigned o = wsum[warp] + incl - n;
+    h4[threadIdx.x] = make_uint4(o, o + v.x, o + v.x + v.y, o + v.x + v.y + v.z);
+}
+__global__ void k_chunk_place(const ChunkDesc* __restrict__ desc, const unsigned short* __restrict__ region,
+                              long long nchunks, unsigned* __restrict__ next, ChunkDesc* __restrict__ order) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t < nchunks) order[atomicAdd(&next[region[t]], 1u)] = desc[t];
 }
 template <typename A>
 __global__ void k_scatter_big(const A* __restrict__ r, const long long* __restrict__ big, long long nbig, A* __restrict__ out) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nbig; k += (long long)gridDim.x * blockDim.x)
         out[big[k]] = r[k];
 }
-// The chunk starts as i64 and, for a few long segments, the order in which
-// the chunk CTAs run.  A segment's rows are spread over the whole source
-// column, so running one segment's chunks after another's would sweep the
-// column once per segment.  Instead chunk (k, c) of long segment k (n_k
-// chunks) runs at the rank of its relative position (2c + 1) / (2 n_k), ties
-// to the lower k: the CTAs resident together then cover the same region of
-// the column in every segment, and a sector fetched for one segment is
-// still in L2 when the others reach it.  Only the schedule changes; each
-// chunk's partial lands at its own index as before.
-// Chunk orders are built for 2..CHUNK_ORDER_MAX_SEGS long segments (each
-// chunk's rank costs one step per long segment), by one CTA from shared
-// memory for the lists @group plans (at most CHUNK_ORDER_SMALL_SEGS).
-constexpr long long CHUNK_ORDER_MAX_SEGS = 2048;
+// The chunk order of a list that @group plans itself (at most
+// CHUNK_ORDER_SMALL_SEGS long segments, all in shared memory): a segment's
+// rows are spread over the whole source column, so running one segment's
+// chunks after another's would sweep the column once per segment.  Instead
+// chunk (k, c) of long segment k (n_k chunks) runs at the rank of its relative
+// position (2c + 1) / (2 n_k), ties to the lower k.  Only the schedule
+// changes; each chunk's partial lands at its own index as before.
 constexpr long long CHUNK_ORDER_SMALL_SEGS = 64;
 // below this many elements the values of a list fit in L2 whatever the
-// order, and the general plan builds none (it costs a launch's worth of work)
+// order, and the general plan builds none (it costs three launches)
 constexpr long long CHUNK_ORDER_MIN_TOTAL = 4ll << 20;
 // order[rank of chunk t] = chunk t's descriptor, for chunk t of nchunks (c0:
 // the long segments' first chunks; seg_first/seg_end(k): long segment k's
@@ -467,51 +537,6 @@ __device__ __forceinline__ void chunk_rank(const unsigned long long* c0, long lo
     const long long len = se - first < TILE_SUM ? se - first : TILE_SUM;
     order[rank] = ChunkDesc{first, (unsigned)len, (unsigned)t};
 }
-// The general plan: ps = the first chunks as i64 and, with `order`, the
-// chunk order of up to CHUNK_ORDER_MAX_SEGS long segments, one warp per chunk
-// (the lanes share the walk over the other segments).
-__global__ void k_chunk_plan(const unsigned long long* __restrict__ c0, long long nbig, unsigned long long nchunks,
-                             const long long* __restrict__ starts, long long ng, long long total,
-                             const long long* __restrict__ big, long long* __restrict__ ps,
-                             ChunkDesc* __restrict__ order) {
-    extern __shared__ unsigned long long sc0[];  // the first chunks, when there is an order to build
-    const long long nth = (long long)gridDim.x * blockDim.x;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nbig; t += nth) ps[t] = (long long)c0[t];
-    if (!order) return;
-    for (long long k = threadIdx.x; k < nbig; k += blockDim.x) sc0[k] = c0[k];
-    __syncthreads();
-    const unsigned lane = lane_id();
-    const long long nwarps = nth >> 5;
-    for (long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; t < (long long)nchunks; t += nwarps) {
-        long long lo = 0, hi = nbig - 1;  // the long segment owning chunk t
-        while (lo < hi) {
-            const long long mid = (lo + hi + 1) >> 1;
-            if ((long long)sc0[mid] <= t) lo = mid; else hi = mid - 1;
-        }
-        const long long k = lo, c = t - (long long)sc0[k];
-        const long long nk = (long long)((k + 1 < nbig ? sc0[k + 1] : nchunks) - sc0[k]);
-        long long part = 0;
-        for (long long k2 = lane; k2 < nbig; k2 += 32) {
-            if (k2 == k) continue;
-            const long long n2 = (long long)((k2 + 1 < nbig ? sc0[k2 + 1] : nchunks) - sc0[k2]);
-            // chunks c2 of segment k2 placed before (k, c): (2 c2 + 1) n_k < (2c + 1) n2, or equal and k2 < k
-            const long long x = (2 * c + 1) * n2 + (k2 < k ? 1 : 0);
-            const long long q = x <= 0xffffffffll ? (long long)((unsigned)(x - 1) / (unsigned)nk) : (x - 1) / nk;
-            const long long cnt = (q + 1) / 2;
-            part += cnt < n2 ? cnt : n2;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) {
-            const long long g = big[k];
-            const long long sf = starts[g], se = (g + 1 < ng) ? starts[g + 1] : total;
-            const long long first = sf + c * TILE_SUM;
-            const long long len = se - first < TILE_SUM ? se - first : TILE_SUM;
-            order[c + part] = ChunkDesc{first, (unsigned)len, (unsigned)t};
-        }
-    }
-}
-
 // The whole plan of a list of at most SEG_PLAN_SMALL segments in one CTA of
 // 1024 threads (four consecutive segments each): the class counts and ids
 // of seg_classes, then the long segments in ascending order with their
@@ -607,7 +632,7 @@ __global__ void __launch_bounds__(1024) k_seg_plan_small(const long long* __rest
         f = sfirst[k];
         e = send[k];
     };
-    if (order && nbig > 1 && nbig <= CHUNK_ORDER_SMALL_SEGS)  // the long segments from shared memory
+    if (nbig <= CHUNK_ORDER_SMALL_SEGS)  // the long segments from shared memory
         for (long long q = t; q < (long long)nchunks; q += 1024) chunk_rank(sc0, nbig, nchunks, q, order, range);
 }
 
@@ -616,85 +641,73 @@ static unsigned gcap(long long n, int per = 256) {
     return g > (unsigned)g_sms * 32 ? (unsigned)g_sms * 32 : g;
 }
 
-// Segment ids by size class (kept with the list when there is one, with a
-// host copy of the class counts so that empty classes launch nothing).
-static I seg_classes(const long long* starts, long long ng, long long total, ListInfo* li, const unsigned** ids,
-                     const unsigned** ccnt) {
-    if (li && li->cls_ids) {
-        *ids = li->cls_ids;
-        *ccnt = li->cls_cnt;
-        return 0;
-    }
-    unsigned* cc = (unsigned*)(li ? dalloc(2 * SEG_CLASSES * 4) : salloc(2 * SEG_CLASSES * 4));
-    unsigned* id = (unsigned*)(li ? dalloc((size_t)ng * 4) : salloc((size_t)ng * 4));
-    if (!cc || !id) return E_DEVICE_OOM;
-    HG_CU(cudaMemsetAsync(cc, 0, 2 * SEG_CLASSES * 4, g_stream));
-    const unsigned gb = (unsigned)((ng + 255) / 256);
-    HG_LAUNCH("seg_class", gb, 256, 0, k_seg_class_count, starts, ng, total, cc);
-    HG_LAUNCH("seg_class_ids", gb, 256, 0, k_seg_class_ids, starts, ng, total, (const unsigned*)cc,
-              cc + SEG_CLASSES, id);
-    *ids = id;
-    *ccnt = cc;
-    if (li) {
+// Segment ids by size class and the split of the segments longer than one
+// tile into chunks, kept with the list: the class counts and the number of
+// chunks come back in one round trip (empty classes then launch nothing),
+// the rest is queued.  `rows` (the row ids behind a gather, or null) gives the
+// chunks their launch order.
+static I seg_plan(const long long* starts, long long ng, long long total, const long long* rows, long long nx,
+                  ListInfo* li) {
+    auto alloc = [li](size_t bytes) { return li->scratch ? salloc(bytes) : dalloc(bytes); };
+    if (!li->cls_ids) {
+        unsigned* cc = (unsigned*)alloc(2 * SEG_CLASSES * 4 + 8);
+        unsigned* id = (unsigned*)alloc((size_t)ng * 4);
+        if (!cc || !id) return E_DEVICE_OOM;
+        unsigned long long* nch = (unsigned long long*)(cc + 2 * SEG_CLASSES);
+        HG_CU(cudaMemsetAsync(cc, 0, 2 * SEG_CLASSES * 4 + 8, g_stream));
+        const unsigned gb = (unsigned)((ng + 255) / 256);
+        HG_LAUNCH("seg_class", gb, 256, 0, k_seg_class_count, starts, ng, total, cc, nch);
+        HG_LAUNCH("seg_class_ids", gb, 256, 0, k_seg_class_ids, starts, ng, total, (const unsigned*)cc,
+                  cc + SEG_CLASSES, id);
+        HG_CHECK(last_launch_error());
+        unsigned long long hn = 0;
+        HG_CHECK(rb_queue(li->cls_host, cc, sizeof(li->cls_host)));
+        HG_CHECK(rb_queue(&hn, nch, 8));
+        HG_CU(stream_sync());
         li->cls_ids = id;
         li->cls_cnt = cc;
-        // a list's segments are reduced several times (one aggregate per
-        // column): read the class counts once, so empty classes are skipped
-        HG_CHECK(rb_queue(li->cls_host, cc, sizeof(li->cls_host)));
-        HG_CU(stream_sync());
         li->cls_known = 1;
-    }
-    return last_launch_error();
-}
-
-// The split of the segments longer than one tile into 4096-element chunks:
-// big[k] = the k-th long segment, chunk0[k] its first chunk, pstarts[k] the
-// same as i64, nchunks in all (kept with the list when there is one).
-struct LongPlan {
-    long long nbig = 0;
-    unsigned long long nchunks = 0;
-    const long long* big = nullptr;
-    const unsigned long long* c0 = nullptr;
-    const long long* pstarts = nullptr;
-    const ChunkDesc* order = nullptr;
-};
-static I seg_plan_long(const long long* starts, long long ng, long long total, ListInfo* li, LongPlan* pl) {
-    if (li && li->planned) {
-        pl->nbig = li->nbig; pl->nchunks = li->nchunks; pl->big = li->big; pl->c0 = li->chunk0; pl->pstarts = li->pstarts;
-        pl->order = li->corder;
-        return 0;
-    }
-    uint8_t* f = (uint8_t*)salloc((size_t)ng);
-    long long* bigs = (long long*)(li ? dalloc((size_t)ng * 8) : salloc((size_t)ng * 8));
-    if (!f || !bigs) return E_DEVICE_OOM;
-    HG_LAUNCH("seg_flags", gcap(ng), 256, 0, k_big_flags, starts, ng, total, f, (unsigned*)nullptr);
-    long long nbig = 0;
-    unsigned long long nchunks = 0;
-    HG_CHECK(compact_rows(f, ng, bigs, &nbig));
-    unsigned* nch = (unsigned*)salloc((size_t)(nbig > 0 ? nbig : 1) * 4);
-    unsigned long long* c0s = (unsigned long long*)(li ? dalloc((size_t)(nbig > 0 ? nbig : 1) * 8) : salloc((size_t)(nbig > 0 ? nbig : 1) * 8));
-    long long* ps = (long long*)(li ? dalloc((size_t)(nbig > 0 ? nbig : 1) * 8) : salloc((size_t)(nbig > 0 ? nbig : 1) * 8));
-    if (!nch || !c0s || !ps) return E_DEVICE_OOM;
-    ChunkDesc* order = nullptr;
-    if (nbig > 0) {
-        HG_LAUNCH("seg_chunks", gcap(nbig), 256, 0, k_big_chunks, starts, ng, total, bigs, nbig, nch);
-        HG_CHECK(scan_exclusive(nch, nbig, c0s, &nchunks));
-        if (nbig > 1 && nbig <= CHUNK_ORDER_MAX_SEGS && total >= CHUNK_ORDER_MIN_TOTAL) {
-            const size_t ob = (size_t)nchunks * sizeof(ChunkDesc);
-            order = (ChunkDesc*)(li ? dalloc(ob) : salloc(ob));
-            if (!order) return E_DEVICE_OOM;
+        if (!li->planned) {
+            li->nbig = li->cls_host[7];
+            li->nchunks = hn;
         }
-        const long long nt = nbig > (long long)nchunks ? nbig : (long long)nchunks;
-        const size_t csm = order ? (size_t)nbig * 8 : 0;  // at most 16 KB
-        const long long nthreads = order ? (long long)nchunks * 32 : nt;  // a warp per chunk for the order
-        HG_LAUNCH("chunk_plan", gcap(nthreads), 256, csm, k_chunk_plan, c0s, nbig, nchunks, starts, ng, total, bigs, ps,
-                  order);
     }
-    pl->nbig = nbig; pl->nchunks = nchunks; pl->big = bigs; pl->c0 = c0s; pl->pstarts = ps; pl->order = order;
-    if (li) {
-        li->planned = 1; li->nbig = nbig; li->nchunks = nchunks; li->big = bigs; li->chunk0 = c0s; li->pstarts = ps;
+    if (li->planned) return 0;
+    const long long nbig = li->nbig;
+    if (nbig > 0) {
+        long long* big = (long long*)alloc((size_t)nbig * 8);
+        unsigned long long* c0 = (unsigned long long*)alloc((size_t)nbig * 8);
+        long long* ps = (long long*)alloc((size_t)nbig * 8);
+        if (!big || !c0 || !ps) return E_DEVICE_OOM;
+        unsigned before = 0;  // ids of the classes below
+        for (int c = 0; c < 7; c++) before += li->cls_host[c];
+        HG_LAUNCH("big_plan", 1, 1024, 0, k_big_plan, starts, ng, total, li->cls_ids + before, nbig, big, c0, ps);
+        const long long nchunks = (long long)li->nchunks;
+        const unsigned cb = grid_for(nchunks, 256);
+        ChunkDesc* order = (ChunkDesc*)alloc((size_t)nchunks * sizeof(ChunkDesc));
+        if (!order) return E_DEVICE_OOM;
+        if (rows && nbig > 1 && total >= CHUNK_ORDER_MIN_TOTAL) {
+            ChunkDesc* desc = (ChunkDesc*)salloc((size_t)nchunks * sizeof(ChunkDesc));
+            unsigned short* region = (unsigned short*)salloc((size_t)nchunks * 2);
+            unsigned* hist = (unsigned*)salloc(CHUNK_BUCKETS * 4);
+            if (!desc || !region || !hist) return E_DEVICE_OOM;
+            int shift = 0;
+            while ((nx >> shift) >= CHUNK_BUCKETS) shift++;
+            HG_CU(cudaMemsetAsync(hist, 0, CHUNK_BUCKETS * 4, g_stream));
+            HG_LAUNCH("chunk_desc", cb, 256, 0, k_chunk_desc, rows, starts, ng, total, big, c0, nbig, nchunks, shift,
+                      desc, region, hist);
+            HG_LAUNCH("chunk_regions", 1, 1024, 0, k_chunk_regions, hist);
+            HG_LAUNCH("chunk_place", cb, 256, 0, k_chunk_place, desc, region, nchunks, hist, order);
+        } else {
+            HG_LAUNCH("chunk_desc", cb, 256, 0, k_chunk_desc, (const long long*)nullptr, starts, ng, total, big, c0,
+                      nbig, nchunks, 0, order, (unsigned short*)nullptr, (unsigned*)nullptr);
+        }
         li->corder = order;
+        li->big = big;
+        li->chunk0 = c0;
+        li->pstarts = ps;
     }
+    li->planned = 1;
     return last_launch_error();
 }
 
@@ -707,11 +720,11 @@ I seg_plan_small(const long long* starts, long long ng, long long total, SmallPl
     p->big = (long long*)dalloc((size_t)ng * 8);
     p->c0 = (unsigned long long*)dalloc((size_t)ng * 8);
     p->ps = (long long*)dalloc((size_t)ng * 8);
-    p->order = ng > 1 ? (ChunkDesc*)dalloc(maxch * sizeof(ChunkDesc)) : nullptr;
+    p->order = (ChunkDesc*)dalloc(maxch * sizeof(ChunkDesc));
     unsigned long long* hd = (unsigned long long*)salloc(16 * 8);
     p->hdr = (unsigned long long*)halloc(16 * 8);
     if (p->hdr) memset(p->hdr, 0, 16 * 8);
-    if (!p->cc || !p->ids || !p->big || !p->c0 || !p->ps || (ng > 1 && !p->order) || !hd || !p->hdr) {
+    if (!p->cc || !p->ids || !p->big || !p->c0 || !p->ps || !p->order || !hd || !p->hdr) {
         *p = SmallPlan{};
         return E_DEVICE_OOM;
     }
@@ -727,65 +740,13 @@ void seg_plan_adopt(ListInfo& li, const SmallPlan& p) {
     li.cls_cnt = p.cc;
     for (int c = 0; c < SEG_CLASSES; c++) li.cls_host[c] = (unsigned)p.hdr[c];
     li.cls_known = 1;
-    li.planned = 1;
     li.nbig = (long long)p.hdr[SEG_CLASSES];
     li.nchunks = p.hdr[SEG_CLASSES + 1];
     li.big = p.big;
     li.chunk0 = p.c0;
     li.pstarts = p.ps;
-    li.corder = (li.nbig > 1 && li.nbig <= CHUNK_ORDER_SMALL_SEGS) ? p.order : nullptr;
-}
-
-// Reduces every segment of (src via rows | src) into out[ng] (device).  When
-// `li` is given, the split of the long segments is computed once per list
-// and kept with it.
-template <typename T, typename A, int OP, bool GATHER>
-static I seg_reduce(const T* src, const long long* rows, long long nx, const long long* starts, long long ng,
-                    long long total, A ident, A* out, ListInfo* li = nullptr) {
-    if (ng == 0) return 0;
-    const unsigned *ids, *ccnt;
-    HG_CHECK(seg_classes(starts, ng, total, li, &ids, &ccnt));
-    const bool known = li && li->cls_known;
-    // warps for the small segments (32 >> c of class c each) and for the
-    // mid-size ones (one each): from the class counts when the host has
-    // them, else as many as ng segments could need.  The kernels stride over
-    // the segments, so the grid decides only how many run at once: with one
-    // thread per segment (8 warps per 256 segments) 64 plans' ~200 mid-size
-    // segments ran on 16 warps, 0.34 ms a launch against 0.01 ms now.
-    long long small_w = ng, mid_w = ng;
-    if (known) {
-        small_w = 0;
-        for (int c = 0; c < 6; c++) small_w += (li->cls_host[c] + (32u >> c) - 1) / (32u >> c);
-        mid_w = li->cls_host[6];
-    }
-    if (small_w)
-        HG_LAUNCH("seg_warps", gcap(small_w * 32), 256, 0, (k_seg_warps<T, A, OP, GATHER>), src, rows, nx, starts, ng,
-                  total, ids, ccnt, ident, out, g_derr);
-    if (mid_w)
-        HG_LAUNCH("seg_mid", gcap(mid_w * 32), 256, 0, (k_seg_mid<T, A, OP, GATHER>), src, rows, nx, starts, ng, total,
-                  ids, ccnt, ident, out, g_derr);
-    if (known && li->cls_host[7] == 0) return last_launch_error();
-    LongPlan pl;
-    HG_CHECK(seg_plan_long(starts, ng, total, li, &pl));
-    const long long nbig = pl.nbig;
-    const unsigned long long nchunks = pl.nchunks;
-    if (nbig == 0) return last_launch_error();
-    A* part = (A*)salloc((size_t)nchunks * sizeof(A));
-    A* res = (A*)salloc((size_t)nbig * sizeof(A));
-    if (!part || !res) return E_DEVICE_OOM;
-    HG_LAUNCH("seg_chunk", (unsigned)nchunks, 256, 0, (k_seg_chunk<T, A, OP, GATHER>), src, rows, nx, starts, ng,
-              total, pl.big, pl.c0, nbig, pl.order, ident, part, g_derr);
-    // partials of each long segment are reduced by the same procedure: at
-    // most 4096 of them per segment (certain when there are at most 4096 in
-    // all) in one launch straight into out, else as segments of their own
-    if (nchunks <= (unsigned long long)TILE_SUM) {
-        HG_LAUNCH("seg_partials", (unsigned)nbig, 256, 0, (k_seg_partials<A, OP>), part, pl.pstarts, pl.big, nbig,
-                  (long long)nchunks, ident, out);
-        return last_launch_error();
-    }
-    HG_CHECK((seg_reduce<A, A, OP, false>(part, nullptr, 0, pl.pstarts, nbig, (long long)nchunks, ident, res)));
-    HG_LAUNCH("scatter_big", gcap(nbig), 256, 0, k_scatter_big<A>, res, pl.big, nbig, out);
-    return last_launch_error();
+    li.corder = p.order;
+    li.planned = li.nbig <= CHUNK_ORDER_SMALL_SEGS;  // else its first aggregation orders the chunks
 }
 
 // ---- several f64 sums over the long segments of one grouping at once.
@@ -794,19 +755,15 @@ static I seg_reduce(const T* src, const long long* rows, long long nx, const lon
 // 16 x ncol gathers of a lane issued before the first add); each column's
 // chunk partial follows the tile tree, so part[col * nchunks + c] is
 // bit-identical to k_seg_chunk's for that column.
-constexpr int SEG_MANY = 4;
 struct SegCols { const double* src[SEG_MANY]; };
 template <int NCOL>
-__global__ void __launch_bounds__(256, 4) k_seg_chunk_many(SegCols cols, int ncol, const long long* __restrict__ rows,
-                                                        long long nx, const long long* __restrict__ starts, long long ng,
-                                                        long long total, const long long* __restrict__ big,
-                                                        const unsigned long long* __restrict__ chunk0, long long nbig,
-                                                        unsigned long long nchunks, const ChunkDesc* __restrict__ order,
-                                                        double* __restrict__ part, unsigned* derr) {
+__global__ void __launch_bounds__(256, 4) k_seg_chunk_many(SegCols cols, const long long* __restrict__ rows, long long nx,
+                                                           unsigned long long nchunks,
+                                                           const ChunkDesc* __restrict__ order,
+                                                           double* __restrict__ part, unsigned* derr) {
     __shared__ double ws[NCOL][256];
-    long long c, base, e;
-    chunk_of_block(order, starts, ng, total, big, chunk0, nbig, c, base, e);
-    const long long first = base + threadIdx.x;
+    const ChunkDesc d = order[blockIdx.x];
+    const long long first = d.first + threadIdx.x, e = d.first + d.len;
     long long r[16];
     bool bad = false;
 #pragma unroll
@@ -833,76 +790,121 @@ __global__ void __launch_bounds__(256, 4) k_seg_chunk_many(SegCols cols, int nco
 #pragma unroll
         for (int v = 0; v < 8; v++) x[v] = ws[q][v * 32 + lane_id()];
         const double r = stile8<double, OP_SUM>(x);
-        if (lane_id() == 0) part[(unsigned long long)q * nchunks + c] = r;
+        if (lane_id() == 0) part[(unsigned long long)q * nchunks + d.chunk] = r;
     }
     if (bad) flag_error(derr, DERR_INDEX);
 }
 
-// the chunk partials of column blockIdx.y, as k_seg_partials does for one
-struct SegOut { double* dst[SEG_MANY]; };
-__global__ void __launch_bounds__(256) k_seg_partials_many(const double* __restrict__ part,
-                                                           const long long* __restrict__ pstarts,
-                                                           const long long* __restrict__ big, long long nbig,
-                                                           long long nchunks, SegOut so) {
-    __shared__ double ws[256];
-    const long long g = blockIdx.x;
-    const double* p = part + (size_t)blockIdx.y * (size_t)nchunks;
-    const long long s = pstarts[g], e = (g + 1 < nbig) ? pstarts[g + 1] : nchunks;
-    bool bad = false;
-    double v[16];
-    seg_load16<double, false>(p, nullptr, 0, s + threadIdx.x, e, v, bad);
-    double acc = 0.0;
-#pragma unroll
-    for (int k = 0; k < 16; k++)
-        if (s + k * 256 + threadIdx.x < e) acc = __dadd_rn(acc, v[k]);
-    acc = sblock8<double, OP_SUM>(acc, ws);
-    if (threadIdx.x == 0) so.dst[blockIdx.y][big[g]] = acc;
-}
-
-// f64 sums of several columns over the segments of one grouping whose
-// segments are all longer than one tile, with at most 4096 chunks in all;
-// sums[q] receives column q's ng sums.  Returns 1 (nothing done) when the
-// grouping is of another shape.
-I seg_sum_f64_many(const double* const* srcs, int ncol, const long long* rows, long long nx, const long long* starts,
-                   long long ng, long long total, ListInfo* li, double* const* sums) {
-    if (ncol < 1 || ncol > SEG_MANY || ng == 0 || !li) return 1;
-    const unsigned *ids, *ccnt;
-    HG_CHECK(seg_classes(starts, ng, total, li, &ids, &ccnt));
-    if (!li->cls_known) return 1;
-    for (int c = 0; c < 7; c++)
-        if (li->cls_host[c]) return 1;
-    LongPlan pl;
-    HG_CHECK(seg_plan_long(starts, ng, total, li, &pl));
-    if (pl.nbig == 0 || pl.nchunks > (unsigned long long)TILE_SUM) return 1;
-    double* part = (double*)salloc((size_t)pl.nchunks * ncol * sizeof(double));
-    if (!part) return E_DEVICE_OOM;
-    SegCols sc{};
-    for (int q = 0; q < ncol; q++) sc.src[q] = srcs[q];
-#define SEG_MANY_LAUNCH(NC)                                                                                          \
-    HG_LAUNCH("seg_chunk_many", (unsigned)pl.nchunks, 256, 0, k_seg_chunk_many<NC>, sc, ncol, rows, nx, starts, ng, total, \
-              pl.big, pl.c0, pl.nbig, pl.nchunks, pl.order, part, g_derr)
-    if (ncol == 1) SEG_MANY_LAUNCH(1);
-    else if (ncol == 2) SEG_MANY_LAUNCH(2);
+// part[q * nchunks + c] = column q's partial of chunk c
+static I seg_chunk_many(const SegCols& sc, int ncol, const long long* rows, long long nx, const ListInfo* li,
+                        double* part) {
+#define SEG_MANY_LAUNCH(NC)                                                                                      \
+    HG_LAUNCH("seg_chunk_many", (unsigned)li->nchunks, 256, 0, k_seg_chunk_many<NC>, sc, rows, nx, li->nchunks, \
+              li->corder, part, g_derr)
+    if (ncol == 2) SEG_MANY_LAUNCH(2);
     else if (ncol == 3) SEG_MANY_LAUNCH(3);
     else SEG_MANY_LAUNCH(4);
 #undef SEG_MANY_LAUNCH
-    SegOut so{};
-    for (int q = 0; q < ncol; q++) so.dst[q] = sums[q];
-    HG_LAUNCH("seg_partials", dim3((unsigned)pl.nbig, (unsigned)ncol), 256, 0, k_seg_partials_many, part, pl.pstarts,
-              pl.big, pl.nbig, (long long)pl.nchunks, so);
     return last_launch_error();
 }
 
-// f64 sums of segments gathered through row ids, for the batched plans: the
-// same kernels and order as hgpuGroupSum.
-I seg_sum_f64(const double* src, const long long* rows, long long nx, const long long* starts, long long ng,
-              long long total, double* out) {
-    return seg_reduce<double, double, OP_SUM, true>(src, rows, nx, starts, ng, total, 0.0, out);
+// Reduces every segment of each of the ncol columns (io.src via rows | io.src)
+// into io.out[.][ng] (device), each class of segments in one launch for all
+// columns.  The plan is kept with `li` when there is one, else it serves this
+// call alone.
+template <typename T, typename A, int OP, bool GATHER>
+static I seg_reduce(const SegIO<T, A>& io, int ncol, const long long* rows, long long nx, const long long* starts,
+                    long long ng, long long total, A ident, ListInfo* li = nullptr) {
+    if (ng == 0) return 0;
+    ListInfo local{};
+    local.scratch = 1;
+    if (!li) li = &local;
+    HG_CHECK(seg_plan(starts, ng, total, GATHER ? rows : nullptr, nx, li));
+    const unsigned *ids = li->cls_ids, *ccnt = li->cls_cnt;
+    // One warp per 32 >> c small segments of class c and per mid-size one.
+    // The kernels stride over the segments, so the grid decides only how many
+    // run at once: with one thread per segment (8 warps per 256 segments) 64
+    // plans' ~200 mid-size segments ran on 16 warps, 0.34 ms a launch against
+    // 0.02 ms now.
+    long long small_w = 0;
+    for (int c = 0; c < 6; c++) small_w += (li->cls_host[c] + (32u >> c) - 1) / (32u >> c);
+    const long long mid_w = li->cls_host[6];
+    const unsigned nc = (unsigned)ncol;
+    if (small_w)
+        HG_LAUNCH("seg_warps", dim3(gcap(small_w * 32), nc), 256, 0, (k_seg_warps<T, A, OP, GATHER>), io, rows, nx,
+                  starts, ng, total, ids, ccnt, ident, g_derr);
+    if (mid_w)
+        HG_LAUNCH("seg_mid", dim3(gcap(mid_w * 32), nc), 256, 0, (k_seg_mid<T, A, OP, GATHER>), io, rows, nx, starts,
+                  ng, total, ids, ccnt, ident, g_derr);
+    const long long nbig = li->nbig;
+    const unsigned long long nchunks = li->nchunks;
+    if (nbig == 0) return last_launch_error();
+    A* part = (A*)salloc((size_t)nchunks * sizeof(A) * nc);
+    if (!part) return E_DEVICE_OOM;
+    bool done = false;
+    if constexpr (GATHER && std::is_same<T, double>::value && OP == OP_SUM) {
+        if (ncol > 1) {  // the columns share one read of the row ids
+            SegCols sc{};
+            for (int q = 0; q < ncol; q++) sc.src[q] = io.src[q];
+            HG_CHECK(seg_chunk_many(sc, ncol, rows, nx, li, part));
+            done = true;
+        }
+    }
+    if (!done)
+        HG_LAUNCH("seg_chunk", dim3((unsigned)nchunks, nc), 256, 0, (k_seg_chunk<T, A, OP, GATHER>), io, rows, nx,
+                  li->corder, ident, part, g_derr);
+    // partials of each long segment are reduced by the same procedure: at
+    // most 4096 of them per segment (certain when there are at most 4096 in
+    // all) in one launch straight into out, else as segments of their own
+    SegIO<A, A> pio{};
+    if (nchunks <= (unsigned long long)TILE_SUM) {
+        for (int q = 0; q < ncol; q++) pio.out[q] = io.out[q];
+        HG_LAUNCH("seg_partials", dim3((unsigned)nbig, nc), 256, 0, (k_seg_partials<A, OP>), part, li->pstarts,
+                  li->big, nbig, (long long)nchunks, ident, pio);
+        return last_launch_error();
+    }
+    for (int q = 0; q < ncol; q++) {
+        pio.src[q] = part + (size_t)q * nchunks;
+        pio.out[q] = (A*)salloc((size_t)nbig * sizeof(A));
+        if (!pio.out[q]) return E_DEVICE_OOM;
+    }
+    HG_CHECK((seg_reduce<A, A, OP, false>(pio, ncol, nullptr, 0, li->pstarts, nbig, (long long)nchunks, ident)));
+    for (int q = 0; q < ncol; q++)
+        HG_LAUNCH("scatter_big", gcap(nbig), 256, 0, k_scatter_big<A>, (const A*)pio.out[q], li->big, nbig, io.out[q]);
+    return last_launch_error();
 }
 
-// f64 sums of contiguous segments (no row indirection), same order
-I seg_sum_f64_direct(const double* src, const long long* starts, long long ng, long long total, double* out) {
-    return seg_reduce<double, double, OP_SUM, false>(src, nullptr, 0, starts, ng, total, 0.0, out);
+// f64 sums of ncol columns over the segments of one grouping, any number of
+// columns, in sets of SEG_MANY; sums[q] receives column q's ng sums.
+template <bool GATHER>
+static I seg_sum_cols(const double* const* srcs, int ncol, const long long* rows, long long nx, const long long* starts,
+                      long long ng, long long total, double* const* sums, ListInfo* li) {
+    ListInfo local{};
+    local.scratch = 1;
+    if (!li) li = &local;
+    for (int c0 = 0; c0 < ncol; c0 += SEG_MANY) {
+        SegIO<double, double> io{};
+        const int nc = ncol - c0 < SEG_MANY ? ncol - c0 : SEG_MANY;
+        for (int q = 0; q < nc; q++) {
+            io.src[q] = srcs[c0 + q];
+            io.out[q] = sums[c0 + q];
+        }
+        HG_CHECK((seg_reduce<double, double, OP_SUM, GATHER>(io, nc, rows, nx, starts, ng, total, 0.0, li)));
+    }
+    return 0;
+}
+
+// f64 sums of several columns over segments gathered through row ids (the
+// batched plans): the same kernels and order as hgpuGroupSum.
+I seg_sum_f64(const double* const* srcs, int ncol, const long long* rows, long long nx, const long long* starts,
+              long long ng, long long total, double* const* sums) {
+    return seg_sum_cols<true>(srcs, ncol, rows, nx, starts, ng, total, sums, nullptr);
+}
+
+// ... over contiguous segments (no row indirection), same order
+I seg_sum_f64_direct(const double* const* srcs, int ncol, const long long* starts, long long ng, long long total,
+                     double* const* sums) {
+    return seg_sum_cols<false>(srcs, ncol, nullptr, 0, starts, ng, total, sums, nullptr);
 }
 
 // ---------------------------------------------------------- finishing steps
@@ -953,7 +955,10 @@ static I agg_typed(int ag, I xt, const T* src, const long long* rows, long long 
     if (ag == AG_SUM || ag == AG_AVG) {
         SA* s = (SA*)salloc((size_t)(ng > 0 ? ng : 1) * sizeof(SA));
         if (!s) return E_DEVICE_OOM;
-        HG_CHECK((seg_reduce<T, SA, OP_SUM, GATHER>(src, rows, nx, starts, ng, total, (SA)0, s, li)));
+        SegIO<T, SA> io{};
+        io.src[0] = src;
+        io.out[0] = s;
+        HG_CHECK((seg_reduce<T, SA, OP_SUM, GATHER>(io, 1, rows, nx, starts, ng, total, (SA)0, li)));
         if (ag == AG_SUM) {
             *typ = isF ? H_F : (isE ? H_E : H_L);
             *out = s;
@@ -971,8 +976,11 @@ static I agg_typed(int ag, I xt, const T* src, const long long* rows, long long 
     T identity;
     if (ag == AG_MIN) identity = std::numeric_limits<T>::has_infinity ? std::numeric_limits<T>::infinity() : std::numeric_limits<T>::max();
     else identity = std::numeric_limits<T>::has_infinity ? -std::numeric_limits<T>::infinity() : std::numeric_limits<T>::lowest();
-    if (ag == AG_MIN) HG_CHECK((seg_reduce<T, T, OP_MIN, GATHER>(src, rows, nx, starts, ng, total, identity, r, li)));
-    else HG_CHECK((seg_reduce<T, T, OP_MAX, GATHER>(src, rows, nx, starts, ng, total, identity, r, li)));
+    SegIO<T, T> io{};
+    io.src[0] = src;
+    io.out[0] = r;
+    if (ag == AG_MIN) HG_CHECK((seg_reduce<T, T, OP_MIN, GATHER>(io, 1, rows, nx, starts, ng, total, identity, li)));
+    else HG_CHECK((seg_reduce<T, T, OP_MAX, GATHER>(io, 1, rows, nx, starts, ng, total, identity, li)));
     unsigned h = 0;
     if (!(li && li->group_rows)) {  // @group never yields an empty group
         unsigned* fl = (unsigned*)salloc(16);
@@ -1160,9 +1168,10 @@ I hgpuGroupLen(V z, V x, V y) { return group_agg(z, x, y, AG_LEN); }
 
 // z[k] = the aggregate aggs[k] (0 sum, 1 avg, 2 min, 3 max, 4 len) of x[k]
 // over the grouping y, each bit for bit what hgpuGroupSum/Avg/Min/Max/Len
-// returns.  The f64 sums and averages over a @group whose groups are all
-// longer than one 4096-row tile share one pass that reads each group's row
-// ids once (the common-index pattern applied to the segmented reductions).
+// returns.  The f64 sums and averages over a list this library made share
+// their launches (one per size class for up to four columns), and the long
+// groups' chunks read the row ids once for all of them (the common-index
+// pattern applied to the segmented reductions).
 I hgpuGroupAggMany(V* z, V* x, V y, const I* aggs, L n) {
     HG_CHECK(ensure_init());
     if (n < 0) return E_LENGTH;
@@ -1181,23 +1190,21 @@ I hgpuGroupAggMany(V* z, V* x, V y, const I* aggs, L n) {
         const void* rows;
         ListInfo* li;
         HG_CHECK(list_segments(y, H_L, &starts, &total, &rows, &li));
-        const long long ng = y->len;
-        const double* srcs[SEG_MANY];
-        double* sums[SEG_MANY];
-        bool in_range = li && li->group_rows;
-        long long nx = -1;
-        for (int q = 0; q < nf; q++) {
-            const void* px;
-            HG_CHECK(in_ptr(x[fused[q]], &px));
-            srcs[q] = (const double*)px;
-            sums[q] = (double*)salloc((size_t)(ng > 0 ? ng : 1) * 8);
-            if (!sums[q]) return E_DEVICE_OOM;
-            nx = nx < 0 ? x[fused[q]]->len : (x[fused[q]]->len < nx ? x[fused[q]]->len : nx);
-        }
-        in_range = in_range && nx >= total;
-        I rc = seg_sum_f64_many(srcs, nf, (const long long*)rows, nx, starts, ng, total, li, sums);
-        if (rc > 1) return rc;
-        if (rc == 0) {
+        if (li) {
+            const long long ng = y->len;
+            const double* srcs[SEG_MANY];
+            double* sums[SEG_MANY];
+            long long nx = -1;
+            for (int q = 0; q < nf; q++) {
+                const void* px;
+                HG_CHECK(in_ptr(x[fused[q]], &px));
+                srcs[q] = (const double*)px;
+                sums[q] = (double*)salloc((size_t)(ng > 0 ? ng : 1) * 8);
+                if (!sums[q]) return E_DEVICE_OOM;
+                nx = nx < 0 ? x[fused[q]]->len : (x[fused[q]]->len < nx ? x[fused[q]]->len : nx);
+            }
+            const bool in_range = li->group_rows && nx >= total;
+            HG_CHECK(seg_sum_cols<true>(srcs, nf, (const long long*)rows, nx, starts, ng, total, sums, li));
             if (!in_range) HG_CHECK(check_device_errors());
             for (int q = 0; q < nf; q++) {
                 const int k = fused[q];
