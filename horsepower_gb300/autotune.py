@@ -10,8 +10,8 @@ Knobs and their search ranges:
   join_filter where the join's presence bitmap is read: 0 through L2, 1 from
               the shared memory of a 16-CTA cluster (dense i32 keys)
   radix_pass  how a radix pass of @group / @order finds each tile's offsets:
-              0 a decoupled look-back, 1 a counting pass and one scan, 2 the
-              counting pass for 32-bit keys only (default)
+              0 a decoupled look-back, 1 and 2 (default) by counting each
+              chunk's digits first
 
 No knob changes a result (stable sorts, order-preserving compaction,
 fixed-order sums), so tuning is a pure search over time: coordinate descent

@@ -20,17 +20,18 @@
 // known from the value range) and packs multi-column integer keys into one
 // u64 after range compression.
 //
-// Radix kernel: onesweep-style LSD (Adinets & Merrill 2022).  One histogram
-// pass gives every digit's global bucket base for all passes; each pass
-// then ranks a 4096-key tile with warp-level __match_any_sync (warps own
-// contiguous sub-ranges, so ranks are stable), resolves per-digit tile
-// offsets with a decoupled look-back (one thread per digit, bounded spin) or
-// from counts taken by a separate pass and one scan, and scatters keys and
-// row ids.
+// The radix passes are the counted ones of radix.cuh; knob HGPU_TUNE_RADIX_PASS
+// 0 takes look-back passes (onesweep, Adinets & Merrill 2022) instead: one
+// histogram pass gives every digit's global bucket base for all passes; each
+// pass then ranks a 4096-key tile with warp-level __match_any_sync (warps own
+// contiguous sub-ranges, so ranks are stable), resolves per-digit tile offsets
+// with a decoupled look-back (one thread per digit, bounded spin) and scatters
+// keys and row ids.
 #include <cstring>
 #include <vector>
 
 #include "dev_common.cuh"
+#include "radix.cuh"
 
 namespace hg {
 
@@ -41,23 +42,20 @@ constexpr int RS_THREADS = 256, RS_ITEMS = 16, RS_TILE = RS_THREADS * RS_ITEMS;
 static int g_digit_bits = 8;  // LSD digit width, 4 - 8 bits (autotuner knob)
 void set_radix_digit_bits(int b) { g_digit_bits = b < 4 ? 4 : (b > 8 ? 8 : b); }
 int get_radix_digit_bits() { return g_digit_bits; }
-// how a pass finds each tile's offset per digit (autotuner knob): 0 a
-// decoupled look-back over the preceding tiles, 1 a counting pass over the
-// keys and one scan of the (digit, tile) counts before the scatter, 2 (the
-// default) the counting pass for 32-bit keys and the look-back for 64-bit
-// ones.  150M rows: the scatter runs 17-23% faster without the look-back;
-// the counting pass reads the keys once more, which leaves @group's 32-bit
-// keys 3% ahead (6.14 -> 5.96 ms) and @order's 64-bit keys even.
+// how a pass finds each tile's offsets (autotuner knob): 0 a decoupled
+// look-back over the preceding tiles, 1 and 2 (the default) the counted
+// passes of radix.cuh
 static int g_radix_pass = 2;
 void set_radix_pass_mode(int m) { g_radix_pass = m < 0 ? 0 : (m > 2 ? 2 : m); }
 int get_radix_pass_mode() { return g_radix_pass; }
 
-template <typename K>
-__global__ void k_key_bits(const K* __restrict__ k, long long n, unsigned long long* orv, unsigned long long* andv) {
+template <typename SRC>
+__global__ void k_key_bits(SRC src, long long n, unsigned long long* orv, unsigned long long* andv) {
     unsigned long long o = 0, a = ~0ull;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        o |= (unsigned long long)k[i];
-        a &= (unsigned long long)k[i];
+        const unsigned long long v = (unsigned long long)src(i);
+        o |= v;
+        a &= v;
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
@@ -108,12 +106,8 @@ __global__ void k_bucket_base(const unsigned long long* __restrict__ hist, unsig
 // result (the last pass of a @group, whose boundaries are read from the
 // keys), RS_OUT_V64 the i64 row ids alone (the last pass of an @order), at
 // position n - 1 - pos when `reverse`.
-//
-// PRE: the offsets are counted beforehand (k_rs_count, one scan): `bucket`
-// then holds every (digit, tile)'s first position, digit-major, tile t =
-// blockIdx.x, and there is no look-back.
 enum { RS_OUT_KV = 0, RS_OUT_KV64 = 1, RS_OUT_V64 = 2 };
-template <typename K, bool FIRST, int OUT, bool PRE>
+template <typename K, bool FIRST, int OUT>
 __global__ void __launch_bounds__(RS_THREADS, (sizeof(K) == 4 ? 4 : 3)) k_onesweep(const K* __restrict__ kin, const unsigned* __restrict__ vin,
                                                          K* __restrict__ kout, unsigned* __restrict__ vout,
                                                          long long* __restrict__ vout64, int reverse, long long n,
@@ -129,7 +123,7 @@ __global__ void __launch_bounds__(RS_THREADS, (sizeof(K) == 4 ? 4 : 3)) k_oneswe
     __shared__ unsigned wscan[8];
     __shared__ long long tile_id;
     for (int i = threadIdx.x; i < 8 * 256; i += RS_THREADS) (&whist[0][0])[i] = 0;
-    if (threadIdx.x == 0) tile_id = PRE ? (long long)blockIdx.x : (long long)atomicAdd(ticket, 1u);
+    if (threadIdx.x == 0) tile_id = (long long)atomicAdd(ticket, 1u);
     __syncthreads();
     const long long t = tile_id;
     const unsigned lane = lane_id(), w = threadIdx.x >> 5;
@@ -172,13 +166,9 @@ __global__ void __launch_bounds__(RS_THREADS, (sizeof(K) == 4 ? 4 : 3)) k_oneswe
         unsigned before = 0;
         for (unsigned ww = 0; ww < w; ww++) before += wscan[ww];
         dstart[d] = before + inc - c;
-        if constexpr (PRE) {
-            dbase[d] = d <= (int)dmask ? bucket[(size_t)d * gridDim.x + (size_t)t] : 0ull;
-        } else {
-            unsigned long long excl = 0;
-            if (d <= (int)dmask) excl = chain_lookback(status + d, 256, t, 0, c, derr);
-            dbase[d] = bucket[d] + excl;
-        }
+        unsigned long long excl = 0;
+        if (d <= (int)dmask) excl = chain_lookback(status + d, 256, t, 0, c, derr);
+        dbase[d] = bucket[d] + excl;
     }
     __syncthreads();
     // place the tile in digit order in shared memory ...
@@ -199,53 +189,17 @@ __global__ void __launch_bounds__(RS_THREADS, (sizeof(K) == 4 ? 4 : 3)) k_oneswe
         K kk = skey[i];
         unsigned d = (unsigned)((unsigned long long)kk >> shift) & dmask;
         unsigned long long pos = dbase[d] + (unsigned long long)(i - (int)dstart[d]);
-        if constexpr (PRE) {  // counted offsets: a position outside the output is an error, not a store
-            if (pos >= (unsigned long long)n) {
-                flag_error(derr, DERR_INDEX);
-                continue;
-            }
-        }
         if constexpr (OUT != RS_OUT_V64) kout[pos] = kk;
         if constexpr (OUT == RS_OUT_KV) vout[pos] = sval[i];
         else vout64[reverse ? (unsigned long long)(n - 1) - pos : pos] = (long long)sval[i];
     }
 }
 
-// The digit counts of every 4096-key tile of one pass, digit-major:
-// counts[d * ntiles + t] (per-warp histograms in shared memory)
-template <typename K>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_count(const K* __restrict__ kin, long long n, int shift, int bits,
-                                                         unsigned* __restrict__ counts) {
-    __shared__ unsigned wh[8][256];
-    for (int i = threadIdx.x; i < 8 * 256; i += RS_THREADS) (&wh[0][0])[i] = 0;
-    __syncthreads();
-    const unsigned dmask = (1u << bits) - 1, w = threadIdx.x >> 5;
-    const long long base = (long long)blockIdx.x * RS_TILE + threadIdx.x;
-    K key[RS_ITEMS];
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; k++) {
-        const long long i = base + (long long)k * RS_THREADS;
-        key[k] = i < n ? kin[i] : K(0);
-    }
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; k++)
-        if (base + (long long)k * RS_THREADS < n)
-            atomicAdd(&wh[w][(unsigned)((unsigned long long)key[k] >> shift) & dmask], 1u);
-    __syncthreads();
-    const unsigned d = threadIdx.x;
-    if (d <= dmask) {
-        unsigned c = 0;
-#pragma unroll
-        for (int q = 0; q < 8; q++) c += wh[q][d];
-        counts[(size_t)d * gridDim.x + blockIdx.x] = c;
-    }
-}
-
 // keeps only the bits set in `mask`, packed to the bottom in order
-template <typename K>
-__global__ void k_squeeze(const K* __restrict__ k, long long n, unsigned long long mask, K* __restrict__ out) {
+template <typename SRC, typename K>
+__global__ void k_squeeze(SRC src, long long n, unsigned long long mask, K* __restrict__ out) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        unsigned long long v = (unsigned long long)k[i], r = 0, m = mask;
+        unsigned long long v = (unsigned long long)src(i), r = 0, m = mask;
         int o = 0;
         while (m) {
             int b = __ffsll((long long)m) - 1;
@@ -286,57 +240,224 @@ struct RadixOut {
     bool keys = true;
 };
 
-// Stable sort of keys[0..n) (row ids travel along).  On return *kres/*vres
-// point to the sorted keys and row ids (scratch).  When no key bit varies
-// the result is the identity permutation.
+template <typename SRC, typename K>
+__global__ void k_copy_keys(SRC src, long long n, K* __restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = (K)src(i);
+}
+
+static int bits_for(unsigned long long range) { return range == 0 ? 1 : 64 - __builtin_clzll(range); }
+
+static unsigned cap8(long long n) {
+    const unsigned grid = grid_for(n, 256);
+    return grid > (unsigned)g_sms * 8 ? (unsigned)g_sms * 8 : grid;
+}
+
+static unsigned rx_chunks(long long ntiles) {
+    const long long c = (long long)RX_PER_SM * g_sms;
+    return (unsigned)(ntiles < c ? ntiles : c);
+}
+
+// One record pass (radix.cuh): digit, modes and the rest as in RxPass, whose
+// offs, ntiles and derr are filled here.
+template <typename SRC, int BITS>
+static I rx_pass_bits(SRC src, RxPass a, unsigned* counts, unsigned* tot) {
+    a.ntiles = (unsigned)(((long long)a.n + RX_TILE - 1) / RX_TILE);
+    a.offs = counts;
+    a.derr = g_derr;
+    const unsigned C = rx_chunks(a.ntiles);
+    const int dsm = RX_TILE * (a.cut ? 10 : 8);
+    HG_LAUNCH("radix_count", C, RX_THREADS, 0, (k_rx_count<SRC, BITS, RX_ITEMS>), src, a.n, a.ntiles, a.kshift, a.bits,
+              counts, tot);
+    HG_LAUNCH("radix_scan", 1u << a.bits, 256, 0, k_rx_scan, counts, C, tot);
+    // the attribute belongs to the current device's context: set it on every call (a host-side write)
+    HG_CU(cudaFuncSetAttribute(k_rx_scatter<SRC, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
+    HG_LAUNCH("radix_scatter", C, RX_THREADS, (size_t)dsm, (k_rx_scatter<SRC, BITS>), src, a);
+    return last_launch_error();
+}
+template <typename SRC>
+static I rx_pass(SRC src, const RxPass& a, unsigned* counts, unsigned* tot) {
+    return a.bits > 8 ? rx_pass_bits<SRC, 9>(src, a, counts, tot) : rx_pass_bits<SRC, 8>(src, a, counts, tot);
+}
+// ... and one two-array pass over 64-bit keys
+static I rx_pass_kv(const unsigned long long* kin, RxPass a, unsigned* counts, unsigned* tot) {
+    a.ntiles = (unsigned)(((long long)a.n + RX_KV_TILE - 1) / RX_KV_TILE);
+    a.offs = counts;
+    a.derr = g_derr;
+    const unsigned C = rx_chunks(a.ntiles);
+    HG_LAUNCH("radix_count", C, RX_THREADS, 0, (k_rx_count<RxKeys<unsigned long long>, 8, RX_KV_ITEMS>),
+              RxKeys<unsigned long long>{kin}, a.n, a.ntiles, a.kshift, a.bits, counts, tot);
+    HG_LAUNCH("radix_scan", 1u << a.bits, 256, 0, k_rx_scan, counts, C, tot);
+    HG_LAUNCH("radix_scatter", C, RX_THREADS, (size_t)RX_KV_TILE * 12, k_rx_scatter_kv, kin, a);
+    return last_launch_error();
+}
+
+// The key bits of src that vary (one OR/AND reduction and a round trip).
+template <typename SRC>
+static I varying_bits(SRC src, long long n, unsigned long long* vary) {
+    unsigned long long* red = (unsigned long long*)salloc(16);
+    if (!red) return E_DEVICE_OOM;
+    HG_CU(cudaMemsetAsync(red, 0, 8, g_stream));
+    HG_CU(cudaMemsetAsync(red + 1, 0xff, 8, g_stream));
+    HG_LAUNCH("key_bits", cap8(n), 256, 0, k_key_bits<SRC>, src, n, red, red + 1);
+    unsigned long long hb[2];
+    HG_CHECK(rb_queue(hb, red, 16));
+    HG_CU(stream_sync());
+    *vary = hb[0] ^ hb[1];
+    return 0;
+}
+
+// The order of equal keys: the identity.  kres/vres as rx_sort's.
+template <typename SRC, typename KR>
+static I identity_order(SRC src, long long n, const KR** kres, const unsigned** vres, const unsigned* init_vals,
+                        const RadixOut* out) {
+    KR* kcopy = (KR*)salloc((size_t)(n > 0 ? n : 1) * sizeof(KR));
+    unsigned* vid = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4);
+    if (!kcopy || !vid) return E_DEVICE_OOM;
+    if (n > 0) {
+        HG_LAUNCH("copy_keys", cap8(n), 256, 0, (k_copy_keys<SRC, KR>), src, n, kcopy);
+        if (init_vals) HG_CU(cudaMemcpyAsync(vid, init_vals, n * 4, cudaMemcpyDeviceToDevice, g_stream));
+        else HG_LAUNCH("iota", cap8(n), 256, 0, k_iota, vid, n);
+        if (out && out->perm64)
+            HG_LAUNCH("widen", cap8(n), 256, 0, k_widen, vid, n, out->perm64, out->reverse ? 1 : 0);
+    }
+    *kres = kcopy;
+    *vres = vid;
+    return last_launch_error();
+}
+
+// Stable sort of the keys of src (row ids travel along), in counted passes.
+// On return *kres/*vres point to the sorted keys (as KR: the bits of them that
+// vary, enough to tell them apart) and row ids, in scratch.  When no key bit
+// varies the result is the identity permutation.
+//   init_vals: the row ids, a permutation of 0 .. n - 1 (null: row i is i);
 //   vary_hint: a superset of the key bits that vary, from bit 0, known to
 //              the caller (0: found with one OR/AND reduction);
-//   hist:      the digit histograms of the plan of vary_hint, already counted
-//              (k_make_keys_hist), or null;
 //   out:       the last pass writes the i64 permutation there instead of
 //              u32 row ids (*vres is then null; *kres too unless out->keys).
-template <typename K>
-I radix_sort_ex(const K* keys, long long n, const K** kres, const unsigned** vres, const unsigned* init_vals,
-                unsigned long long vary_hint, unsigned long long* hist_ready, const RadixOut* out) {
-    unsigned grid = grid_for(n, 256);
-    if (grid > (unsigned)g_sms * 8) grid = g_sms * 8;
+template <typename SRC, typename KR>
+static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, const unsigned* init_vals,
+                 unsigned long long vary_hint, const RadixOut* out) {
+    using K = typename SRC::key_t;
     unsigned long long vary = vary_hint;
-    if (!vary_hint && n > 1) {
-        unsigned long long* red = (unsigned long long*)salloc(16);
-        if (!red) return E_DEVICE_OOM;
-        unsigned long long init[2] = {0, ~0ull};
-        HG_CU(cudaMemcpyAsync(red, init, 16, cudaMemcpyHostToDevice, g_stream));
-        HG_LAUNCH("key_bits", grid, 256, 0, k_key_bits<K>, keys, n, red, red + 1);
-        unsigned long long hb[2];
-        HG_CHECK(rb_queue(hb, red, 16));
-        HG_CU(stream_sync());
-        vary = hb[0] ^ hb[1];
-    }
-    unsigned* vid = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4);
-    if (!vid) return E_DEVICE_OOM;
-    if (vary == 0 || n <= 1) {
-        // all keys equal: identity order
-        K* kcopy = (K*)salloc((size_t)(n > 0 ? n : 1) * sizeof(K));
-        if (!kcopy) return E_DEVICE_OOM;
-        if (n > 0) HG_CU(cudaMemcpyAsync(kcopy, keys, n * sizeof(K), cudaMemcpyDeviceToDevice, g_stream));
-        if (n > 0) {
-            if (init_vals) HG_CU(cudaMemcpyAsync(vid, init_vals, n * 4, cudaMemcpyDeviceToDevice, g_stream));
-            else HG_LAUNCH("iota", grid, 256, 0, k_iota, vid, n);
-            if (out && out->perm64)
-                HG_LAUNCH("widen", grid, 256, 0, k_widen, vid, n, out->perm64, out->reverse ? 1 : 0);
-        }
-        *kres = kcopy;
-        *vres = vid;
-        return last_launch_error();
-    }
+    if (!vary_hint && n > 1) HG_CHECK(varying_bits(src, n, &vary));
+    if (vary == 0 || n <= 1) return identity_order<SRC, KR>(src, n, kres, vres, init_vals, out);
     RadixPlan pl = radix_plan(vary);
-    int nvar = __builtin_popcountll(vary);
-    if (!hist_ready && (nvar + pl.bits - 1) / pl.bits < pl.npass) {
+    const int nvar = __builtin_popcountll(vary);
+    if (!vary_hint && (nvar + pl.bits - 1) / pl.bits < pl.npass) {
         // bits that never change inside the range: squeeze them out (order
         // preserving, injective) and sort the shorter keys
         K* sq = (K*)salloc((size_t)n * sizeof(K));
         if (!sq) return E_DEVICE_OOM;
-        HG_LAUNCH("squeeze_keys", grid, 256, 0, k_squeeze<K>, keys, n, vary, sq);
+        HG_LAUNCH("squeeze_keys", cap8(n), 256, 0, (k_squeeze<SRC, K>), src, n, vary, sq);
+        return rx_sort<RxKeys<K>, KR>(RxKeys<K>{sq}, n, kres, vres, init_vals,
+                                      nvar >= 64 ? ~0ull : (1ull << nvar) - 1, out);
+    }
+    const bool perm = out && out->perm64, keep = !(perm && !out->keys);
+    const int total = pl.hi - pl.lo, rb = bits_for((unsigned long long)n - 1);
+    // 9-bit digits where they save a pass (150M rows: 0.85 ms a pass against
+    // 0.69 ms, each with a count of 0.20 ms; 45 bits take 5.3 ms in five passes
+    // and would take that in six as well, but the five leave room for the row
+    // id); only at the default digit width
+    if (pl.bits == 8 && (total + 8) / 9 < pl.npass) {
+        pl.npass = (total + 8) / 9;
+        pl.bits = (total + pl.npass - 1) / pl.npass;
+    }
+    // a record holds what is left of the key above the row id, after the
+    // first pass at the latest (a kept key in full)
+    const bool fits = total + rb - (keep || pl.npass == 1 ? 0 : pl.bits) <= 64;
+    if (!fits) {
+        pl.bits = pl.bits > 8 ? 8 : pl.bits;
+        pl.npass = (total + pl.bits - 1) / pl.bits;
+    }
+    unsigned* counts = (unsigned*)salloc((size_t)RX_PER_SM * g_sms * RX_MAX_DIGITS * 4);
+    unsigned* tot = (unsigned*)salloc((size_t)pl.npass * RX_MAX_DIGITS * 4);
+    // key or record buffers, and u32 row ids where they are a result or
+    // travel beside the keys; the last pass of a permutation alone writes neither
+    const bool sep_vals = !fits;
+    void* kb[2] = {nullptr, nullptr};
+    unsigned* vb[2] = {nullptr, nullptr};
+    for (int p = 0; p < pl.npass; p++) {
+        const bool last = p == pl.npass - 1;
+        if (!kb[p & 1] && !(last && !keep)) {
+            kb[p & 1] = salloc((size_t)n * 8);
+            if (!kb[p & 1]) return E_DEVICE_OOM;
+        }
+        if (!vb[p & 1] && !(last && perm) && (sep_vals || last)) {
+            vb[p & 1] = (unsigned*)salloc((size_t)n * 4);
+            if (!vb[p & 1]) return E_DEVICE_OOM;
+        }
+    }
+    if (!counts || !tot) return E_DEVICE_OOM;
+    HG_CU(cudaMemsetAsync(tot, 0, (size_t)pl.npass * RX_MAX_DIGITS * 4, g_stream));
+    RxPass a{};
+    a.n = (unsigned)n;
+    a.rb = rb;
+    a.kw = (int)sizeof(KR);
+    a.vin = init_vals;
+    const unsigned long long* kin = nullptr;  // keys or records of the pass before
+    if (!fits) {
+        if constexpr (std::is_same<SRC, RxKeys<unsigned long long>>::value) {
+            kin = src.p;
+        } else {
+            unsigned long long* k = (unsigned long long*)salloc((size_t)n * 8);
+            if (!k) return E_DEVICE_OOM;
+            HG_LAUNCH("copy_keys", cap8(n), 256, 0, (k_copy_keys<SRC, unsigned long long>), src, n, k);
+            kin = k;
+        }
+    }
+    for (int p = 0; p < pl.npass; p++) {
+        const bool last = p == pl.npass - 1;
+        a.bits = total - p * pl.bits < pl.bits ? total - p * pl.bits : pl.bits;
+        a.mode = !last ? (fits ? RX_REC : RX_KV) : perm ? (out->keys ? RX_KV64 : RX_V64) : RX_KV;
+        a.out = kb[p & 1];
+        a.vout = vb[p & 1];
+        a.perm64 = perm && last ? out->perm64 : nullptr;
+        a.reverse = perm && last && out->reverse;
+        unsigned* t = tot + (size_t)p * RX_MAX_DIGITS;
+        if (!fits) {
+            a.kshift = pl.lo + p * pl.bits;
+            HG_CHECK(rx_pass_kv(kin, a, counts, t));
+            a.vin = a.vout;
+        } else if (p == 0) {
+            // the record's key: without its constant low bits, and without
+            // the first digit when that is what makes it fit
+            const bool cut = total + rb > 64;
+            a.kshift = pl.lo;
+            a.cut = cut;
+            a.drop = pl.lo + (cut ? a.bits : 0);
+            const int left = total - (cut ? a.bits : 0);
+            a.kmask = left >= 64 ? ~0ull : (1ull << left) - 1;
+            HG_CHECK(rx_pass(src, a, counts, t));
+            a.kshift = rb + (cut ? 0 : a.bits);
+            a.drop = a.cut = 0;
+            a.vin = nullptr;
+        } else {
+            HG_CHECK(rx_pass(RxRec{kin}, a, counts, t));
+            a.kshift += a.bits;
+        }
+        kin = (const unsigned long long*)kb[p & 1];
+    }
+    *kres = keep ? (const KR*)kin : nullptr;
+    *vres = perm ? nullptr : vb[(pl.npass - 1) & 1];
+    return 0;
+}
+
+// The same by look-back passes (HGPU_TUNE_RADIX_PASS 0), over an array of keys.
+//   hist: the digit histograms of the plan of vary_hint, already counted
+//         (k_make_keys_hist), or null
+template <typename K>
+static I lookback_sort(const K* keys, long long n, const K** kres, const unsigned** vres, const unsigned* init_vals,
+                       unsigned long long vary_hint, unsigned long long* hist_ready, const RadixOut* out) {
+    unsigned long long vary = vary_hint;
+    if (!vary_hint && n > 1) HG_CHECK(varying_bits(RxKeys<K>{keys}, n, &vary));
+    if (vary == 0 || n <= 1) return identity_order<RxKeys<K>, K>(RxKeys<K>{keys}, n, kres, vres, init_vals, out);
+    RadixPlan pl = radix_plan(vary);
+    int nvar = __builtin_popcountll(vary);
+    if (!hist_ready && (nvar + pl.bits - 1) / pl.bits < pl.npass) {
+        K* sq = (K*)salloc((size_t)n * sizeof(K));
+        if (!sq) return E_DEVICE_OOM;
+        HG_LAUNCH("squeeze_keys", cap8(n), 256, 0, (k_squeeze<RxKeys<K>, K>), RxKeys<K>{keys}, n, vary, sq);
         keys = sq;
         pl = radix_plan(nvar >= 64 ? ~0ull : (1ull << nvar) - 1);
     }
@@ -346,33 +467,20 @@ I radix_sort_ex(const K* keys, long long n, const K** kres, const unsigned** vre
         hist = (unsigned long long*)salloc((size_t)npass * 256 * 8 * 2);
         if (!hist) return E_DEVICE_OOM;
         HG_CU(cudaMemsetAsync(hist, 0, (size_t)npass * 256 * 8, g_stream));
-        HG_LAUNCH("radix_hist", grid, 256, 0, k_radix_hist<K>, keys, n, lo, bits, npass, hist);
+        HG_LAUNCH("radix_hist", cap8(n), 256, 0, k_radix_hist<K>, keys, n, lo, bits, npass, hist);
     }
     unsigned long long* bucket = hist + npass * 256;
     HG_LAUNCH("bucket_base", npass, 256, 0, k_bucket_base, hist, bucket);
     long long ntiles = (n + RS_TILE - 1) / RS_TILE;
     K* kb[2] = {(K*)salloc(n * sizeof(K)), (K*)salloc(n * sizeof(K))};
-    unsigned* vb[2] = {vid, (unsigned*)salloc(n * 4)};
+    unsigned* vb[2] = {(unsigned*)salloc(n * 4), (unsigned*)salloc(n * 4)};
     char* st = (char*)salloc((size_t)ntiles * 256 * 8 + 64);
-    if (!kb[0] || !kb[1] || !vb[1] || !st) return E_DEVICE_OOM;
+    if (!kb[0] || !kb[1] || !vb[0] || !vb[1] || !st) return E_DEVICE_OOM;
     const K* kin = keys;
     const unsigned* vin = init_vals;
     const int dsm = (int)((size_t)RS_TILE * (sizeof(K) + 4));
-    const bool counted = g_radix_pass == 1 || (g_radix_pass == 2 && sizeof(K) == 4);
-    unsigned* cnts = nullptr;
-    unsigned long long* offs = nullptr;
-    if (counted) {
-        cnts = (unsigned*)salloc((size_t)ntiles * 256 * 4);
-        offs = (unsigned long long*)salloc(((size_t)ntiles * 256 + 1) * 8);
-        if (!cnts || !offs) return E_DEVICE_OOM;
-    }
     for (int p = 0; p < npass; p++) {
-        if (counted) {  // the (digit, tile) offsets of this pass, from the keys it reads
-            HG_LAUNCH("radix_count", (unsigned)ntiles, RS_THREADS, 0, k_rs_count<K>, kin, n, lo + p * bits, bits, cnts);
-            HG_CHECK(scan_exclusive(cnts, (long long)ntiles << bits, offs, nullptr));
-        } else {
-            HG_CU(cudaMemsetAsync(st, 0, (size_t)ntiles * 256 * 8 + 64, g_stream));
-        }
+        HG_CU(cudaMemsetAsync(st, 0, (size_t)ntiles * 256 * 8 + 64, g_stream));
         K* ko = kb[p & 1];
         unsigned* vo = vb[p & 1];
         unsigned* ticket = (unsigned*)(st + (size_t)ntiles * 256 * 8);
@@ -380,17 +488,12 @@ I radix_sort_ex(const K* keys, long long n, const K** kres, const unsigned** vre
         const int mode = (p == npass - 1 && out && out->perm64) ? (out->keys ? RS_OUT_KV64 : RS_OUT_V64) : RS_OUT_KV;
         long long* v64 = mode == RS_OUT_KV ? nullptr : out->perm64;
         const int rev = (mode != RS_OUT_KV && out->reverse) ? 1 : 0;
-#define RS_PASS1(F, M, PR, BASE)                                                                                     \
+#define RS_PASS(F, M)                                                                                                \
     do {                                                                                                             \
         /* the attribute belongs to the current device's context: set it on every call (a host-side write) */      \
-        HG_CU(cudaFuncSetAttribute(k_onesweep<K, F, M, PR>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));      \
-        HG_LAUNCH("onesweep", (unsigned)ntiles, RS_THREADS, (size_t)dsm, (k_onesweep<K, F, M, PR>), kin, vin, ko, vo, \
-                  v64, rev, n, lo + p * bits, bits, BASE, (unsigned long long*)st, ticket, g_derr);                  \
-    } while (0)
-#define RS_PASS(F, M)                                            \
-    do {                                                         \
-        if (counted) RS_PASS1(F, M, true, offs);                 \
-        else RS_PASS1(F, M, false, bucket + p * 256);            \
+        HG_CU(cudaFuncSetAttribute(k_onesweep<K, F, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));          \
+        HG_LAUNCH("onesweep", (unsigned)ntiles, RS_THREADS, (size_t)dsm, (k_onesweep<K, F, M>), kin, vin, ko, vo,    \
+                  v64, rev, n, lo + p * bits, bits, bucket + p * 256, (unsigned long long*)st, ticket, g_derr);      \
     } while (0)
         if (first) {
             if (mode == RS_OUT_KV) RS_PASS(true, RS_OUT_KV);
@@ -402,7 +505,6 @@ I radix_sort_ex(const K* keys, long long n, const K** kres, const unsigned** vre
             else RS_PASS(false, RS_OUT_V64);
         }
 #undef RS_PASS
-#undef RS_PASS1
         kin = ko;
         vin = vo;
         if (mode == RS_OUT_V64) kin = nullptr;
@@ -416,7 +518,8 @@ I radix_sort_ex(const K* keys, long long n, const K** kres, const unsigned** vre
 
 template <typename K>
 I radix_sort(const K* keys, long long n, const K** kres, const unsigned** vres, const unsigned* init_vals = nullptr) {
-    return radix_sort_ex<K>(keys, n, kres, vres, init_vals, 0, nullptr, nullptr);
+    if (g_radix_pass == 0) return lookback_sort<K>(keys, n, kres, vres, init_vals, 0, nullptr, nullptr);
+    return rx_sort<RxKeys<K>, K>(RxKeys<K>{keys}, n, kres, vres, init_vals, 0, nullptr);
 }
 
 template I radix_sort<unsigned>(const unsigned*, long long, const unsigned**, const unsigned**, const unsigned*);
@@ -520,19 +623,21 @@ __device__ __forceinline__ unsigned long long spec_key(const KeySpec& s, long lo
     }
 }
 
-__global__ void k_minmax_i64(const void* p, int typ, long long n, long long* mn, long long* mx) {
-    long long a = LLONG_MAX, b = LLONG_MIN;
+// mm[0] = the smallest order-preserving unsigned image of a value, mm[1] =
+// the smallest complement of one (both start at all ones)
+__global__ void k_minmax_i64(const void* p, int typ, long long n, unsigned long long* mm) {
+    unsigned long long a = ~0ull, b = ~0ull;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long v = ival(p, typ, i);
-        a = v < a ? v : a;
-        b = v > b ? v : b;
+        const unsigned long long u = (unsigned long long)ival(p, typ, i) ^ (1ull << 63);
+        a = u < a ? u : a;
+        b = ~u < b ? ~u : b;
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
-        long long o = __shfl_xor_sync(0xffffffffu, a, s); a = o < a ? o : a;
-        long long q = __shfl_xor_sync(0xffffffffu, b, s); b = q > b ? q : b;
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, a, s); a = o < a ? o : a;
+        const unsigned long long q = __shfl_xor_sync(0xffffffffu, b, s); b = q < b ? q : b;
     }
-    if (lane_id() == 0) { atomicMin(mn, a); atomicMax(mx, b); }
+    if (lane_id() == 0) { atomicMin(&mm[0], a); atomicMin(&mm[1], b); }
 }
 
 // ------------------------------------------------------------- permutations
@@ -676,24 +781,57 @@ struct SortResult {
 template <typename K>
 static I sort_keys_spec(const KeySpec& s, long long n, unsigned long long vary_hint, const RadixOut* ro,
                         SortResult* r) {
+    const K* ks = nullptr;
+    const unsigned long long hint0 = n > 1 ? vary_hint : 0;
+    r->perm64 = ro ? ro->perm64 : nullptr;
+    if (g_radix_pass != 0) {
+        // the first counted pass reads the columns themselves where the key
+        // is one integer column's bits or two range-compressed ones packed
+        // (150M rows: writing and reading a key array took 0.5 - 1 ms)
+        const int w0 = esize(s.typ[0]);
+        I rc = -1;
+        if (s.ncol == 1 && s.shift[0] == 0) {
+            if (s.xf[0] == XF_RAW32 && w0 == 4 && sizeof(K) == 4)
+                rc = rx_sort<RxKeys<unsigned>, unsigned>(RxKeys<unsigned>{(const unsigned*)s.col[0]}, n,
+                                                         (const unsigned**)&ks, &r->perm, nullptr, hint0, ro);
+            else if (s.xf[0] == XF_LOW32 && w0 == 8 && sizeof(K) == 4)
+                rc = rx_sort<RxLow32, unsigned>(RxLow32{(const long long*)s.col[0]}, n, (const unsigned**)&ks, &r->perm,
+                                                nullptr, hint0, ro);
+            else if (s.xf[0] == XF_RAW64 && w0 == 8 && sizeof(K) == 8)
+                rc = rx_sort<RxKeys<unsigned long long>, unsigned long long>(
+                    RxKeys<unsigned long long>{(const unsigned long long*)s.col[0]}, n, (const unsigned long long**)&ks,
+                    &r->perm, nullptr, hint0, ro);
+        } else if (s.ncol == 2 && s.xf[0] == XF_RANGE && s.xf[1] == XF_RANGE && s.shift[1] == 0 && w0 >= 4 &&
+                   esize(s.typ[1]) >= 4 && s.typ[0] != H_F && s.typ[1] != H_F) {
+            const RxPair p{s.col[0], s.col[1], s.desc[0] ? s.hi[0] : s.lo[0], s.desc[1] ? s.hi[1] : s.lo[1],
+                           w0 == 8, esize(s.typ[1]) == 8, s.desc[0], s.desc[1], s.shift[0]};
+            rc = rx_sort<RxPair, K>(p, n, &ks, &r->perm, nullptr, hint0, ro);
+        }
+        if (rc >= 0) {
+            r->keys = ks;
+            return rc ? rc : last_launch_error();
+        }
+    }
     K* k = (K*)salloc((size_t)(n > 0 ? n : 1) * sizeof(K));
     if (!k) return E_DEVICE_OOM;
+    if (g_radix_pass != 0) {
+        if (n > 0) HG_LAUNCH("make_keys", gcap(n), 256, 0, k_make_keys<K>, s, n, k);
+        HG_CHECK((rx_sort<RxKeys<K>, K>(RxKeys<K>{k}, n, &ks, &r->perm, nullptr, hint0, ro)));
+        r->keys = ks;
+        return last_launch_error();
+    }
     unsigned long long* hist = nullptr;
-    if (n > 1 && vary_hint) {  // the digit plan is known: count the histograms while making the keys
-        const RadixPlan pl = radix_plan(vary_hint);
+    if (hint0) {  // the digit plan is known: count the histograms while making the keys
+        const RadixPlan pl = radix_plan(hint0);
         hist = (unsigned long long*)salloc((size_t)pl.npass * 256 * 8 * 2);
         if (!hist) return E_DEVICE_OOM;
         HG_CU(cudaMemsetAsync(hist, 0, (size_t)pl.npass * 256 * 8, g_stream));
-        unsigned grid = grid_for(n, 256);
-        if (grid > (unsigned)g_sms * 8) grid = g_sms * 8;
-        HG_LAUNCH("make_keys", grid, 256, 0, k_make_keys_hist<K>, s, n, k, pl.lo, pl.bits, pl.npass, hist);
+        HG_LAUNCH("make_keys", cap8(n), 256, 0, k_make_keys_hist<K>, s, n, k, pl.lo, pl.bits, pl.npass, hist);
     } else if (n > 0) {
         HG_LAUNCH("make_keys", gcap(n), 256, 0, k_make_keys<K>, s, n, k);
     }
-    const K* ks;
-    HG_CHECK(radix_sort_ex<K>(k, n, &ks, &r->perm, nullptr, n > 1 ? vary_hint : 0, hist, ro));
+    HG_CHECK(lookback_sort<K>(k, n, &ks, &r->perm, nullptr, hint0, hist, ro));
     r->keys = ks;
-    r->perm64 = ro ? ro->perm64 : nullptr;
     return last_launch_error();
 }
 
@@ -707,20 +845,26 @@ static I sort_by_spec(const KeySpec& s, long long n, int total_bits, SortResult*
     return sort_keys_spec<unsigned>(s, n, vary_hint, ro, r);
 }
 
-static int bits_for(unsigned long long range) { return range == 0 ? 1 : 64 - __builtin_clzll(range); }
-
-static I col_minmax(const void* p, I typ, long long n, long long* mn, long long* mx) {
-    long long* d = (long long*)salloc(16);
+// The value ranges of nc integer columns (at most KMAXC), in one round trip;
+// an empty column gives [LLONG_MAX, LLONG_MIN].
+static I cols_minmax(int nc, const void* const* p, const int* typ, long long n, long long* mn, long long* mx) {
+    unsigned long long* d = (unsigned long long*)salloc(16 * KMAXC);
     if (!d) return E_DEVICE_OOM;
-    long long init[2] = {LLONG_MAX, LLONG_MIN};
-    HG_CU(cudaMemcpyAsync(d, init, 16, cudaMemcpyHostToDevice, g_stream));
-    if (n > 0) HG_LAUNCH("minmax", gcap(n), 256, 0, k_minmax_i64, p, (int)typ, n, d, d + 1);
-    long long h[2];
-    HG_CHECK(rb_queue(h, d, 16));
+    HG_CU(cudaMemsetAsync(d, 0xff, (size_t)16 * nc, g_stream));
+    if (n > 0)
+        for (int c = 0; c < nc; c++) HG_LAUNCH("minmax", gcap(n), 256, 0, k_minmax_i64, p[c], typ[c], n, d + 2 * c);
+    unsigned long long h[2 * KMAXC];
+    HG_CHECK(rb_queue(h, d, (size_t)16 * nc));
     HG_CU(stream_sync());
-    *mn = h[0];
-    *mx = h[1];
+    for (int c = 0; c < nc; c++) {
+        mn[c] = (long long)(h[2 * c] ^ (1ull << 63));
+        mx[c] = (long long)(~h[2 * c + 1] ^ (1ull << 63));
+    }
     return 0;
+}
+static I col_minmax(const void* p, I typ, long long n, long long* mn, long long* mx) {
+    const int t = (int)typ;
+    return cols_minmax(1, &p, &t, n, mn, mx);
 }
 
 // Single-column keys following the reference's radix rules (i32 / i64).
@@ -761,23 +905,30 @@ static I column_spec(int ncol, V* cols, const void** ptrs, const B* asc, long lo
     if (ncol > KMAXC) return set_error(E_NOT_IMPL, "ordering by more than %d columns", KMAXC);
     memset(s, 0, sizeof *s);
     s->ncol = ncol;
-    int shift = 0;
-    for (int c = ncol - 1; c >= 0; c--) {
-        int width;
+    const void* ip[KMAXC];
+    int it[KMAXC], ic[KMAXC], ni = 0;  // the integer columns
+    for (int c = 0; c < ncol; c++) {
         s->col[c] = ptrs[c];
         s->typ[c] = cols[c]->typ;
         s->desc[c] = asc ? !asc[c] : 0;
-        if (cols[c]->typ == H_F || cols[c]->typ == H_E) {
-            s->xf[c] = XF_FLOAT;
-            width = 64;
-        } else {
-            long long mn, mx;
-            HG_CHECK(col_minmax(ptrs[c], cols[c]->typ, n, &mn, &mx));
-            s->xf[c] = XF_RANGE;
-            s->lo[c] = mn;
-            s->hi[c] = mx;
-            width = n > 0 ? bits_for((unsigned long long)mx - (unsigned long long)mn) : 1;
-        }
+        s->xf[c] = XF_FLOAT;
+        if (cols[c]->typ == H_F || cols[c]->typ == H_E) continue;
+        s->xf[c] = XF_RANGE;
+        ip[ni] = ptrs[c];
+        it[ni] = cols[c]->typ;
+        ic[ni++] = c;
+    }
+    long long mn[KMAXC], mx[KMAXC];
+    if (ni) HG_CHECK(cols_minmax(ni, ip, it, n, mn, mx));
+    for (int k = 0; k < ni; k++) {
+        s->lo[ic[k]] = mn[k];
+        s->hi[ic[k]] = mx[k];
+    }
+    int shift = 0;
+    for (int c = ncol - 1; c >= 0; c--) {
+        int width = 64;
+        if (s->xf[c] == XF_RANGE)
+            width = n > 0 ? bits_for((unsigned long long)s->hi[c] - (unsigned long long)s->lo[c]) : 1;
         s->shift[c] = shift;
         shift += width;
     }

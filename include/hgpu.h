@@ -217,8 +217,8 @@ I hgpuGroupLen(V z, V x, V y);
  * common-index pattern, pattern.cc:558-672, applied to the segmented
  * reductions of pattern.cc:63-105).  z[k] = hgpuGroupSum / Avg / Min / Max /
  * Len (x[k], y) for aggs[k] = HGPU_AGG_SUM .. HGPU_AGG_LEN, bit for bit; f64
- * sums and averages over a @group whose groups are all longer than 4096 rows
- * read the groups' row ids once for all of them. */
+ * sums and averages over a list this library made share their launches, and
+ * the long groups' row ids are read once for all of them. */
 #define HGPU_AGG_SUM 0
 #define HGPU_AGG_AVG 1
 #define HGPU_AGG_MIN 2
@@ -365,7 +365,8 @@ double hgpuTimerStop(void);
  * Values outside a knob's range are clamped; hgpuGetTuning returns the
  * value in force. */
 #define HGPU_TUNE_HASH_LOAD  0   /* hash-table load factor, 0.5 - 0.8 (default 0.5) */
-#define HGPU_TUNE_RADIX_BITS 1   /* LSD radix digit width of @group/@order, 4 - 8 bits (default 8) */
+#define HGPU_TUNE_RADIX_BITS 1   /* LSD radix digit width of @group/@order, 4 - 8 bits (default 8; at 8 the
+                                    counted passes take 9 bits where that saves a pass) */
 #define HGPU_TUNE_TILE_ROWS  2   /* probe rows per thread of the tiled join probes: 8, 16, 32
                                     (tile = 256 x that; default 8) */
 #define HGPU_TUNE_L2_FETCH   3   /* largest L2 fetch from DRAM, bytes: 32, 64 or 128 (default 64;
@@ -373,8 +374,7 @@ double hgpuTimerStop(void);
 #define HGPU_TUNE_JOIN_FILTER 4 /* @join_index presence bitmap on dense i32 keys: 0 read through L2
                                     (default), 1 held in the shared memory of a 16-CTA cluster */
 #define HGPU_TUNE_RADIX_PASS 5  /* radix pass of @group/@order: 0 tile offsets by a decoupled look-back,
-                                    1 by a counting pass and one scan before the scatter, 2 (default)
-                                    1 for 32-bit keys and 0 for 64-bit ones */
+                                    1 and 2 (default) by counting each chunk's digits first */
 I    hgpuSetTuning(I knob, E value);
 E    hgpuGetTuning(I knob);
 

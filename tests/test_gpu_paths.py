@@ -54,3 +54,60 @@ def test_mid_size_groups(libs, sizes):
         assert sums[gi].tobytes() == np.float64(want).tobytes(), (len(rows), sums[gi], want)
         assert lo[gi] == ipay[rows].min() and hi[gi] == x.max()
     gpu.free_inputs()
+
+
+def key_column(rng, n, lo_bit, hi_bit, negative=False):
+    """n i64 keys whose varying bits are lo_bit .. hi_bit - 1 (repeats included)."""
+    top = rng.integers(0, 1 << min(hi_bit - lo_bit, 62), n, dtype=np.int64)
+    top[rng.random(n) < 0.2] = top[0]
+    top[:2] = [0, (1 << (hi_bit - lo_bit)) - 1]
+    key = top << lo_bit
+    return -key if negative else key
+
+
+@pytest.mark.parametrize("n", [2, 31, 4095, 4096, 4097, 70_001, 2_000_003])
+@pytest.mark.parametrize("lo_bit,hi_bit", [(0, 1), (0, 8), (0, 9), (0, 17), (3, 20), (0, 32), (0, 33), (5, 45), (0, 45),
+                                           (0, 53), (0, 62)])
+def test_radix_keys(libs, n, lo_bit, hi_bit):
+    """@order and @group of one i64 key for key widths on either side of what
+    a 64-bit record holds beside the row id (whole, without the first digit,
+    not at all), constant low bits, and tile and chunk remainders: the stable
+    argsort, its reverse when descending, and its runs."""
+    gpu = libs[0]
+    rng = np.random.default_rng(n + 100 * hi_bit + lo_bit)
+    key = key_column(rng, n, lo_bit, hi_bit)
+    want = np.argsort(key, kind="stable")
+    k = gpu.vec(key, H_L)
+    up = gpu.to_py(gpu.call("pfnOrderBy", k, gpu.vec(np.array([1], bool), H_B)))
+    assert np.array_equal(up, want)
+    down = gpu.to_py(gpu.call("pfnOrderBy", k, gpu.vec(np.array([0], bool), H_B)))
+    assert np.array_equal(down, want[::-1])
+    if n > 100_000 and hi_bit > 20:
+        gpu.free_inputs()
+        return  # a million one-row groups say no more than the small sizes
+    g = gpu.to_py(gpu.call("pfnGroup", k))
+    heads = np.flatnonzero(np.r_[True, key[want][1:] != key[want][:-1]])
+    assert np.array_equal(g[1], want[heads])
+    assert np.array_equal(np.concatenate(g[2]), want)
+    assert [len(v) for v in g[2]] == list(np.diff(np.r_[heads, n]))
+    gpu.free_inputs()
+
+
+@pytest.mark.parametrize("t0,t1", [(H_I, H_I), (H_L, H_I), (H_I, H_L), (H_L, H_L)])
+@pytest.mark.parametrize("dirs", [(1, 1), (0, 1), (1, 0), (0, 0)])
+@pytest.mark.parametrize("span0,span1", [(1 << 8, 1 << 8), (1 << 16, 1 << 18), (1 << 29, 1 << 16), (1 << 30, 1 << 30)])
+def test_radix_pairs(libs, t0, t1, dirs, span0, span1):
+    """@order of two integer columns of every width and direction, packed keys
+    of 16 to 60 bits, negative values included: the oracle's permutation."""
+    gpu, ora = libs
+    rng = np.random.default_rng(span0 % 97 + 7 * dirs[0] + dirs[1])
+    n = 40_009
+    a = (rng.integers(0, span0, n) - span0 // 2).astype(np.int32 if t0 == H_I else np.int64)
+    b = (rng.integers(0, span1, n) - span1 // 3).astype(np.int32 if t1 == H_I else np.int64)
+    a[: n // 2] = a[rng.integers(0, 50, n // 2)]
+    out = []
+    for L in (gpu, ora):
+        z = L.call("pfnOrderBy", L.list([L.vec(a, t0), L.vec(b, t1)]), L.vec(np.array(dirs, bool), H_B))
+        out.append(L.to_py(z))
+        L.free_inputs()
+    assert np.array_equal(out[0], out[1])
