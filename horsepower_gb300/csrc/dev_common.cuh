@@ -9,6 +9,11 @@ namespace hg {
 
 constexpr double H_EPSILON = 1e-13;  // src/horseir/v3/backend/h_system.cc:9
 
+// First statement of every kernel, in every thread: waits for the kernel
+// before this one in the stream (see HG_LAUNCH), whose results and buffers the
+// rest may then touch.  A plain launch has waited already.
+__device__ __forceinline__ void grid_entry() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void flag_error(unsigned* derr, unsigned bit) { atomicOr(derr, bit); }
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }

@@ -15,6 +15,7 @@
 #pragma once
 #include <cstdint>
 #include <cstddef>
+#include <tuple>
 #include <cuda_runtime.h>
 #include "hgpu.h"
 
@@ -128,10 +129,38 @@ struct LaunchScope {
     explicit LaunchScope(const char* n);
     ~LaunchScope();
 };
-#define HG_LAUNCH(name, grid, block, smem, kern, ...)                           \
-    do {                                                                        \
-        ::hg::LaunchScope ls_(name);                                            \
-        kern<<<(grid), (block), (smem), ::hg::g_stream>>>(__VA_ARGS__);         \
+// Every kernel is launched with programmatic stream serialisation and begins
+// with grid_entry() (dev_common.cuh), which waits until the kernel before it
+// has finished and its memory is visible.  The launch itself then overlaps
+// that kernel's run: GB300, dependent kernels of a few microseconds: 4.1 us
+// apart with plain launches, 1.45 us this way.
+inline cudaError_t launch_kernel_args(const void* kern, dim3 grid, dim3 block, size_t smem, void** args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = g_stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelExC(&c, kern, args);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    std::tuple<P...> p(static_cast<P>(args)...);
+    return std::apply(
+        [&](P&... q) {
+            void* ptrs[] = {(void*)&q...};
+            return launch_kernel_args((const void*)kern, grid, block, smem, ptrs);
+        },
+        p);
+}
+#define HG_LAUNCH(name, grid, block, smem, kern, ...)                     \
+    do {                                                                  \
+        ::hg::LaunchScope ls_(name);                                      \
+        ::hg::launch_kernel(kern, (grid), (block), (smem), __VA_ARGS__);  \
     } while (0)
 I last_launch_error();
 

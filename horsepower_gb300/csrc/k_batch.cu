@@ -79,6 +79,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // ---------------------------------------------------------------- stage 0/1
 __global__ void k_b_minmax(const DPlan* __restrict__ P, const long long* __restrict__ tile_first, int np,
                            long long* __restrict__ mm) {
+    grid_entry();
     const long long t = blockIdx.x;
     const int p = plan_of_tile(tile_first, np, t);
     const long long r0 = (t - tile_first[p]) * BT;
@@ -107,6 +108,7 @@ __global__ void k_b_minmax(const DPlan* __restrict__ P, const long long* __restr
 // counts them (the length of the compressed key column)
 __global__ void k_b_build(const DPlan* __restrict__ P, const long long* __restrict__ tile_first, int np,
                           unsigned* __restrict__ dup, unsigned long long* __restrict__ nsel) {
+    grid_entry();
     const long long t = blockIdx.x;
     const int p = plan_of_tile(tile_first, np, t);
     const DPlan& q = P[p];
@@ -143,6 +145,7 @@ __global__ void k_b_build(const DPlan* __restrict__ P, const long long* __restri
 template <int R>
 __global__ void __launch_bounds__(256) k_b_probe(const DPlan* __restrict__ P, const long long* __restrict__ tile_first,
                                                  int np, unsigned* __restrict__ bits, unsigned* __restrict__ counts) {
+    grid_entry();
     extern __shared__ unsigned bp_smem[];
     unsigned(*koff)[256] = reinterpret_cast<unsigned(*)[256]>(bp_smem);            // key - kmin, NONE when out of range
     unsigned(*word)[256] = reinterpret_cast<unsigned(*)[256]>(bp_smem + R * 256);  // presence word of the key
@@ -206,6 +209,7 @@ __global__ void __launch_bounds__(256) k_b_emit(const EmitPlan* __restrict__ E, 
                                                 int np, const unsigned* __restrict__ bits,
                                                 const unsigned long long* __restrict__ offs, unsigned* __restrict__ fi,
                                                 unsigned long long* __restrict__ mcount) {
+    grid_entry();
     __shared__ unsigned wc[8];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const long long t = blockIdx.x;
@@ -243,6 +247,7 @@ __global__ void __launch_bounds__(256) k_b_emit(const EmitPlan* __restrict__ E, 
 constexpr unsigned short NO_DATE = 0xffffu;
 
 __global__ void k_sh_minmax(const int* __restrict__ a, const int* __restrict__ b, long long n, long long* mm) {
+    grid_entry();
     long long amin = LLONG_MAX, amax = LLONG_MIN, bmin = LLONG_MAX, bmax = LLONG_MIN;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long x = a[i], y = b[i];
@@ -267,6 +272,7 @@ __global__ void k_sh_minmax(const int* __restrict__ a, const int* __restrict__ b
 __global__ void k_sh_build(const int* __restrict__ pk, const int* __restrict__ date, long long nd, long long kmin,
                            int dmin, int drange, unsigned short* __restrict__ dt, unsigned* __restrict__ dimhist,
                            unsigned* dup) {
+    grid_entry();
     extern __shared__ unsigned sh_hist[];
     const bool local = drange <= 8192;
     if (local) for (int i = threadIdx.x; i < drange; i += blockDim.x) sh_hist[i] = 0;
@@ -289,6 +295,7 @@ __global__ void k_sh_build(const int* __restrict__ pk, const int* __restrict__ d
 __global__ void k_sh_probe(const int* __restrict__ fk, long long nf, long long kmin, unsigned long long kspan,
                            const unsigned short* __restrict__ dt, int drange, unsigned short* __restrict__ dd,
                            unsigned* __restrict__ facthist) {
+    grid_entry();
     extern __shared__ unsigned sh_hist[];
     const bool local = drange <= 8192;
     if (local) for (int i = threadIdx.x; i < drange; i += blockDim.x) sh_hist[i] = 0;
@@ -336,6 +343,7 @@ constexpr long long SG_TILE = 256LL * SG_R;
 // presence bits of the codes (flag << 8 | status) over the fact table
 __global__ void k_sg_codes(const int8_t* __restrict__ flag, const int8_t* __restrict__ status, long long n,
                            unsigned* __restrict__ bits) {
+    grid_entry();
     __shared__ unsigned sb[2048];
     for (int i = threadIdx.x; i < 2048; i += blockDim.x) sb[i] = 0;
     __syncthreads();
@@ -395,6 +403,7 @@ __global__ void __launch_bounds__(256) k_sg_count(const unsigned short* __restri
                                                   const unsigned char* __restrict__ dense, long long nf,
                                                   const int* __restrict__ wins, int npl, int G,
                                                   unsigned* __restrict__ counts, long long ntiles) {
+    grid_entry();
     __shared__ unsigned wc[8][SG_MAXP * SG_MAXG];
     const unsigned w = threadIdx.x >> 5;
     const long long t = blockIdx.x, base = t * SG_TILE + (long long)w * (32 * SG_R);
@@ -416,6 +425,7 @@ __global__ void __launch_bounds__(256) k_sg_count(const unsigned short* __restri
 __global__ void __launch_bounds__(1024) k_sg_scan(const unsigned* __restrict__ counts, long long ntiles,
                                                   unsigned long long* __restrict__ offs,
                                                   unsigned long long* __restrict__ totals) {
+    grid_entry();
     __shared__ unsigned long long wsum[32];
     __shared__ unsigned long long carry;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -468,6 +478,7 @@ __global__ void __launch_bounds__(256) k_sg_scatter(const unsigned short* __rest
                                                     const unsigned long long* __restrict__ base, long long ntiles,
                                                     double* __restrict__ vq, double* __restrict__ vp,
                                                     double* __restrict__ vd) {
+    grid_entry();
     __shared__ unsigned wc[8][SG_MAXP * SG_MAXG];
     const unsigned lane = lane_id(), w = threadIdx.x >> 5;
     const long long t = blockIdx.x, rbase = t * SG_TILE + (long long)w * (32 * SG_R);
@@ -530,6 +541,7 @@ struct CPlan {
 template <int R>
 __global__ void __launch_bounds__(256) k_sh_select(const CPlan* __restrict__ P, const long long* __restrict__ tile_first,
                                                    int np, unsigned* __restrict__ bits, unsigned* __restrict__ counts) {
+    grid_entry();
     __shared__ unsigned wc[8];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const long long t = blockIdx.x;
@@ -562,6 +574,7 @@ __global__ void __launch_bounds__(256) k_sh_select(const CPlan* __restrict__ P, 
 
 // exclusive prefix of the per-plan match counts (one block)
 __global__ void k_b_offsets(const unsigned long long* __restrict__ mcount, int np, long long* __restrict__ moff) {
+    grid_entry();
     if (threadIdx.x == 0) {
         long long acc = 0;
         for (int p = 0; p < np; p++) { moff[p] = acc; acc += (long long)mcount[p]; }
@@ -576,6 +589,7 @@ __global__ void k_b_gather(const DPlan* __restrict__ P, const long long* __restr
                            const unsigned* __restrict__ fi, const unsigned long long* __restrict__ mcount,
                            const long long* __restrict__ moff, unsigned* __restrict__ code, double* __restrict__ qty,
                            double* __restrict__ price, double* __restrict__ disc) {
+    grid_entry();
     // codes seen by this block, merged into the plan's presence bits once
     // at the end (a few atomics per block instead of a few per warp)
     __shared__ unsigned seen[2048];
@@ -633,6 +647,7 @@ __global__ void k_b_gather(const DPlan* __restrict__ P, const long long* __restr
 
 // code -> dense group id (ascending codes), one block per plan
 __global__ void k_b_dense(const DPlan* __restrict__ P, unsigned* __restrict__ ngroups, unsigned* __restrict__ codes) {
+    grid_entry();
     const int p = blockIdx.x;
     const DPlan& q = P[p];
     __shared__ unsigned wsum[8];
@@ -664,6 +679,7 @@ __global__ void k_b_dense(const DPlan* __restrict__ P, unsigned* __restrict__ ng
 __global__ void k_b_hist(const DPlan* __restrict__ P, const long long* __restrict__ tile_first, int np,
                          const unsigned long long* __restrict__ mcount, const long long* __restrict__ moff,
                          const unsigned* __restrict__ code, unsigned* __restrict__ hist) {
+    grid_entry();
     __shared__ unsigned h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -677,6 +693,7 @@ __global__ void k_b_hist(const DPlan* __restrict__ P, const long long* __restric
 }
 
 __global__ void k_b_bucket(const unsigned* __restrict__ hist, unsigned* __restrict__ bucket) {
+    grid_entry();
     __shared__ unsigned s[256];
     const int p = blockIdx.x, d = threadIdx.x;
     s[d] = hist[p * 256 + d];
@@ -697,6 +714,7 @@ __global__ void __launch_bounds__(256) k_b_sort(const DPlan* __restrict__ P, con
                                                 const long long* __restrict__ moff, const unsigned* __restrict__ code,
                                                 const unsigned* __restrict__ bucket, long long* __restrict__ rows,
                                                 unsigned long long* status, unsigned* ticket, unsigned* derr) {
+    grid_entry();
     __shared__ unsigned whist[8][256];
     __shared__ unsigned long long dbase[256];
     __shared__ long long tile_id;
@@ -745,6 +763,7 @@ __global__ void __launch_bounds__(256) k_b_sort(const DPlan* __restrict__ P, con
 __global__ void k_b_starts(const long long* __restrict__ moff, const unsigned* __restrict__ bucket,
                            const unsigned* __restrict__ ngroups, const long long* __restrict__ segoff, int np,
                            long long* __restrict__ starts) {
+    grid_entry();
     const int p = blockIdx.x, g = threadIdx.x;
     if (g < (int)ngroups[p]) starts[segoff[p] + g] = moff[p] + bucket[p * 256 + g];
 }
@@ -752,6 +771,7 @@ __global__ void k_b_starts(const long long* __restrict__ moff, const unsigned* _
 // avg = sum / count per group (k_avg_seg's division)
 __global__ void k_b_avg(const double* __restrict__ s, const long long* __restrict__ starts, long long ng, long long total,
                         double* __restrict__ avg) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
         long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
         avg[g] = __ddiv_rn(s[g], (double)m);

@@ -42,6 +42,7 @@ __device__ __forceinline__ uint4 load_mask16(const uint8_t* __restrict__ mask, l
 // pass 1: selected rows per 4096-row tile
 __global__ void __launch_bounds__(CT_THREADS) k_compact_count(const uint8_t* __restrict__ mask, long long n,
                                                               unsigned* __restrict__ counts) {
+    grid_entry();
     __shared__ unsigned warp_tot[8];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const long long base = (long long)blockIdx.x * CT_TILE;
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_compact_count(const uint8_t* __r
 // even 2^31 rows make only 2^19 counts); out[ntiles] = total
 __global__ void __launch_bounds__(1024) k_scan_counts(const unsigned* __restrict__ in, long long n,
                                                       unsigned long long* __restrict__ out) {
+    grid_entry();
     // Rounds of 8192 counts, element k * 1024 + t of a round held by thread
     // t, so that every load and store of a warp covers 32 consecutive
     // counts.  The round's order is k-major: the exclusive prefix of element
@@ -152,6 +154,7 @@ __device__ __forceinline__ void scatter_col(const void* __restrict__ src, void* 
 __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter(const uint8_t* __restrict__ mask, long long n,
                                                                 CompactCols cols,
                                                                 const unsigned long long* __restrict__ offs) {
+    grid_entry();
     __shared__ __align__(16) uint8_t smask[CT_TILE];
     __shared__ unsigned warp_tot[8];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -189,6 +192,7 @@ template <int ES>
 __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter1(const uint8_t* __restrict__ mask, long long n,
                                                                  const void* __restrict__ src, void* __restrict__ dst,
                                                                  const unsigned long long* __restrict__ offs) {
+    grid_entry();
     using E = typename std::conditional<ES == 1, uint8_t,
               typename std::conditional<ES == 2, uint16_t,
               typename std::conditional<ES == 4, uint32_t, unsigned long long>::type>::type>::type;

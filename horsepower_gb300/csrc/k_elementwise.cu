@@ -131,6 +131,7 @@ __device__ __forceinline__ T arith_op(int op, T a, T b, bool& divzero) {
 template <typename T>
 __global__ void __launch_bounds__(256) k_compare(const T* __restrict__ x, const T* __restrict__ y,
                                                  bool* __restrict__ z, long long n, int op, int mode, T sx, T sy) {
+    grid_entry();
     long long nchunks = (n + 15) / 16;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nchunks;
          c += (long long)gridDim.x * blockDim.x) {
@@ -155,6 +156,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_arith(const T* __restrict__ x, const T* __restrict__ y,
                                                T* __restrict__ z, long long n, int op, int mode, T sx, T sy,
                                                unsigned* derr) {
+    grid_entry();
     long long nchunks = (n + 15) / 16;
     bool dz = false;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nchunks;
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(256) k_arith(const T* __restrict__ x, const T*
 __global__ void __launch_bounds__(256) k_logic(const uint8_t* __restrict__ x, const uint8_t* __restrict__ y,
                                                uint8_t* __restrict__ z, long long n, int op, int mode,
                                                uint8_t sx, uint8_t sy) {
+    grid_entry();
     long long nchunks = (n + 15) / 16;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nchunks;
          c += (long long)gridDim.x * blockDim.x) {
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(256) k_logic(const uint8_t* __restrict__ x, co
 // promotion of a vector of type `st` to T (promoteValueWithIndex, h_system.cc:168-252)
 template <typename T>
 __global__ void k_convert(const void* __restrict__ src, int st, T* __restrict__ dst, long long n) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         T v;
         switch (st) {
@@ -311,6 +315,7 @@ F64Cmp f64_cmp_thresholds(double s, bool scalar_first) {
 // a double vector against a fixed double, by the integer thresholds
 __global__ void __launch_bounds__(256) k_compare_f64_fixed(const double* __restrict__ x, bool* __restrict__ z,
                                                            long long n, int op, F64Cmp t) {
+    grid_entry();
     long long nchunks = (n + 15) / 16;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nchunks;
          c += (long long)gridDim.x * blockDim.x) {

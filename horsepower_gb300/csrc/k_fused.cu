@@ -358,6 +358,7 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
                "* part, " + A + " ident, unsigned* derr, unsigned* done, " + A + "* result) {\n"
                "    __shared__ " + A + " ws[8];\n"
                "    __shared__ bool last;\n"
+               "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"  // as grid_entry
                "    const long long base = (long long)blockIdx.x * 4096;\n" + hoist +
                "    #pragma unroll\n"
                "    for (int k = 0; k < 16; k++) {\n"
@@ -426,7 +427,8 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
                           "] : (" + ctype(types[k]) + ")0;\n";
         }
         src += "extern \"C\" __global__ void __launch_bounds__(256) chain_kernel(const void* const* cols, long long n, "
-               "unsigned char* mask, void* const* outs, unsigned* derr) {\n    bool dz = false;\n"
+               "unsigned char* mask, void* const* outs, unsigned* derr) {\n"
+               "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n    bool dz = false;\n"
                "    const long long stride = (long long)gridDim.x * blockDim.x;\n"
                "    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += " +
                std::to_string(CH_UNROLL) + " * stride) {\n" + ld + body + "    }\n    if (dz) atomicOr(derr, 4u);\n}\n";
@@ -516,7 +518,7 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
         if (grid > (unsigned)g_sms * 16) grid = g_sms * 16;
         {
             LaunchScope ls("chain");
-            HG_CU(cudaLaunchKernel((const void*)cm->kern, dim3(grid), dim3(256), args, 0, g_stream));
+            HG_CU(launch_kernel_args((const void*)cm->kern, dim3(grid), dim3(256), 0, args));
         }
         HG_CHECK(last_launch_error());
         if (cm->may_fail) {  // a division by zero fails the call, as the builtin's checkZero does
@@ -546,7 +548,7 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
         if (grid > (unsigned)g_sms * 16) grid = g_sms * 16;
         {
             LaunchScope ls("chain");
-            HG_CU(cudaLaunchKernel((const void*)cm->kern, dim3(grid), dim3(256), args, 0, g_stream));
+            HG_CU(launch_kernel_args((const void*)cm->kern, dim3(grid), dim3(256), 0, args));
         }
         HG_CHECK(check_device_errors());
         if (!zs_many) return set_error(E_DOMAIN, "chain: compress writes several outputs; use hgpuChainRunMany");
@@ -595,7 +597,7 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
     void* args[] = {&dcols, &nn, &part, &ident, &g_derr, &done, &rptr};
     {
         LaunchScope ls("chain");
-        HG_CU(cudaLaunchKernel((const void*)cm->kern, dim3((unsigned)tiles), dim3(256), args, 0, g_stream));
+        HG_CU(launch_kernel_args((const void*)cm->kern, dim3((unsigned)tiles), dim3(256), 0, args));
     }
     if (!one_launch) {
         int op = cm->sink == "min" ? 1 : cm->sink == "max" ? 2 : 0;

@@ -20,6 +20,7 @@ __device__ __forceinline__ long long load_idx(const void* y, long long i) {
 template <typename ET, typename IT>
 __global__ void __launch_bounds__(256) k_gather(const ET* __restrict__ x, long long nx, const void* __restrict__ y,
                                                 ET* __restrict__ z, long long n, unsigned* derr, int vec) {
+    grid_entry();
     bool bad = false;
     long long stride = (long long)gridDim.x * blockDim.x * 4;
     for (long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i0 < n; i0 += stride) {
@@ -140,6 +141,7 @@ __device__ __forceinline__ void gm_column(const void* src, long long nx, void* d
 template <typename IT>
 __global__ void __launch_bounds__(256) k_gather_many(GatherCols c, const void* __restrict__ y, long long n, unsigned* derr,
                                                      int vec) {
+    grid_entry();
     bool bad = false;
     const long long stride = (long long)gridDim.x * blockDim.x * 4;
     for (long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i0 < n; i0 += stride) {

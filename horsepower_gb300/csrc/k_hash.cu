@@ -256,6 +256,7 @@ __device__ __forceinline__ long long table_find(const Table<K>& t, K k, long lon
 
 template <typename K>
 __global__ void k_build(Table<K> t, const void* __restrict__ x, int typ, long long n, unsigned* derr) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         K k;
         if (key_at<K>(x, typ, i, &k)) table_insert<K>(t, k, (unsigned)i, derr);
@@ -263,6 +264,7 @@ __global__ void k_build(Table<K> t, const void* __restrict__ x, int typ, long lo
 }
 
 __global__ void k_key_minmax(const void* __restrict__ x, int typ, long long n, long long* mm) {
+    grid_entry();
     long long a = LLONG_MAX, b = LLONG_MIN;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long v;
@@ -376,6 +378,7 @@ __device__ __forceinline__ void note_miss(unsigned* miss, bool missed) {
 template <typename K>
 __global__ void k_index_of(Table<K> t, const void* __restrict__ y, int typ, long long n, long long lenX,
                            long long* __restrict__ z, unsigned* miss) {
+    grid_entry();
     bool missed = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         K k;
@@ -395,6 +398,7 @@ __global__ void k_index_of(Table<K> t, const void* __restrict__ y, int typ, long
 // flags == 1)
 template <typename T>
 __global__ void k_order_flags(const T* __restrict__ x, long long n, unsigned* flags) {
+    grid_entry();
     bool up = false, down = false, eq = false;
     for (long long i = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         T a = x[i - 1], b = x[i];
@@ -420,6 +424,7 @@ __device__ __forceinline__ unsigned long long bucket_of(long long v, long long x
 template <typename T>
 __global__ void k_bucket_firsts(const T* __restrict__ x, long long n, long long x0, int s, unsigned* __restrict__ bst,
                                 unsigned long long nb) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned long long b = bucket_of((long long)x[i], x0, s);
         if (i == 0 || bucket_of((long long)x[i - 1], x0, s) != b) bst[b] = (unsigned)i;
@@ -430,6 +435,7 @@ __global__ void k_bucket_firsts(const T* __restrict__ x, long long n, long long 
 template <typename T>
 __global__ void k_bucket_fill(const T* __restrict__ x, long long n, long long x0, int s, unsigned* __restrict__ bst,
                               unsigned long long nb) {
+    grid_entry();
     for (unsigned long long b = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; b < nb;
          b += (unsigned long long)gridDim.x * blockDim.x) {
         if (bst[b] != ~0u) continue;
@@ -446,6 +452,7 @@ template <typename T>
 __global__ void k_search_bucketed(const T* __restrict__ x, long long lenX, long long x0, long long xl, int s,
                                   const unsigned* __restrict__ bst, const void* __restrict__ y, int ytyp, long long n,
                                   long long* __restrict__ z, unsigned* miss) {
+    grid_entry();
     bool missed = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long v;
@@ -490,6 +497,7 @@ __device__ __forceinline__ long long probe_val(const void* __restrict__ y, int y
 template <typename T>
 __global__ void k_rank_bits(const T* __restrict__ x, long long x0, const unsigned* __restrict__ bst, unsigned long long nw,
                             ulonglong2* __restrict__ ent) {
+    grid_entry();
     for (unsigned long long w = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; w < nw;
          w += (unsigned long long)gridDim.x * blockDim.x) {
         const unsigned lo = bst[w], hi = bst[w + 1];
@@ -500,6 +508,7 @@ __global__ void k_rank_bits(const T* __restrict__ x, long long x0, const unsigne
 }
 __global__ void k_search_rank(long long x0, long long xl, const ulonglong2* __restrict__ ent, const void* __restrict__ y,
                               int ytyp, long long n, long long lenX, long long* __restrict__ z, unsigned* miss) {
+    grid_entry();
     bool missed = false;
 #pragma unroll 1
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -524,6 +533,7 @@ template <typename K, bool FILTER>
 __global__ void k_index_of_direct(const unsigned* __restrict__ rows, const unsigned* __restrict__ filter, long long kmin,
                                   long long kmax, const void* __restrict__ y, int typ, long long n, long long lenX,
                                   long long* __restrict__ z, unsigned* miss) {
+    grid_entry();
     bool missed = false;
 #pragma unroll 1
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -552,6 +562,7 @@ __global__ void k_index_of_direct(const unsigned* __restrict__ rows, const unsig
 template <typename T>
 __global__ void k_search_ordered(const T* __restrict__ x, long long lenX, const void* __restrict__ y, int ytyp,
                                  long long n, long long* __restrict__ z, unsigned* miss) {
+    grid_entry();
     bool missed = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long v;
@@ -580,11 +591,13 @@ __global__ void k_search_ordered(const T* __restrict__ x, long long lenX, const 
 }
 
 __global__ void k_first_false(const bool* __restrict__ x, long long n, unsigned long long* first) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         if (!x[i]) atomicMin(first, (unsigned long long)i);
 }
 __global__ void k_index_of_bool(const bool* __restrict__ y, long long n, const unsigned long long* first,
                                 long long lenX, long long* __restrict__ z, unsigned* miss) {
+    grid_entry();
     long long f = (*first == ~0ull) ? lenX : (long long)*first;
     bool missed = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -603,6 +616,7 @@ static unsigned grid_cap(long long n) {
 // ------------------------------------------------------------------ member
 template <typename K>
 __global__ void k_member(Table<K> t, const void* __restrict__ y, int typ, long long n, bool* __restrict__ z) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         K k;
         bool r = false;
@@ -615,6 +629,7 @@ __global__ void k_member(Table<K> t, const void* __restrict__ y, int typ, long l
 // sets of one or two elements: direct == compares (lib_member_fast1/2, h_libs.cc:900-945)
 template <typename T>
 __global__ void k_member_small(const T* __restrict__ y, long long n, T a, T b, int m, bool* __restrict__ z) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         T v = y[i];
         z[i] = (m >= 1 && v == a) || (m >= 2 && v == b);
@@ -622,6 +637,7 @@ __global__ void k_member_small(const T* __restrict__ y, long long n, T a, T b, i
 }
 __global__ void k_member_bool(const bool* __restrict__ x, long long nx, const bool* __restrict__ y, long long n,
                               unsigned* seen, bool* __restrict__ z, int phase) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (phase ? n : nx); i += (long long)gridDim.x * blockDim.x) {
         if (phase == 0) atomicOr(seen, x[i] ? 2u : 1u);
         else z[i] = (*seen & (y[i] ? 2u : 1u)) != 0;
@@ -661,6 +677,7 @@ __global__ void __launch_bounds__(JT_THREADS, (R > 16 ? 2 : 4)) k_join_probe(
     Table<K> t, LinearBuild lin, int mode, const void* __restrict__ y, int ytyp, long long n,
     long long* __restrict__ zb, long long* __restrict__ zp, unsigned long long* status, unsigned* ticket,
     unsigned long long* total, unsigned* derr) {
+    grid_entry();
     constexpr long long SUB = 32LL * R;  // rows per warp sub-tile
     __shared__ long long tile_id;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -719,6 +736,7 @@ __global__ void __launch_bounds__(JT_THREADS, (R > 16 ? 2 : 4)) k_join_probe(
 template <typename K>
 __global__ void k_csr_fill(Table<K> t, const void* __restrict__ x, int typ, long long n,
                            const unsigned long long* __restrict__ start, unsigned* fillc, unsigned* rows) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         K k;
         if (!key_at<K>(x, typ, i, &k)) continue;
@@ -731,6 +749,7 @@ __global__ void k_csr_fill(Table<K> t, const void* __restrict__ x, int typ, long
 }
 template <typename K>
 __global__ void k_slot_counts(Table<K> t, const void* __restrict__ x, int typ, long long n) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         K k;
         if (!key_at<K>(x, typ, i, &k)) continue;
@@ -741,6 +760,7 @@ __global__ void k_slot_counts(Table<K> t, const void* __restrict__ x, int typ, l
 }
 __global__ void k_csr_sort(const unsigned long long* __restrict__ start, const unsigned* __restrict__ cnt,
                            long long nslots, unsigned* rows) {
+    grid_entry();
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         unsigned c = cnt[s];
         if (c < 2) continue;
@@ -756,6 +776,7 @@ __global__ void k_csr_sort(const unsigned long long* __restrict__ start, const u
 template <typename K>
 __global__ void k_join_count(Table<K> t, const void* __restrict__ y, int ytyp, long long n,
                              unsigned* __restrict__ c, unsigned* __restrict__ slot) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         K k;
         unsigned cc = 0, ss = 0;
@@ -773,6 +794,7 @@ __global__ void k_join_write(const unsigned* __restrict__ c, const unsigned* __r
                              const unsigned long long* __restrict__ off, long long n,
                              const unsigned long long* __restrict__ start, const unsigned* __restrict__ rows,
                              long long* __restrict__ zb, long long* __restrict__ zp) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned cc = c[i];
         unsigned long long o = off[i], s0 = start[slot[i]];
@@ -823,6 +845,7 @@ template <int R>
 __global__ void __launch_bounds__(JT_THREADS) k_jp_stage(Table<unsigned> t, const int* __restrict__ y, long long n,
                                                          uint2* __restrict__ stage, unsigned* __restrict__ wcounts,
                                                          unsigned* __restrict__ wpre, unsigned* __restrict__ tcounts) {
+    grid_entry();
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const long long wid = (long long)blockIdx.x * (JT_THREADS / 32) + warp;
     const long long base = wid * (32 * R);
@@ -883,6 +906,7 @@ __global__ void __launch_bounds__(JT_THREADS) k_jp_stage_dsmem(Table<unsigned> t
                                                                long long ntiles, unsigned nwords, int shift,
                                                                uint2* __restrict__ stage, unsigned* __restrict__ wcounts,
                                                                unsigned* __restrict__ wpre, unsigned* __restrict__ tcounts) {
+    grid_entry();
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned qs_bits[];
     __shared__ const unsigned* peer[QC];
@@ -1006,6 +1030,7 @@ __global__ void __launch_bounds__(256) k_jp_unstage(const uint2* __restrict__ st
                                                     const unsigned* __restrict__ wpre,
                                                     const unsigned long long* __restrict__ toffs, long long nwarps, int per,
                                                     long long* __restrict__ zb, long long* __restrict__ zp) {
+    grid_entry();
     const unsigned lane = lane_id();
     const long long w0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * JU_GROUP;
     if (w0 >= nwarps) return;
@@ -1405,6 +1430,7 @@ struct PackSpec {
     int nc;
 };
 __global__ void k_pack_rows(PackSpec s, long long n, unsigned long long* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned long long key = 0;
         bool ok = true;
@@ -1423,6 +1449,7 @@ __global__ void k_pack_rows(PackSpec s, long long n, unsigned long long* __restr
     }
 }
 __global__ void k_fill_i64(long long* __restrict__ z, long long n, long long v) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) z[i] = v;
 }
 
@@ -1646,6 +1673,7 @@ template <typename T>
 __global__ void k_pair_keep(const void* __restrict__ x, int xt, const void* __restrict__ y, int yt,
                             const long long* __restrict__ a, const long long* __restrict__ b, long long m, int op,
                             uint8_t* __restrict__ keep) {
+    grid_entry();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
         const T u = elem_as<T>(x, xt, a[k]), v = elem_as<T>(y, yt, b[k]);
         bool r;

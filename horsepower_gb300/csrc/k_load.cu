@@ -252,6 +252,7 @@ I csv_symbols(const char* dbuf, const unsigned long long* spans, long long rows,
 unsigned grid_of(long long n);
 
 __global__ void k_text_lengths(const long long* __restrict__ sz, long long n, unsigned* __restrict__ lens) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         lens[i] = (unsigned)sz[i] + 1u;
 }
@@ -259,6 +260,7 @@ __global__ void k_text_lengths(const long long* __restrict__ sz, long long n, un
 __global__ void k_text_spans(const char* __restrict__ blob, const long long* __restrict__ sz,
                              const unsigned long long* __restrict__ offs, long long n,
                              unsigned long long* __restrict__ spans, unsigned* bad) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long o = offs[i];
         const int k = (int)sz[i];
@@ -494,6 +496,7 @@ __device__ unsigned nl_count_seg(const char* __restrict__ buf, long long n, long
     return c;
 }
 __global__ void k_nl_count(const char* __restrict__ buf, long long n, unsigned* __restrict__ counts) {
+    grid_entry();
     const long long t0 = (long long)blockIdx.x * NL_TILE + (long long)threadIdx.x * NL_PER;
     unsigned c = nl_count_seg(buf, n, t0);
     c = __reduce_add_sync(0xffffffffu, c);
@@ -510,6 +513,7 @@ __global__ void k_nl_count(const char* __restrict__ buf, long long n, unsigned* 
 // positions of the newlines of each tile, in order (offs: exclusive tile prefix)
 __global__ void k_nl_scatter(const char* __restrict__ buf, long long n, const unsigned long long* __restrict__ offs,
                              long long* __restrict__ pos) {
+    grid_entry();
     const long long t0 = (long long)blockIdx.x * NL_TILE + (long long)threadIdx.x * NL_PER;
     const unsigned c = nl_count_seg(buf, n, t0);
     // exclusive prefix of c over the block (thread order = byte order)
@@ -769,6 +773,7 @@ __device__ __forceinline__ unsigned byte_mask(long long o, long long lo, long lo
 }
 
 __global__ void k_csv_parse(CsvArgs a) {
+    grid_entry();
     extern __shared__ unsigned csv_fields[];
     const int warp = threadIdx.x >> 5, lane = lane_id();
     const int nc = a.ncols;
@@ -1081,6 +1086,7 @@ __device__ unsigned long long exact_decimal(const char* p_, int n, int p, Big& D
 
 __global__ void k_csv_slow(const char* __restrict__ buf, const unsigned long long* __restrict__ slow, unsigned nslow,
                            const CsvCol* __restrict__ cols, Big* __restrict__ work) {
+    grid_entry();
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < nslow; t += gridDim.x * blockDim.x) {
         const unsigned long long span = slow[2 * t], meta = slow[2 * t + 1];
         const char* f = buf + (span >> 16);
@@ -1107,6 +1113,7 @@ __device__ __forceinline__ unsigned long long span_hash(const char* buf, unsigne
 __global__ void k_sym_insert(const char* __restrict__ buf, const unsigned long long* __restrict__ spans, long long rows,
                              unsigned long long* __restrict__ keys, unsigned long long* __restrict__ first,
                              unsigned long long mask, unsigned* derr) {
+    grid_entry();
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x) {
         const unsigned long long h = span_hash(buf, spans[r]);
         unsigned long long sl = (h * 0x9e3779b97f4a7c15ull) >> 20 & mask;
@@ -1126,6 +1133,7 @@ __global__ void k_sym_insert(const char* __restrict__ buf, const unsigned long l
 __global__ void k_sym_rep(const char* __restrict__ buf, const unsigned long long* __restrict__ spans, long long rows,
                           const unsigned long long* __restrict__ keys, const unsigned long long* __restrict__ first,
                           unsigned long long mask, long long* __restrict__ rep, uint8_t* __restrict__ is_first) {
+    grid_entry();
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x) {
         const unsigned long long h = span_hash(buf, spans[r]);
         unsigned long long sl = (h * 0x9e3779b97f4a7c15ull) >> 20 & mask;
@@ -1142,6 +1150,7 @@ __global__ void k_sym_rep(const char* __restrict__ buf, const unsigned long long
 __global__ void k_sym_pack(const char* __restrict__ buf, const unsigned long long* __restrict__ spans,
                            const long long* __restrict__ drows, long long nd, const unsigned long long* __restrict__ offs,
                            char* __restrict__ blob, unsigned* __restrict__ dpos) {
+    grid_entry();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nd; k += (long long)gridDim.x * blockDim.x) {
         const long long r = drows[k];
         const unsigned long long sp = spans[r];
@@ -1155,6 +1164,7 @@ __global__ void k_sym_pack(const char* __restrict__ buf, const unsigned long lon
 }
 __global__ void k_sym_lengths(const unsigned long long* __restrict__ spans, const long long* __restrict__ drows, long long nd,
                               unsigned* __restrict__ lens) {
+    grid_entry();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nd; k += (long long)gridDim.x * blockDim.x)
         lens[k] = (unsigned)(spans[drows[k]] & 0xffffull) + 1u;
 }
@@ -1162,6 +1172,7 @@ __global__ void k_sym_lengths(const unsigned long long* __restrict__ spans, cons
 __global__ void k_sym_ids(const char* __restrict__ buf, const unsigned long long* __restrict__ spans, long long rows,
                           const long long* __restrict__ rep, const unsigned* __restrict__ dpos,
                           const long long* __restrict__ ids, long long* __restrict__ out, unsigned* __restrict__ bad) {
+    grid_entry();
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x) {
         const long long f = rep[r];
         out[r] = ids[dpos[f]];
@@ -1175,6 +1186,7 @@ __global__ void k_sym_ids(const char* __restrict__ buf, const unsigned long long
     }
 }
 __global__ void k_str_lengths(const unsigned long long* __restrict__ spans, long long rows, unsigned* __restrict__ lens) {
+    grid_entry();
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x)
         lens[r] = (unsigned)(spans[r] & 0xffffull) + 1u;
 }
@@ -1184,6 +1196,7 @@ __global__ void k_str_pack(const char* __restrict__ buf, const unsigned long lon
                            const unsigned long long* __restrict__ offs, char* __restrict__ dblob,
                            unsigned long long host_base, unsigned long long* __restrict__ ptrs,
                            unsigned long long* __restrict__ bspans) {
+    grid_entry();
     const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     const int lane = lane_id();

@@ -74,11 +74,13 @@ __device__ __forceinline__ int qs_cmp(unsigned long long a, unsigned long long b
 // img[p] = image of col[perm[p]] (perm null: row p)
 __global__ void k_qs_image(const void* __restrict__ col, int typ, const unsigned* __restrict__ perm, long long n,
                            unsigned long long flip, unsigned long long* __restrict__ img, unsigned* nanflag) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
         img[p] = qs_image(col, typ, perm ? (long long)perm[p] : p, nanflag) ^ flip;
 }
 
 __global__ void k_qs_iota(unsigned* __restrict__ v, long long n) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
         v[p] = (unsigned)p;
 }
@@ -97,6 +99,7 @@ __device__ __forceinline__ unsigned long long qs_flag(const unsigned* __restrict
 
 __global__ void __launch_bounds__(QS_THREADS) k_qs_count(const unsigned* __restrict__ lo, const unsigned long long* __restrict__ K,
                                                          long long n, unsigned long long* __restrict__ tile_sum) {
+    grid_entry();
     __shared__ unsigned long long ws[QS_THREADS / 32];
     const long long base = (long long)blockIdx.x * QS_TILE + (long long)threadIdx.x * QS_ITEMS;
     unsigned long long s = 0;
@@ -115,6 +118,7 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_count(const unsigned* __restr
 
 // exclusive scan of the nt tile sums in place (one block); tile_sum[nt] = total
 __global__ void __launch_bounds__(1024) k_qs_scan_sums(unsigned long long* __restrict__ ts, long long nt) {
+    grid_entry();
     __shared__ unsigned long long wsum[32];
     const long long per = (nt + 1023) / 1024;
     const long long a = (long long)threadIdx.x * per, b = a + per < nt ? a + per : nt;
@@ -138,6 +142,7 @@ __global__ void __launch_bounds__(1024) k_qs_scan_sums(unsigned long long* __res
 __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __restrict__ lo, const unsigned long long* __restrict__ K,
                                                           long long n, const unsigned long long* __restrict__ tile_sum,
                                                           long long nt, unsigned long long* __restrict__ S) {
+    grid_entry();
     __shared__ unsigned long long ws[QS_THREADS / 32];
     const long long base = (long long)blockIdx.x * QS_TILE + (long long)threadIdx.x * QS_ITEMS;
     unsigned long long v[QS_ITEMS], s = 0;
@@ -169,6 +174,7 @@ __device__ __forceinline__ unsigned qs_lt(unsigned long long s) { return (unsign
 __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __restrict__ hi,
                          const unsigned long long* __restrict__ K, const unsigned long long* __restrict__ S, long long n,
                          unsigned* __restrict__ Lpos, unsigned* __restrict__ Rpos, unsigned* derr) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned l = lo[p];
         if (l == QS_DONE || (long long)l == p) continue;
@@ -194,6 +200,7 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
                           const unsigned* __restrict__ Lpos, const unsigned* __restrict__ Rpos,
                           unsigned long long* __restrict__ K2, unsigned* __restrict__ P2, unsigned* __restrict__ fin,
                           unsigned* __restrict__ active, unsigned* derr) {
+    grid_entry();
     unsigned still = 0;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned l = lo[p];
@@ -249,6 +256,7 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
 // ---- ranges (segments) of a list sort
 // seg[p] = index of the segment holding position p (starts ascending)
 __global__ void k_qs_segid(const long long* __restrict__ starts, long long ns, long long n, unsigned* __restrict__ seg) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         long long a = 0, b = ns - 1;  // last start <= p
         while (a < b) {
@@ -261,6 +269,7 @@ __global__ void k_qs_segid(const long long* __restrict__ starts, long long ns, l
 // lib_order_by_sorted per segment: up[s] / down[s] = some neighbour pair rises / falls
 __global__ void k_qs_updown(const unsigned long long* __restrict__ img, const unsigned* __restrict__ seg, long long n,
                             uint8_t* __restrict__ up, uint8_t* __restrict__ down) {
+    grid_entry();
     for (long long p = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned s = seg[p];
         if (s != seg[p - 1]) continue;
@@ -275,6 +284,7 @@ enum : uint8_t { QS_SORT = 0, QS_KEEP = 1, QS_REVERSE = 2 };
 // ascend (images fall, never rise) is reversed; every other one is sorted
 __global__ void k_qs_mode(const uint8_t* __restrict__ up, const uint8_t* __restrict__ down, long long ns, int desc,
                           uint8_t* __restrict__ mode, unsigned* __restrict__ nrev) {
+    grid_entry();
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < ns; s += (long long)gridDim.x * blockDim.x) {
         uint8_t m = QS_SORT;
         if (!desc && up[s] && !down[s]) m = QS_KEEP;
@@ -285,6 +295,7 @@ __global__ void k_qs_mode(const uint8_t* __restrict__ up, const uint8_t* __restr
 __global__ void k_qs_reverse(const unsigned* __restrict__ perm, const unsigned* __restrict__ seg,
                              const long long* __restrict__ starts, long long ns, long long n, const uint8_t* __restrict__ mode,
                              unsigned* __restrict__ out) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned s = seg[p];
         long long q = p;
@@ -300,6 +311,7 @@ __global__ void k_qs_reverse(const unsigned* __restrict__ perm, const unsigned* 
 __global__ void k_qs_ranges(const unsigned* __restrict__ seg, const long long* __restrict__ starts, long long ns, long long n,
                             const uint8_t* __restrict__ mode, const unsigned* __restrict__ perm,
                             unsigned* __restrict__ lo, unsigned* __restrict__ hi, unsigned* __restrict__ fin) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned s = seg ? seg[p] : 0;
         const long long a = seg ? starts[s] : 0, b = seg ? (s + 1 < ns ? starts[s + 1] : n) : n;
@@ -317,6 +329,7 @@ __global__ void k_qs_ranges(const unsigned* __restrict__ seg, const long long* _
 __global__ void k_qs_skey(const unsigned long long* __restrict__ img, const unsigned* __restrict__ seg,
                           const long long* __restrict__ starts, long long ns, long long n, const uint8_t* __restrict__ mode,
                           int min_len, unsigned long long* __restrict__ key) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned s = seg[p];
         const long long a = starts[s], b = s + 1 < ns ? starts[s + 1] : n;
@@ -325,11 +338,13 @@ __global__ void k_qs_skey(const unsigned long long* __restrict__ img, const unsi
 }
 __global__ void k_qs_gather_seg(const unsigned* __restrict__ seg, const unsigned* __restrict__ pos, long long n,
                                 unsigned* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = seg[pos[i]];
 }
 __global__ void k_qs_permute(const unsigned* __restrict__ perm, const unsigned* __restrict__ pos, long long n,
                              unsigned* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = perm[pos[i]];
 }
@@ -337,6 +352,7 @@ __global__ void k_qs_permute(const unsigned* __restrict__ perm, const unsigned* 
 // exchange on a[rtn[i]] > a[rtn[j]], one thread per sorted segment
 __global__ void k_qs_char_small(const int8_t* __restrict__ a, const long long* __restrict__ starts, long long ns, long long n,
                                 const uint8_t* __restrict__ mode, unsigned* __restrict__ perm) {
+    grid_entry();
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < ns; s += (long long)gridDim.x * blockDim.x) {
         const long long lo = starts[s], hi = s + 1 < ns ? starts[s + 1] : n;
         if (mode[s] != QS_SORT || hi - lo >= 10 || hi - lo < 2) continue;
@@ -352,6 +368,7 @@ __global__ void k_qs_char_small(const int8_t* __restrict__ a, const long long* _
 // run heads of the next column: a new segment or a new image value
 __global__ void k_qs_heads(const unsigned long long* __restrict__ img, const unsigned* __restrict__ seg, long long n,
                            uint8_t* __restrict__ head) {
+    grid_entry();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
         head[p] = p == 0 || seg[p] != seg[p - 1] || img[p] != img[p - 1];
 }

@@ -49,6 +49,7 @@ __device__ __forceinline__ A warp_red(A v) {
 // Block = 256 threads, one 4096-element tile per block.
 template <typename T, typename A, int OP>
 __global__ void __launch_bounds__(256) k_tile_reduce(const T* __restrict__ x, long long n, A* __restrict__ out, A ident) {
+    grid_entry();
     __shared__ A ws[8];
     const long long base = (long long)blockIdx.x * TILE_SUM;
     A acc = ident;
@@ -159,6 +160,7 @@ __device__ __forceinline__ unsigned long long fx_round(Fx128 a, int sexp) {
 // Block = 256 threads, one 4096-element tile per block.
 __global__ void __launch_bounds__(256) k_tile_sum_fx(const unsigned long long* __restrict__ x, long long n,
                                                      double* __restrict__ out) {
+    grid_entry();
     __shared__ unsigned s_e[8], s_f[8];
     __shared__ Fx128 s_acc[8];
     const long long base = (long long)blockIdx.x * TILE_SUM;
@@ -328,6 +330,7 @@ __device__ __forceinline__ long long block_max_i64(long long v) {
 template <typename T, int OP>
 __global__ void __launch_bounds__(256) k_tile_minmax_f(const T* __restrict__ x, long long n, long long* __restrict__ onan,
                                                        long long* __restrict__ okey, long long* __restrict__ opos) {
+    grid_entry();
     const long long base = (long long)blockIdx.x * TILE_SUM;
     const int lim = (int)min((long long)TILE_SUM, n - base);
     T v[16];
@@ -393,6 +396,7 @@ __global__ void __launch_bounds__(256) k_minmax_combine(const long long* __restr
                                                         const long long* __restrict__ ipos, long long m,
                                                         long long* __restrict__ onan, long long* __restrict__ okey,
                                                         long long* __restrict__ opos) {
+    grid_entry();
     const long long base = (long long)blockIdx.x * TILE_SUM;
     long long J = -1;
     for (int k = 0; k < 16; k++) {
@@ -413,6 +417,7 @@ __global__ void __launch_bounds__(256) k_minmax_combine(const long long* __restr
 
 template <typename T>
 __global__ void k_minmax_pick(const T* __restrict__ x, const long long* nan, const long long* pos, T* out) {
+    grid_entry();
     *out = x[*pos >= 0 ? *pos : *nan];
 }
 
@@ -465,6 +470,7 @@ static I tree_reduce(const T* x, long long n, A ident, A* result) {
 // avg = sum / len (pfnAvg, h_primitive.cc:792-797)
 template <typename A>
 __global__ void k_avg_final(const A* s, long long n, void* out) {
+    grid_entry();
     if constexpr (std::is_same<A, long long>::value) *(double*)out = __ddiv_rn((double)*s * 1.0, (double)n);
     else if constexpr (std::is_same<A, float>::value) *(float*)out = __fdiv_rn(*s, (float)n);
     else *(double*)out = __ddiv_rn(*s, (double)n);

@@ -11,6 +11,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_scan_u32(const unsigned* __restr
                                                          unsigned long long* __restrict__ out,
                                                          unsigned long long* status, unsigned* ticket,
                                                          unsigned long long* total, unsigned* derr) {
+    grid_entry();
     __shared__ unsigned long long warp_tot[8];
     __shared__ unsigned long long tile_off;
     __shared__ long long tile_id;
@@ -72,6 +73,7 @@ I scan_exclusive(const unsigned* in, long long n, unsigned long long* out, unsig
 // block-wide look-back of the scans and compactions; mode 1: the per-digit
 // chain look-back of the radix passes.
 __global__ void k_selftest_wait(unsigned long long* status, unsigned* ticket, int mode, long long limit, unsigned* derr) {
+    grid_entry();
     __shared__ long long tile;
     if (threadIdx.x == 0) tile = atomicAdd(ticket, 1u);
     __syncthreads();

@@ -178,6 +178,7 @@ __device__ __forceinline__ int seg_class(long long m) {
 // ones, in all (*nch)
 __global__ void k_seg_class_count(const long long* __restrict__ starts, long long ng, long long total,
                                   unsigned* __restrict__ cnt, unsigned long long* __restrict__ nch) {
+    grid_entry();
     __shared__ unsigned sc[SEG_CLASSES];
     __shared__ unsigned long long snch;
     if (threadIdx.x < SEG_CLASSES) sc[threadIdx.x] = 0;
@@ -199,6 +200,7 @@ __global__ void k_seg_class_count(const long long* __restrict__ starts, long lon
 __global__ void k_seg_class_ids(const long long* __restrict__ starts, long long ng, long long total,
                                 const unsigned* __restrict__ cnt, unsigned* __restrict__ cur,
                                 unsigned* __restrict__ ids) {
+    grid_entry();
     __shared__ unsigned sc[SEG_CLASSES], sbase[SEG_CLASSES];
     if (threadIdx.x < SEG_CLASSES) sc[threadIdx.x] = 0;
     __syncthreads();
@@ -230,6 +232,7 @@ __global__ void __launch_bounds__(256) k_seg_warps(SegIO<T, A> io, const long lo
                                                    long long total, const unsigned* __restrict__ ids,
                                                    const unsigned* __restrict__ cnt, A ident,
                                                    unsigned* derr) {
+    grid_entry();
     const T* __restrict__ src = io.src[blockIdx.y];
     A* __restrict__ out = io.out[blockIdx.y];
     __shared__ long long wfirst[7];  // first warp of each class 0-5; wfirst[6] = warps in all
@@ -282,6 +285,7 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long l
                                                  long long total, const unsigned* __restrict__ ids,
                                                  const unsigned* __restrict__ cnt, A ident,
                                                  unsigned* derr) {
+    grid_entry();
     const T* __restrict__ src = io.src[blockIdx.y];
     A* __restrict__ out = io.out[blockIdx.y];
     __shared__ unsigned first;
@@ -356,6 +360,7 @@ template <typename A, int OP>
 __global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ parts, const long long* __restrict__ pstarts,
                                                       const long long* __restrict__ big, long long nbig,
                                                       long long nchunks, A ident, SegIO<A, A> io) {
+    grid_entry();
     __shared__ A ws[256];
     const long long g = blockIdx.x;
     const A* __restrict__ part = parts + (size_t)blockIdx.y * (size_t)nchunks;
@@ -379,6 +384,7 @@ template <typename T, typename A, int OP, bool GATHER>
 __global__ void __launch_bounds__(256, 4) k_seg_chunk(SegIO<T, A> io, const long long* __restrict__ rows,
                                                       long long nx, const ChunkDesc* __restrict__ order, A ident,
                                                       A* __restrict__ part, unsigned* derr) {
+    grid_entry();
     const T* __restrict__ src = io.src[blockIdx.y];
     part += (size_t)blockIdx.y * gridDim.x;
     __shared__ A ws[256];
@@ -403,6 +409,7 @@ __global__ void __launch_bounds__(1024) k_big_plan(const long long* __restrict__
                                                    const unsigned* __restrict__ ids, long long nbig,
                                                    long long* __restrict__ big, unsigned long long* __restrict__ c0,
                                                    long long* __restrict__ ps) {
+    grid_entry();
     __shared__ unsigned long long wsum[32];
     __shared__ unsigned long long carry;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -453,6 +460,7 @@ __global__ void k_chunk_desc(const long long* __restrict__ rows, const long long
                              const unsigned long long* __restrict__ c0, long long nbig, long long nchunks, int shift,
                              ChunkDesc* __restrict__ desc, unsigned short* __restrict__ region,
                              unsigned* __restrict__ hist) {
+    grid_entry();
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= nchunks) return;
     long long lo = 0, hi = nbig - 1;  // the long segment owning chunk t
@@ -472,6 +480,7 @@ __global__ void k_chunk_desc(const long long* __restrict__ rows, const long long
     }
 }
 __global__ void __launch_bounds__(1024) k_chunk_regions(unsigned* __restrict__ hist) {
+    grid_entry();
     __shared__ unsigned wsum[32];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     uint4* h4 = reinterpret_cast<uint4*>(hist);  // CHUNK_BUCKETS = 4 per thread
@@ -489,11 +498,13 @@ __global__ void __launch_bounds__(1024) k_chunk_regions(unsigned* __restrict__ h
 }
 __global__ void k_chunk_place(const ChunkDesc* __restrict__ desc, const unsigned short* __restrict__ region,
                               long long nchunks, unsigned* __restrict__ next, ChunkDesc* __restrict__ order) {
+    grid_entry();
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t < nchunks) order[atomicAdd(&next[region[t]], 1u)] = desc[t];
 }
 template <typename A>
 __global__ void k_scatter_big(const A* __restrict__ r, const long long* __restrict__ big, long long nbig, A* __restrict__ out) {
+    grid_entry();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nbig; k += (long long)gridDim.x * blockDim.x)
         out[big[k]] = r[k];
 }
@@ -547,6 +558,7 @@ __global__ void __launch_bounds__(1024) k_seg_plan_small(const long long* __rest
                                                          unsigned* __restrict__ ids, long long* __restrict__ big,
                                                          unsigned long long* __restrict__ c0, long long* __restrict__ ps,
                                                          ChunkDesc* __restrict__ order, unsigned long long* __restrict__ hdr) {
+    grid_entry();
     __shared__ unsigned sc[SEG_CLASSES], soff[SEG_CLASSES], scur[SEG_CLASSES];
     __shared__ unsigned wb[32];
     __shared__ unsigned long long wc[32];
@@ -761,6 +773,7 @@ __global__ void __launch_bounds__(256, 4) k_seg_chunk_many(SegCols cols, const l
                                                            unsigned long long nchunks,
                                                            const ChunkDesc* __restrict__ order,
                                                            double* __restrict__ part, unsigned* derr) {
+    grid_entry();
     __shared__ double ws[NCOL][256];
     const ChunkDesc d = order[blockIdx.x];
     const long long first = d.first + threadIdx.x, e = d.first + d.len;
@@ -911,6 +924,7 @@ I seg_sum_f64_direct(const double* const* srcs, int ncol, const long long* start
 template <typename A>
 __global__ void k_avg_seg(const A* __restrict__ s, const long long* __restrict__ starts, long long ng, long long total,
                           void* __restrict__ out) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
         long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
         if constexpr (std::is_same<A, long long>::value) ((double*)out)[g] = __ddiv_rn((double)s[g] * 1.0, (double)m);
@@ -919,6 +933,7 @@ __global__ void k_avg_seg(const A* __restrict__ s, const long long* __restrict__
     }
 }
 __global__ void k_len_seg(const long long* __restrict__ starts, long long ng, long long total, long long* __restrict__ out) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x)
         out[g] = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
 }
@@ -926,6 +941,7 @@ __global__ void k_len_seg(const long long* __restrict__ starts, long long ng, lo
 template <typename T>
 __global__ void k_minmax_fix(const T* __restrict__ r, const long long* __restrict__ starts, long long ng, long long total,
                              int op, int to_long, void* __restrict__ out) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
         long long m = ((g + 1 < ng) ? starts[g + 1] : total) - starts[g];
         if (to_long) ((long long*)out)[g] = m ? (long long)r[g] : (op == AG_MIN ? LLONG_MAX : LLONG_MIN);
@@ -935,6 +951,7 @@ __global__ void k_minmax_fix(const T* __restrict__ r, const long long* __restric
     }
 }
 __global__ void k_any_empty(const long long* __restrict__ starts, long long ng, long long total, unsigned* flag) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x)
         if (((g + 1 < ng) ? starts[g + 1] : total) == starts[g]) atomicOr(flag, 1u);
 }
@@ -1015,6 +1032,7 @@ static I agg_dispatch(int ag, I xt, const void* src, const long long* rows, long
 
 // ------------------------------------------------ lists -> contiguous segments
 __global__ void k_node_lens(const V0* __restrict__ nodes, long long ng, unsigned* __restrict__ lens) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x)
         lens[g] = (unsigned)nodes[g].len;
 }
@@ -1025,6 +1043,7 @@ __global__ void k_node_lens(const V0* __restrict__ nodes, long long ng, unsigned
 template <typename T>
 __global__ void k_node_copy(const V0* __restrict__ nodes, long long ng, unsigned long long host_base,
                             const unsigned long long* __restrict__ off, T* __restrict__ data) {
+    grid_entry();
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long g = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ng; g += warps) {
         const V0 v = nodes[g];
@@ -1034,6 +1053,7 @@ __global__ void k_node_copy(const V0* __restrict__ nodes, long long ng, unsigned
     }
 }
 __global__ void k_offsets_i64(const unsigned long long* __restrict__ a, long long n, long long* __restrict__ b) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         b[i] = (long long)a[i];
 }
@@ -1103,6 +1123,7 @@ static I list_segments(V y, I typ, const long long** starts, long long* total, c
 // points at its own host node)
 __global__ void k_scalar_nodes(const char* __restrict__ vals, long long ng, int es, I typ, V0* __restrict__ out,
                                unsigned long long host_base) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
         V0 v;
         v.len = 1;
@@ -1116,6 +1137,7 @@ __global__ void k_scalar_nodes(const char* __restrict__ vals, long long ng, int 
 // segment nodes over a contiguous payload (inline when one element)
 __global__ void k_segment_nodes(const char* __restrict__ data, const long long* __restrict__ starts, long long ng,
                                 long long total, int es, I typ, V0* __restrict__ out, unsigned long long host_base) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
         long long s = starts[g], e = (g + 1 < ng) ? starts[g + 1] : total;
         V0 v;

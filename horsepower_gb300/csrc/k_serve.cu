@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(256) k_s_q6(const int* __restrict__ ship, cons
                                               const double* __restrict__ disc, const double* __restrict__ price,
                                               long long n, const int* __restrict__ lohi, int nw,
                                               double* __restrict__ part, long long ntiles, F64Cmp d_lo, F64Cmp d_hi) {
+    grid_entry();
     __shared__ int s_lo[SQ_MAXW], s_hi[SQ_MAXW];
     __shared__ double ws[SQ_MAXW][8];
     for (int w = threadIdx.x; w < nw; w += 256) {
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(256) k_s_q6(const int* __restrict__ ship, cons
 // in[w][0..m) -> out[w][0..m2), block (tile, w).
 __global__ void __launch_bounds__(256) k_s_rows(const double* __restrict__ in, long long m, double* __restrict__ out,
                                                 long long m2) {
+    grid_entry();
     __shared__ double ws[8];
     const long long w = blockIdx.y, base = (long long)blockIdx.x * TILE_SUM;
     const double* x = in + w * m;
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(256) k_s_rows(const double* __restrict__ in, l
 // are counted in shared memory first (the hot bins of skewed keys).
 __global__ void k_s_hist(const void* __restrict__ col, int is64, long long n, long long kmin, long long range,
                          unsigned* __restrict__ hist) {
+    grid_entry();
     __shared__ unsigned sh[4096];
     for (int i = threadIdx.x; i < 4096; i += blockDim.x) sh[i] = 0;
     __syncthreads();
@@ -124,6 +127,7 @@ __global__ void k_s_hist(const void* __restrict__ col, int is64, long long n, lo
 }
 
 __global__ void k_s_minmax(const void* __restrict__ col, int is64, long long n, long long* mm) {
+    grid_entry();
     long long a = LLONG_MAX, b = LLONG_MIN;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long v = is64 ? ((const long long*)col)[i] : (long long)((const int*)col)[i];
@@ -155,6 +159,7 @@ __global__ void __launch_bounds__(256) k_s_topk_collect(const long long* __restr
                                                         const long long* __restrict__ base,
                                                         const long long* __restrict__ cap, long long* __restrict__ rows,
                                                         unsigned long long* __restrict__ cnt, unsigned* derr) {
+    grid_entry();
     __shared__ long long s_a[TK_MAXR], s_b[TK_MAXR];
     for (int r = threadIdx.x; r < nr; r += blockDim.x) { s_a[r] = rng[2 * r]; s_b[r] = rng[2 * r + 1]; }
     __syncthreads();

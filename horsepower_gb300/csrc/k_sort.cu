@@ -51,6 +51,7 @@ int get_radix_pass_mode() { return g_radix_pass; }
 
 template <typename SRC>
 __global__ void k_key_bits(SRC src, long long n, unsigned long long* orv, unsigned long long* andv) {
+    grid_entry();
     unsigned long long o = 0, a = ~0ull;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long v = (unsigned long long)src(i);
@@ -68,6 +69,7 @@ __global__ void k_key_bits(SRC src, long long n, unsigned long long* orv, unsign
 template <typename K>
 __global__ void k_radix_hist(const K* __restrict__ k, long long n, int lo, int bits, int npass,
                              unsigned long long* __restrict__ hist) {
+    grid_entry();
     __shared__ unsigned sh[8][256];
     for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&sh[0][0])[i] = 0;
     __syncthreads();
@@ -83,6 +85,7 @@ __global__ void k_radix_hist(const K* __restrict__ k, long long n, int lo, int b
 
 // exclusive scan of each pass's 256 bins (one block per pass)
 __global__ void k_bucket_base(const unsigned long long* __restrict__ hist, unsigned long long* __restrict__ base) {
+    grid_entry();
     __shared__ unsigned long long s[256];
     const int p = blockIdx.x, d = threadIdx.x;
     s[d] = hist[p * 256 + d];
@@ -113,6 +116,7 @@ __global__ void __launch_bounds__(RS_THREADS, (sizeof(K) == 4 ? 4 : 3)) k_oneswe
                                                          long long* __restrict__ vout64, int reverse, long long n,
                                                          int shift, int bits, const unsigned long long* __restrict__ bucket,
                                                          unsigned long long* status, unsigned* ticket, unsigned* derr) {
+    grid_entry();
     // dynamic shared memory: the tile's keys and row ids in digit order
     extern __shared__ __align__(16) unsigned char os_smem[];
     K* skey = reinterpret_cast<K*>(os_smem);
@@ -198,6 +202,7 @@ __global__ void __launch_bounds__(RS_THREADS, (sizeof(K) == 4 ? 4 : 3)) k_oneswe
 // keeps only the bits set in `mask`, packed to the bottom in order
 template <typename SRC, typename K>
 __global__ void k_squeeze(SRC src, long long n, unsigned long long mask, K* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned long long v = (unsigned long long)src(i), r = 0, m = mask;
         int o = 0;
@@ -211,6 +216,7 @@ __global__ void k_squeeze(SRC src, long long n, unsigned long long mask, K* __re
 }
 
 __global__ void k_iota(unsigned* v, long long n) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         v[i] = (unsigned)i;
 }
@@ -242,6 +248,7 @@ struct RadixOut {
 
 template <typename SRC, typename K>
 __global__ void k_copy_keys(SRC src, long long n, K* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = (K)src(i);
 }
@@ -567,6 +574,7 @@ __device__ __forceinline__ double fval(const void* p, int typ, long long i) {
 __device__ __forceinline__ unsigned long long spec_key(const KeySpec& s, long long i);
 template <typename K>
 __global__ void k_make_keys(KeySpec s, long long n, K* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = (K)spec_key(s, i);
 }
@@ -576,6 +584,7 @@ __global__ void k_make_keys(KeySpec s, long long n, K* __restrict__ out) {
 template <typename K>
 __global__ void k_make_keys_hist(KeySpec s, long long n, K* __restrict__ out, int lo, int bits, int npass,
                                  unsigned long long* __restrict__ hist) {
+    grid_entry();
     __shared__ unsigned sh[8][256];
     for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&sh[0][0])[i] = 0;
     __syncthreads();
@@ -626,6 +635,7 @@ __device__ __forceinline__ unsigned long long spec_key(const KeySpec& s, long lo
 // mm[0] = the smallest order-preserving unsigned image of a value, mm[1] =
 // the smallest complement of one (both start at all ones)
 __global__ void k_minmax_i64(const void* p, int typ, long long n, unsigned long long* mm) {
+    grid_entry();
     unsigned long long a = ~0ull, b = ~0ull;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long u = (unsigned long long)ival(p, typ, i) ^ (1ull << 63);
@@ -642,6 +652,7 @@ __global__ void k_minmax_i64(const void* p, int typ, long long n, unsigned long 
 
 // ------------------------------------------------------------- permutations
 __global__ void k_widen(const unsigned* __restrict__ v, long long n, long long* __restrict__ out, int reverse) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = reverse ? (long long)v[n - 1 - i] : (long long)v[i];
 }
@@ -649,6 +660,7 @@ __global__ void k_widen(const unsigned* __restrict__ v, long long n, long long* 
 // group boundary flags: row i starts a group when its key differs from row i-1
 template <typename K>
 __global__ void k_bound_keys(const K* __restrict__ k, long long n, uint8_t* __restrict__ f) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         f[i] = (i == 0) || (k[i] != k[i - 1]);
 }
@@ -660,6 +672,7 @@ struct ColSet {
     int ncol;
 };
 __global__ void k_bound_cols(ColSet c, const unsigned* __restrict__ perm, long long n, uint8_t* __restrict__ f) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         bool b = i == 0;
         if (!b) {
@@ -678,6 +691,7 @@ __global__ void k_bound_cols(ColSet c, const unsigned* __restrict__ perm, long l
 __global__ void k_group_nodes(const long long* __restrict__ starts, long long ng, long long n,
                               const long long* __restrict__ perm, long long* __restrict__ keys, V0* __restrict__ nodes,
                               unsigned long long host_base) {
+    grid_entry();
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
         long long s = starts[g], e = (g + 1 < ng) ? starts[g + 1] : n;
         long long first = perm[s];
@@ -699,6 +713,7 @@ __global__ void k_group_nodes(const long long* __restrict__ starts, long long ng
 // the reference's char sort of fewer than ten rows (h_libs.cc:388-390):
 // all-pairs exchange on a[rtn[i]] > a[rtn[j]], which leaves them descending
 __global__ void k_char_small(const int8_t* __restrict__ a, long long n, unsigned* __restrict__ perm) {
+    grid_entry();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     unsigned r[10];
     for (long long i = 0; i < n; i++) r[i] = (unsigned)i;
@@ -723,6 +738,7 @@ static unsigned gcap(long long n) {
 // with fully tied rows in their run's row order.
 __global__ void k_updown(const void* __restrict__ col, int typ, const unsigned* __restrict__ perm,
                          const unsigned* __restrict__ rid, long long n, unsigned* __restrict__ flags) {
+    grid_entry();
     for (long long i = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned r0 = rid ? rid[i - 1] : 0, r1 = rid ? rid[i] : 0;
         if (r0 != r1) continue;
@@ -735,6 +751,7 @@ __global__ void k_updown(const void* __restrict__ col, int typ, const unsigned* 
 // order is reversed: flip the direction bit of its rows
 __global__ void k_flip(const unsigned* __restrict__ perm, const unsigned* __restrict__ rid, long long n,
                        const unsigned* __restrict__ flags, uint8_t* __restrict__ dirbit) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned r = perm ? perm[i] : (unsigned)i;
         unsigned f = flags[rid ? rid[i] : 0];
@@ -744,18 +761,22 @@ __global__ void k_flip(const unsigned* __restrict__ perm, const unsigned* __rest
     }
 }
 __global__ void k_run_ids(const uint8_t* __restrict__ bflag, long long n, unsigned* __restrict__ one) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         one[i] = (i > 0 && bflag[i]) ? 1u : 0u;
 }
 __global__ void k_add_u32(unsigned* __restrict__ a, const unsigned* __restrict__ b, long long n) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         a[i] += b[i];
 }
 __global__ void k_u64_to_u32(const unsigned long long* __restrict__ a, long long n, unsigned* __restrict__ b) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         b[i] = (unsigned)a[i];
 }
 __global__ void k_tiebreak(const uint8_t* __restrict__ dirbit, long long n, unsigned* __restrict__ tb, unsigned* any) {
+    grid_entry();
     bool f = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         tb[i] = dirbit[i] ? (unsigned)(n - 1 - i) : (unsigned)i;
@@ -765,6 +786,7 @@ __global__ void k_tiebreak(const uint8_t* __restrict__ dirbit, long long n, unsi
 }
 template <typename K>
 __global__ void k_gather_keys(const K* __restrict__ k, const unsigned* __restrict__ perm, long long n, K* __restrict__ out) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = k[perm[i]];
 }
@@ -1167,6 +1189,7 @@ struct CodeInt {
 };
 template <typename Code>
 __global__ void k_trie_present(Code code_of, long long n, unsigned* __restrict__ bitmap) {
+    grid_entry();
     __shared__ unsigned sb[2048];
     for (int i = threadIdx.x; i < 2048; i += blockDim.x) sb[i] = 0;
     __syncthreads();
@@ -1190,6 +1213,7 @@ __device__ void load_rank(TrieRank& s, const TrieRank* g) {
 template <typename Code>
 __global__ void __launch_bounds__(256) k_trie_count(Code code_of, long long n, const TrieRank* __restrict__ rk, int G,
                                                     long long T, unsigned* __restrict__ counts) {
+    grid_entry();
     __shared__ TrieRank r;
     __shared__ unsigned cnt[TS_MAXG];
     load_rank(r, rk);
@@ -1211,6 +1235,7 @@ template <typename Code>
 __global__ void __launch_bounds__(256) k_trie_scatter(Code code_of, long long n, const TrieRank* __restrict__ rk, int G,
                                                       long long T, const unsigned long long* __restrict__ offs,
                                                       long long* __restrict__ perm) {
+    grid_entry();
     __shared__ TrieRank r;
     __shared__ unsigned wcnt[8][TS_MAXG];  // per warp: rows of each bucket, then the warp's base
     __shared__ unsigned long long toff[TS_MAXG];  // the tile's first position in each bucket
@@ -1252,6 +1277,7 @@ __global__ void __launch_bounds__(256) k_trie_scatter(Code code_of, long long n,
     }
 }
 __global__ void k_trie_starts(const unsigned long long* __restrict__ offs, int G, long long T, long long* __restrict__ starts) {
+    grid_entry();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < G) starts[b] = (long long)offs[(long long)b * T];
 }

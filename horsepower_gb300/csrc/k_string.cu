@@ -111,6 +111,7 @@ I sym_ranks(const long long** rank, L* n_out) {
 __global__ void k_cmp_sym(const long long* __restrict__ x, long long xs, bool xone, const long long* __restrict__ y,
                           long long ys, bool yone, long long n, const long long* __restrict__ rank, long long nsym, int op,
                           bool* __restrict__ z, unsigned* derr) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long a = xone ? xs : x[i], b = yone ? ys : y[i];
         bool r;
@@ -176,6 +177,7 @@ __device__ bool like_match(const LikeProg& p, const unsigned char* s, int n) {
 // one text per thread: texts given by (offset << 16 | length) spans into blob
 __global__ void k_like_spans(LikeProg prog, const char* __restrict__ blob, const unsigned long long* __restrict__ spans,
                              long long n, bool* __restrict__ z) {
+    grid_entry();
     __shared__ LikeProg p;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) p.cls[i] = prog.cls[i];
     if (threadIdx.x == 0) { p.star = prog.star; p.m = prog.m; }
@@ -190,6 +192,7 @@ __global__ void k_like_spans(LikeProg prog, const char* __restrict__ blob, const
 // symbol columns: the per-id result gathered by the column's ids
 __global__ void k_like_gather(const bool* __restrict__ by_id, long long nsym, const long long* __restrict__ ids, long long n,
                               bool* __restrict__ z, unsigned* derr) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long id = ids[i];
         if (id < 0 || id >= nsym) { flag_error(derr, DERR_INDEX); z[i] = false; }

@@ -44,6 +44,7 @@ __device__ __forceinline__ unsigned long long feistel(unsigned long long x, int 
 
 __global__ void k_synth_dim(unsigned long long seed, long long nd, int h, int* __restrict__ pk, int* __restrict__ date,
                             unsigned* derr) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nd; i += (long long)gridDim.x * blockDim.x) {
         unsigned long long x = (unsigned long long)i;
         int guard = 0;
@@ -59,6 +60,7 @@ __global__ void k_synth_dim(unsigned long long seed, long long nd, int h, int* _
 __global__ void k_synth_fact(unsigned long long seed, long long nf, long long nd, int* __restrict__ fk,
                              int8_t* __restrict__ flag, int8_t* __restrict__ status, double* __restrict__ qty,
                              double* __restrict__ price, double* __restrict__ disc) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nf; i += (long long)gridDim.x * blockDim.x) {
         fk[i] = (int)(rnd(seed, 2, i) % (unsigned long long)nd);
         flag[i] = (int8_t)(rnd(seed, 3, i) % 3ull);
@@ -75,6 +77,7 @@ __global__ void k_synth_fact(unsigned long long seed, long long nf, long long nd
 // in [0, 1); sec uniform over [0, 2^20].
 __global__ void k_synth_order(unsigned long long seed, long long n, const double* __restrict__ cdf, long long nr,
                               long long* __restrict__ key, int* __restrict__ sec) {
+    grid_entry();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double u = (double)(rnd(seed, 8, i) >> 11) * (1.0 / 9007199254740992.0);
         long long lo = 0, hi = nr;  // first index with cdf > u

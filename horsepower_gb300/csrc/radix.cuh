@@ -103,6 +103,7 @@ constexpr int RX_KV_ITEMS = 12, RX_KV_TILE = RX_THREADS * RX_KV_ITEMS;
 template <typename SRC, int BITS, int ITEMS>
 __global__ void __launch_bounds__(RX_THREADS) k_rx_count(SRC src, unsigned n, unsigned ntiles, int shift, int bits,
                                                          unsigned* __restrict__ counts, unsigned* __restrict__ tot) {
+    grid_entry();
     using K = typename SRC::key_t;
     constexpr int D = 1 << BITS, TILE = RX_THREADS * ITEMS;
     __shared__ unsigned wh[RX_WARPS][D];
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(RX_THREADS) k_rx_count(SRC src, unsigned n, un
 // rows of all lower digits (positions fit 32 bits: row ids do)
 __global__ void __launch_bounds__(256) k_rx_scan(unsigned* __restrict__ counts, unsigned C,
                                                  const unsigned* __restrict__ tot) {
+    grid_entry();
     __shared__ unsigned ws[8], wb[8];
     const unsigned lane = lane_id(), w = threadIdx.x >> 5, d = blockIdx.x;
     unsigned below = 0;
@@ -229,6 +231,7 @@ struct RxPass {
 };
 template <typename SRC, int BITS>
 __global__ void __launch_bounds__(RX_THREADS, RX_PER_SM) k_rx_scatter(SRC src, RxPass a) {
+    grid_entry();
     constexpr bool FIRST = !std::is_same<SRC, RxRec>::value;
     constexpr int D = 1 << BITS;
     extern __shared__ __align__(16) unsigned char rx_smem[];
@@ -335,6 +338,7 @@ __global__ void __launch_bounds__(RX_THREADS, RX_PER_SM) k_rx_scatter(SRC src, R
 // in two arrays.  mode: RX_KV, RX_KV64 or RX_V64.
 __global__ void __launch_bounds__(RX_THREADS, RX_PER_SM)
 k_rx_scatter_kv(const unsigned long long* __restrict__ kin, RxPass a) {
+    grid_entry();
     constexpr int D = 256, ITEMS = RX_KV_ITEMS, TILE = RX_KV_TILE;
     extern __shared__ __align__(16) unsigned char rx_smem[];
     unsigned long long* skey = reinterpret_cast<unsigned long long*>(rx_smem);

@@ -10,7 +10,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "hgpu_internal.cuh"
+#include "dev_common.cuh"
 
 // the symbol table (getSymbol / getSymbolStr): texts by id, ids by text
 static std::unordered_map<std::string, L>* g_sym_ids;
@@ -532,6 +532,7 @@ static unsigned char* g_rbmap = nullptr;   // its device address
 static unsigned g_rbused = 0;
 
 __global__ void k_read_back(RbList l, unsigned char* dst) {
+    grid_entry();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (w >= l.n) return;
     const unsigned char* src = l.src[w];
@@ -578,7 +579,7 @@ cudaError_t stream_sync() {
     const int n = g_rbl.n;
     if (n > 0) {
         ::hg::LaunchScope ls_("read_back");
-        k_read_back<<<1, 32 * RB_ITEMS, 0, g_stream>>>(g_rbl, g_rbmap);
+        launch_kernel(k_read_back, 1, 32 * RB_ITEMS, 0, g_rbl, g_rbmap);
     }
     g_rbl.n = 0;
     g_rbused = 0;
