@@ -23,6 +23,13 @@
 // partitioned at once: a flag pair per element (<= P, < P), one scan over
 // all ranges, the trade partners from the scan's ranks, and the next depth's
 // ranges.  Depths repeat until no range of two or more elements is left.
+//
+// The same step runs at three scales: ranges above QS_BLOCK elements together
+// in global memory (four launches a depth), ranges of up to QS_BLOCK in one
+// CTA's shared memory and ranges of up to 32 in one warp's registers, both to
+// their end without another launch.  (With every depth in global memory 114K
+// random rows took 48 depths of five launches: what bounded the call was
+// launch latency.)
 // A NaN key makes the reference's comparator non-reflexive and its scans
 // leave the range (undefined behaviour), so NaN keys return E_NOT_IMPL.
 #include "dev_common.cuh"
@@ -35,13 +42,48 @@ I compact_rows(const uint8_t* mask, long long n, long long* out, long long* coun
 
 constexpr unsigned QS_DONE = 0xffffffffu;
 constexpr int QS_THREADS = 256, QS_ITEMS = 8, QS_TILE = QS_THREADS * QS_ITEMS;
-constexpr int QS_SPLIT_LEVELS = 8;  // recursion depths issued between two reads of the active count
-// A recursion deeper than max(8192, 2^36 / n) levels (first-element pivots
-// on nearly ordered keys, where the reference's own sort is quadratic) is
-// refused, which bounds a call to about 2^36 element visits.
+constexpr int QS_WARP = 32;         // largest range one warp sorts
+constexpr int QS_BLOCK = 4096;      // largest range one CTA sorts in shared memory
+constexpr int QB_THREADS = 1024, QB_ITEMS = QS_BLOCK / QB_THREADS, QB_WARPS = QB_THREADS / 32;
+// A range handed to a CTA or a warp: positions [lo, hi), the recursion depth
+// at which it was made, and whether its elements lie in the local buffers
+// (made by a partition) or in the sort's own (a range it started with).
+struct QsRange {
+    unsigned lo, hi, depth, local;
+};
+// counters of one sort, in device memory
+struct QsCounters {
+    unsigned nblock, nwarp;  // ranges listed for CTAs and warps
+    unsigned nbig;           // ranges the sort starts with that neither takes
+    unsigned depth;          // recursion depth reached by the listed ranges
+    unsigned nrev, nan;      // segments to reverse; a NaN key was seen
+};
+struct QsLists {
+    QsRange* block;
+    QsRange* warp;
+    QsCounters* cnt;
+};
+__device__ __forceinline__ void qs_list(const QsLists& q, unsigned lo, unsigned hi, unsigned depth, unsigned local) {
+    const unsigned m = hi - lo;
+    if (m > QS_WARP) q.block[atomicAdd(&q.cnt->nblock, 1u)] = QsRange{lo, hi, depth, local};
+    else q.warp[atomicAdd(&q.cnt->nwarp, 1u)] = QsRange{lo, hi, depth, local};
+}
+// A recursion deeper than max(8192, 2^36 / n) levels, rounded up to a multiple
+// of 8 (first-element pivots on nearly ordered keys, where the reference's own
+// sort is quadratic) is refused, which bounds a call to about 2^36 element
+// visits.
 static long long qs_max_levels(long long n) {
     const long long m = (1LL << 36) / (n > 0 ? n : 1);
-    return m > 8192 ? m : 8192;
+    return ((m > 8192 ? m : 8192) + 7) / 8 * 8;
+}
+// Depths issued before the host reads the active count: a random range of n
+// rows needs about 2 log2(n / QS_BLOCK) of them to come down to QS_BLOCK at
+// its worst place; after these the count is read every QS_ROUND depths.
+constexpr int QS_ROUND = 4, QS_MAX_ROUND = 64;
+static int qs_first_round(long long n) {
+    int d = 2;
+    for (long long m = n; m > QS_BLOCK && d < QS_MAX_ROUND; m >>= 1) d += 2;
+    return d;
 }
 
 __device__ __forceinline__ long long qs_ival(const void* p, int typ, long long i) {
@@ -116,34 +158,13 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_count(const unsigned* __restr
     }
 }
 
-// exclusive scan of the nt tile sums in place (one block); tile_sum[nt] = total
-__global__ void __launch_bounds__(1024) k_qs_scan_sums(unsigned long long* __restrict__ ts, long long nt) {
-    grid_entry();
-    __shared__ unsigned long long wsum[32];
-    const long long per = (nt + 1023) / 1024;
-    const long long a = (long long)threadIdx.x * per, b = a + per < nt ? a + per : nt;
-    unsigned long long s = 0;
-    for (long long i = a; i < b; i++) s += ts[i];
-    const unsigned long long incl = warp_incl_scan64(s);
-    if (lane_id() == 31) wsum[threadIdx.x >> 5] = incl;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const unsigned long long w = wsum[threadIdx.x];
-        const unsigned long long wi = warp_incl_scan64(w);
-        wsum[threadIdx.x] = wi - w;
-    }
-    __syncthreads();
-    unsigned long long off = wsum[threadIdx.x >> 5] + incl - s;
-    for (long long i = a; i < b; i++) { const unsigned long long v = ts[i]; ts[i] = off; off += v; }
-    if (threadIdx.x == 1023) ts[nt] = off;
-}
-
-// S[p] = exclusive prefix of the flag pairs; S[n] = total
+// S[p] = exclusive prefix of the flag pairs; S[n] = total.  Each block sums
+// the tiles before its own.
 __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __restrict__ lo, const unsigned long long* __restrict__ K,
                                                           long long n, const unsigned long long* __restrict__ tile_sum,
-                                                          long long nt, unsigned long long* __restrict__ S) {
+                                                          unsigned long long* __restrict__ S) {
     grid_entry();
-    __shared__ unsigned long long ws[QS_THREADS / 32];
+    __shared__ unsigned long long ws[QS_THREADS / 32], wb[QS_THREADS / 32];
     const long long base = (long long)blockIdx.x * QS_TILE + (long long)threadIdx.x * QS_ITEMS;
     unsigned long long v[QS_ITEMS], s = 0;
 #pragma unroll
@@ -151,17 +172,22 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __rest
         v[k] = base + k < n ? qs_flag(lo, K, base + k) : 0;
         s += v[k];
     }
+    unsigned long long before = 0;
+    for (long long t = threadIdx.x; t < blockIdx.x; t += QS_THREADS) before += tile_sum[t];
+    before = warp_sum(before);
     const unsigned long long incl = warp_incl_scan64(s);
     if (lane_id() == 31) ws[threadIdx.x >> 5] = incl;
+    if (lane_id() == 0) wb[threadIdx.x >> 5] = before;
     __syncthreads();
-    unsigned long long off = tile_sum[blockIdx.x] + incl - s;
-    for (unsigned w = 0; w < (threadIdx.x >> 5); w++) off += ws[w];
+    unsigned long long off = incl - s;
+#pragma unroll
+    for (unsigned w = 0; w < QS_THREADS / 32; w++) off += wb[w] + (w < (threadIdx.x >> 5) ? ws[w] : 0ull);
 #pragma unroll
     for (int k = 0; k < QS_ITEMS; k++) {
         if (base + k < n) S[base + k] = off;
         off += v[k];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) S[n] = tile_sum[nt];
+    if (base < n && base + QS_ITEMS >= n) S[n] = off;  // the thread of the last element
 }
 
 __device__ __forceinline__ unsigned qs_le(unsigned long long s) { return (unsigned)s; }
@@ -193,13 +219,15 @@ __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __rest
 }
 
 // Moves every element of the partitioned ranges to its place, records the
-// next depth's range of every element (or its final place) and counts the
-// elements still in a range of two or more.
+// next depth's range of every element (or its final place; ranges of up to
+// QS_BLOCK elements go to the local buffers and lists) and counts the elements
+// still in a larger range.
 __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, const unsigned long long* __restrict__ K,
                           const unsigned* __restrict__ P, const unsigned long long* __restrict__ S, long long n,
                           const unsigned* __restrict__ Lpos, const unsigned* __restrict__ Rpos,
                           unsigned long long* __restrict__ K2, unsigned* __restrict__ P2, unsigned* __restrict__ fin,
-                          unsigned* __restrict__ active, unsigned* derr) {
+                          unsigned* __restrict__ active, unsigned depth, unsigned long long* __restrict__ KL,
+                          unsigned* __restrict__ PL, QsLists lists, unsigned* derr) {
     grid_entry();
     unsigned still = 0;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
@@ -241,6 +269,11 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
         if (p == j || nh - nl < 2) {
             fin[p] = P[q];
             lo[p] = QS_DONE;
+        } else if (nh - nl <= QS_BLOCK) {
+            PL[p] = P[q];
+            KL[p] = K[q];
+            lo[p] = QS_DONE;
+            if (p == nl) qs_list(lists, (unsigned)nl, (unsigned)nh, depth + 1, 1);
         } else {
             P2[p] = P[q];
             K2[p] = K[q];
@@ -251,6 +284,225 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
     }
     still = warp_sum(still);
     if (lane_id() == 0 && still) atomicAdd(active, still);
+}
+
+// ---- one warp's range: m <= 32 elements, element i in lane i (key k, row p).
+// Partitions it to its end; p is then the row of position `lane`.  sl/sr: the
+// warp's 32 slots for each side of the trades.  Returns the depths it took.
+__device__ __forceinline__ unsigned qs_warp_range(unsigned long long k, unsigned& p, unsigned m, volatile uint8_t* sl,
+                                                  volatile uint8_t* sr) {
+    const unsigned lane = lane_id();
+    unsigned lo = lane < m ? 0u : lane, hi = m, depths = 0;
+    bool act = lane < m && m > 1;
+    while (__any_sync(0xffffffffu, act)) {
+        depths++;
+        const unsigned long long kp = __shfl_sync(0xffffffffu, k, lo);
+        const int c = act ? qs_cmp(k, kp) : 0;
+        const unsigned le = __ballot_sync(0xffffffffu, act && lane != lo && c <= 0);
+        const unsigned lt = __ballot_sync(0xffffffffu, act && lane != lo && c < 0);
+        const unsigned seg = (hi >= 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u);  // the range's lanes
+        const unsigned cle = __popc(le & seg), j = act ? lo + cle : lane;
+        const bool same = cle == hi - lo - 1 && !(lt & seg);
+        auto below = [&](unsigned x) { return (unsigned)__popc(le & seg & ((1u << x) - 1u)); };  // le elements before x
+        const bool up = act && !same && lane != lo && lane <= j && c > 0, down = act && !same && lane > j && c <= 0;
+        if (up) sl[lo + (lane - lo - 1) - below(lane)] = (uint8_t)lane;
+        if (down) sr[lo + cle - below(lane) - 1] = (uint8_t)lane;
+        const unsigned long long kj = __shfl_sync(0xffffffffu, k, j);
+        __syncwarp();
+        unsigned q = lane;
+        if (act && !same) {
+            if (lane == lo) q = (j > lo && qs_cmp(kj, kp) > 0) ? sr[lo + (j - lo - 1) - below(j)] : j;
+            else if (lane == j) q = lo;
+            else if (up) q = sr[lo + (lane - lo - 1) - below(lane)];
+            else if (down) q = sl[lo + cle - below(lane) - 1];
+        }
+        __syncwarp();
+        k = __shfl_sync(0xffffffffu, k, q);
+        p = __shfl_sync(0xffffffffu, p, q);
+        if (act) {
+            if (lane < j) hi = j;
+            else if (lane > j) lo = j + 1;
+            if (same || lane == j || hi - lo < 2) act = false;
+        }
+    }
+    return depths;
+}
+
+// the listed ranges of 2 to 32 elements, one warp each
+__global__ void __launch_bounds__(256) k_qs_warps(QsLists lists, const unsigned long long* __restrict__ K0,
+                                                  const unsigned* __restrict__ P0,
+                                                  const unsigned long long* __restrict__ KL,
+                                                  const unsigned* __restrict__ PL, unsigned* __restrict__ fin) {
+    grid_entry();
+    __shared__ uint8_t slots[8][64];
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5, n = lists.cnt->nwarp;
+    unsigned deep = 0;
+    for (unsigned r = blockIdx.x * 8 + w; r < n; r += gridDim.x * 8) {
+        const QsRange g = lists.warp[r];
+        const unsigned m = g.hi - g.lo;
+        unsigned long long k = 0;
+        unsigned p = 0;
+        if (lane < m) {
+            k = (g.local ? KL : K0)[g.lo + lane];
+            p = (g.local ? PL : P0)[g.lo + lane];
+        }
+        const unsigned d = g.depth + qs_warp_range(k, p, m, slots[w], slots[w] + 32);
+        deep = d > deep ? d : deep;
+        if (lane < m) fin[g.lo + lane] = p;
+    }
+    if (lane == 0 && deep) atomicMax(&lists.cnt->depth, deep);
+}
+
+// The listed ranges of 33 to QS_BLOCK elements, one CTA each, in shared memory:
+// position w * 128 + 32 k + lane of the range belongs to item k of the thread,
+// so the prefixes are ballots.  Ranges that reach 32 elements wait in a list
+// for the CTA's warps.  What bounds a depth is its five barriers.
+struct QsBlockSmem {
+    unsigned long long K[QS_BLOCK];
+    unsigned P[QS_BLOCK];
+    unsigned S[QS_BLOCK + 1];         // exclusive prefix: (<= P) in the low half, (< P) in the high half
+    unsigned short L[QS_BLOCK], R[QS_BLOCK];
+    unsigned small[QS_BLOCK / 2];     // lo | (size - 1) << 12 | depth << 17
+    unsigned wt[QB_WARPS];
+    uint8_t slots[QB_WARPS][64];
+    unsigned nsmall, depth;
+};
+static_assert(QS_BLOCK <= 4096 && QS_WARP <= 32, "packing of QsBlockSmem::small");
+__global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, const unsigned long long* __restrict__ K0,
+                                                             const unsigned* __restrict__ P0,
+                                                             const unsigned long long* __restrict__ KL,
+                                                             const unsigned* __restrict__ PL, unsigned* __restrict__ fin,
+                                                             unsigned* derr) {
+    grid_entry();
+    extern __shared__ __align__(16) unsigned char qb_smem[];
+    QsBlockSmem& sm = *reinterpret_cast<QsBlockSmem*>(qb_smem);
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5, p0 = w * (32 * QB_ITEMS) + lane;
+    auto le = [](unsigned s) { return s & 0xffffu; };
+    auto lt = [](unsigned s) { return s >> 16; };
+    const unsigned n = lists.cnt->nblock;
+    for (unsigned r = blockIdx.x; r < n; r += gridDim.x) {
+        const QsRange g = lists.block[r];
+        const unsigned m = g.hi - g.lo;
+        if (threadIdx.x == 0) sm.nsmall = sm.depth = 0;
+        unsigned long long key[QB_ITEMS];
+        unsigned row[QB_ITEMS], lo[QB_ITEMS], hi[QB_ITEMS], act = 0;
+#pragma unroll
+        for (int k = 0; k < QB_ITEMS; k++) {
+            const unsigned p = p0 + 32 * k;
+            key[k] = 0;
+            row[k] = lo[k] = hi[k] = 0;
+            if (p < m) {
+                key[k] = (g.local ? KL : K0)[g.lo + p];
+                row[k] = (g.local ? PL : P0)[g.lo + p];
+                hi[k] = m;
+                act |= 1u << k;
+                sm.K[p] = key[k];
+                sm.P[p] = row[k];
+            }
+        }
+        __syncthreads();
+        unsigned depths = 0;
+        for (; __syncthreads_or((int)act); depths++) {
+            unsigned pre[QB_ITEMS], run = 0;
+            int c[QB_ITEMS];
+#pragma unroll
+            for (int k = 0; k < QB_ITEMS; k++) {
+                const unsigned p = p0 + 32 * k;
+                const bool a = (act >> k) & 1u;
+                c[k] = a && p != lo[k] ? qs_cmp(key[k], sm.K[lo[k]]) : 2;  // 2: the pivot, or finished
+                const unsigned ble = __ballot_sync(0xffffffffu, c[k] <= 0), blt = __ballot_sync(0xffffffffu, c[k] < 0);
+                pre[k] = run + ((unsigned)__popc(ble & lanemask_lt()) | ((unsigned)__popc(blt & lanemask_lt()) << 16));
+                run += (unsigned)__popc(ble) | ((unsigned)__popc(blt) << 16);
+            }
+            if (lane == 0) sm.wt[w] = run;
+            __syncthreads();
+            unsigned base = 0, all = 0;
+#pragma unroll
+            for (int q = 0; q < QB_WARPS; q++) {
+                const unsigned t = sm.wt[q];
+                if (q < (int)w) base += t;
+                all += t;
+            }
+#pragma unroll
+            for (int k = 0; k < QB_ITEMS; k++)
+                if (p0 + 32 * k < m) sm.S[p0 + 32 * k] = base + pre[k];
+            if (threadIdx.x == 0) sm.S[m] = all;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < QB_ITEMS; k++) {
+                if (!((act >> k) & 1u) || c[k] == 2) continue;
+                const unsigned p = p0 + 32 * k, l = lo[k];
+                const unsigned le_lo = le(sm.S[l]), le_hi = le(sm.S[hi[k]]), le_p = le(base + pre[k]);
+                const unsigned j = l + (le_hi - le_lo);
+                if (p <= j && c[k] > 0) sm.L[l + (p - l - 1) - (le_p - le_lo)] = (unsigned short)p;
+                else if (p > j && c[k] <= 0) sm.R[l + (le_hi - le_p) - 1] = (unsigned short)p;
+            }
+            __syncthreads();
+            unsigned long long nkey[QB_ITEMS];
+            unsigned nrow[QB_ITEMS];
+#pragma unroll
+            for (int k = 0; k < QB_ITEMS; k++) {
+                nkey[k] = key[k];
+                nrow[k] = row[k];
+                if (!((act >> k) & 1u)) continue;
+                const unsigned p = p0 + 32 * k, l = lo[k], h = hi[k];
+                const unsigned sl = sm.S[l], sh = sm.S[h], cle = le(sh) - le(sl), j = l + cle;
+                if (cle == h - l - 1 && lt(sh) == lt(sl)) {  // leftSame: every element equals the pivot
+                    lo[k] = hi[k] = 0;
+                    continue;
+                }
+                unsigned q = p;
+                if (p == l) {
+                    q = j;
+                    if (j > l && qs_cmp(sm.K[j], key[k]) > 0) q = sm.R[l + (j - l - 1) - (le(sm.S[j]) - le(sl))];
+                } else if (p == j) {
+                    q = l;
+                } else if (p < j && c[k] > 0) {
+                    q = sm.R[l + (p - l - 1) - (le(base + pre[k]) - le(sl))];
+                } else if (p > j && c[k] <= 0) {
+                    q = sm.L[l + (le(sh) - le(base + pre[k])) - 1];
+                }
+                if (q < l || q >= h) { flag_error(derr, DERR_INDEX); q = p; }
+                nkey[k] = sm.K[q];
+                nrow[k] = sm.P[q];
+                if (p < j) hi[k] = j;
+                else { lo[k] = p == j ? j : j + 1; if (p == j) hi[k] = j; }  // an empty range for the pivot's place
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < QB_ITEMS; k++) {
+                if (!((act >> k) & 1u)) continue;
+                const unsigned p = p0 + 32 * k, sz = hi[k] - lo[k];
+                key[k] = nkey[k];
+                row[k] = nrow[k];
+                sm.K[p] = key[k];
+                sm.P[p] = row[k];
+                if (sz > QS_WARP) continue;
+                act &= ~(1u << k);
+                if (sz < 2) fin[g.lo + p] = row[k];
+                else if (p == lo[k]) sm.small[atomicAdd(&sm.nsmall, 1u)] = p | ((sz - 1) << 12) | ((depths + 1) << 17);
+            }
+        }
+        // every range of 2 to 32 elements left in the CTA
+        unsigned deep = depths;
+        const unsigned ns = sm.nsmall;
+        for (unsigned q = w; q < ns; q += QB_WARPS) {
+            const unsigned v = sm.small[q], a = v & 4095u, mm = ((v >> 12) & 31u) + 1;
+            unsigned long long k = 0;
+            unsigned p = 0;
+            if (lane < mm) {
+                k = sm.K[a + lane];
+                p = sm.P[a + lane];
+            }
+            const unsigned d = (v >> 17) + qs_warp_range(k, p, mm, sm.slots[w], sm.slots[w] + 32);
+            deep = d > deep ? d : deep;
+            if (lane < mm) fin[g.lo + a + lane] = p;
+        }
+        if (lane == 0) atomicMax(&sm.depth, deep);
+        __syncthreads();
+        if (threadIdx.x == 0) atomicMax(&lists.cnt->depth, g.depth + sm.depth);
+        __syncthreads();
+    }
 }
 
 // ---- ranges (segments) of a list sort
@@ -281,15 +533,49 @@ __global__ void k_qs_updown(const unsigned long long* __restrict__ img, const un
 enum : uint8_t { QS_SORT = 0, QS_KEEP = 1, QS_REVERSE = 2 };
 // mode of each segment: an ascending-ordered segment (rises, never falls)
 // is kept; for a descending key (images complemented) a segment whose values
-// ascend (images fall, never rise) is reversed; every other one is sorted
-__global__ void k_qs_mode(const uint8_t* __restrict__ up, const uint8_t* __restrict__ down, long long ns, int desc,
-                          uint8_t* __restrict__ mode, unsigned* __restrict__ nrev) {
+// ascend (images fall, never rise) is reversed; every other one is sorted, and
+// listed when it holds min_len or more elements (those above QS_BLOCK are only
+// counted)
+__global__ void k_qs_mode(const uint8_t* __restrict__ up, const uint8_t* __restrict__ down,
+                          const long long* __restrict__ starts, long long ns, long long n, int desc, int min_len,
+                          uint8_t* __restrict__ mode, QsLists lists) {
     grid_entry();
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < ns; s += (long long)gridDim.x * blockDim.x) {
         uint8_t m = QS_SORT;
         if (!desc && up[s] && !down[s]) m = QS_KEEP;
-        if (desc && down[s] && !up[s]) { m = QS_REVERSE; atomicAdd(nrev, 1u); }
+        if (desc && down[s] && !up[s]) { m = QS_REVERSE; atomicAdd(&lists.cnt->nrev, 1u); }
         mode[s] = m;
+        const long long a = starts[s], b = s + 1 < ns ? starts[s + 1] : n;
+        if (m == QS_SORT && b - a >= min_len) {
+            if (b - a > QS_BLOCK) atomicAdd(&lists.cnt->nbig, 1u);
+            else qs_list(lists, (unsigned)a, (unsigned)b, 0, 0);
+        }
+    }
+}
+// the only range of a vector sort (one thread)
+__global__ void k_qs_whole(long long n, QsLists lists) {
+    grid_entry();
+    if (n > QS_BLOCK) lists.cnt->nbig = 1;
+    else if (n >= 2) qs_list(lists, 0, (unsigned)n, 0, 0);
+}
+// the listed segments of 2 to 32 elements in stable order, one warp each: an
+// element's place is the number of smaller images and of equal ones before it
+__global__ void __launch_bounds__(256) k_qs_stable_small(QsLists lists, const unsigned long long* __restrict__ img,
+                                                         unsigned* __restrict__ perm) {
+    grid_entry();
+    const unsigned lane = lane_id(), n = lists.cnt->nwarp;
+    for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
+        const QsRange g = lists.warp[r];
+        const unsigned m = g.hi - g.lo;
+        const unsigned long long k = lane < m ? img[g.lo + lane] : ~0ull;
+        const unsigned row = lane < m ? perm[g.lo + lane] : 0u;
+        unsigned at = 0;
+        for (unsigned j = 0; j < m; j++) {
+            const unsigned long long kj = __shfl_sync(0xffffffffu, k, j);
+            at += kj < k || (kj == k && j < lane);
+        }
+        __syncwarp();
+        if (lane < m) perm[g.lo + at] = row;
     }
 }
 __global__ void k_qs_reverse(const unsigned* __restrict__ perm, const unsigned* __restrict__ seg,
@@ -306,8 +592,9 @@ __global__ void k_qs_reverse(const unsigned* __restrict__ perm, const unsigned* 
         out[p] = perm[q];
     }
 }
-// range of each position for the quicksort: its segment when that is sorted
-// and holds two or more elements; finished positions keep their row
+// range of each position for the quicksort's depths in global memory (with
+// `lo`): its segment when that is sorted and larger than QS_BLOCK.  Positions
+// of segments that are not sorted keep their row.
 __global__ void k_qs_ranges(const unsigned* __restrict__ seg, const long long* __restrict__ starts, long long ns, long long n,
                             const uint8_t* __restrict__ mode, const unsigned* __restrict__ perm,
                             unsigned* __restrict__ lo, unsigned* __restrict__ hi, unsigned* __restrict__ fin) {
@@ -315,11 +602,10 @@ __global__ void k_qs_ranges(const unsigned* __restrict__ seg, const long long* _
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned s = seg ? seg[p] : 0;
         const long long a = seg ? starts[s] : 0, b = seg ? (s + 1 < ns ? starts[s + 1] : n) : n;
-        if ((mode && mode[s] != QS_SORT) || b - a < 2) {
-            lo[p] = QS_DONE;
-            fin[p] = perm[p];
-        } else {
-            lo[p] = (unsigned)a;
+        const bool sorted = !(mode && mode[s] != QS_SORT) && b - a >= 2;
+        if (!sorted) fin[p] = perm[p];
+        if (lo) {
+            lo[p] = sorted && b - a > QS_BLOCK ? (unsigned)a : QS_DONE;
             hi[p] = (unsigned)b;
         }
     }
@@ -378,46 +664,102 @@ static unsigned qs_grid(long long n) {
     return g > (unsigned)g_sms * 16 ? (unsigned)g_sms * 16 : g;
 }
 
-// The quicksort of every range at once.  perm/img: the elements in their
-// current order (consumed); lo/hi: each position's range (QS_DONE: not in
-// one, fin already holds its row).  On return fin holds every position's row.
-static I qs_run(long long n, unsigned* perm, unsigned long long* img, unsigned* lo, unsigned* hi, unsigned* fin) {
-    const long long nt = (n + QS_TILE - 1) / QS_TILE;
-    unsigned* P2 = (unsigned*)salloc((size_t)n * 4);
-    unsigned long long* K2 = (unsigned long long*)salloc((size_t)n * 8);
-    unsigned long long* S = (unsigned long long*)salloc((size_t)(n + 1) * 8);
-    unsigned long long* ts = (unsigned long long*)salloc((size_t)(nt + 1) * 8);
-    unsigned* Lpos = (unsigned*)salloc((size_t)n * 4);
-    unsigned* Rpos = (unsigned*)salloc((size_t)n * 4);
-    unsigned* act = (unsigned*)salloc(QS_SPLIT_LEVELS * 4);
-    if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos || !act) return E_DEVICE_OOM;
-    unsigned* Pc = perm;
-    unsigned long long* Kc = img;
+static I qs_too_deep(long long levels) {
+    return set_error(E_NOT_IMPL, "the reference's quicksort recursion is deeper than %lld levels here "
+                     "(first-element pivots on nearly ordered keys)", levels);
+}
+
+static I qs_lists_alloc(long long n, QsLists* q) {
+    q->block = (QsRange*)salloc((size_t)(n / QS_WARP + 1) * sizeof(QsRange));
+    q->warp = (QsRange*)salloc((size_t)(n / 2 + 1) * sizeof(QsRange));
+    q->cnt = (QsCounters*)salloc(sizeof(QsCounters));
+    return q->block && q->warp && q->cnt ? 0 : E_DEVICE_OOM;
+}
+
+// NaN keys, from counters already read back
+static I qs_nan_check(const QsCounters& h) {
+    if (h.nan) return set_error(E_NOT_IMPL, "NaN sort key: the reference's quicksort compares NaN as greater than "
+                                "itself and scans outside the range");
+    return 0;
+}
+
+// The quicksort of every sorted range at once.  perm/img: the elements in
+// their current order (consumed); lists/h: the ranges listed so far and their
+// counters as the host has read them; seg, starts, mode: the segments, for
+// those too large to list (null: the whole).  On return fin holds every
+// position's row.
+static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsigned* seg, const long long* starts,
+                long long ns, const uint8_t* mode, const QsLists& lists, QsCounters* h, unsigned* fin) {
     const unsigned g = qs_grid(n);
     const long long max_levels = qs_max_levels(n);
-    for (long long level = 0;; level += QS_SPLIT_LEVELS) {
-        if (level >= max_levels)
-            return set_error(E_NOT_IMPL, "the reference's quicksort recursion is deeper than %lld levels here "
-                             "(first-element pivots on nearly ordered keys)", max_levels);
-        HG_CU(cudaMemsetAsync(act, 0, QS_SPLIT_LEVELS * 4, g_stream));
-        for (int d = 0; d < QS_SPLIT_LEVELS; d++) {
-            HG_LAUNCH("qs_count", (unsigned)nt, QS_THREADS, 0, k_qs_count, lo, Kc, n, ts);
-            HG_LAUNCH("qs_scan_sums", 1, 1024, 0, k_qs_scan_sums, ts, nt);
-            HG_LAUNCH("qs_prefix", (unsigned)nt, QS_THREADS, 0, k_qs_prefix, lo, Kc, n, ts, nt, S);
-            HG_LAUNCH("qs_pos", g, 256, 0, k_qs_pos, lo, hi, Kc, S, n, Lpos, Rpos, g_derr);
-            unsigned* Pn = Pc == perm ? P2 : perm;
-            unsigned long long* Kn = Kc == img ? K2 : img;
-            HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, Lpos, Rpos, Kn, Pn, fin, act + d, g_derr);
-            Pc = Pn;
-            Kc = Kn;
-        }
-        HG_CHECK(last_launch_error());
-        unsigned h = 0;
-        HG_CHECK(rb_queue(&h, act + QS_SPLIT_LEVELS - 1, 4));
-        HG_CU(stream_sync());
-        if (h == 0) break;
+    unsigned long long* KL = nullptr;  // the elements of listed ranges that a partition has made
+    unsigned* PL = nullptr;
+    unsigned *lo = nullptr, *hi = nullptr;
+    if (h->nbig) {
+        lo = (unsigned*)salloc((size_t)n * 4);
+        hi = (unsigned*)salloc((size_t)n * 4);
+        if (!lo || !hi) return E_DEVICE_OOM;
     }
-    return check_device_errors();
+    HG_LAUNCH("qs_ranges", g, 256, 0, k_qs_ranges, seg, starts, ns, n, mode, perm, lo, hi, fin);
+    if (h->nbig) {
+        const long long nt = (n + QS_TILE - 1) / QS_TILE;
+        unsigned* P2 = (unsigned*)salloc((size_t)n * 4);
+        unsigned long long* K2 = (unsigned long long*)salloc((size_t)n * 8);
+        unsigned long long* S = (unsigned long long*)salloc((size_t)(n + 1) * 8);
+        unsigned long long* ts = (unsigned long long*)salloc((size_t)nt * 8);
+        unsigned* Lpos = (unsigned*)salloc((size_t)n * 4);
+        unsigned* Rpos = (unsigned*)salloc((size_t)n * 4);
+        unsigned* act = (unsigned*)salloc(QS_MAX_ROUND * 4);
+        KL = (unsigned long long*)salloc((size_t)n * 8);
+        PL = (unsigned*)salloc((size_t)n * 4);
+        if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos || !act || !KL || !PL) return E_DEVICE_OOM;
+        // the ranges listed at the start are read from perm/img, which the
+        // depths below reuse only at the positions of larger ranges
+        unsigned* Pc = perm;
+        unsigned long long* Kc = img;
+        int round = qs_first_round(n);
+        for (long long level = 0;; level += round, round = QS_ROUND) {
+            if (level >= max_levels) return qs_too_deep(max_levels);
+            if (level + round > max_levels) round = (int)(max_levels - level);
+            HG_CU(cudaMemsetAsync(act, 0, QS_MAX_ROUND * 4, g_stream));
+            for (int d = 0; d < round; d++) {
+                HG_LAUNCH("qs_count", (unsigned)nt, QS_THREADS, 0, k_qs_count, lo, Kc, n, ts);
+                HG_LAUNCH("qs_prefix", (unsigned)nt, QS_THREADS, 0, k_qs_prefix, lo, Kc, n, ts, S);
+                HG_LAUNCH("qs_pos", g, 256, 0, k_qs_pos, lo, hi, Kc, S, n, Lpos, Rpos, g_derr);
+                unsigned* Pn = Pc == perm ? P2 : perm;
+                unsigned long long* Kn = Kc == img ? K2 : img;
+                HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, Lpos, Rpos, Kn, Pn, fin, act + d,
+                          (unsigned)(level + d), KL, PL, lists, g_derr);
+                Pc = Pn;
+                Kc = Kn;
+            }
+            HG_CHECK(last_launch_error());
+            unsigned left = 0;
+            HG_CHECK(rb_queue(&left, act + round - 1, 4));
+            HG_CHECK(rb_queue(h, lists.cnt, sizeof *h));
+            HG_CU(stream_sync());
+            if (left == 0) break;
+        }
+    }
+    if (h->nblock) {
+        const int dsm = (int)sizeof(QsBlockSmem);
+        // the attribute belongs to the current device's context: set it on every call (a host-side write)
+        HG_CU(cudaFuncSetAttribute(k_qs_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
+        const unsigned cap = 2u * (unsigned)g_sms;
+        HG_LAUNCH("qs_blocks", h->nblock < cap ? h->nblock : cap, QB_THREADS, (size_t)dsm, k_qs_blocks, lists, img, perm, KL,
+                  PL, fin, g_derr);
+    }
+    if (h->nwarp) {
+        const unsigned cap = 16u * (unsigned)g_sms, want = grid_for(h->nwarp, 8);
+        HG_LAUNCH("qs_warps", want < cap ? want : cap, 256, 0, k_qs_warps, lists, img, perm, KL, PL, fin);
+    }
+    HG_CHECK(last_launch_error());
+    // read again with the caller's next wait, for qs_depth_check
+    return rb_queue(h, lists.cnt, sizeof *h);
+}
+// after the wait that follows a qs_run: the depths of the listed ranges count
+static I qs_depth_check(long long n, const QsCounters& h) {
+    return (long long)h.depth > qs_max_levels(n) ? qs_too_deep(qs_max_levels(n)) : 0;
 }
 
 static I qs_image_of(const void* col, I typ, const unsigned* perm, long long n, bool desc, unsigned long long* img,
@@ -427,15 +769,6 @@ static I qs_image_of(const void* col, I typ, const unsigned* perm, long long n, 
     return last_launch_error();
 }
 
-static I qs_nan_check(unsigned* nanflag) {
-    unsigned h = 0;
-    HG_CHECK(rb_queue(&h, nanflag, 4));
-    HG_CU(stream_sync());
-    if (h) return set_error(E_NOT_IMPL, "NaN sort key: the reference's quicksort compares NaN as greater than "
-                            "itself and scans outside the range");
-    return 0;
-}
-
 // lib_order_by_vector (h_libs.cc:730-736) on a key its quicksort sorts:
 // rows 0..n-1 in order, then lib_quicksort_other over [0, n).
 I qs_sort_vector(const void* col, I typ, long long n, bool asc, const unsigned** perm_out) {
@@ -443,19 +776,22 @@ I qs_sort_vector(const void* col, I typ, long long n, bool asc, const unsigned**
     unsigned* perm = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4);
     unsigned* fin = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4);
     unsigned long long* img = (unsigned long long*)salloc((size_t)(n > 0 ? n : 1) * 8);
-    unsigned* lo = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4);
-    unsigned* hi = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4);
-    unsigned* nanflag = (unsigned*)salloc(16);
-    if (!perm || !fin || !img || !lo || !hi || !nanflag) return E_DEVICE_OOM;
+    QsLists lists;
+    if (!perm || !fin || !img) return E_DEVICE_OOM;
+    HG_CHECK(qs_lists_alloc(n, &lists));
     *perm_out = fin;
     if (n == 0) return 0;
-    HG_CU(cudaMemsetAsync(nanflag, 0, 4, g_stream));
+    HG_CU(cudaMemsetAsync(lists.cnt, 0, sizeof(QsCounters), g_stream));
     HG_LAUNCH("qs_iota", qs_grid(n), 256, 0, k_qs_iota, perm, n);
-    HG_CHECK(qs_image_of(col, typ, nullptr, n, !asc, img, nanflag));
-    HG_CHECK(qs_nan_check(nanflag));
-    HG_LAUNCH("qs_ranges", qs_grid(n), 256, 0, k_qs_ranges, (const unsigned*)nullptr, (const long long*)nullptr, 0LL, n,
-              (const uint8_t*)nullptr, perm, lo, hi, fin);
-    return qs_run(n, perm, img, lo, hi, fin);
+    HG_CHECK(qs_image_of(col, typ, nullptr, n, !asc, img, &lists.cnt->nan));
+    HG_LAUNCH("qs_whole", 1, 1, 0, k_qs_whole, n, lists);
+    QsCounters h;
+    HG_CHECK(rb_queue(&h, lists.cnt, sizeof h));
+    HG_CU(stream_sync());
+    HG_CHECK(qs_nan_check(h));
+    HG_CHECK(qs_run(n, perm, img, nullptr, nullptr, 0, nullptr, lists, &h, fin));
+    HG_CHECK(check_device_errors());
+    return qs_depth_check(n, h);
 }
 
 // lib_quicksort_list (h_libs.cc:637-697) over nc columns: for each column in
@@ -463,8 +799,11 @@ I qs_sort_vector(const void* col, I typ, long long n, bool asc, const unsigned**
 // lib_order_by_sorted (kept, or reversed for a descending column whose values
 // ascend) and otherwise sorted -- i32/i64 columns by the stable merge sort,
 // char columns by lib_quicksort_char, the rest by the quicksort -- and its
-// runs of equal values form the next column's ranges.
-I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, long long n, const unsigned** perm_out) {
+// runs of equal values form the next column's ranges.  *checked: the device
+// error word has been read since the last pass that can set it.
+I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, long long n, const unsigned** perm_out,
+               bool* checked) {
+    *checked = true;
     if (n >= (1LL << 31)) return set_error(E_NOT_IMPL, "quicksort order of 2^31 or more rows");
     const size_t nn = (size_t)(n > 0 ? n : 1);
     unsigned* perm = (unsigned*)salloc(nn * 4);
@@ -473,16 +812,15 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
     unsigned long long* img = (unsigned long long*)salloc(nn * 8);
     long long* starts = (long long*)salloc(nn * 8);
     uint8_t* flags = (uint8_t*)salloc(nn * 3);
-    unsigned* aux = (unsigned*)salloc(64);
-    if (!perm || !tmp || !seg || !img || !starts || !flags || !aux) return E_DEVICE_OOM;
+    QsLists lists;
+    if (!perm || !tmp || !seg || !img || !starts || !flags) return E_DEVICE_OOM;
+    HG_CHECK(qs_lists_alloc(n, &lists));
     *perm_out = perm;
     if (n == 0) return 0;
     uint8_t* up = flags;
     uint8_t* down = flags + nn;
     uint8_t* mode = flags + 2 * nn;
-    unsigned* nanflag = aux;
-    unsigned* nrev = aux + 1;
-    HG_CU(cudaMemsetAsync(nanflag, 0, 4, g_stream));
+    unsigned* nanflag = &lists.cnt->nan;
     const unsigned g = qs_grid(n);
     HG_LAUNCH("qs_iota", g, 256, 0, k_qs_iota, perm, n);
     long long ns = 1;  // segments: runs of rows equal on the columns sorted so far
@@ -493,22 +831,35 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
         const bool desc = asc && !asc[c];
         if (typ == H_C && desc)
             return set_error(E_NOT_IMPL, "descending char column in a list order (the reference indexes past the range)");
+        const bool stable = typ == H_I || typ == H_L || typ == H_C;
+        bool ran = false;  // a quicksort whose counters the next wait reads into h
+        HG_CU(cudaMemsetAsync(lists.cnt, 0, sizeof(QsCounters), g_stream));
         HG_CHECK(qs_image_of(cols[c], typ, perm, n, desc, img, nanflag));
         // lib_order_by_sorted
         HG_CU(cudaMemsetAsync(flags, 0, 2 * nn, g_stream));
-        HG_CU(cudaMemsetAsync(nrev, 0, 4, g_stream));
         HG_LAUNCH("qs_updown", g, 256, 0, k_qs_updown, img, seg, n, up, down);
-        HG_LAUNCH("qs_mode", qs_grid(ns), 256, 0, k_qs_mode, up, down, ns, desc ? 1 : 0, mode, nrev);
-        unsigned hrev = 0;
-        HG_CHECK(rb_queue(&hrev, nrev, 4));
+        HG_LAUNCH("qs_mode", qs_grid(ns), 256, 0, k_qs_mode, up, down, starts, ns, n, desc ? 1 : 0, typ == H_C ? 10 : 2,
+                  mode, lists);
+        QsCounters h;
+        HG_CHECK(rb_queue(&h, lists.cnt, sizeof h));
         HG_CU(stream_sync());
-        HG_CHECK(qs_nan_check(nanflag));
-        if (hrev) {
+        HG_CHECK(qs_nan_check(h));
+        if (h.nrev) {
             HG_LAUNCH("qs_reverse", g, 256, 0, k_qs_reverse, perm, seg, starts, ns, n, mode, tmp);
             unsigned* t = perm; perm = tmp; tmp = t;
             HG_CHECK(qs_image_of(cols[c], typ, perm, n, desc, img, nanflag));
         }
-        if (typ == H_I || typ == H_L || typ == H_C) {
+        if (!h.nbig && !h.nblock && (!h.nwarp || stable)) {
+            // nothing is left to sort, or only short segments in stable order
+            if (h.nwarp) {
+                const unsigned cap = 16u * (unsigned)g_sms, want = grid_for(h.nwarp, 8);
+                HG_LAUNCH("qs_stable_small", want < cap ? want : cap, 256, 0, k_qs_stable_small, lists, img, perm);
+            }
+            if (typ == H_C)
+                HG_LAUNCH("qs_char_small", qs_grid(ns), 256, 0, k_qs_char_small, (const int8_t*)cols[c], starts, ns, n,
+                          mode, perm);
+        } else
+        if (stable) {
             // stable by (segment, image): radix sort on the image, then on
             // the segment index; kept, reversed and small char segments have
             // key 0 and do not move
@@ -518,6 +869,7 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
             HG_LAUNCH("qs_skey", g, 256, 0, k_qs_skey, img, seg, starts, ns, n, mode, typ == H_C ? 10 : 2, key);
             const unsigned long long* k1;
             const unsigned* pos1;
+            *checked = c + 1 < nc;  // the next column's waits read the error word
             HG_CHECK(radix_sort<unsigned long long>(key, n, &k1, &pos1, nullptr));
             HG_LAUNCH("qs_gather_seg", g, 256, 0, k_qs_gather_seg, seg, pos1, n, sk);
             const unsigned* k2;
@@ -529,18 +881,19 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
                 HG_LAUNCH("qs_char_small", qs_grid(ns), 256, 0, k_qs_char_small, (const int8_t*)cols[c], starts, ns, n,
                           mode, perm);
         } else {
-            unsigned* lo = (unsigned*)salloc(nn * 4);
-            unsigned* hi = (unsigned*)salloc(nn * 4);
-            if (!lo || !hi) return E_DEVICE_OOM;
-            HG_LAUNCH("qs_ranges", g, 256, 0, k_qs_ranges, seg, starts, ns, n, mode, perm, lo, hi, tmp);
-            HG_CHECK(qs_run(n, perm, img, lo, hi, tmp));
+            HG_CHECK(qs_run(n, perm, img, seg, starts, ns, mode, lists, &h, tmp));
+            ran = true;
             unsigned* t = perm; perm = tmp; tmp = t;
         }
         if (c + 1 < nc) {  // the runs of equal values become the next column's segments
             HG_CHECK(qs_image_of(cols[c], typ, perm, n, desc, img, nanflag));
             HG_LAUNCH("qs_heads", g, 256, 0, k_qs_heads, img, seg, n, up);
-            HG_CHECK(compact_rows(up, n, starts, &ns));
+            HG_CHECK(compact_rows(up, n, starts, &ns));  // waits, and reads the device errors
+            if (ran) HG_CHECK(qs_depth_check(n, h));
             HG_LAUNCH("qs_segid", g, 256, 0, k_qs_segid, starts, ns, n, seg);
+        } else if (ran) {
+            HG_CHECK(check_device_errors());
+            HG_CHECK(qs_depth_check(n, h));
         }
     }
     HG_CHECK(last_launch_error());

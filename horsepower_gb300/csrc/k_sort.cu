@@ -535,7 +535,8 @@ template I radix_sort<unsigned long long>(const unsigned long long*, long long, 
 
 // the reference's comparison sorts (k_qsort.cu)
 I qs_sort_vector(const void* col, I typ, long long n, bool asc, const unsigned** perm_out);
-I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, long long n, const unsigned** perm_out);
+I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, long long n, const unsigned** perm_out,
+               bool* checked);
 
 // ---------------------------------------------------------------- sort keys
 enum KeyXf : int {
@@ -1131,14 +1132,15 @@ static I order_prealloc(V z, long long n, bool reverse, RadixOut* ro, void** d) 
     return 0;
 }
 
-static I order_output(V z, const SortResult& r, long long n, bool reverse, void* d_pre = nullptr) {
+// checked: the device error word has been read since the sort's last pass
+static I order_output(V z, const SortResult& r, long long n, bool reverse, void* d_pre = nullptr, bool checked = false) {
     void* d = d_pre;
     if (!d) HG_CHECK(alloc_out(z, H_L, n, &d));
     if (n > 0 && !r.perm64) HG_LAUNCH("widen", gcap(n), 256, 0, k_widen, r.perm, n, (long long*)d, reverse ? 1 : 0);
     HG_CHECK(last_launch_error());
     // a radix pass whose look-back gave up leaves a wrong permutation: read
     // the device error word before the result is marked as in range
-    HG_CHECK(check_device_errors());
+    if (!checked) HG_CHECK(check_device_errors());
     register_bound(d, n, n);
     return finish_out(z, d);
 }
@@ -1418,7 +1420,8 @@ I pfnGroupBasic(V z, V x) {
             I typs[KMAXC];
             B up[KMAXC];
             for (int i = 0; i < nc; i++) { typs[i] = c[i].typ; up[i] = 1; }
-            HG_CHECK(qs_sort_list(nc, ptrs, typs, up, n, &r.perm));
+            bool checked;
+            HG_CHECK(qs_sort_list(nc, ptrs, typs, up, n, &r.perm, &checked));
             r.keys = nullptr;
             r.key64 = 0;
             r.key_injective = false;
@@ -1478,7 +1481,7 @@ static I order_basic(V z, V x, V y) {
     }
     if (is_real(x->typ) || is_dtime(x->typ)) {  // lib_order_by_vector: the reference's quicksort
         HG_CHECK(qs_sort_vector(p, x->typ, n, asc, &r.perm));
-        return order_output(z, r, n, false);
+        return order_output(z, r, n, false, nullptr, true);
     }
     return set_error(E_NOT_IMPL, "order on this type is outside the path");
 }
@@ -1490,12 +1493,14 @@ I pfnOrderBy(V z, V x, V y) {
         if (!list_of_basic(x)) return E_DOMAIN;
         int nc = (int)x->len;
         V0* c = host_nodes(x);
-        const void* pb;
-        HG_CHECK(in_ptr(y, &pb));
         B dir[KMAXC + 1];
         if (nc > KMAXC) return set_error(E_NOT_IMPL, "order by more than %d columns", KMAXC);
-        if (nc > 0) {
-            HG_CU(cudaMemcpyAsync(dir, pb, nc, cudaMemcpyDefault, g_stream));
+        if (nc > 0 && (is_inline(y) || !is_device_ptr(y->g))) {  // plain host memory
+            memcpy(dir, y->g, (size_t)nc);
+        } else if (nc > 0) {
+            const void* pb;
+            HG_CHECK(in_ptr(y, &pb));
+            HG_CHECK(rb_queue(dir, pb, (size_t)nc));
             HG_CU(stream_sync());
         }
         long long n = nc ? c[0].len : 0;
@@ -1534,8 +1539,9 @@ I pfnOrderBy(V z, V x, V y) {
         if (!all_int) {  // lib_quicksort_list with the quicksort or the char sort on some column
             I typs[KMAXC];
             for (int i = 0; i < nc; i++) typs[i] = c[i].typ;
-            HG_CHECK(qs_sort_list(nc, ptrs, typs, dir, n, &r.perm));
-            return order_output(z, r, n, false);
+            bool checked;
+            HG_CHECK(qs_sort_list(nc, ptrs, typs, dir, n, &r.perm, &checked));
+            return order_output(z, r, n, false, nullptr, checked);
         }
         bool all_asc = true;
         for (int i = 0; i < nc; i++) all_asc = all_asc && dir[i];

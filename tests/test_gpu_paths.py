@@ -111,3 +111,59 @@ def test_radix_pairs(libs, t0, t1, dirs, span0, span1):
         out.append(L.to_py(z))
         L.free_inputs()
     assert np.array_equal(out[0], out[1])
+
+
+def quick_keys(rng, n, shape):
+    x = rng.standard_normal(n)
+    if shape == "ties":
+        x = np.round(x * 3) / 2
+    elif shape == "few":
+        x = rng.integers(0, 3, n) * 0.5
+    elif shape == "equal":
+        x = np.full(n, -0.0)
+        x[::3] = 0.0
+    elif shape == "rising":  # first-element pivots: one element per depth
+        x = np.sort(x)
+        x[: n // 3] = x[0]
+    elif shape == "falling":
+        x = np.sort(x)[::-1].copy()
+    return x
+
+
+@pytest.mark.parametrize("shape", ["plain", "ties", "few", "equal", "rising", "falling"])
+@pytest.mark.parametrize("n", [2, 3, 31, 32, 33, 64, 65, 1000, 4095, 4096, 4097, 4200, 9000])
+def test_quicksort_scales(libs, n, shape):
+    """The quicksort in a warp, in a CTA and in global memory: f64 keys on
+    either side of 32 and 4096 rows, both directions, against the oracle's
+    sequential quicksort (its order of equal keys included)."""
+    gpu, ora = libs
+    x = quick_keys(np.random.default_rng(n), n, shape)
+    for up in (1, 0):
+        out = []
+        for L in (gpu, ora):
+            out.append(L.to_py(L.call("pfnOrderBy", L.vec(x, H_E), L.vec(np.array([up], bool), H_B))))
+            L.free_inputs()
+        assert np.array_equal(out[0], out[1]), up
+
+
+@pytest.mark.parametrize("dirs", [(1, 1), (0, 1), (1, 0), (0, 0)])
+@pytest.mark.parametrize("second", ["i32", "f64", "char"])
+@pytest.mark.parametrize("run", [1, 2, 9, 10, 32, 33, 700, 5000])
+def test_quicksort_lists(libs, run, second, dirs):
+    """Lists led by an f64 column whose runs of equal values have about `run`
+    rows: short runs only (sorted by a warp each), longer ones, and no repeats
+    at all, with a stable, a quicksort and a char column behind it."""
+    gpu, ora = libs
+    if second == "char" and not dirs[1]:
+        pytest.skip("descending char columns are refused")
+    rng = np.random.default_rng(run + 3 * dirs[0] + dirs[1])
+    n = 12_007
+    a = rng.permutation(n) // run * 0.25
+    b = {"i32": (rng.integers(-4, 4, n).astype(np.int32), H_I), "f64": (rng.integers(-4, 4, n) * 1.5, H_E),
+         "char": (rng.integers(97, 103, n).astype(np.int8), H_C)}[second]
+    out = []
+    for L in (gpu, ora):
+        z = L.call("pfnOrderBy", L.list([L.vec(a, H_E), L.vec(*b)]), L.vec(np.array(dirs, bool), H_B))
+        out.append(L.to_py(z))
+        L.free_inputs()
+    assert np.array_equal(out[0], out[1])
