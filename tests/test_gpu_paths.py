@@ -167,3 +167,66 @@ def test_quicksort_lists(libs, run, second, dirs):
         out.append(L.to_py(z))
         L.free_inputs()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nfact,groups", [(2047, 6), (2048, 8), (2049, 1), (100_003, 6), (300_001, 8)])
+def test_shared_windows(libs, nfact, groups):
+    """Plans over one table set, date windows from none to all of the rows (a
+    tile's selection fits one list, or is taken in parts): each plan's rows
+    equal the same plan through its builtins, bit for bit."""
+    from horsepower_gb300 import batch as B, data as D, plans as P
+    gpu = libs[0]
+    dim, fact = D.join_tables(nfact=nfact, ndim=max(2, nfact // 3), seed=nfact)
+    rng = np.random.default_rng(groups)
+    g = rng.integers(0, groups, nfact)
+    fact["flag"], fact["status"] = (g // 2).astype(np.int8), (g % 2).astype(np.int8)
+    ddim, dfact = B.device_tables(gpu, dim, fact)
+    spans = [1, 30, 365, 620, 640, 700, 1300, 2525, 2526]
+    wins = [(D.DAYS0 + int(rng.integers(0, D.NDAYS - s + 1)), s) for s in spans]
+    wins = [(lo, lo + s) for lo, s in wins] + [(D.WIN_LO, D.WIN_LO), (D.DAYS0 - 9, D.DAYS0 + 5000)]
+    got = B.run_batch(gpu, [B.make_plan(ddim, dfact, lo, hi) for lo, hi in wins])
+    for (lo, hi), r in zip(wins, got):
+        if not np.isin(fact["fk"], dim["pk"][(dim["date"] >= lo) & (dim["date"] < hi)]).any():
+            assert len(r[0]) == 0
+            continue
+        want = [gpu.to_py(o) for o in P.join_group(gpu, ddim, dfact, lo, hi)]
+        for a, b in zip(r, want):
+            assert np.array_equal(a, b), (lo, hi)
+    gpu.free_inputs()
+
+
+@pytest.mark.parametrize("nreq", [1, 7, 8, 9, 40])
+def test_served_windows(libs, nreq):
+    """Served filter-aggregates, any number of windows folded together: each
+    equals the fused chain of its window bit for bit.  Served top-k rows equal
+    the first rows of the stable (key, sec) order in the key range."""
+    from horsepower_gb300 import data as D, plans as P, serve as S
+    gpu = libs[0]
+    rng = np.random.default_rng(nreq)
+    line = S.line_table(gpu, 50_021, seed=nreq)
+    from horsepower_gb300 import batch as B
+    dim, fact = B.device_tables(gpu, *D.join_tables(nfact=3000, ndim=700, seed=3))
+    n = 200_003
+    key = np.minimum(rng.zipf(1.2, n), 1 << 40).astype(np.int64)
+    sec = rng.integers(0, 1000, n).astype(np.int32)
+    order = dict(key=B.to_device(gpu, key, H_L), sec=B.to_device(gpu, sec, H_I))
+    srv = S.Server(gpu, line, dim, fact, order, budget=1 << 30)
+    reqs = []
+    for _ in range(nreq):
+        lo = int(D.DAYS0 + rng.integers(0, D.NDAYS))
+        reqs.append(S.Request(S.FILTER_AGG, lo, lo + int(rng.integers(0, 900)), 0, 0, 0.0))
+        a = int(rng.choice([1, 2, 50, 10_000, 1 << 30]))
+        reqs.append(S.Request(S.TOPK_ORDER, 0, 0, a, a + int(rng.choice([0, 1, 100, 1 << 35])), 0.0))
+    got, _, _ = srv.run(reqs)
+    for r, v in zip(reqs, got):
+        if r.kind == S.FILTER_AGG:
+            ch = P.Chain(gpu, P.Q6_CHAIN.format(lo=r.lo, hi=r.hi)) if nreq < 10 else None
+            if ch:
+                f = gpu.to_py(ch.run([line["shipdate"], line["qty"], line["disc"], line["price"]]))[0]
+                assert v == f, (r.lo, r.hi)
+        else:
+            rows = np.flatnonzero((key >= r.klo) & (key < r.khi))
+            want = rows[np.lexsort((sec[rows], key[rows]))][: S.TOPK]
+            assert np.array_equal(v, want), (r.klo, r.khi)
+    srv.close()
+    gpu.free_inputs()
