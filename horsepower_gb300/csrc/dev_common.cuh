@@ -180,13 +180,14 @@ __device__ __forceinline__ unsigned long long chain_lookback(unsigned long long*
 // ---- compareFloat (h_primitive.cc:1061) against a fixed double s without
 // FP64 arithmetic.  With s fixed, compareFloat(v, s) is a non-decreasing step
 // function of v (-1, then 0, then 1) and compareFloat(s, v) a non-increasing
-// one, so both reduce to two thresholds on an integer image of v that keeps
-// the IEEE order: c = ord(v) < ta ? ca : (ord(v) < tb ? cb : cc).  The host
-// finds the thresholds by bisection, evaluating compareFloat itself in
-// double arithmetic; NaN compares as 1 either way round.
-struct F64Cmp {
-    long long ta, tb;
-    int ca, cb, cc;
+// one, and NaN compares as 1 either way round.  So on an unsigned image of v
+// that keeps the IEEE order (the NaNs outside the infinities, at both ends)
+// each of the six compares is true inside one range of images, or outside it:
+// a subtraction and a compare decide it.  The host finds the range's ends by
+// bisection, evaluating compareFloat itself in double arithmetic.
+struct F64Range {
+    unsigned long long base, span;  // images in [base, base + span), wrapping
+    int inv;                        // 1: true outside
 };
 __host__ __device__ __forceinline__ long long f64_ord(unsigned long long b) {
     return (b >> 63) ? -(long long)(b & 0x7fffffffffffffffull) : (long long)b;  // -0.0 and +0.0 both map to 0
@@ -194,13 +195,15 @@ __host__ __device__ __forceinline__ long long f64_ord(unsigned long long b) {
 __host__ __device__ __forceinline__ bool f64_nan_bits(unsigned long long b) {
     return (b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull;
 }
-__device__ __forceinline__ int f64_cmp_fixed(double v, const F64Cmp& t) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    if (f64_nan_bits(b)) return 1;
-    const long long o = f64_ord(b);
-    return o < t.ta ? t.ca : (o < t.tb ? t.cb : t.cc);
+__host__ __device__ __forceinline__ bool f64_range_bits(unsigned long long b, const F64Range& r) {
+    const unsigned long long u = b ^ ((unsigned long long)((long long)b >> 63) | (1ull << 63));
+    return (u - r.base < r.span) != (r.inv != 0);
 }
-F64Cmp f64_cmp_thresholds(double s, bool scalar_first);  // host (k_elementwise.cu)
+__device__ __forceinline__ bool f64_in_range(double v, const F64Range& r) {
+    return f64_range_bits((unsigned long long)__double_as_longlong(v), r);
+}
+// op 0..5: <, <=, >, >=, ==, != of (v, s), or of (s, v) when scalar_first
+F64Range f64_cmp_range(double s, bool scalar_first, int op);  // host (k_elementwise.cu)
 
 // ---- fixed-order deterministic tile sum (used by @sum/@avg and every
 // segmented sum).  A chunk of up to TILE_SUM = 4096 elements is summed as:

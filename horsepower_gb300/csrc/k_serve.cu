@@ -47,7 +47,7 @@ constexpr int SQ_MAXW = 256;  // request windows per shared-scan launch
 __global__ void __launch_bounds__(256) k_s_q6(const int* __restrict__ ship, const int* __restrict__ qty,
                                               const double* __restrict__ disc, const double* __restrict__ price,
                                               long long n, const int* __restrict__ lohi, int nw,
-                                              double* __restrict__ part, long long ntiles, F64Cmp d_lo, F64Cmp d_hi) {
+                                              double* __restrict__ part, long long ntiles, F64Range d_lo, F64Range d_hi) {
     grid_entry();
     __shared__ int s_lo[SQ_MAXW], s_hi[SQ_MAXW];
     __shared__ double ws[SQ_MAXW][8];
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) k_s_q6(const int* __restrict__ ship, cons
 #pragma unroll
     for (int k = 0; k < 16; k++) {
         const long long i = base + k * 256 + threadIdx.x;
-        const bool c = i < n && q[k] < 24 && f64_cmp_fixed(dc[k], d_lo) >= 0 && f64_cmp_fixed(dc[k], d_hi) <= 0;
+        const bool c = i < n && q[k] < 24 && f64_in_range(dc[k], d_lo) && f64_in_range(dc[k], d_hi);
         v[k] = c ? __dmul_rn(v[k], dc[k]) : 0.0;
         live |= (unsigned)c << k;
     }
@@ -517,7 +517,7 @@ static I filter_aggs(const hgpu_server_s* s, const hgpuRequest* req, const std::
     double* part = (double*)salloc((size_t)nw * ntiles * 8);
     if (!dl || !part) return E_DEVICE_OOM;
     HG_CU(cudaMemcpyAsync(dl, lohi.data(), 8 * nw, cudaMemcpyHostToDevice, g_stream));
-    const F64Cmp d_lo = f64_cmp_thresholds(0.05, false), d_hi = f64_cmp_thresholds(0.07, false);
+    const F64Range d_lo = f64_cmp_range(0.05, false, 3), d_hi = f64_cmp_range(0.07, false, 1);  // >=, <=
     for (long long c0 = 0; c0 < nw; c0 += SQ_MAXW) {
         int cw = (int)std::min<long long>(SQ_MAXW, nw - c0);
         HG_LAUNCH("serve_q6", (unsigned)ntiles, 256, 0, k_s_q6, t.l_shipdate, t.l_qty, t.l_disc, t.l_price, t.nline,

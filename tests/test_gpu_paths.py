@@ -10,7 +10,7 @@ import os
 import numpy as np
 import pytest
 
-from horsepower_gb300.abi import Builtins, H_B, H_C, H_E, H_I, H_L  # noqa: F401
+from horsepower_gb300.abi import (Builtins, DTYPE, H_B, H_C, H_E, H_F, H_H, H_I, H_J, H_L)  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -230,3 +230,49 @@ def test_served_windows(libs, nreq):
             assert np.array_equal(v, want), (r.klo, r.khi)
     srv.close()
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("typ", [H_B, H_J, H_H, H_I, H_L, H_F, H_E])
+@pytest.mark.parametrize("n", [2, 15, 31, 511, 512, 513, 4096 + 7, 70_001])
+def test_elementwise_chunks(libs, typ, n):
+    """Compare, arithmetic, logic and not around the 512-element chunks, from
+    16-byte-aligned columns and from views that start one element later, for
+    vector and scalar operands on either side: equal to the oracle."""
+    from horsepower_gb300 import batch as B
+    gpu, ora = libs
+    rng = np.random.default_rng(n + typ)
+    dt = DTYPE[typ]
+    cols = []
+    for _ in range(2):
+        if typ == H_B:
+            cols.append(rng.random(n + 1) < 0.5)
+        elif typ in (H_F, H_E):
+            c = np.round(rng.standard_normal(n + 1), 1).astype(dt)
+            c[rng.random(n + 1) < 0.05] = np.nan
+            cols.append(c)
+        else:
+            cols.append(rng.integers(-5, 6, n + 1).astype(dt))
+    names = ["pfnLt", "pfnLeq", "pfnGt", "pfnGeq", "pfnEq", "pfnNeq", "pfnPlus", "pfnMinus", "pfnMul"]
+    names += ["pfnAnd", "pfnOr", "pfnXor", "pfnNand", "pfnNor"] if typ == H_B else ["pfnDiv"]
+    for skip in (0, 1):
+        a, b = cols[0][skip:], cols[1][skip:]
+        if typ != H_B:
+            b = np.where(b == 0, dt(3), b)      # divisors
+        s = b[0] if b[0] == b[0] else dt(0.1)
+
+        def view(c, skip=skip):
+            d = B.to_device(gpu, np.concatenate([c[:1]] * skip + [c]), typ)
+            d.g, d.len = d.g + skip * c.itemsize, c.size
+            return d
+
+        da, db = view(a), view(b)
+        for f in names:
+            for x, y, hx, hy in ((da, db, a, b), (da, s, a, s), (s, db, s, b)):
+                dev = [gpu.scalar(v, typ) if isinstance(v, np.generic) else v for v in (x, y)]
+                host = [ora.scalar(v, typ) if isinstance(v, np.generic) else ora.vec(v, typ) for v in (hx, hy)]
+                got, want = gpu.to_py(gpu.call(f, *dev)), ora.to_py(ora.call(f, *host))
+                assert got.dtype == want.dtype and np.array_equal(got, want, equal_nan=got.dtype.kind == "f"), (f, skip)
+        if typ == H_B:
+            assert np.array_equal(gpu.to_py(gpu.call("pfnNot", da)), ~a)
+    gpu.free_inputs()
+    ora.free_inputs()
