@@ -43,6 +43,9 @@ enum : unsigned {
     DERR_CAPACITY = 8u,    // a hash table or buffer ran out of slots
 };
 extern unsigned* g_derr;   // device word
+// words behind it in the same zeroed 256 bytes: counters that a kernel leaves
+// at zero for the next launch
+enum { DW_CHAIN = 32 };    // blocks of a fused reduction that have finished
 I check_device_errors();   // syncs, reads and clears g_derr, maps to E_* codes
 // iteration limit for every device-side spin-wait
 constexpr long long SPIN_LIMIT = 1LL << 24;

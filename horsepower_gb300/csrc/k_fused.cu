@@ -203,6 +203,29 @@ struct Gen {
 // Device helpers shared by every generated kernel (same semantics as
 // k_elementwise.cu and k_reduce.cu).
 static const char* kPrelude = R"(
+// *p when `on`, else 0.  Volatile, so that the loads of all rows are issued
+// where they stand and not sunk into the branches that use them.
+template <int B> struct hg_ldn;
+template <> struct hg_ldn<8> { static __device__ __forceinline__ unsigned long long at(const void* p, bool on) {
+    unsigned long long v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.u64 %0, 0;\n@q ld.global.nc.u64 %0, [%1];\n}" : "=&l"(v) : "l"(p), "r"((unsigned)on));
+    return v; } };
+template <> struct hg_ldn<4> { static __device__ __forceinline__ unsigned at(const void* p, bool on) {
+    unsigned v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.u32 %0, 0;\n@q ld.global.nc.u32 %0, [%1];\n}" : "=&r"(v) : "l"(p), "r"((unsigned)on));
+    return v; } };
+template <> struct hg_ldn<2> { static __device__ __forceinline__ unsigned short at(const void* p, bool on) {
+    unsigned short v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.u16 %0, 0;\n@q ld.global.nc.u16 %0, [%1];\n}" : "=&h"(v) : "l"(p), "r"((unsigned)on));
+    return v; } };
+template <> struct hg_ldn<1> { static __device__ __forceinline__ unsigned char at(const void* p, bool on) {
+    unsigned v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.u32 %0, 0;\n@q ld.global.nc.u8 %0, [%1];\n}" : "=&r"(v) : "l"(p), "r"((unsigned)on));
+    return (unsigned char)v; } };
+template <typename T> __device__ __forceinline__ T hg_ld(const T* p, bool on) {
+    union { decltype(hg_ldn<sizeof(T)>::at(p, on)) u; T t; } x;
+    x.u = hg_ldn<sizeof(T)>::at(p, on);
+    return x.t; }
 template <typename T> struct hg_is_f { static const bool v = false; };
 template <> struct hg_is_f<float> { static const bool v = true; };
 template <> struct hg_is_f<double> { static const bool v = true; };
@@ -254,6 +277,7 @@ struct Compiled {
     int acc_typ = H_E;      // accumulator / result type
     std::vector<int> out_typ;
     bool may_fail = false;  // some operation can flag an error (division by zero)
+    bool by_value = false;  // pointers as kernel parameters
 };
 
 }  // namespace hg
@@ -279,15 +303,25 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
     cm->sink = r->op;
     std::string body, red;
     const int nin = (int)types.size();
-    std::string loads;
-    auto gen_loads = [&]() {
-        loads.clear();
-        for (int k = 0; k < nin; k++)
-            if (g.used[k])
-                loads += std::string("        ") + ctype(types[k]) + " v" + std::to_string(k) + " = ((const " + ctype(types[k]) +
-                         "*)cols[" + std::to_string(k) + "])[i];\n";
+    // the column and output pointers are kernel parameters (a parameter list
+    // holds 32 KB; programs with more take them from device memory)
+    const size_t nouts = (r->op == "map") ? r->kids.size() : r->op == "compress" ? r->kids.size() - 1 : 0;
+    cm->by_value = nin <= 1024 && nouts <= 1024;
+    auto pointers = [&](const char* name, size_t count, bool in) {
+        return cm->by_value ? std::string("struct Hg_") + name + " { " + (in ? "const " : "") + "void* p[" +
+                                  std::to_string(count ? count : 1) + "]; };\n"
+                            : std::string();
+    };
+    auto param = [&](const char* name, bool in) {
+        return cm->by_value ? std::string("Hg_") + name + " " + name + "_v"
+                            : std::string(in ? "const " : "") + "void* const* " + name;
+    };
+    auto bind = [&](const char* name, bool in) {
+        return cm->by_value ? std::string("    ") + (in ? "const " : "") + "void* const* " + name + " = " + name + "_v.p;\n"
+                            : std::string();
     };
     std::string src = kPrelude;
+    src += pointers("cols", (size_t)nin, true) + pointers("outs", nouts, false);
     if (r->op == "sum" || r->op == "min" || r->op == "max" || r->op == "count") {
         std::string val, mask;
         if (r->op == "count") {
@@ -312,15 +346,19 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
                 while (!st.empty()) { Node* q = st.back(); st.pop_back(); if (q->op == "x") in_val[q->col] = true; for (auto& k : q->kids) st.push_back(k.get()); }
             }
         }
-        std::string vloads, hoist, preload, unpack;
+        std::string hoist, preload, unpack, vdecl, vload, vunpack;
         for (int k = 0; k < nin; k++) {
             const std::string K = std::to_string(k), T = ctype(types[k]);
             if (in_mask[k] || in_val[k]) hoist += "    const " + T + "* __restrict__ c" + K + " = (const " + T + "*)cols[" + K + "];\n";
-            if (in_val[k] && !in_mask[k]) vloads += "                " + T + " v" + K + " = c" + K + "[i];\n";
             if (in_mask[k]) {
-                preload += "        a" + K + "[k] = in ? c" + K + "[i] : (" + T + ")0;\n";
-                hoist += "    " + T + " a" + K + "[16];\n";
-                unpack += "            " + T + " v" + K + " = a" + K + "[k];\n";
+                preload += " a" + K + "[k] = hg_ld(c" + K + " + i, in);";
+                hoist += "    " + T + " a" + K + "[4];\n";
+                unpack += "                const " + T + " v" + K + " = a" + K + "[k];\n";
+            }
+            if (in_val[k]) {
+                vdecl += "        " + T + " b" + K + "[4];\n";
+                vload += "            b" + K + "[k] = " + (in_mask[k] ? "a" + K + "[k]" : "hg_ld(c" + K + " + i, (m >> k) & 1u)") + ";\n";
+                vunpack += "                const " + T + " v" + K + " = b" + K + "[k];\n";
             }
         }
         int vt = r->op == "count" ? H_L : arith_rank(r->kids[0]->typ);
@@ -331,46 +369,75 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
                         : (at == H_E ? "__dadd_rn(a, b)" : at == H_F ? "__fadd_rn(a, b)" : "(long long)((unsigned long long)a + (unsigned long long)b)");
         std::string ident = r->op == "min" ? "ident" : r->op == "max" ? "ident" : std::string("(") + A + ")0";
         // Each block reduces one 4096-row tile in the tile-tree order: lane t
-        // takes rows t, t+256, ..., t+3840 (the mask columns of all 16 rows
-        // are loaded before the first is used, so the loads overlap), then a
-        // xor butterfly and the pairwise combine of the 8 warps.  With
-        // `result` set, the block that finishes last reduces the tile
-        // partials by the same tree (one tile of partials: at most 4096
-        // blocks) and writes the result, so the chain is one launch.
-        auto tree = [&](const std::string& dest) {
-            return std::string("    {\n") +
-                   "    for (int o = 16; o > 0; o >>= 1) acc = hg_op(acc, __shfl_xor_sync(0xffffffffu, acc, o));\n"
-                   "    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;\n"
-                   "    __syncthreads();\n"
-                   "    if (threadIdx.x == 0) " + dest + " = hg_op(hg_op(hg_op(ws[0], ws[1]), hg_op(ws[2], ws[3])),"
-                   " hg_op(hg_op(ws[4], ws[5]), hg_op(ws[6], ws[7])));\n"
-                   "    }\n";
+        // takes rows t, t+256, ..., t+3840, then a xor butterfly and the
+        // pairwise combine of the 8 warps, which warp 0 folds for all of them
+        // at once (9 operations instead of 40; the operand pairs are those of
+        // the separate butterflies).  What bounds it is memory latency, so
+        // the rows go in rounds of 4: the value columns of a round's selected
+        // rows and the mask columns of the next round are all in flight
+        // before the first value is added.  0.377 -> 0.278 ms for the 60M-row q6 (each selected value
+        // loaded where it is added before; rounds of 8 or 16 rows hold too few
+        // warps, 0.302 and 0.44 ms).  With `result` set, the block that finishes last reduces the tile partials by the same
+        // tree (one tile of partials: at most 4096 blocks) and writes the
+        // result, so the chain is one launch.
+        const bool sum = r->op == "sum" || r->op == "count";
+        src += std::string("__device__ __forceinline__ ") + A + " hg_op(" + A + " a, " + A + " b) { return " + opf + "; }\n" +
+               "__device__ __forceinline__ " + A + " hg_lane(" + A + " own, " + A + " other, bool upper) { return " +
+               (sum ? "hg_op(own, other)" : "upper ? hg_op(other, own) : hg_op(own, other)") + "; }\n" +
+               "__device__ __forceinline__ " + A + " hg_tile(" + A + " acc, " + A + "* ws) {\n"
+               "    ws[threadIdx.x] = acc;\n"
+               "    __syncthreads();\n"
+               "    if (threadIdx.x >= 32) return acc;\n"
+               "    " + A + " x[8], a[4], b[2], c;\n"
+               "    for (int v = 0; v < 8; v++) x[v] = ws[v * 32 + threadIdx.x];\n"
+               "    const bool u16 = threadIdx.x & 16, u8 = threadIdx.x & 8, u4 = threadIdx.x & 4;\n"
+               "    for (int i = 0; i < 4; i++)\n"
+               "        a[i] = hg_lane(u16 ? x[i + 4] : x[i], __shfl_xor_sync(0xffffffffu, u16 ? x[i] : x[i + 4], 16), u16);\n"
+               "    for (int i = 0; i < 2; i++)\n"
+               "        b[i] = hg_lane(u8 ? a[i + 2] : a[i], __shfl_xor_sync(0xffffffffu, u8 ? a[i] : a[i + 2], 8), u8);\n"
+               "    c = hg_lane(u4 ? b[1] : b[0], __shfl_xor_sync(0xffffffffu, u4 ? b[0] : b[1], 4), u4);\n"
+               "    c = hg_lane(c, __shfl_xor_sync(0xffffffffu, c, 2), threadIdx.x & 2);\n"
+               "    c = hg_lane(c, __shfl_xor_sync(0xffffffffu, c, 1), threadIdx.x & 1);\n"
+               "    for (int o = 4; o < 32; o <<= 1) c = hg_op(c, __shfl_down_sync(0xffffffffu, c, o));\n"
+               "    return c;\n}\n";
+        auto load_round = [&](const std::string& h, const std::string& pad) {
+            return pad + "#pragma unroll\n" + pad + "for (int k = 0; k < 4; k++) { const long long i = base + (" + h +
+                   " + k) * 256; const bool in = i < n;" + preload + " }\n";
         };
-        src += std::string("__device__ __forceinline__ ") + A + " hg_op(" + A + " a, " + A + " b) { return " + opf + "; }\n";
-        src += std::string("extern \"C\" __global__ void __launch_bounds__(256) chain_kernel(const void* const* cols, long long n, ") + A +
-               "* part, " + A + " ident, unsigned* derr, unsigned* done, " + A + "* result) {\n"
-               "    __shared__ " + A + " ws[8];\n"
-               "    __shared__ bool last;\n"
+        src += std::string("extern \"C\" __global__ void __launch_bounds__(256) chain_kernel(") + param("cols", true) +
+               ", long long n, " + A + "* part, " + A + " ident, unsigned* derr, unsigned* done, " + A + "* result) {\n"
                "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"  // as grid_entry
-               "    const long long base = (long long)blockIdx.x * 4096;\n" + hoist +
-               "    #pragma unroll\n"
-               "    for (int k = 0; k < 16; k++) {\n"
-               "        const long long i = base + k * 256 + threadIdx.x;\n"
-               "        const bool in = i < n;\n" + preload +
-               "    }\n"
-               "    " + A + " acc = " + ident + ";\n    bool dz = false;\n"
-               "    #pragma unroll\n"
-               "    for (int k = 0; k < 16; k++) {\n"
-               "        const long long i = base + k * 256 + threadIdx.x;\n"
-               "        if (i < n) {\n" + unpack +
-               "            if (" + mask + ") {\n" + vloads + "                acc = hg_op(acc, (" + A + ")(" + val + "));\n            }\n"
+               "    __shared__ " + A + " ws[256];\n"
+               "    __shared__ bool last;\n" + bind("cols", true) +
+               "    const long long base = (long long)blockIdx.x * 4096 + threadIdx.x;\n" + hoist +
+               "    " + A + " acc = " + ident + ";\n    bool dz = false;\n" + load_round("0", "    ") +
+               "    #pragma unroll 1\n"
+               "    for (int h = 0; h < 16; h += 4) {\n"
+               "        unsigned m = 0;\n" + vdecl +
+               "        #pragma unroll\n"
+               "        for (int k = 0; k < 4; k++) {\n"
+               "            if (base + (h + k) * 256 < n) {\n" + unpack +
+               "                if (" + mask + ") m |= 1u << k;\n"
+               "            }\n"
                "        }\n"
-               "    }\n" + tree("part[blockIdx.x]") +
+               "        #pragma unroll\n"
+               "        for (int k = 0; k < 4; k++) {\n"
+               "            const long long i = base + (h + k) * 256;\n" + vload +
+               "        }\n"
+               "        if (h < 12) {\n" + load_round("h + 4", "            ") + "        }\n"
+               "        #pragma unroll\n"
+               "        for (int k = 0; k < 4; k++)\n"
+               "            if ((m >> k) & 1u) {\n" + vunpack +
+               "                acc = hg_op(acc, (" + A + ")(" + val + "));\n"
+               "            }\n"
+               "    }\n"
+               "    acc = hg_tile(acc, ws);\n"
                "    if (dz) atomicOr(derr, 4u);\n"
+               "    if (threadIdx.x == 0) part[blockIdx.x] = acc;\n"
                "    if (!result) return;\n"
                "    __threadfence();\n"
                "    __syncthreads();\n"
-               "    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;\n"
+               "    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;\n"  // back to 0 by the last
                "    __syncthreads();\n"
                "    if (!last) return;\n"
                "    __threadfence();\n"
@@ -379,7 +446,8 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
                "        const long long i = k * 256 + threadIdx.x;\n"
                "        acc = hg_op(acc, i < gridDim.x ? ((volatile " + A + "*)part)[i] : ident);\n"
                "    }\n"
-               "    __syncthreads();\n" + tree("*result") + "}\n";
+               "    acc = hg_tile(acc, ws);\n"
+               "    if (threadIdx.x == 0) *result = acc;\n}\n";
     } else if (r->op == "compress" || r->op == "map") {
         if (r->kids.empty()) return set_error(E_DOMAIN, "chain: %s needs operands", r->op.c_str());
         bool isc = r->op == "compress";
@@ -416,12 +484,13 @@ static I compile_chain(hgpu_chain_s* c, const std::vector<int>& types, std::shar
             for (int k = 0; k < nin; k++)
                 if (g.used[k])
                     ld += std::string("        const ") + ctype(types[k]) + " v" + std::to_string(k) + "_" + std::to_string(u) +
-                          " = " + iu + " < n ? ((const " + ctype(types[k]) + "*)cols[" + std::to_string(k) + "])[" + iu +
-                          "] : (" + ctype(types[k]) + ")0;\n";
+                          " = hg_ld((const " + ctype(types[k]) + "*)cols[" + std::to_string(k) + "] + " + iu + ", " + iu +
+                          " < n);\n";
         }
-        src += "extern \"C\" __global__ void __launch_bounds__(256) chain_kernel(const void* const* cols, long long n, "
-               "unsigned char* mask, void* const* outs, unsigned* derr) {\n"
-               "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n    bool dz = false;\n"
+        src += "extern \"C\" __global__ void __launch_bounds__(256) chain_kernel(" + param("cols", true) + ", long long n, "
+               "unsigned char* mask, " + param("outs", false) + ", unsigned* derr) {\n"
+               "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n    bool dz = false;\n" +
+               bind("cols", true) + bind("outs", false) +
                "    const long long stride = (long long)gridDim.x * blockDim.x;\n"
                "    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += " +
                std::to_string(CH_UNROLL) + " * stride) {\n" + ld + body + "    }\n    if (dz) atomicOr(derr, 4u);\n}\n";
@@ -488,9 +557,22 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
     }
     std::shared_ptr<Compiled> cm;
     HG_CHECK(compile_chain(c, types, &cm));
-    const void** dcols = (const void**)salloc(16 + nin * sizeof(void*));
-    if (!dcols) return E_DEVICE_OOM;
-    if (nin) HG_CU(cudaMemcpyAsync(dcols, ptrs.data(), nin * sizeof(void*), cudaMemcpyHostToDevice, g_stream));
+    // a pointer array as the kernel takes it: by value, or a device copy
+    void *dcols = nullptr, *douts = nullptr;
+    auto pass = [&](const void* host, size_t count, void** dev, void** arg) -> I {
+        if (cm->by_value) {
+            static const void* const none[1] = {nullptr};
+            *arg = (void*)(count ? host : none);
+            return 0;
+        }
+        *dev = salloc(16 + count * sizeof(void*));
+        if (!*dev) return E_DEVICE_OOM;
+        if (count) HG_CU(cudaMemcpyAsync(*dev, host, count * sizeof(void*), cudaMemcpyHostToDevice, g_stream));
+        *arg = dev;
+        return 0;
+    };
+    void *acols, *aouts;
+    HG_CHECK(pass(ptrs.data(), nin, &dcols, &acols));
     if (cm->sink == "map") {
         // the values go straight into the outputs; with no operation that
         // can fail there is nothing to read back, so no wait
@@ -501,12 +583,10 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
         std::vector<void*> outs(no);
         const long long mark = out_mark();
         for (size_t k = 0; k < no; k++) HG_CHECK(alloc_out(zs[k], cm->out_typ[k], n, &outs[k]));
-        void** douts = (void**)salloc(16 + no * sizeof(void*));
-        if (!douts) return E_DEVICE_OOM;
-        HG_CU(cudaMemcpyAsync(douts, outs.data(), no * sizeof(void*), cudaMemcpyHostToDevice, g_stream));
+        HG_CHECK(pass(outs.data(), no, &douts, &aouts));
         long long nn = n;
         unsigned char* nomask = nullptr;
-        void* args[] = {&dcols, &nn, &nomask, &douts, &g_derr};
+        void* args[] = {acols, &nn, &nomask, aouts, &g_derr};
         unsigned grid = grid_for(n, 256);
         if (grid > (unsigned)g_sms * 16) grid = g_sms * 16;
         {
@@ -531,12 +611,11 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
             outs[k] = salloc((size_t)(n > 0 ? n : 1) * esize(cm->out_typ[k]));
             if (!outs[k]) return E_DEVICE_OOM;
         }
-        void** douts = (void**)salloc(16 + no * sizeof(void*));
         uint8_t* mask = (uint8_t*)salloc((size_t)(n > 0 ? n : 1));
-        if (!douts || !mask) return E_DEVICE_OOM;
-        HG_CU(cudaMemcpyAsync(douts, outs.data(), no * sizeof(void*), cudaMemcpyHostToDevice, g_stream));
+        if (!mask) return E_DEVICE_OOM;
+        HG_CHECK(pass(outs.data(), no, &douts, &aouts));
         long long nn = n;
-        void* args[] = {&dcols, &nn, &mask, &douts, &g_derr};
+        void* args[] = {acols, &nn, &mask, aouts, &g_derr};
         unsigned grid = grid_for(n, 256);
         if (grid > (unsigned)g_sms * 16) grid = g_sms * 16;
         {
@@ -583,11 +662,9 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
     // up to one tile of tile partials: the last block reduces them in the
     // same launch; more: a separate tree over the partials
     const bool one_launch = tiles <= TILE_SUM;
-    unsigned* done = (unsigned*)salloc(16);
-    if (!done) return E_DEVICE_OOM;
+    unsigned* done = g_derr + DW_CHAIN;  // zero between launches
     void* rptr = one_launch ? res : nullptr;
-    if (one_launch) HG_CU(cudaMemsetAsync(done, 0, 4, g_stream));
-    void* args[] = {&dcols, &nn, &part, &ident, &g_derr, &done, &rptr};
+    void* args[] = {acols, &nn, &part, &ident, &g_derr, &done, &rptr};
     {
         LaunchScope ls("chain");
         HG_CU(launch_kernel_args((const void*)cm->kern, dim3((unsigned)tiles), dim3(256), 0, args));
@@ -596,10 +673,15 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
         int op = cm->sink == "min" ? 1 : cm->sink == "max" ? 2 : 0;
         HG_CHECK(tree_reduce_any(cm->acc_typ, op, part, tiles, res));
     }
-    HG_CHECK(check_device_errors());
+    uint64_t bits = 0;
+    HG_CHECK(rb_queue(&bits, res, (size_t)es));
+    HG_CHECK(check_device_errors());  // one wait for both
     z->typ = cm->acc_typ;
     z->len = 1;
-    return finish_out(z, res);
+    z->i64 = 0;
+    memcpy(&z->b, &bits, (size_t)es);
+    z->g = (G)&z->b;
+    return apply_residency(z);
 }
 
 }  // namespace hg

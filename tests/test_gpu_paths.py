@@ -276,3 +276,37 @@ def test_elementwise_chunks(libs, typ, n):
             assert np.array_equal(gpu.to_py(gpu.call("pfnNot", da)), ~a)
     gpu.free_inputs()
     ora.free_inputs()
+
+
+@pytest.mark.parametrize("n", [1, 255, 1023, 1025, 4096, 4097, 50_001])
+@pytest.mark.parametrize("text,typs", [
+    ("(sum (mul x2 x1) (and (lt x0 3:i32) (gt x1 0.25:f64)))", (H_I, H_E, H_E)),   # a value column the mask also reads
+    ("(max x1 (lt x0 x2))", (H_H, H_F, H_J)),
+    ("(min x0 (neq x0 2:i64))", (H_L,)),
+    ("(count (or x0 (lt x1 0:i32)))", (H_B, H_I)),
+])
+def test_chain_rounds(libs, n, text, typs):
+    """A fused reduction's rounds of four rows, last tile ragged, one and
+    several tiles: the f64 sum bit-identical to the fixed tile tree over the
+    rows with unselected ones as -0.0, the others to numpy."""
+    from horsepower_gb300 import plans as P
+    gpu, ora = libs
+    rng = np.random.default_rng(n)
+    x = [rng.random(n) < 0.3 if t == H_B else (rng.standard_normal(n).astype(DTYPE[t]) if t in (H_F, H_E)
+         else rng.integers(-9, 10, n).astype(DTYPE[t])) for t in typs]
+    got = gpu.to_py(P.Chain(gpu, text).run([gpu.vec(c, t) for c, t in zip(x, typs)]))[0]
+    if text.startswith("(sum"):
+        m = (x[0] < 3) & (x[1] - 0.25 >= 1e-13)
+        v = np.where(m, x[2] * x[1], -0.0)
+        want = ora.lib.hgoTreeSumF64(np.ascontiguousarray(v).ctypes.data, n)
+        assert got == want, (got, want)
+    elif text.startswith("(max"):
+        m = x[0] < x[2]
+        if m.any():
+            assert got == x[1][m].max()
+    elif text.startswith("(min"):
+        if (x[0] != 2).any():
+            assert got == x[0][x[0] != 2].min()
+    else:
+        assert got == (x[0] | (x[1] < 0)).sum()
+    gpu.free_inputs()

@@ -35,4 +35,4 @@ def test_every_kernel_waits_first():
 def test_generated_kernels_wait():
     """The chain compiler's kernels hold the same wait (one per kernel text)."""
     text = open(os.path.join(CSRC, "k_fused.cu")).read()
-    assert text.count("chain_kernel(const void* const* cols") == text.count("griddepcontrol.wait") == 2
+    assert text.count("__global__ void __launch_bounds__(256) chain_kernel(") == text.count("griddepcontrol.wait") == 2
