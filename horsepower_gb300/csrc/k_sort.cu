@@ -260,8 +260,8 @@ static unsigned cap8(long long n) {
     return grid > (unsigned)g_sms * 8 ? (unsigned)g_sms * 8 : grid;
 }
 
-static unsigned rx_chunks(long long ntiles) {
-    const long long c = (long long)RX_PER_SM * g_sms;
+static unsigned rx_chunks(long long ntiles, int per_sm) {
+    const long long c = (long long)per_sm * g_sms;
     return (unsigned)(ntiles < c ? ntiles : c);
 }
 
@@ -269,12 +269,13 @@ static unsigned rx_chunks(long long ntiles) {
 // offs, ntiles and derr are filled here.
 template <typename SRC, int BITS>
 static I rx_pass_bits(SRC src, RxPass a, unsigned* counts, unsigned* tot) {
-    a.ntiles = (unsigned)(((long long)a.n + RX_TILE - 1) / RX_TILE);
+    using Shape = RxShape<BITS>;
+    a.ntiles = (unsigned)(((long long)a.n + Shape::TILE - 1) / Shape::TILE);
     a.offs = counts;
     a.derr = g_derr;
-    const unsigned C = rx_chunks(a.ntiles);
-    const int dsm = RX_TILE * (a.cut ? 10 : 8);
-    HG_LAUNCH("radix_count", C, RX_THREADS, 0, (k_rx_count<SRC, BITS, RX_ITEMS>), src, a.n, a.ntiles, a.kshift, a.bits,
+    const unsigned C = rx_chunks(a.ntiles, Shape::PER_SM);
+    const int dsm = Shape::TILE * (a.cut ? 10 : 8);
+    HG_LAUNCH("radix_count", C, RX_THREADS, 0, (k_rx_count<SRC, BITS, Shape::ITEMS>), src, a.n, a.ntiles, a.kshift, a.bits,
               counts, tot);
     HG_LAUNCH("radix_scan", 1u << a.bits, 256, 0, k_rx_scan, counts, C, tot);
     // the attribute belongs to the current device's context: set it on every call (a host-side write)
@@ -291,7 +292,7 @@ static I rx_pass_kv(const unsigned long long* kin, RxPass a, unsigned* counts, u
     a.ntiles = (unsigned)(((long long)a.n + RX_KV_TILE - 1) / RX_KV_TILE);
     a.offs = counts;
     a.derr = g_derr;
-    const unsigned C = rx_chunks(a.ntiles);
+    const unsigned C = rx_chunks(a.ntiles, RX_MAX_PER_SM);
     HG_LAUNCH("radix_count", C, RX_THREADS, 0, (k_rx_count<RxKeys<unsigned long long>, 8, RX_KV_ITEMS>),
               RxKeys<unsigned long long>{kin}, a.n, a.ntiles, a.kshift, a.bits, counts, tot);
     HG_LAUNCH("radix_scan", 1u << a.bits, 256, 0, k_rx_scan, counts, C, tot);
@@ -362,10 +363,10 @@ static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, c
     }
     const bool perm = out && out->perm64, keep = !(perm && !out->keys);
     const int total = pl.hi - pl.lo, rb = bits_for((unsigned long long)n - 1);
-    // 9-bit digits where they save a pass (150M rows: 0.85 ms a pass against
-    // 0.69 ms, each with a count of 0.20 ms; 45 bits take 5.3 ms in five passes
-    // and would take that in six as well, but the five leave room for the row
-    // id); only at the default digit width
+    // 9-bit digits where they save a pass (150M rows: 0.676 ms a pass against
+    // 0.585 ms, each with a count of 0.20 ms, so 45 bits take 4.4 ms in five
+    // passes and 4.7 ms in six); the others keep 8 or fewer.  Only at the
+    // default digit width.
     if (pl.bits == 8 && (total + 8) / 9 < pl.npass) {
         pl.npass = (total + 8) / 9;
         pl.bits = (total + pl.npass - 1) / pl.npass;
@@ -377,7 +378,7 @@ static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, c
         pl.bits = pl.bits > 8 ? 8 : pl.bits;
         pl.npass = (total + pl.bits - 1) / pl.bits;
     }
-    unsigned* counts = (unsigned*)salloc((size_t)RX_PER_SM * g_sms * RX_MAX_DIGITS * 4);
+    unsigned* counts = (unsigned*)salloc((size_t)RX_MAX_PER_SM * g_sms * RX_MAX_DIGITS * 4);
     unsigned* tot = (unsigned*)salloc((size_t)pl.npass * RX_MAX_DIGITS * 4);
     // key or record buffers, and u32 row ids where they are a result or
     // travel beside the keys; the last pass of a permutation alone writes neither
@@ -413,9 +414,11 @@ static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, c
             kin = k;
         }
     }
+    int done = 0;  // key bits sorted by the passes before
     for (int p = 0; p < pl.npass; p++) {
         const bool last = p == pl.npass - 1;
-        a.bits = total - p * pl.bits < pl.bits ? total - p * pl.bits : pl.bits;
+        a.bits = pl.bits > 8 ? (total - done + pl.npass - p - 1) / (pl.npass - p)
+                             : total - done < pl.bits ? total - done : pl.bits;
         a.mode = !last ? (fits ? RX_REC : RX_KV) : perm ? (out->keys ? RX_KV64 : RX_V64) : RX_KV;
         a.out = kb[p & 1];
         a.vout = vb[p & 1];
@@ -423,7 +426,7 @@ static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, c
         a.reverse = perm && last && out->reverse;
         unsigned* t = tot + (size_t)p * RX_MAX_DIGITS;
         if (!fits) {
-            a.kshift = pl.lo + p * pl.bits;
+            a.kshift = pl.lo + done;
             HG_CHECK(rx_pass_kv(kin, a, counts, t));
             a.vin = a.vout;
         } else if (p == 0) {
@@ -444,6 +447,7 @@ static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, c
             a.kshift += a.bits;
         }
         kin = (const unsigned long long*)kb[p & 1];
+        done += a.bits;
     }
     *kres = keep ? (const KR*)kin : nullptr;
     *vres = perm ? nullptr : vb[(pl.npass - 1) & 1];

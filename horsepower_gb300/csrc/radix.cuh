@@ -22,13 +22,15 @@
 // template parameter, so the first pass reads the columns themselves (packed
 // and range-compressed in registers) and no key array is made.
 //
-// What bounds a pass is the ALU: ranking takes eight or nine ballots a row,
-// some 40 of its 100 instructions (ncu: 0.57 instructions per cycle and
-// scheduler, DRAM 47%).  __match_any_sync, peers collected by shared-memory
-// atomics and larger tiles were all slower or even.  150M rows: a pass of
-// 8-bit digits 0.69 ms, of 9-bit digits 0.85 ms, its count 0.20 ms; @order of
-// (i64 key, i32 secondary) 11.2 -> 5.7 ms and @group of the i64 keys 6.0 ->
-// 3.8 ms against look-back and counted passes over separate keys and row ids.
+// What bounds a pass is the ranking: without it the same kernel moves 150M
+// records in 0.40 ms, with it in 0.585 (8-bit digits) and 0.676 (9 bits); the
+// ballots are half of its 70 instructions a row, and the warp's counter of a
+// digit is read and written once a row, a chain through shared memory (ncu:
+// short scoreboard 3.8 of 11.5 cycles an instruction, DRAM 51%).
+// __match_any_sync, peers or counters by shared-memory atomics and other tiles
+// were all slower or even.  A pass's count takes 0.20 ms.  150M rows: @order
+// of (i64 key, i32 secondary) 11.2 -> 5.0 ms and @group of the i64 keys 6.0 ->
+// 3.5 ms against look-back passes over separate keys and row ids.
 #pragma once
 #include "dev_common.cuh"
 
@@ -79,24 +81,41 @@ __device__ __forceinline__ unsigned rx_first_tile(unsigned ntiles, unsigned c, u
 // before is computed again instead of held in registers across a phase
 __device__ __forceinline__ void rx_forget(unsigned long long& v) { asm volatile("" : "+l"(v)); }
 
-// the lanes whose BITS-bit digit equals this lane's (every lane takes part)
+// The lanes whose BITS-bit digit equals this lane's (every lane takes part).
+// Each ballot comes from a predicate set straight from the bit, and the same
+// predicate turns the ballot round for a lane whose bit is clear: 3.5
+// instructions a bit.  With an all-ones word per bit as the mask of both, as
+// the compiler makes of the C++ form, a bit takes 5 (150M rows, 8-bit pass:
+// 0.69 ms against 0.585).
 template <int BITS>
 __device__ __forceinline__ unsigned rx_match(unsigned d) {
-    unsigned peers = 0xffffffffu;
+    unsigned same[BITS], peers = 0xffffffffu;
 #pragma unroll
-    for (int b = 0; b < BITS; b++) {
-        const unsigned bit = (unsigned)((int)(d << (31 - b)) >> 31);  // all ones when bit b is set
-        peers &= ~(__ballot_sync(0xffffffffu, bit != 0) ^ bit);
-    }
+    for (int b = 0; b < BITS; b++)
+        asm volatile(
+            "{\n.reg .pred p;\n.reg .b32 t;\n"
+            "and.b32 t, %1, %2;\nsetp.ne.u32 p, t, 0;\n"
+            "vote.sync.ballot.b32 %0, p, 0xffffffff;\n"
+            "@!p not.b32 %0, %0;\n}"
+            : "=r"(same[b]) : "r"(d), "r"(1u << b));
+#pragma unroll
+    for (int b = 0; b < BITS; b++) peers &= same[b];
     return peers;
 }
 
-// Three CTAs per SM of 16 rows per thread: with four (64 registers) the
-// records spill, and larger tiles make fewer warps (150M-row pair order, ms:
-// 4 x 16 6.7, 4 x 14 6.5, 3 x 16 5.7, 3 x 20 6.1, 2 x 24 5.6; the i64 group 7.7,
-// 7.5, 7.4, 7.7, 7.6 with its sums).
-constexpr int RX_THREADS = 256, RX_WARPS = RX_THREADS / 32, RX_PER_SM = 3, RX_MAX_DIGITS = 512;
-constexpr int RX_ITEMS = 16, RX_TILE = RX_THREADS * RX_ITEMS;
+// Eight-bit digits: three CTAs per SM of 16 rows per thread; with four (64
+// registers) the records spill and larger tiles make fewer warps.  Nine-bit
+// digits: two of 24, so that a digit's run in a tile is 12 rows instead of 8
+// and the bigger histogram's registers do not spill.  One pass over 150M
+// records, ms, 8 and 9 bits:  3 x 16 0.585 and 0.84;  3 x 12 0.63, 1.01;
+// 2 x 20 0.61, 0.71;  2 x 24 0.60, 0.676;  2 x 28 0.61, 0.71;  2 x 32 0.67,
+// 0.75;  4 x 10 0.73, 1.2.
+constexpr int RX_THREADS = 256, RX_WARPS = RX_THREADS / 32, RX_MAX_PER_SM = 3, RX_MAX_DIGITS = 512;
+template <int BITS>
+struct RxShape {
+    static constexpr int PER_SM = BITS > 8 ? 2 : RX_MAX_PER_SM, ITEMS = BITS > 8 ? 24 : 16;
+    static constexpr int TILE = RX_THREADS * ITEMS;
+};
 constexpr int RX_KV_ITEMS = 12, RX_KV_TILE = RX_THREADS * RX_KV_ITEMS;
 
 // counts[d * C + c] = rows of chunk c with digit d; tot[d] += them (tot zeroed before)
@@ -230,10 +249,10 @@ struct RxPass {
     unsigned* derr;
 };
 template <typename SRC, int BITS>
-__global__ void __launch_bounds__(RX_THREADS, RX_PER_SM) k_rx_scatter(SRC src, RxPass a) {
+__global__ void __launch_bounds__(RX_THREADS, RxShape<BITS>::PER_SM) k_rx_scatter(SRC src, RxPass a) {
     grid_entry();
     constexpr bool FIRST = !std::is_same<SRC, RxRec>::value;
-    constexpr int D = 1 << BITS;
+    constexpr int D = 1 << BITS, RX_ITEMS = RxShape<BITS>::ITEMS, RX_TILE = RxShape<BITS>::TILE;
     extern __shared__ __align__(16) unsigned char rx_smem[];
     unsigned long long* stage = reinterpret_cast<unsigned long long*>(rx_smem);  // the tile in digit order
     unsigned short* sdig = reinterpret_cast<unsigned short*>(stage + RX_TILE);   // its digits, when dropped
@@ -336,7 +355,7 @@ __global__ void __launch_bounds__(RX_THREADS, RX_PER_SM) k_rx_scatter(SRC src, R
 
 // The same for 64-bit keys that leave no room for a row id: keys and row ids
 // in two arrays.  mode: RX_KV, RX_KV64 or RX_V64.
-__global__ void __launch_bounds__(RX_THREADS, RX_PER_SM)
+__global__ void __launch_bounds__(RX_THREADS, RX_MAX_PER_SM)
 k_rx_scatter_kv(const unsigned long long* __restrict__ kin, RxPass a) {
     grid_entry();
     constexpr int D = 256, ITEMS = RX_KV_ITEMS, TILE = RX_KV_TILE;
