@@ -224,8 +224,21 @@ __global__ void k_seg_class_ids(const long long* __restrict__ starts, long long 
 // Segments of classes 0-5 in one launch.  Class c (at most P = 2^c
 // elements): the segment's elements sit in lanes 0..m-1 of warp 0 of the
 // 256-lane tile and every other lane and warp holds the identity, so the
-// tile tree reduces to the xor butterfly over the first P lanes; a warp
-// reduces 32 / P such segments in sub-warps of P lanes.
+// tile tree reduces to the xor butterfly over the first P lanes.  Here a lane
+// holds up to four of a segment's places, L = P / 4 apart (one lane a segment
+// of up to 4, eight of up to 32): the butterfly's first two steps are its own
+// and the rest go over L lanes.  What bounds the kernel is latency (segment
+// id, start, row id and value are loads one behind the other) and the FP64
+// unit, which takes a warp's instruction every 16 cycles however few lanes
+// matter: four loads in flight per lane, and 1.5 additions a segment of 17 to
+// 32 rows against 6 with one place per lane.  5.8M groups of 1 to 32 rows (18M
+// rows) of a 150M-row Zipf grouping: 0.65-0.77 ms with one place per lane,
+// 0.555-0.69 now, where the values' random sectors take 0.40 (the chip loads 41 to
+// 45 G/s of them from columns of 1 GB and more, whatever is in flight; so
+// four sets of segments at a time, or a pipeline over the four loads, gained
+// nothing).
+constexpr int SEG_LANE_ITEMS = 4;
+__host__ __device__ constexpr int seg_lanes(int c) { return c <= 2 ? 1 : (1 << c) / SEG_LANE_ITEMS; }  // L of class c
 template <typename T, typename A, int OP, bool GATHER>
 __global__ void __launch_bounds__(256) k_seg_warps(SegIO<T, A> io, const long long* __restrict__ rows,
                                                    long long nx, const long long* __restrict__ starts, long long ng,
@@ -236,14 +249,15 @@ __global__ void __launch_bounds__(256) k_seg_warps(SegIO<T, A> io, const long lo
     const T* __restrict__ src = io.src[blockIdx.y];
     A* __restrict__ out = io.out[blockIdx.y];
     __shared__ long long wfirst[7];  // first warp of each class 0-5; wfirst[6] = warps in all
-    __shared__ unsigned cfirst[6];   // first id of each class
+    __shared__ unsigned cfirst[6], ccnt[6];  // first id and number of ids of each class
     if (threadIdx.x == 0) {
         long long w = 0;
         unsigned o = 0;
         for (int c = 0; c < 6; c++) {
             wfirst[c] = w;
             cfirst[c] = o;
-            const long long per = 32 >> c;  // segments per warp
+            ccnt[c] = cnt[c];
+            const long long per = 32 / seg_lanes(c);  // segments per warp
             w += ((long long)cnt[c] + per - 1) / per;
             o += cnt[c];
         }
@@ -251,23 +265,50 @@ __global__ void __launch_bounds__(256) k_seg_warps(SegIO<T, A> io, const long lo
     }
     __syncthreads();
     const unsigned lane = lane_id();
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5), wend = wfirst[6];
     bool bad = false;
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < wfirst[6]; w += warps) {
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < wend; w += warps) {
         int c = 0;
         while (c < 5 && w >= wfirst[c + 1]) c++;
-        const int P = 1 << c;
-        const unsigned q = lane >> c, j = lane & (P - 1);
-        const long long k = (w - wfirst[c]) * (32 >> c) + q;
-        A acc = ident;
-        long long g = -1;
-        if (k < (long long)cnt[c]) {
-            g = ids[cfirst[c] + k];
-            const long long s = starts[g], e = (g + 1 < ng) ? starts[g + 1] : total;
-            if ((long long)j < e - s) acc = sop<A, OP>(ident, (A)seg_elem<T, GATHER>(src, rows, nx, s + j, bad));
+        const int lb = c <= 2 ? 0 : c - 2;  // log2 of the lanes of a segment
+        const unsigned l = lane & ((1u << lb) - 1);
+        const long long k = (w - wfirst[c]) * (32 >> lb) + (lane >> lb);
+        const bool have = k < (long long)ccnt[c];
+        const unsigned g = ids[cfirst[c] + (have ? k : 0)];  // a class without segments has no warps
+        const long long s = starts[g], e = ((long long)g + 1 < ng) ? starts[g + 1] : total;
+        const long long m = have ? e - s : 0;
+        bool in[SEG_LANE_ITEMS];
+        long long at[SEG_LANE_ITEMS];
+        T v[SEG_LANE_ITEMS];
+#pragma unroll
+        for (int q = 0; q < SEG_LANE_ITEMS; q++) {
+            at[q] = l + ((unsigned)q << lb);
+            in[q] = at[q] < m;
+            at[q] += s;
         }
-        for (int o = P >> 1; o > 0; o >>= 1) acc = sop<A, OP>(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-        if (j == 0 && g >= 0) out[g] = acc;
+        if constexpr (GATHER) {
+#pragma unroll
+            for (int q = 0; q < SEG_LANE_ITEMS; q++) at[q] = in[q] ? rows[at[q]] : 0;
+#pragma unroll
+            for (int q = 0; q < SEG_LANE_ITEMS; q++) {
+                const bool ok = at[q] >= 0 && at[q] < nx;
+                bad |= in[q] && !ok;
+                in[q] = in[q] && ok;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < SEG_LANE_ITEMS; q++) v[q] = in[q] ? src[at[q]] : T(0);
+        A x[SEG_LANE_ITEMS];
+#pragma unroll
+        for (int q = 0; q < SEG_LANE_ITEMS; q++) {
+            x[q] = ident;
+            if (in[q]) x[q] = sop<A, OP>(ident, (A)v[q]);
+        }
+        A acc = x[0];
+        if (c == 1) acc = sop<A, OP>(x[0], x[1]);
+        else if (c >= 2) acc = sop<A, OP>(sop<A, OP>(x[0], x[2]), sop<A, OP>(x[1], x[3]));
+        for (int o = (1 << lb) >> 1; o > 0; o >>= 1) acc = sop<A, OP>(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+        if (l == 0 && have) out[g] = acc;
     }
     if (bad) flag_error(derr, DERR_INDEX);
 }
@@ -834,13 +875,16 @@ static I seg_reduce(const SegIO<T, A>& io, int ncol, const long long* rows, long
     if (!li) li = &local;
     HG_CHECK(seg_plan(starts, ng, total, GATHER ? rows : nullptr, nx, li));
     const unsigned *ids = li->cls_ids, *ccnt = li->cls_cnt;
-    // One warp per 32 >> c small segments of class c and per mid-size one.
+    // One warp per 32 / seg_lanes(c) small segments of class c and per mid-size one.
     // The kernels stride over the segments, so the grid decides only how many
     // run at once: with one thread per segment (8 warps per 256 segments) 64
     // plans' ~200 mid-size segments ran on 16 warps, 0.34 ms a launch against
     // 0.02 ms now.
     long long small_w = 0;
-    for (int c = 0; c < 6; c++) small_w += (li->cls_host[c] + (32u >> c) - 1) / (32u >> c);
+    for (int c = 0; c < 6; c++) {
+        const unsigned per = 32u / seg_lanes(c);
+        small_w += (li->cls_host[c] + per - 1) / per;
+    }
     const long long mid_w = li->cls_host[6];
     const unsigned nc = (unsigned)ncol;
     if (small_w)

@@ -310,3 +310,46 @@ def test_chain_rounds(libs, n, text, typs):
     else:
         assert got == (x[0] | (x[1] < 0)).sum()
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("copies", [1, 7, 33])
+def test_small_groups(libs, copies):
+    """Groups of 1 to 33 rows, any number of each size: sums equal the fixed
+    tile tree of their rows bit for bit, min and max follow the xor butterfly's
+    operand order (which decides where NaN goes)."""
+    gpu, ora = libs
+    rng = np.random.default_rng(copies)
+    sizes = np.repeat(np.arange(1, 34), copies)
+    key = np.repeat(np.arange(sizes.size, dtype=np.int32), sizes)
+    rng.shuffle(key)
+    pay = rng.standard_normal(key.size) * 10.0 ** rng.integers(-8, 8, key.size)
+    pay[rng.random(key.size) < 0.05] = -0.0
+    nanp = np.where(rng.random(key.size) < 0.2, np.nan, pay)
+    g = gpu.call("pfnGroup", gpu.vec(key, H_I))
+    vals, keys = gpu.call("pfnValues", g), gpu.to_py(gpu.call("pfnKeys", g))
+    sums = gpu.to_py(gpu.call("hgpuGroupSum", gpu.vec(pay, H_E), vals))
+    isum = gpu.to_py(gpu.call("hgpuGroupSum", gpu.vec(key, H_I), vals))
+    lo = gpu.to_py(gpu.call("hgpuGroupMin", gpu.vec(nanp, H_E), vals))
+    hi = gpu.to_py(gpu.call("hgpuGroupMax", gpu.vec(nanp, H_E), vals))
+
+    def butterfly(x, op, ident):
+        p = 1 << max(0, (len(x) - 1).bit_length())
+        x = [op(ident, v) for v in x] + [ident] * (p - len(x))
+        while p > 1:
+            p //= 2
+            x = [op(x[j], x[j + p]) for j in range(p)]
+        return x[0]
+
+    top = np.inf
+    for gi, first in enumerate(keys):
+        rows = np.flatnonzero(key == key[first])
+        x = np.ascontiguousarray(pay[rows])
+        want = ora.lib.hgoTreeSumF64(x.ctypes.data, x.size)
+        assert sums[gi].tobytes() == np.float64(want).tobytes(), (len(rows), sums[gi], want)
+        assert isum[gi] == len(rows) * int(key[first])
+        if len(rows) <= 32:
+            for got, op, ident in ((lo[gi], lambda a, b: a if a < b else b, top),
+                                   (hi[gi], lambda a, b: a if a > b else b, -top)):
+                want = butterfly(list(nanp[rows]), op, ident)
+                assert got == want or (got != got and want != want), (len(rows), got, want)
+    gpu.free_inputs()
