@@ -357,66 +357,85 @@ __global__ void k_sg_codes(const int8_t* __restrict__ flag, const int8_t* __rest
         if (sb[i]) atomicOr(&bits[i], sb[i]);
 }
 
-// The tile preamble shared by both passes: each lane's SG_R date offsets,
-// and in lane c (c < G) the ballot of "row has group c" for each round k
-// (mygb[k]), so that a (plan, group c) count is a popc in lane c.
-__device__ __forceinline__ void sg_tile(const unsigned short* __restrict__ dd, const int8_t* __restrict__ flag,
-                                        const int8_t* __restrict__ status, const unsigned char* __restrict__ dense,
-                                        long long nf, long long base, int G, unsigned short (&d)[SG_R],
-                                        unsigned (&mygb)[SG_R], unsigned char (&g)[SG_R]) {
-    const unsigned lane = lane_id();
+// The windows' ends cut the date axis into intervals: interval i holds the
+// dates with exactly i ends at or before them, and plan pl selects the rows of
+// intervals lo[pl] .. hi[pl] - 1, bit pl of mask[i].
+struct SgWins {
+    int npl, G, nb;  // plans, groups, ends (distinct, ascending)
+    unsigned short end[2 * SG_MAXP];
+    unsigned mask[2 * SG_MAXP + 1];
+    unsigned char lo[SG_MAXP], hi[SG_MAXP];
+};
+constexpr int SG_IV = 2 * SG_MAXP + 1;
+static SgWins sg_windows(const int* lo, const int* hi, int npl, int G) {
+    SgWins w{};
+    w.npl = npl;
+    w.G = G;
+    std::vector<int> e;
+    for (int k = 0; k < npl; k++)
+        if (lo[k] < hi[k]) { e.push_back(lo[k]); e.push_back(hi[k]); }
+    std::sort(e.begin(), e.end());
+    e.erase(std::unique(e.begin(), e.end()), e.end());
+    w.nb = (int)e.size();
+    for (int i = 0; i < w.nb; i++) w.end[i] = (unsigned short)e[i];
+    for (int k = 0; k < npl; k++) {
+        if (lo[k] >= hi[k]) continue;  // lo == hi == 0: no interval
+        w.lo[k] = (unsigned char)(std::lower_bound(e.begin(), e.end(), lo[k]) - e.begin() + 1);
+        w.hi[k] = (unsigned char)(std::lower_bound(e.begin(), e.end(), hi[k]) - e.begin() + 1);
+        for (int i = w.lo[k]; i < w.hi[k]; i++) w.mask[i] |= 1u << k;
+    }
+    return w;
+}
+// iv[d] = the interval of date offset d; NO_DATE lies behind every window
+__global__ void k_sg_intervals(const __grid_constant__ SgWins wins, unsigned char* __restrict__ iv) {
+    grid_entry();
+    const unsigned d = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned n = 0;
+    for (int i = 0; i < wins.nb; i++) n += wins.end[i] <= d;
+    iv[d] = (unsigned char)n;
+}
+
+// pass 1: counts[(pl * G + g) * ntiles + t] = rows of plan pl and group g in
+// tile t, from the tile's histogram over (interval, group): the work per row
+// does not grow with the plans.  (60M rows, 19 plans, 6 groups: 0.155 ms; with
+// a ballot per plan and 32 rows 0.50 ms.)
+__global__ void __launch_bounds__(256) k_sg_count(const unsigned short* __restrict__ dd, const int8_t* __restrict__ flag,
+                                                  const int8_t* __restrict__ status,
+                                                  const unsigned char* __restrict__ dense,
+                                                  const unsigned char* __restrict__ iv, long long nf,
+                                                  const __grid_constant__ SgWins wins, unsigned* __restrict__ counts,
+                                                  long long ntiles) {
+    grid_entry();
+    __shared__ unsigned hist[SG_MAXG][SG_IV + 1];  // then, per group, the rows of all lower intervals
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5;
+    const long long t = blockIdx.x, base = t * SG_TILE + threadIdx.x;
+    for (int i = threadIdx.x; i < SG_MAXG * (SG_IV + 1); i += 256) (&hist[0][0])[i] = 0;
+    __syncthreads();
+    unsigned v[SG_R], g[SG_R];
 #pragma unroll
     for (int k = 0; k < SG_R; k++) {
-        long long i = base + k * 32 + lane;
-        d[k] = 0xffffu;
-        g[k] = 0xff;
+        const long long i = base + k * 256;
+        v[k] = g[k] = 0xffu;
         if (i < nf) {
-            d[k] = __ldcs(dd + i);
-            g[k] = __ldg(dense + (((unsigned)(uint8_t)flag[i] << 8) | (unsigned)(uint8_t)status[i]));
+            v[k] = __ldg(iv + __ldcs(dd + i));
+            g[k] = __ldg(dense + (((unsigned)(uint8_t)__ldcs(flag + i) << 8) | (unsigned)(uint8_t)__ldcs(status + i)));
         }
-        mygb[k] = 0;
     }
 #pragma unroll
     for (int k = 0; k < SG_R; k++)
-        for (int c = 0; c < G; c++) {
-            const unsigned b = __ballot_sync(0xffffffffu, g[k] == c);
-            if ((int)lane == c) mygb[k] = b;
-        }
-}
-
-// this warp's rows of every (plan, group): wc[w][pl * G + c]
-__device__ __forceinline__ void sg_warp_counts(const unsigned short (&d)[SG_R], const unsigned (&mygb)[SG_R],
-                                               const int* __restrict__ wins, int npl, int G, unsigned* wcw) {
-    const unsigned lane = lane_id();
-    for (int pl = 0; pl < npl; pl++) {
-        const int lo = wins[2 * pl], hi = wins[2 * pl + 1];
-        unsigned n = 0;
-#pragma unroll
-        for (int k = 0; k < SG_R; k++) n += __popc(__ballot_sync(0xffffffffu, (int)d[k] >= lo && (int)d[k] < hi) & mygb[k]);
-        if ((int)lane < G) wcw[pl * G + lane] = n;
-    }
-}
-
-// pass 1: counts[(pl * G + g) * ntiles + t] = rows of plan pl and group g in tile t
-__global__ void __launch_bounds__(256) k_sg_count(const unsigned short* __restrict__ dd, const int8_t* __restrict__ flag,
-                                                  const int8_t* __restrict__ status,
-                                                  const unsigned char* __restrict__ dense, long long nf,
-                                                  const int* __restrict__ wins, int npl, int G,
-                                                  unsigned* __restrict__ counts, long long ntiles) {
-    grid_entry();
-    __shared__ unsigned wc[8][SG_MAXP * SG_MAXG];
-    const unsigned w = threadIdx.x >> 5;
-    const long long t = blockIdx.x, base = t * SG_TILE + (long long)w * (32 * SG_R);
-    unsigned short d[SG_R];
-    unsigned mygb[SG_R];
-    unsigned char g[SG_R];
-    sg_tile(dd, flag, status, dense, nf, base, G, d, mygb, g);
-    sg_warp_counts(d, mygb, wins, npl, G, wc[w]);
+        if (v[k] != 0xffu) atomicAdd(&hist[g[k] & (SG_MAXG - 1)][v[k]], 1u);
     __syncthreads();
-    for (int j = threadIdx.x; j < npl * G; j += blockDim.x) {
-        unsigned n = 0;
-        for (int v = 0; v < 8; v++) n += wc[v][j];
-        counts[(long long)j * ntiles + t] = n;
+    unsigned carry = 0;
+    for (int i0 = 0; i0 < SG_IV + 1; i0 += 32) {  // warp w: group w
+        const int i = i0 + (int)lane;
+        const unsigned x = i < SG_IV + 1 ? hist[w][i] : 0u, incl = warp_incl_scan(x);
+        if (i < SG_IV + 1) hist[w][i] = carry + incl - x;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < wins.npl * wins.G; j += 256) {
+        const int pl = j / wins.G, c = j - pl * wins.G;
+        counts[(long long)j * ntiles + t] = hist[c][wins.hi[pl]] - hist[c][wins.lo[pl]];
     }
 }
 
@@ -466,27 +485,43 @@ __global__ void __launch_bounds__(1024) k_sg_scan(const unsigned* __restrict__ c
 
 // pass 2: every plan's matching rows of the tile, values written to
 // base[j] + offs[j * ntiles + t] + (rows of the same (plan, group) earlier in
-// the tile).  The tile's values, date offsets and groups are staged in shared
-// memory and each warp takes whole plans: it lists the plan's rows of the tile
-// (densely, one ballot a round), places the list in group order (row order
-// within a group) and writes the listed rows' values with consecutive lanes at
-// consecutive positions.  What bounds it is instruction issue, about 1200 a
-// plan and tile (19 windows of 365 days over 60M rows: 1.6 GB read, 4.0 GB
-// written).  Storing each round's few matching rows as they were found made
-// 500M partial-sector stores: 3.9 ms.
-constexpr int SG_LIST = 512;  // rows of one list: a quarter of the tile, so that four of them always do
+// the tile).  The tile's values are staged in shared memory while its rows are put
+// in group order (row order within a group), each with the mask of the plans
+// that select it; a 32 x 32 bit transpose turns 32 rows' masks into one word of rows per plan.  A
+// warp then takes half a tile of one plan at a time: it lists the words' rows
+// densely and writes their values with consecutive lanes at consecutive
+// positions.  (19 windows of 365 days over 60M rows: 1.6 GB read, 4.0 GB
+// written.)  What bounds it is the shared-memory pipe, 72% busy: a warp's 32
+// selected rows lie in random banks, seven wavefronts per column.  With a
+// ballot per plan and 32 rows and the groups sorted once per plan it was
+// instruction issue, 3100 a plan and tile against 1450, and 2.37 ms against
+// 1.71; storing each round's few matching rows as they were found made 500M
+// partial-sector stores, 3.9 ms.
+constexpr int SG_WORDS = (int)SG_TILE / 32;  // of 32 rows
+constexpr int SG_LIST = 512;                 // rows of one list; a half with more takes a second
 struct SgSmem {
     double q[SG_TILE], p[SG_TILE], d[SG_TILE];
-    unsigned dg[SG_TILE];                  // date offset << 16 | group
-    unsigned short a[8][SG_LIST], b[8][SG_LIST];  // row | group << 11, in row order and in group order
-    unsigned next[8][SG_MAXG];             // each group's next place in b
+    union {
+        unsigned mask[SG_TILE];           // the plans of each row, until they are transposed
+        unsigned short list[8][SG_LIST];  // per warp: rows, each with its group as in `row`
+    };
+    unsigned bits[SG_WORDS][SG_MAXP + 1];  // [word][plan]: the word's rows that the plan selects
+    unsigned long long pos[SG_MAXP * SG_MAXG];  // first position of (plan, group)
+    unsigned cnt[SG_MAXP * SG_MAXG];            // its rows in the tile
+    unsigned gw[8][SG_MAXG];               // per warp and group: rows, then the first place
+    unsigned short row[SG_TILE];           // by place in group order: row | group << 11
 };
-static_assert(SG_TILE == 4 * SG_LIST && SG_TILE <= 2048 && SG_MAXG <= 8, "packing of SgSmem's lists");
+static_assert(SG_TILE == 2048 && SG_R == 8 && SG_MAXG == 8 && SG_MAXP == 32, "the tile is 8 warps x 8 x 32 rows");
+// 8 bytes from global to shared memory, complete after cp.async.wait_all
+__device__ __forceinline__ void sg_copy8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 __global__ void __launch_bounds__(256, 3) k_sg_scatter(const unsigned short* __restrict__ dd, const int8_t* __restrict__ flag,
                                                     const int8_t* __restrict__ status,
-                                                    const unsigned char* __restrict__ dense, const double* __restrict__ qty,
+                                                    const unsigned char* __restrict__ dense,
+                                                    const unsigned char* __restrict__ iv, const double* __restrict__ qty,
                                                     const double* __restrict__ price, const double* __restrict__ disc,
-                                                    long long nf, const int* __restrict__ wins, int npl, int G,
+                                                    long long nf, const __grid_constant__ SgWins wins,
                                                     const unsigned long long* __restrict__ offs,
                                                     const unsigned long long* __restrict__ totals,
                                                     const unsigned long long* __restrict__ base, long long ntiles,
@@ -495,92 +530,124 @@ __global__ void __launch_bounds__(256, 3) k_sg_scatter(const unsigned short* __r
     grid_entry();
     extern __shared__ __align__(16) unsigned char sg_smem[];
     SgSmem& sm = *reinterpret_cast<SgSmem*>(sg_smem);
+    __shared__ unsigned imask[SG_IV];
     const unsigned lane = lane_id(), w = threadIdx.x >> 5;
-    const long long t = blockIdx.x, rbase = t * SG_TILE;
+    const long long t = blockIdx.x, rbase = t * SG_TILE + w * (32 * SG_R) + lane;
+    const int npl = wins.npl, G = wins.G;
+    unsigned v[SG_R], g[SG_R];
 #pragma unroll
     for (int k = 0; k < SG_R; k++) {
-        const int r = k * 256 + (int)threadIdx.x;
-        const long long i = rbase + r;
-        const bool ok = i < nf;
-        unsigned d = NO_DATE, g = 0;
-        if (ok) {
-            d = __ldcs(dd + i);
-            g = __ldg(dense + (((unsigned)(uint8_t)flag[i] << 8) | (unsigned)(uint8_t)status[i]));
+        const long long i = rbase + k * 32;
+        v[k] = 0;           // interval 0 is in no window
+        g[k] = SG_MAXG - 1;  // rows past the end come last
+        if (i < nf) {
+            v[k] = __ldcs(dd + i);
+            g[k] = ((unsigned)(uint8_t)__ldcs(flag + i) << 8) | (unsigned)(uint8_t)__ldcs(status + i);
         }
-        sm.q[r] = ok ? __ldcs(qty + i) : 0.0;
-        sm.p[r] = ok ? __ldcs(price + i) : 0.0;
-        sm.d[r] = ok ? __ldcs(disc + i) : 0.0;
-        sm.dg[r] = (d << 16) | (g & 7u);
+    }
+#pragma unroll
+    for (int k = 0; k < SG_R; k++) {  // the values go to shared memory by themselves
+        const long long i = rbase + k * 32;
+        const int r = (int)w * (32 * SG_R) + k * 32 + (int)lane;
+        if (i < nf) {
+            sg_copy8(&sm.q[r], qty + i);
+            sg_copy8(&sm.p[r], price + i);
+            sg_copy8(&sm.d[r], disc + i);
+        }
+    }
+    if ((int)threadIdx.x < npl * G) {
+        const long long j = threadIdx.x;
+        const unsigned long long o = offs[j * ntiles + t];
+        sm.pos[j] = base[j] + o;
+        sm.cnt[j] = (unsigned)((t + 1 < ntiles ? offs[j * ntiles + t + 1] : totals[j]) - o);
+    }
+    if (threadIdx.x < SG_IV) imask[threadIdx.x] = wins.mask[threadIdx.x];
+    if (lane < SG_MAXG) sm.gw[w][lane] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < SG_R; k++)
+        if (rbase + k * 32 < nf) {
+            v[k] = __ldg(iv + v[k]);
+            g[k] = __ldg(dense + g[k]) & (SG_MAXG - 1);
+        }
+    unsigned rank[SG_R];  // among the warp's rows of the group
+#pragma unroll
+    for (int k = 0; k < SG_R; k++) {
+        unsigned peers = 0xffffffffu;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const unsigned bal = __ballot_sync(0xffffffffu, (g[k] >> b) & 1u);
+            peers &= (g[k] >> b) & 1u ? bal : ~bal;
+        }
+        const unsigned before = __popc(peers & lanemask_lt()), pre = sm.gw[w][g[k]];
+        rank[k] = pre + before;
+        __syncwarp();
+        if (before == 0) sm.gw[w][g[k]] = pre + __popc(peers);
+        __syncwarp();
     }
     __syncthreads();
-    unsigned short *la = sm.a[w], *lb = sm.b[w];
-    unsigned* next = sm.next[w];
-    for (int pl = (int)w; pl < npl; pl += 8) {
-        const unsigned lo = (unsigned)wins[2 * pl], hi = (unsigned)wins[2 * pl + 1];
-        const unsigned span = hi > lo ? hi - lo : 0u;
-        unsigned long long pos = 0;  // lane c < G: next position of group c
-        unsigned cnt = 0;            // ... and its rows in the tile
-        if ((int)lane < G) {
-            const long long j = (long long)pl * G + (int)lane;
-            const unsigned long long o = offs[j * ntiles + t];
-            pos = base[j] + o;
-            cnt = (unsigned)((t + 1 < ntiles ? offs[j * ntiles + t + 1] : totals[j]) - o);
-        }
-        const unsigned total = warp_sum(cnt);
-        const int parts = total <= (unsigned)SG_LIST ? 1 : 4, rounds = SG_TILE / 32 / parts;
-        for (int part = 0; part < parts; part++) {
-            unsigned m = 0;
-#pragma unroll 8
-            for (int k = part * rounds; k < (part + 1) * rounds; k++) {
-                const unsigned dg = sm.dg[k * 32 + lane];
-                const bool in = (dg >> 16) - lo < span;
-                const unsigned mb = __ballot_sync(0xffffffffu, in);
-                if (in) la[m + __popc(mb & lanemask_lt())] = (unsigned short)((k * 32 + lane) | ((dg & 7u) << 11));
-                m += __popc(mb);
-            }
-            __syncwarp();
-            if (parts > 1) {  // the part's rows per group
-                cnt = 0;
-                for (unsigned i0 = 0; i0 < m; i0 += 32) {
-                    const unsigned g = i0 + lane < m ? la[i0 + lane] >> 11 : 0xffu;
-                    for (int c = 0; c < G; c++) {
-                        const unsigned b = __popc(__ballot_sync(0xffffffffu, g == (unsigned)c));
-                        if ((int)lane == c) cnt += b;
-                    }
-                }
-            }
-            const unsigned first = warp_incl_scan(cnt) - cnt;  // lane c: group c's first place in lb
-            if ((int)lane < SG_MAXG) next[lane] = first;
-            __syncwarp();
-            for (unsigned i0 = 0; i0 < m; i0 += 32) {
-                const bool ok = i0 + lane < m;
-                const unsigned e = ok ? la[i0 + lane] : 0u, g = e >> 11;
-                unsigned peers = __ballot_sync(0xffffffffu, ok);
+    if (w == 0) {  // first places: groups in order, the warps' rows of a group in order
+        unsigned c[8], sum = 0;
 #pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    const unsigned bal = __ballot_sync(0xffffffffu, (g >> b) & 1u);
-                    peers &= (g >> b) & 1u ? bal : ~bal;
-                }
-                const unsigned place = next[g] + __popc(peers & lanemask_lt());
-                __syncwarp();
-                if (ok) {
-                    lb[place] = (unsigned short)e;
-                    if (!(peers >> lane >> 1)) next[g] = place + 1;  // the group's last lane
-                }
-                __syncwarp();
-            }
-            const unsigned long long at0 = pos - first;  // list entry i of group c goes to at0 + i
-            for (unsigned i0 = 0; i0 < m; i0 += 32) {
-                const unsigned i = i0 + lane, e = i < m ? lb[i] : 0u, r = e & 2047u;
-                const unsigned long long at = __shfl_sync(0xffffffffu, at0, e >> 11) + i;
-                if (i < m) {
+        for (int x = 0; x < 8; x++) {
+            c[x] = lane < SG_MAXG ? sm.gw[x][lane] : 0u;
+            sum += c[x];
+        }
+        unsigned first = warp_incl_scan(sum) - sum;
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            if (lane < SG_MAXG) sm.gw[x][lane] = first;
+            first += c[x];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SG_R; k++) {
+        const unsigned at = sm.gw[w][g[k]] + rank[k];
+        sm.row[at] = (unsigned short)((w * (32 * SG_R) + k * 32 + lane) | (g[k] << 11));
+        sm.mask[at] = imask[v[k]];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SG_R; k++) {
+        const int word = (int)w * SG_R + k;
+        unsigned x = sm.mask[word * 32 + lane], m = 0x0000ffffu;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1, m ^= m << s) {
+            const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
+            x = lane & s ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y << s) & ~m);
+        }
+        sm.bits[word][lane] = x;  // lane pl: bit r = plan pl selects row r of the word
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // also: the masks are read, lists take their place
+    unsigned short* list = sm.list[w];
+    for (int u = (int)w; u < 2 * npl; u += 8) {
+        const int pl = u >> 1, half = u & 1;
+        const unsigned wd = sm.bits[half * 32 + lane][pl];
+        const unsigned before = half ? __reduce_add_sync(0xffffffffu, __popc(sm.bits[lane][pl])) : 0u;
+        const unsigned n = __popc(wd), incl = warp_incl_scan(n), m = __shfl_sync(0xffffffffu, incl, 31);
+        if (m == 0) continue;
+        const unsigned cnt = (int)lane < G ? sm.cnt[pl * G + lane] : 0u;
+        // the plan's i-th selected row of the tile, of group c, goes to at0 (of lane c) + i
+        const unsigned long long at0 =
+            ((int)lane < G ? sm.pos[pl * G + lane] : 0ull) - (warp_incl_scan(cnt) - cnt) + before;
+        for (unsigned l0 = 0; l0 < m; l0 += SG_LIST) {
+            unsigned i = incl - n - l0;  // wraps below l0: never under SG_LIST
+            for (unsigned b = wd; b; b &= b - 1, i++)
+                if (i < (unsigned)SG_LIST) list[i] = sm.row[half * 1024 + lane * 32 + __ffs(b) - 1];
+            __syncwarp();
+            const unsigned lm = m - l0 < (unsigned)SG_LIST ? m - l0 : (unsigned)SG_LIST;
+            for (unsigned i0 = 0; i0 < lm; i0 += 32) {
+                const unsigned k = i0 + lane, x = k < lm ? list[k] : 0u, r = x & 2047u;
+                const unsigned long long at = __shfl_sync(0xffffffffu, at0, x >> 11) + l0 + k;
+                if (k < lm) {
                     vq[at] = sm.q[r];
                     vp[at] = sm.p[r];
                     vd[at] = sm.d[r];
                 }
             }
-            pos += cnt;
-            __syncwarp();  // the lists are rewritten
+            __syncwarp();  // the list is rewritten
         }
     }
 }
@@ -963,17 +1030,16 @@ static I shared_grouped(const hgpuJoinGroupPlan* plans, const std::vector<int>& 
         ScratchScope inner;
         const int npl = (int)std::min<size_t>(SG_MAXP, ps.size() - c0);
         const int nj = npl * G;
-        std::vector<int> hw(2 * npl);
-        for (int k = 0; k < npl; k++) { hw[2 * k] = plo[c0 + k]; hw[2 * k + 1] = phi[c0 + k]; }
-        int* wins = (int*)salloc(8 * npl);
+        const SgWins wins = sg_windows(&plo[c0], &phi[c0], npl, G);
+        unsigned char* iv = (unsigned char*)salloc(65536);
         unsigned* counts = (unsigned*)salloc((size_t)nj * ntiles * 4);
         unsigned long long* offs = (unsigned long long*)salloc((size_t)nj * ntiles * 8);
         unsigned long long* totals = (unsigned long long*)salloc((size_t)nj * 8);
         unsigned long long* base = (unsigned long long*)salloc((size_t)nj * 8);
-        if (!wins || !counts || !offs || !totals || !base) return E_DEVICE_OOM;
-        HG_CU(cudaMemcpyAsync(wins, hw.data(), 8 * npl, cudaMemcpyHostToDevice, g_stream));
+        if (!iv || !counts || !offs || !totals || !base) return E_DEVICE_OOM;
+        HG_LAUNCH("sg_intervals", 256, 256, 0, k_sg_intervals, wins, iv);
         HG_LAUNCH("sg_count", (unsigned)ntiles, 256, 0, k_sg_count, dd, (const int8_t*)q0.flag,
-                  (const int8_t*)q0.status, (const unsigned char*)dense, nf, (const int*)wins, npl, G, counts, ntiles);
+                  (const int8_t*)q0.status, (const unsigned char*)dense, (const unsigned char*)iv, nf, wins, counts, ntiles);
         HG_LAUNCH("sg_scan", (unsigned)nj, 1024, 0, k_sg_scan, (const unsigned*)counts, ntiles, offs, totals);
         std::vector<unsigned long long> ht(nj), hbase(nj);
         HG_CU(cudaMemcpyAsync(ht.data(), totals, (size_t)nj * 8, cudaMemcpyDeviceToHost, g_stream));
@@ -1000,8 +1066,8 @@ static I shared_grouped(const hgpuJoinGroupPlan* plans, const std::vector<int>& 
             // the attribute belongs to the current device's context: set it on every call (a host-side write)
             HG_CU(cudaFuncSetAttribute(k_sg_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
             HG_LAUNCH("sg_scatter", (unsigned)ntiles, 256, (size_t)dsm, k_sg_scatter, dd, (const int8_t*)q0.flag,
-                      (const int8_t*)q0.status, (const unsigned char*)dense, q0.qty, q0.price, q0.disc, nf,
-                      (const int*)wins, npl, G, (const unsigned long long*)offs, (const unsigned long long*)totals,
+                      (const int8_t*)q0.status, (const unsigned char*)dense, (const unsigned char*)iv,
+                      q0.qty, q0.price, q0.disc, nf, wins, (const unsigned long long*)offs, (const unsigned long long*)totals,
                       (const unsigned long long*)base, ntiles, vq, vp, vd);
             HG_CU(cudaMemcpyAsync(st, seg_start.data(), (size_t)nseg * 8, cudaMemcpyHostToDevice, g_stream));
             const double* cols[3] = {vq, vp, vd};

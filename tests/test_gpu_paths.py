@@ -353,3 +353,26 @@ def test_small_groups(libs, copies):
                 want = butterfly(list(nanp[rows]), op, ident)
                 assert got == want or (got != got and want != want), (len(rows), got, want)
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("nplans,nfact", [(32, 30_001), (33, 5_000), (40, 120_013)])
+def test_shared_many_windows(libs, nplans, nfact):
+    """As many windows as one pass over the fact table takes, and more (random
+    ends, all distinct or shared, empty and full windows among them): each
+    plan's rows equal the same plan alone, bit for bit."""
+    from horsepower_gb300 import batch as B, data as D, plans as P
+    gpu = libs[0]
+    dim, fact = D.join_tables(nfact=nfact, ndim=max(2, nfact // 4), seed=nplans)
+    rng = np.random.default_rng(nplans)
+    ddim, dfact = B.device_tables(gpu, dim, fact)
+    ends = np.sort(rng.integers(D.DAYS0 - 5, D.DAYS0 + 2531, (nplans, 2)), axis=1)
+    ends[0], ends[1], ends[2] = (D.DAYS0, D.DAYS0 + 2526), (9000, 9000), ends[3]
+    got = B.run_batch(gpu, [B.make_plan(ddim, dfact, int(lo), int(hi)) for lo, hi in ends])
+    for (lo, hi), r in zip(ends, got):
+        sel = dim["pk"][(dim["date"] >= lo) & (dim["date"] < hi)]
+        if not np.isin(fact["fk"], sel).any():
+            assert len(r[0]) == 0
+            continue
+        for a, b in zip(r, P.join_group(gpu, ddim, dfact, int(lo), int(hi))):
+            assert np.array_equal(a, gpu.to_py(b)), (lo, hi)
+    gpu.free_inputs()
