@@ -160,6 +160,21 @@ inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size
         },
         p);
 }
+// A kernel whose blocks wait for one another: launched whole or not at all
+// (an error when the blocks do not fit the device together).
+inline cudaError_t launch_cooperative_args(const void* kern, dim3 grid, dim3 block, size_t smem, void** args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = g_stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelExC(&c, kern, args);
+}
 #define HG_LAUNCH(name, grid, block, smem, kern, ...)                     \
     do {                                                                  \
         ::hg::LaunchScope ls_(name);                                      \

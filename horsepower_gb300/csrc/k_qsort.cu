@@ -25,7 +25,8 @@
 // ranges.  Depths repeat until no range of two or more elements is left.
 //
 // The same step runs at three scales: ranges above QS_BLOCK elements together
-// in global memory (four launches a depth), ranges of up to QS_BLOCK in one
+// in global memory (all depths in one launch of resident blocks while the
+// elements fit them, else four launches a depth), ranges of up to QS_BLOCK in one
 // CTA's shared memory and ranges of up to 32 in one warp's registers, both to
 // their end without another launch.  (With every depth in global memory 114K
 // random rows took 48 depths of five launches: what bounded the call was
@@ -284,6 +285,239 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
     }
     still = warp_sum(still);
     if (lane_id() == 0 && still) atomicAdd(active, still);
+}
+
+// ---- every depth of a sort whose elements the chip's threads hold: one launch
+// Thread t of block b keeps E elements in registers, those of positions
+// b * per + k * 1024 + t (per = 1024 E), and the blocks pass the same four
+// steps as above, depth after depth, with a barrier over the grid where a step
+// reads what other blocks wrote: after the block-relative prefixes, after the
+// trade partners and after the moves.  What bounds a depth is latency, three
+// barriers and half a dozen dependent loads: 8 us, against 13 to 15 for the
+// four launches (114K random rows, 15 depths: 0.12 ms against 0.22, and no
+// host waits between).  Loads of shared arrays bypass L1 (ld.cg).  A barrier
+// that gives up ends the block with DERR_TIMEOUT; the others then give up too.
+constexpr int QD_THREADS = 1024, QD_WARPS = QD_THREADS / 32, QD_ROUND = 256, QD_MAX_BLOCKS = 256;
+struct QsDepths {
+    unsigned *lo, *hi;
+    unsigned long long* K[2];  // images and rows by position, of even and odd depths of this launch
+    unsigned* P[2];
+    unsigned long long *S, *ts;  // block-relative prefixes, the blocks' totals
+    unsigned *Lpos, *Rpos, *fin;
+    unsigned *act, *bar;  // elements left after each depth of this launch; the barrier's arrivals (all zero)
+    unsigned* done;       // depths run, then elements left
+    unsigned long long* KL;
+    unsigned* PL;
+    QsLists lists;
+    unsigned* derr;
+    unsigned n, level, maxd;
+};
+__device__ __forceinline__ bool qd_barrier(unsigned* bar, unsigned& target, unsigned* derr) {
+    __shared__ bool ok;
+    target += gridDim.x;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ok = true;
+        atomicAdd(bar, 1u);
+        long long spins = 0;
+        unsigned v;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if (v >= target) break;
+            if (++spins > SPIN_LIMIT) { flag_error(derr, DERR_TIMEOUT); ok = false; break; }
+        }
+    }
+    __syncthreads();
+    return ok;
+}
+template <int E>
+__global__ void __launch_bounds__(QD_THREADS, 1) k_qs_depths(const __grid_constant__ QsDepths a) {
+    grid_entry();
+    constexpr int SHIFT = E == 2 ? 11 : 12;
+    static_assert(1 << SHIFT == QD_THREADS * E, "positions of a block");
+    __shared__ unsigned long long wsum[E * QD_WARPS];    // per round and warp: the flag pairs before it in the block
+    __shared__ unsigned long long pre[QD_MAX_BLOCKS + 1];  // the flag pairs before each block; [gridDim.x]: all
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5, C = gridDim.x, n = a.n;
+    const unsigned base = (blockIdx.x << SHIFT) + threadIdx.x;
+    unsigned lo[E], hi[E], row[E], target = 0;
+    unsigned long long key[E];
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        const unsigned p = base + k * QD_THREADS;
+        lo[k] = QS_DONE;
+        hi[k] = row[k] = 0;
+        key[k] = 0;
+        if (p < n) {
+            lo[k] = a.lo[p];
+            if (lo[k] != QS_DONE) {
+                hi[k] = a.hi[p];
+                key[k] = a.K[0][p];
+                row[k] = a.P[0][p];
+            }
+        }
+    }
+    unsigned d = 0, left = 0;
+    while (d < a.maxd) {
+        const unsigned long long* K = a.K[d & 1];
+        const unsigned* P = a.P[d & 1];
+        unsigned long long rel[E], kp[E];
+        int c[E];
+#pragma unroll
+        for (int k = 0; k < E; k++) kp[k] = lo[k] != QS_DONE ? __ldcg(K + lo[k]) : 0;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const bool in = lo[k] != QS_DONE && lo[k] != base + k * QD_THREADS;
+            c[k] = qs_cmp(key[k], kp[k]);
+            const unsigned le = __ballot_sync(0xffffffffu, in && c[k] <= 0), lt = __ballot_sync(0xffffffffu, in && c[k] < 0);
+            rel[k] = (unsigned long long)__popc(le & lanemask_lt()) | ((unsigned long long)__popc(lt & lanemask_lt()) << 32);
+            if (lane == 0) wsum[k * QD_WARPS + w] = (unsigned long long)__popc(le) | ((unsigned long long)__popc(lt) << 32);
+        }
+        __syncthreads();
+        if (w == 0) {
+            unsigned long long v[E], sum = 0;
+#pragma unroll
+            for (int q = 0; q < E; q++) {
+                v[q] = wsum[lane * E + q];
+                sum += v[q];
+            }
+            unsigned long long off = warp_incl_scan64(sum);
+            if (lane == 31) a.ts[blockIdx.x] = off;
+            off -= sum;
+#pragma unroll
+            for (int q = 0; q < E; q++) {
+                wsum[lane * E + q] = off;
+                off += v[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const unsigned p = base + k * QD_THREADS;
+            rel[k] += wsum[k * QD_WARPS + w];
+            if (p < n) a.S[p] = rel[k];  // of finished positions too: a range may end at one
+        }
+        if (!qd_barrier(a.bar, target, a.derr)) return;
+        if (w == 0) {
+            constexpr int PER = QD_MAX_BLOCKS / 32;
+            unsigned long long v[PER], sum = 0;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const unsigned b = lane * PER + q;
+                v[q] = b < C ? __ldcg(a.ts + b) : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < PER; q++) sum += v[q];
+            unsigned long long off = warp_incl_scan64(sum) - sum;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                pre[lane * PER + q] = off;
+                off += v[q];
+            }
+            if (lane == 31) pre[QD_MAX_BLOCKS] = off;
+        }
+        __syncthreads();
+        auto prefix = [&](unsigned x) { return x >= n ? pre[C] : __ldcg(a.S + x) + pre[x >> SHIFT]; };
+        unsigned long long sl[E], sh[E];
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const bool on = lo[k] != QS_DONE;
+            rel[k] += pre[blockIdx.x];
+            sl[k] = on ? prefix(lo[k]) : 0;
+            sh[k] = on ? prefix(hi[k]) : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const unsigned l = lo[k], p = base + k * QD_THREADS;
+            if (l == QS_DONE || l == p) continue;
+            const unsigned le_p = qs_le(rel[k]);
+            const long long j = (long long)l + (qs_le(sh[k]) - qs_le(sl[k]));
+            long long slot = -1;
+            unsigned* dst = nullptr;
+            if (p <= j && c[k] > 0) { slot = (long long)l + (long long)(p - l - 1) - (long long)(le_p - qs_le(sl[k])); dst = a.Lpos; }
+            else if (p > j && c[k] <= 0) { slot = (long long)l + (long long)qs_le(sh[k]) - (long long)le_p - 1; dst = a.Rpos; }
+            if (!dst) continue;
+            if (slot >= (long long)l && slot < (long long)hi[k]) dst[slot] = p;
+            else flag_error(a.derr, DERR_INDEX);
+        }
+        if (!qd_barrier(a.bar, target, a.derr)) return;
+        unsigned still = 0;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const unsigned l = lo[k], p = base + k * QD_THREADS, h = hi[k];
+            if (l == QS_DONE) continue;
+            const unsigned cle = qs_le(sh[k]) - qs_le(sl[k]);
+            const long long j = (long long)l + cle;
+            if (cle == h - l - 1 && qs_lt(sh[k]) == qs_lt(sl[k])) {  // leftSame: every element equals the pivot
+                a.fin[p] = row[k];
+                lo[k] = QS_DONE;
+                continue;
+            }
+            auto left_slot = [&](long long x, unsigned le_x) { return (long long)l + (x - l - 1) - (long long)(le_x - qs_le(sl[k])); };
+            long long q = p, slot = -1;
+            const unsigned* from = nullptr;
+            if (p == l) {
+                q = j;
+                if (j > (long long)l && qs_cmp(__ldcg(K + j), kp[k]) > 0) {
+                    slot = left_slot(j, qs_le(prefix((unsigned)j)));
+                    from = a.Rpos;
+                }
+            } else if (p == j) {
+                q = l;
+            } else if (p < j && c[k] > 0) {
+                slot = left_slot(p, qs_le(rel[k]));
+                from = a.Rpos;
+            } else if (p > j && c[k] <= 0) {
+                slot = (long long)l + (long long)qs_le(sh[k]) - (long long)qs_le(rel[k]) - 1;
+                from = a.Lpos;
+            }
+            if (from) {
+                if (slot >= (long long)l && slot < (long long)h) q = __ldcg(from + slot);
+                else { flag_error(a.derr, DERR_INDEX); q = p; }
+            }
+            if (q < (long long)l || q >= (long long)h) { flag_error(a.derr, DERR_INDEX); q = p; }
+            if (q != (long long)p) {
+                row[k] = __ldcg(P + q);
+                key[k] = __ldcg(K + q);
+            }
+            unsigned nl = l, nh = (unsigned)j;
+            if (p >= j) { nl = (unsigned)j + 1; nh = h; }
+            if (p == j || nh - nl < 2) {
+                a.fin[p] = row[k];
+                lo[k] = QS_DONE;
+            } else if (nh - nl <= (unsigned)QS_BLOCK) {
+                a.PL[p] = row[k];
+                a.KL[p] = key[k];
+                lo[k] = QS_DONE;
+                if (p == nl) qs_list(a.lists, nl, nh, a.level + d + 1, 1);
+            } else {
+                a.P[(d & 1) ^ 1][p] = row[k];
+                a.K[(d & 1) ^ 1][p] = key[k];
+                lo[k] = nl;
+                hi[k] = nh;
+                still++;
+            }
+        }
+        still = warp_sum(still);
+        if (lane == 0 && still) atomicAdd(a.act + d, still);
+        if (!qd_barrier(a.bar, target, a.derr)) return;
+        left = __ldcg(a.act + d);
+        d++;
+        if (left == 0) break;
+    }
+    if (left)
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const unsigned p = base + k * QD_THREADS;
+            if (p < n) {
+                a.lo[p] = lo[k];
+                a.hi[p] = hi[k];
+            }
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.done[0] = d;
+        a.done[1] = left;
+    }
 }
 
 // ---- one warp's range: m <= 32 elements, element i in lane i (key k, row p).
@@ -683,6 +917,24 @@ static I qs_nan_check(const QsCounters& h) {
     return 0;
 }
 
+// Launches k_qs_depths when n elements fit one block per SM of at most 4 per
+// thread; false when they do not, or the device does not take the blocks
+// together.  @order of random f64 keys, us, with four launches a depth and
+// with this: 6000 rows 182 and 162, 20K 225 and 191, 114K 351 and 287, 300K 407
+// and 326, 600K 635 and 511; with 8 per thread (the registers spill) 600K 767,
+// 1.2M 1064 against 1045.
+static bool qs_depths_launch(long long n, QsDepths& q) {
+    void* args[] = {&q};
+    const long long most = (long long)(g_sms < QD_MAX_BLOCKS ? g_sms : QD_MAX_BLOCKS) * QD_THREADS;
+    const int e = n <= 2 * most ? 2 : 4;
+    if (n > e * most) return false;
+    const void* kern = e == 2 ? (const void*)k_qs_depths<2> : (const void*)k_qs_depths<4>;
+    LaunchScope ls("qs_depths");
+    if (launch_cooperative_args(kern, grid_for(n, QD_THREADS * e), QD_THREADS, 0, args) == cudaSuccess) return true;
+    cudaGetLastError();  // clears the refused launch's own error
+    return false;
+}
+
 // The quicksort of every sorted range at once.  perm/img: the elements in
 // their current order (consumed); lists/h: the ranges listed so far and their
 // counters as the host has read them; seg, starts, mode: the segments, for
@@ -706,10 +958,10 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
         unsigned* P2 = (unsigned*)salloc((size_t)n * 4);
         unsigned long long* K2 = (unsigned long long*)salloc((size_t)n * 8);
         unsigned long long* S = (unsigned long long*)salloc((size_t)(n + 1) * 8);
-        unsigned long long* ts = (unsigned long long*)salloc((size_t)nt * 8);
+        unsigned long long* ts = (unsigned long long*)salloc((size_t)(nt > QD_MAX_BLOCKS ? nt : QD_MAX_BLOCKS) * 8);
         unsigned* Lpos = (unsigned*)salloc((size_t)n * 4);
         unsigned* Rpos = (unsigned*)salloc((size_t)n * 4);
-        unsigned* act = (unsigned*)salloc(QS_MAX_ROUND * 4);
+        unsigned* act = (unsigned*)salloc((QD_ROUND + 3) * 4);  // counts, then k_qs_depths' barrier and result
         KL = (unsigned long long*)salloc((size_t)n * 8);
         PL = (unsigned*)salloc((size_t)n * 4);
         if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos || !act || !KL || !PL) return E_DEVICE_OOM;
@@ -718,8 +970,35 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
         unsigned* Pc = perm;
         unsigned long long* Kc = img;
         int round = qs_first_round(n);
+        bool resident = true;  // k_qs_depths takes the depths, while the elements fit the chip's threads
         for (long long level = 0;; level += round, round = QS_ROUND) {
             if (level >= max_levels) return qs_too_deep(max_levels);
+            if (resident) {
+                round = (int)(max_levels - level < QD_ROUND ? max_levels - level : QD_ROUND);
+                HG_CU(cudaMemsetAsync(act, 0, (QD_ROUND + 3) * 4, g_stream));
+                QsDepths q{lo, hi, {Kc, Kc == img ? K2 : img}, {Pc, Pc == perm ? P2 : perm}, S, ts, Lpos, Rpos, fin,
+                           act, act + QD_ROUND, act + QD_ROUND + 1, KL, PL, lists, g_derr, (unsigned)n, (unsigned)level,
+                           (unsigned)round};
+                resident = qs_depths_launch(n, q);
+                if (resident) {
+                    unsigned res[2];
+                    HG_CHECK(rb_queue(res, q.done, 8));
+                    HG_CHECK(rb_queue(h, lists.cnt, sizeof *h));
+                    HG_CU(stream_sync());
+                    if (res[0] == 0) {  // a barrier gave up
+                        HG_CHECK(check_device_errors());
+                        return set_error(E_DEVICE, "the quicksort's grid barrier did not complete");
+                    }
+                    if (res[1] == 0) break;
+                    if (res[0] & 1) {
+                        Kc = q.K[1];
+                        Pc = q.P[1];
+                    }
+                    round = (int)res[0];
+                    continue;
+                }
+                round = level == 0 ? qs_first_round(n) : QS_ROUND;
+            }
             if (level + round > max_levels) round = (int)(max_levels - level);
             HG_CU(cudaMemsetAsync(act, 0, QS_MAX_ROUND * 4, g_stream));
             for (int d = 0; d < round; d++) {

@@ -376,3 +376,25 @@ def test_shared_many_windows(libs, nplans, nfact):
         for a, b in zip(r, P.join_group(gpu, ddim, dfact, int(lo), int(hi))):
             assert np.array_equal(a, gpu.to_py(b)), (lo, hi)
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("n,kind", [
+    (4097, "random"), (65_536, "few"), (311_296, "random"), (311_297, "few"), (622_592, "random"), (622_593, "random"),
+    (5_000, "sorted"), (9_000, "organ"),                         # deeper than one launch runs
+])
+def test_quicksort_depths(libs, n, kind):
+    """Quicksort orders whose partitions above one CTA's size run in one launch
+    of resident blocks (two or four elements a thread, or past them with four
+    launches a depth), and recursions deeper than a launch: the reference's
+    order of equal keys, both directions."""
+    gpu, ora = libs
+    rng = np.random.default_rng(n)
+    x = {"random": lambda: rng.standard_normal(n), "few": lambda: rng.integers(0, 40, n) / 8.0,
+         "sorted": lambda: np.arange(n) / 3.0, "organ": lambda: np.minimum(np.arange(n), n - np.arange(n)) * 1.0}[kind]()
+    for up in (True, False):
+        d = np.array([up])
+        a = gpu.to_py(gpu.call("pfnOrderBy", gpu.vec(x, H_E), gpu.vec(d, H_B)))
+        b = ora.to_py(ora.call("pfnOrderBy", ora.vec(x, H_E), ora.vec(d, H_B)))
+        assert np.array_equal(a, b), up
+    gpu.free_inputs()
+    ora.free_inputs()
