@@ -45,7 +45,10 @@ enum : unsigned {
 extern unsigned* g_derr;   // device word
 // words behind it in the same zeroed 256 bytes: counters that a kernel leaves
 // at zero for the next launch
-enum { DW_CHAIN = 32 };    // blocks of a fused reduction that have finished
+enum {
+    DW_CHAIN = 32,  // blocks of a fused reduction that have finished
+    DW_STATS = 33,  // blocks of k_key_stats that have finished
+};
 I check_device_errors();   // syncs, reads and clears g_derr, maps to E_* codes
 // iteration limit for every device-side spin-wait
 constexpr long long SPIN_LIMIT = 1LL << 24;

@@ -398,3 +398,25 @@ def test_quicksort_depths(libs, n, kind):
         assert np.array_equal(a, b), up
     gpu.free_inputs()
     ora.free_inputs()
+
+
+@pytest.mark.parametrize("n", [4096, 5000, 300_001])
+@pytest.mark.parametrize("lo,hi,mul", [(-70_000, -1, 1), (-70_000, 70_000, 1), (0, 70_000, 1 << 12), (1 << 30, (1 << 30) + 9, 1),
+                                       (-1, 1, 1 << 31), (5, 6, 1)])
+def test_group_key_stats(libs, n, lo, hi, mul):
+    """@group of i32 and i64 keys whose varying bits come with their range:
+    negative, mixed signs, constant low bits, constant bits inside, one value.
+    Keys and row lists are those of the stable sort of the reference's order."""
+    gpu, ora = libs
+    rng = np.random.default_rng(n)
+    for typ in (H_I, H_L):
+        key = rng.integers(lo, hi, n) * mul
+        if typ == H_I:
+            key = key.astype(np.int32).astype(np.int64)
+        key = key.astype(DTYPE[typ])
+        a, b = gpu.call("pfnGroup", gpu.vec(key, typ)), ora.call("pfnGroup", ora.vec(key, typ))
+        assert np.array_equal(gpu.to_py(gpu.call("pfnKeys", a)), ora.to_py(ora.call("pfnKeys", b))), typ
+        for x, y in zip(gpu.to_py(gpu.call("pfnValues", a)), ora.to_py(ora.call("pfnValues", b))):
+            assert np.array_equal(x, y)
+        gpu.free_inputs()
+        ora.free_inputs()
