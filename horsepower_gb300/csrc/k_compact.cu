@@ -9,10 +9,10 @@
 //
 // GB300 kernels: a tile is 4096 rows handled by 8 warps; each lane reads its
 // 16 mask bytes with one 128-bit load and counts them with popc.  A count
-// pass writes the tiles' counts, one block scans them, and a scatter pass
-// re-reads the mask (1 byte a row) and writes each tile's selected rows from
-// its offset: each warp walks its 512 rows in rounds of 32, and selected
-// lanes write to consecutive positions found with ballot/popc.  Values are
+// pass writes the tiles' counts, one block scans them (or, of few tiles, each
+// sums those before its own), and a scatter pass re-reads the mask (1 byte a
+// row) and writes each tile's selected rows from its offset: each warp walks
+// its 512 rows in rounds of 32, and selected lanes write to consecutive positions found with ballot/popc.  Values are
 // only read for selected rows, so a sparse mask reads a fraction of the
 // value column.
 #include "dev_common.cuh"
@@ -124,6 +124,37 @@ I scan_counts(const unsigned* counts, long long n, unsigned long long* offs) {
     return last_launch_error();
 }
 
+// A tile's offset: from the scanned counts, or (offs null) the sum of the
+// counts before it, found by the tile's own block, whose last one then writes
+// the total.  Up to CT_DIRECT tiles that costs less than the scan's launch
+// (two selections of a call, with and without the scan: of 60K rows 112 and
+// 102 us, of 6M rows 136 and 132); the reads grow with the square of the
+// tiles, 8.4 MB of L2 at the line.
+constexpr long long CT_DIRECT = 2048;
+struct CompactOffs {
+    const unsigned* counts;
+    const unsigned long long* offs;
+    unsigned long long* total;
+};
+__device__ __forceinline__ unsigned long long compact_offset(const CompactOffs& o) {
+    if (o.offs) return o.offs[blockIdx.x];
+    __shared__ unsigned ws[CT_THREADS / 32];
+    unsigned s = 0;
+#pragma unroll
+    for (int k = 0; k < CT_DIRECT / CT_THREADS; k++) {
+        const unsigned t = k * CT_THREADS + threadIdx.x;
+        s += t < blockIdx.x ? o.counts[t] : 0u;
+    }
+    s = warp_sum(s);
+    if (lane_id() == 0) ws[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0;
+#pragma unroll
+    for (int w = 0; w < CT_THREADS / 32; w++) s += ws[w];
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *o.total = s + o.counts[blockIdx.x];
+    return s;
+}
+
 // pass 2: each tile writes its selected rows from its known offset; each warp
 // walks its 512 rows in rounds of 32 and selected lanes write to consecutive
 // positions found with ballot/popc
@@ -152,8 +183,7 @@ __device__ __forceinline__ void scatter_col(const void* __restrict__ src, void* 
 }
 
 __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter(const uint8_t* __restrict__ mask, long long n,
-                                                                CompactCols cols,
-                                                                const unsigned long long* __restrict__ offs) {
+                                                                CompactCols cols, CompactOffs offs) {
     grid_entry();
     __shared__ __align__(16) uint8_t smask[CT_TILE];
     __shared__ unsigned warp_tot[8];
@@ -164,8 +194,8 @@ __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter(const uint8_t* _
     *reinterpret_cast<uint4*>(smask + lofs) = m4;
     unsigned c = warp_sum(__popc(m4.x) + __popc(m4.y) + __popc(m4.z) + __popc(m4.w));
     if (lane == 0) warp_tot[warp] = c;
+    unsigned long long off = compact_offset(offs);
     __syncthreads();
-    unsigned long long off = offs[blockIdx.x];
     for (unsigned w = 0; w < warp; w++) off += warp_tot[w];
     const int wbase = (int)warp * 512;
     unsigned selbits = 0;  // bit k: row wbase + 32 k + lane is selected
@@ -191,7 +221,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter(const uint8_t* _
 template <int ES>
 __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter1(const uint8_t* __restrict__ mask, long long n,
                                                                  const void* __restrict__ src, void* __restrict__ dst,
-                                                                 const unsigned long long* __restrict__ offs) {
+                                                                 CompactOffs offs) {
     grid_entry();
     using E = typename std::conditional<ES == 1, uint8_t,
               typename std::conditional<ES == 2, uint16_t,
@@ -206,6 +236,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter1(const uint8_t* 
     *reinterpret_cast<uint4*>(smask + lofs) = m4;
     unsigned c = warp_sum(__popc(m4.x) + __popc(m4.y) + __popc(m4.z) + __popc(m4.w));
     if (lane == 0) warp_tot[warp] = c;
+    const unsigned long long first = compact_offset(offs);
     __syncthreads();
     unsigned loc = 0, total = 0;
     for (unsigned w = 0; w < 8; w++) {
@@ -226,12 +257,12 @@ __global__ void __launch_bounds__(CT_THREADS) k_compact_scatter1(const uint8_t* 
         loc += __popc(bal);
     }
     __syncthreads();
-    E* out = reinterpret_cast<E*>(dst) + offs[blockIdx.x];
+    E* out = reinterpret_cast<E*>(dst) + first;
     for (unsigned k = threadIdx.x; k < total; k += CT_THREADS) out[k] = sbuf[k];
 }
 
 // Compaction in two passes with no dependence between tiles: count per
-// tile, scan the counts, scatter.  (A single pass with a decoupled look-back
+// tile, scan the counts where they are many, scatter.  (A single pass with a decoupled look-back
 // across tiles measured several times slower here: the tiles waited on the
 // look-back chain rather than on memory.)  *count receives the number of
 // selected rows.
@@ -242,11 +273,13 @@ static I compact(const uint8_t* mask, long long n, CompactCols& cols, long long*
     unsigned long long* offs = (unsigned long long*)salloc((ntiles + 1) * 8);
     if (!counts || !offs) return E_DEVICE_OOM;
     HG_LAUNCH("compact_count", (unsigned)ntiles, CT_THREADS, 0, k_compact_count, mask, n, counts);
-    HG_LAUNCH("compact_scan", 1, 1024, 0, k_scan_counts, counts, ntiles, offs);
+    const bool scan = ntiles > CT_DIRECT;
+    if (scan) HG_LAUNCH("compact_scan", 1, 1024, 0, k_scan_counts, counts, ntiles, offs);
+    const CompactOffs co{counts, scan ? offs : nullptr, offs + ntiles};
     if (cols.ncol == 1 && cols.es[0] == 0) {  // @where: staged row numbers (measured 0.094 -> 0.074 ms at 60M)
-        HG_LAUNCH("compact", (unsigned)ntiles, CT_THREADS, 0, k_compact_scatter1<0>, mask, n, cols.src[0], cols.dst[0], offs);
+        HG_LAUNCH("compact", (unsigned)ntiles, CT_THREADS, 0, k_compact_scatter1<0>, mask, n, cols.src[0], cols.dst[0], co);
     } else {  // value columns: direct stores measured faster than staging for 8-byte values
-        HG_LAUNCH("compact", (unsigned)ntiles, CT_THREADS, 0, k_compact_scatter, mask, n, cols, offs);
+        HG_LAUNCH("compact", (unsigned)ntiles, CT_THREADS, 0, k_compact_scatter, mask, n, cols, co);
     }
     HG_CHECK(last_launch_error());
     unsigned long long h = 0;

@@ -420,3 +420,20 @@ def test_group_key_stats(libs, n, lo, hi, mul):
             assert np.array_equal(x, y)
         gpu.free_inputs()
         ora.free_inputs()
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 255, 257, 2047, 2048, 2049])
+@pytest.mark.parametrize("cut", [0, 1, 4095])
+def test_compact_offsets(libs, tiles, cut):
+    """@where and @compress with as many tiles as find their offsets
+    themselves, and more: against numpy, rows selected up to the last."""
+    gpu = libs[0]
+    n = tiles * 4096 - cut
+    rng = np.random.default_rng(tiles + cut)
+    m = rng.random(n) < 0.01
+    m[-1] = True
+    v = np.arange(n, dtype=np.int16)
+    dm = gpu.vec(m, H_B)
+    assert np.array_equal(gpu.to_py(gpu.call("pfnWhere", dm)), np.flatnonzero(m))
+    assert np.array_equal(gpu.to_py(gpu.call("pfnCompress", dm, gpu.vec(v, H_H))), v[m])
+    gpu.free_inputs()
