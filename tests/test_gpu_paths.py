@@ -437,3 +437,28 @@ def test_compact_offsets(libs, tiles, cut):
     assert np.array_equal(gpu.to_py(gpu.call("pfnWhere", dm)), np.flatnonzero(m))
     assert np.array_equal(gpu.to_py(gpu.call("pfnCompress", dm, gpu.vec(v, H_H))), v[m])
     gpu.free_inputs()
+
+
+def test_topk_sizes(libs):
+    """Top-k requests with 1 to more than 4096 candidates (one CTA sorts up to
+    4096; ties on the key, the second column and the row), negative keys and
+    second columns: the first rows of the stable order."""
+    from horsepower_gb300 import batch as B, data as D, serve as S
+    gpu = libs[0]
+    rng = np.random.default_rng(5)
+    counts = [1, 2, 3, 31, 33, 999, 1000, 1001, 2047, 2048, 2049, 4095, 4096, 4097, 9000]
+    key = np.repeat(np.arange(len(counts), dtype=np.int64) * 3 - 20, counts)
+    sec = rng.choice(np.array([-2 ** 31, -7, 0, 5, 2 ** 31 - 1]), key.size).astype(np.int32)
+    p = rng.permutation(key.size)
+    key, sec = key[p], sec[p]
+    line = S.line_table(gpu, 5000, seed=1)
+    dim, fact = B.device_tables(gpu, *D.join_tables(nfact=300, ndim=70, seed=3))
+    srv = S.Server(gpu, line, dim, fact, dict(key=B.to_device(gpu, key, H_L), sec=B.to_device(gpu, sec, H_I)), budget=1 << 30)
+    reqs = [S.Request(S.TOPK_ORDER, 0, 0, int(k), int(k) + w, 0.0) for k in np.unique(key) for w in (1, 4, 100)]
+    got, _, _ = srv.run(reqs)
+    for r, v in zip(reqs, got):
+        rows = np.flatnonzero((key >= r.klo) & (key < r.khi))
+        want = rows[np.lexsort((rows, sec[rows], key[rows]))][: S.TOPK]
+        assert np.array_equal(v, want), (r.klo, r.khi)
+    srv.close()
+    gpu.free_inputs()
