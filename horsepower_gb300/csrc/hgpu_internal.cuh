@@ -63,6 +63,10 @@ cudaError_t stream_sync();
 constexpr int RB_ITEMS = 8;
 constexpr unsigned RB_BYTES = 16384;
 I rb_queue(void* host_dst, const void* dev, size_t bytes);
+// the same for any number of values of any size (larger ones by copies into
+// pinned staging, delivered by the same wait)
+constexpr size_t RB_STAGE = 512 * 1024;
+I rb_fetch(void* host_dst, const void* dev, size_t bytes);
 cudaError_t rb_init();
 extern int g_sms;
 I ensure_init();

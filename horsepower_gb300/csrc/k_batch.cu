@@ -1012,7 +1012,7 @@ static I shared_grouped(const hgpuJoinGroupPlan* plans, const std::vector<int>& 
     if (gr > (unsigned)g_sms * 4) gr = g_sms * 4;
     HG_LAUNCH("sg_codes", gr, 256, 0, k_sg_codes, (const int8_t*)q0.flag, (const int8_t*)q0.status, nf, bits);
     std::vector<unsigned> hb(2048);
-    HG_CU(cudaMemcpyAsync(hb.data(), bits, 2048 * 4, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(hb.data(), bits, 2048 * 4));
     HG_CHECK(check_device_errors());
     std::vector<unsigned char> hd(65536, 0xff);
     std::vector<unsigned> code_of;
@@ -1042,7 +1042,7 @@ static I shared_grouped(const hgpuJoinGroupPlan* plans, const std::vector<int>& 
                   (const int8_t*)q0.status, (const unsigned char*)dense, (const unsigned char*)iv, nf, wins, counts, ntiles);
         HG_LAUNCH("sg_scan", (unsigned)nj, 1024, 0, k_sg_scan, (const unsigned*)counts, ntiles, offs, totals);
         std::vector<unsigned long long> ht(nj), hbase(nj);
-        HG_CU(cudaMemcpyAsync(ht.data(), totals, (size_t)nj * 8, cudaMemcpyDeviceToHost, g_stream));
+        HG_CHECK(rb_fetch(ht.data(), totals, (size_t)nj * 8));
         HG_CHECK(check_device_errors());
         // each plan's groups in ascending code order, plans one after another
         unsigned long long tot = 0;
@@ -1077,7 +1077,7 @@ static I shared_grouped(const hgpuJoinGroupPlan* plans, const std::vector<int>& 
                       (const long long*)st, nseg, (long long)tot, res + nseg);
         }
         std::vector<double> hr((size_t)(nseg ? nseg : 1) * 3);
-        if (nseg > 0) HG_CU(cudaMemcpyAsync(hr.data(), res, (size_t)nseg * 3 * 8, cudaMemcpyDeviceToHost, g_stream));
+        if (nseg > 0) HG_CHECK(rb_fetch(hr.data(), res, (size_t)nseg * 3 * 8));
         HG_CHECK(check_device_errors());
         for (int k = 0; k < npl; k++) {
             hgpuJoinGroupResult& r = out[ps[c0 + k]];
@@ -1136,7 +1136,7 @@ static I shared_probe(const hgpuJoinGroupPlan* plans, int np, std::vector<char>*
         HG_LAUNCH("sh_minmax", gr, 256, 0, k_sh_minmax, q.dim_pk, q.dim_date, q.ndim, mm + 4 * g);
     }
     std::vector<long long> hmm(4 * ng);
-    HG_CU(cudaMemcpyAsync(hmm.data(), mm, (size_t)ng * 32, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(hmm.data(), mm, (size_t)ng * 32));
     HG_CU(stream_sync());
     struct Built { int g; long long kmin; unsigned long long kspan; int dmin, drange; unsigned* dimhist; unsigned* facthist;
                    unsigned* dup; unsigned short* dd; };
@@ -1169,7 +1169,7 @@ static I shared_probe(const hgpuJoinGroupPlan* plans, int np, std::vector<char>*
     if (built.empty()) return 0;
     for (Built& b : built) {
         std::vector<unsigned> h((size_t)b.drange * 2 + 1);
-        HG_CU(cudaMemcpyAsync(h.data(), b.dimhist, ((size_t)b.drange * 2 + 1) * 4, cudaMemcpyDeviceToHost, g_stream));
+        HG_CHECK(rb_fetch(h.data(), b.dimhist, ((size_t)b.drange * 2 + 1) * 4));
         HG_CHECK(check_device_errors());
         std::vector<unsigned long long> cd(b.drange + 1, 0), cf(b.drange + 1, 0);
         for (int i = 0; i < b.drange; i++) {
@@ -1270,7 +1270,7 @@ extern "C" I hgpuBatchJoinGroup(const hgpuJoinGroupPlan* plans, L nplans, hgpuJo
     HG_CU(cudaMemsetAsync(dup, 0, np * 4, g_stream));
     if (dtiles[np] > 0) HG_LAUNCH("b_minmax", (unsigned)dtiles[np], 256, 0, k_b_minmax, dP, dT, np, mm);
     std::vector<long long> hmm(2 * np);
-    HG_CU(cudaMemcpyAsync(hmm.data(), mm, np * 16, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(hmm.data(), mm, np * 16));
     HG_CU(stream_sync());
     // presence bitmaps and code tables
     long long bm_words = 0;
@@ -1370,11 +1370,11 @@ extern "C" I hgpuBatchJoinGroup(const hgpuJoinGroupPlan* plans, L nplans, hgpuJo
     HG_LAUNCH("b_offsets", 1, 32, 0, k_b_offsets, mcount, np, moff);
     // gather (over the fact tile map: a plan has at most as many matches as rows)
     std::vector<unsigned long long> hm(np);
-    HG_CU(cudaMemcpyAsync(hm.data(), mcount, np * 8, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(hm.data(), mcount, np * 8));
     std::vector<unsigned> hdup(np);
     std::vector<unsigned long long> hsel(np);
-    HG_CU(cudaMemcpyAsync(hdup.data(), dup, np * 4, cudaMemcpyDeviceToHost, g_stream));
-    HG_CU(cudaMemcpyAsync(hsel.data(), nsel, np * 8, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(hdup.data(), dup, np * 4));
+    HG_CHECK(rb_fetch(hsel.data(), nsel, np * 8));
     HG_CHECK(check_device_errors());
     // A repeated dimension key emits several rows per fact row, and a
     // compressed key column longer than the fact table makes @join_index
@@ -1417,7 +1417,7 @@ extern "C" I hgpuBatchJoinGroup(const hgpuJoinGroupPlan* plans, L nplans, hgpuJo
                   (unsigned long long*)st2, (unsigned*)(st2 + (size_t)mtiles[np] * 256 * 8), g_derr);
     }
     std::vector<unsigned> hg(np);
-    HG_CU(cudaMemcpyAsync(hg.data(), ngroups, np * 4, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(hg.data(), ngroups, np * 4));
     HG_CHECK(check_device_errors());
     std::vector<long long> segoff(np + 1);
     segoff[0] = 0;
@@ -1450,11 +1450,11 @@ extern "C" I hgpuBatchJoinGroup(const hgpuJoinGroupPlan* plans, L nplans, hgpuJo
     std::vector<double> hq(nseg > 0 ? nseg : 1), hpv(nseg > 0 ? nseg : 1), hd(nseg > 0 ? nseg : 1);
     std::vector<unsigned> hcodes((size_t)np * 256);
     if (nseg > 0) {
-        HG_CU(cudaMemcpyAsync(hst.data(), starts, nseg * 8, cudaMemcpyDeviceToHost, g_stream));
-        HG_CU(cudaMemcpyAsync(hq.data(), sq, nseg * 8, cudaMemcpyDeviceToHost, g_stream));
-        HG_CU(cudaMemcpyAsync(hpv.data(), sp, nseg * 8, cudaMemcpyDeviceToHost, g_stream));
-        HG_CU(cudaMemcpyAsync(hd.data(), sd, nseg * 8, cudaMemcpyDeviceToHost, g_stream));
-        HG_CU(cudaMemcpyAsync(hcodes.data(), codes, (size_t)np * 256 * 4, cudaMemcpyDeviceToHost, g_stream));
+        HG_CHECK(rb_fetch(hst.data(), starts, nseg * 8));
+        HG_CHECK(rb_fetch(hq.data(), sq, nseg * 8));
+        HG_CHECK(rb_fetch(hpv.data(), sp, nseg * 8));
+        HG_CHECK(rb_fetch(hd.data(), sd, nseg * 8));
+        HG_CHECK(rb_fetch(hcodes.data(), codes, (size_t)np * 256 * 4));
     }
     HG_CHECK(check_device_errors());
     for (int p = 0; p < np; p++) {

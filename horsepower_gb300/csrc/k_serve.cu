@@ -532,10 +532,10 @@ static I topk_batch(const hgpu_server_s* s, const hgpuRequest* req, const std::v
                   s->t.o_key, s->t.o_sec, s->t.norder, top, g_derr);
         HG_CHECK(last_launch_error());
         ht.resize(HGPU_TOPK * nr);
-        HG_CU(cudaMemcpyAsync(ht.data(), top, 8 * HGPU_TOPK * nr, cudaMemcpyDeviceToHost, g_stream));
+        HG_CHECK(rb_fetch(ht.data(), top, 8 * HGPU_TOPK * nr));
     }
     std::vector<unsigned long long> cnt(nr);
-    HG_CU(cudaMemcpyAsync(cnt.data(), d_cnt, 8 * nr, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(cnt.data(), d_cnt, 8 * nr));
     HG_CHECK(check_device_errors());
     for (long long k = 0; k < nr; k++) {
         if ((long long)cnt[k] != cap[k]) return set_error(E_GENERAL, "top-k candidate count %llu, expected %lld", cnt[k], cap[k]);
@@ -622,7 +622,7 @@ static I filter_aggs(const hgpu_server_s* s, const hgpuRequest* req, const std::
         m = m2;
     }
     std::vector<double> res(nw);
-    HG_CU(cudaMemcpyAsync(res.data(), cur, nw * 8, cudaMemcpyDeviceToHost, g_stream));
+    HG_CHECK(rb_fetch(res.data(), cur, nw * 8));
     HG_CHECK(check_device_errors());
     for (long long w = 0; w < nw; w++) out[ids[w]].value = res[w];
     return 0;
