@@ -462,3 +462,27 @@ def test_topk_sizes(libs):
         assert np.array_equal(v, want), (r.klo, r.khi)
     srv.close()
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("typ", [H_H, H_I, H_L, H_F, H_E])
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 70_001])
+@pytest.mark.parametrize("wide", [False, True])
+def test_member_rounds(libs, typ, n, wide):
+    """@member in rounds of eight keys a lane, sets of a narrow range (the
+    presence bit answers) and of a wide one (hashed), keys outside the range
+    and NaN: equal to the oracle."""
+    gpu, ora = libs
+    rng = np.random.default_rng(n + typ)
+    span = {H_H: 30_000, H_I: 2 ** 31 - 1, H_L: 2 ** 62, H_F: 1e6, H_E: 1e9}[typ] if wide else 3000
+    make = lambda m, s: (rng.integers(-s, s, m) if typ in (H_H, H_I, H_L) else np.round(rng.uniform(-s, s, m))).astype(DTYPE[typ])  # noqa: E731
+    x = make(1000, span)
+    y = np.where(rng.random(n) < 0.5, rng.choice(x, n), make(n, min(4 * span, 32_000) if typ == H_H else span))
+    if typ in (H_F, H_E):
+        x[3] = np.nan
+        y[rng.random(n) < 0.1] = np.nan
+    y = y.astype(DTYPE[typ])
+    a = gpu.to_py(gpu.call("pfnMember", gpu.vec(x, typ), gpu.vec(y, typ)))
+    b = ora.to_py(ora.call("pfnMember", ora.vec(x, typ), ora.vec(y, typ)))
+    assert np.array_equal(a, b)
+    gpu.free_inputs()
+    ora.free_inputs()
