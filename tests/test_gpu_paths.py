@@ -486,3 +486,29 @@ def test_member_rounds(libs, typ, n, wide):
     assert np.array_equal(a, b)
     gpu.free_inputs()
     ora.free_inputs()
+
+
+@pytest.mark.parametrize("ndim,span", [(2, 2), (7, 8), (255, 2040), (1000, 63_999)])
+@pytest.mark.parametrize("repeat", [False, True])
+def test_shared_probe_keys(libs, ndim, span, repeat):
+    """The shared date table filled by plain stores: key ranges with empty
+    places and odd lengths, negative keys, and a repeated key, which sends the
+    plans to their builtins.  Fact keys outside the dimension match nothing."""
+    from horsepower_gb300 import batch as B, data as D, plans as P
+    gpu = libs[0]
+    dim, fact = D.join_tables(nfact=5000, ndim=ndim, seed=ndim)
+    rng = np.random.default_rng(span)
+    dim["pk"] = (rng.choice(span, ndim, replace=False) - span // 2).astype(np.int32)
+    if repeat:
+        dim["pk"][-1] = dim["pk"][0]
+    fact["fk"] = np.where(rng.random(5000) < 0.9, rng.choice(dim["pk"], 5000), span).astype(np.int32)
+    ddim, dfact = B.device_tables(gpu, dim, fact)
+    wins = [(D.DAYS0, D.DAYS0 + 2526), (D.DAYS0 + 100, D.DAYS0 + 1500), (D.DAYS0, D.DAYS0 + 2526)]
+    got = B.run_batch(gpu, [B.make_plan(ddim, dfact, lo, hi) for lo, hi in wins])
+    for (lo, hi), r in zip(wins, got):
+        if not np.isin(fact["fk"], dim["pk"][(dim["date"] >= lo) & (dim["date"] < hi)]).any():
+            assert len(r[0]) == 0
+            continue
+        for a, b in zip(r, P.join_group(gpu, ddim, dfact, lo, hi)):
+            assert np.array_equal(a, gpu.to_py(b)), (lo, hi)
+    gpu.free_inputs()
