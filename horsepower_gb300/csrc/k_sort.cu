@@ -36,7 +36,7 @@
 
 namespace hg {
 
-I compact_rows(const uint8_t* mask, long long n, long long* out, long long* count);
+I scan_counts(const unsigned* counts, long long n, unsigned long long* offs);
 I scan_exclusive(const unsigned* in, long long n, unsigned long long* out, unsigned long long* total_h);
 
 constexpr int RS_THREADS = 256, RS_ITEMS = 16, RS_TILE = RS_THREADS * RS_ITEMS;
@@ -747,25 +747,89 @@ __global__ void k_bound_keys(const K* __restrict__ k, long long n, uint8_t* __re
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         f[i] = (i == 0) || (k[i] != k[i - 1]);
 }
-// ... or when any column value differs between the rows perm[i-1] and perm[i]
-// (equality as the reference's comparator: == on values)
+// The boundaries of a grouping, one bit a row (word w: rows 32 w .. 32 w + 31)
+// and their number per 4096-row tile.  As bytes they were written once and
+// read twice, and the starts went through a full-length array and a copy (150M
+// rows, 8.6M groups: 0.34 ms from sorted keys to starts, 0.22 now).
+constexpr int GB_TILE = 4096;
+template <typename K>
+struct BoundKeys {  // row i starts a group when its key differs from row i-1's
+    const K* k;
+    using value_t = K;
+    __device__ __forceinline__ K at(long long i) const { return k[i]; }
+    __device__ __forceinline__ bool differ(K a, K b) const { return a != b; }
+};
 struct ColSet {
     const void* col[KMAXC];
     int typ[KMAXC];
     int ncol;
 };
-__global__ void k_bound_cols(ColSet c, const unsigned* __restrict__ perm, long long n, uint8_t* __restrict__ f) {
-    grid_entry();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        bool b = i == 0;
-        if (!b) {
-            long long a = perm[i - 1], q = perm[i];
-            for (int j = 0; j < c.ncol && !b; j++) {
-                if (c.typ[j] == H_F || c.typ[j] == H_E) b = fval(c.col[j], c.typ[j], a) != fval(c.col[j], c.typ[j], q);
-                else b = ival(c.col[j], c.typ[j], a) != ival(c.col[j], c.typ[j], q);
-            }
+struct BoundCols {  // ... or when any column value differs between the rows perm[i-1]
+                    // and perm[i] (equality as the reference's comparator: == on values)
+    ColSet c;
+    const unsigned* perm;
+    using value_t = unsigned;
+    __device__ __forceinline__ unsigned at(long long i) const { return perm[i]; }
+    __device__ __forceinline__ bool differ(unsigned a, unsigned q) const {
+        bool b = false;
+        for (int j = 0; j < c.ncol && !b; j++) {
+            if (c.typ[j] == H_F || c.typ[j] == H_E) b = fval(c.col[j], c.typ[j], a) != fval(c.col[j], c.typ[j], q);
+            else b = ival(c.col[j], c.typ[j], a) != ival(c.col[j], c.typ[j], q);
         }
-        f[i] = b;
+        return b;
+    }
+};
+template <typename F>
+__global__ void __launch_bounds__(256) k_bound_bits(const __grid_constant__ F f, long long n, unsigned* __restrict__ bits,
+                                                    unsigned* __restrict__ counts) {
+    grid_entry();
+    __shared__ unsigned ws[8];
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5;
+    const long long base = (long long)blockIdx.x * GB_TILE + w * 512;  // a warp's 16 words
+    using V = typename F::value_t;
+    V v[16], before = V(0);
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[k] = base + k * 32 + lane < n ? f.at(base + k * 32 + lane) : V(0);
+    if (lane == 0 && base > 0 && base <= n) before = f.at(base - 1);
+    unsigned cnt = 0, mine = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const long long i = base + k * 32 + lane;
+        V prev = __shfl_up_sync(0xffffffffu, v[k], 1);
+        if (lane == 0) prev = before;
+        const unsigned word = __ballot_sync(0xffffffffu, i < n && (i == 0 || f.differ(prev, v[k])));
+        before = __shfl_sync(0xffffffffu, v[k], 31);
+        cnt += __popc(word);
+        if ((int)lane == k) mine = word;
+    }
+    if (lane < 16) bits[base / 32 + lane] = mine;
+    if (lane == 0) ws[w] = cnt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 8; q++) cnt += ws[q];
+        counts[blockIdx.x] = cnt;
+    }
+}
+// the rows of the set bits from the tiles' scanned counts: a warp takes 16
+// words, word by word, lane l writing the row of bit l (a lane walking its own
+// words' bits waits for the densest word: 0.10 - 0.12 ms, 0.073 now)
+__global__ void __launch_bounds__(256) k_bound_starts(const unsigned* __restrict__ bits,
+                                                      const unsigned long long* __restrict__ offs,
+                                                      long long* __restrict__ starts) {
+    grid_entry();
+    __shared__ unsigned ws[8];
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5;
+    const unsigned mine = lane < 16 ? bits[(long long)blockIdx.x * (GB_TILE / 32) + w * 16 + lane] : 0u;
+    const unsigned c = __popc(mine), incl = warp_incl_scan(c);
+    if (lane == 31) ws[w] = incl;
+    __syncthreads();
+    unsigned long long first = offs[blockIdx.x];
+    for (unsigned q = 0; q < w; q++) first += ws[q];
+    const long long row = (long long)blockIdx.x * GB_TILE + w * 512 + lane;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const unsigned word = __shfl_sync(0xffffffffu, mine, k), at = __shfl_sync(0xffffffffu, incl - c, k);
+        if ((word >> lane) & 1u) starts[first + at + __popc(word & lanemask_lt())] = row + k * 32;
     }
 }
 
@@ -1181,22 +1245,27 @@ static I group_finish(V z, long long* starts, long long G, long long* perm, long
 // perm_pre: the output-arena buffer for the i64 permutation, allocated by
 // the caller before the sort (r.perm64 is set when the sort wrote it)
 static I group_dict(V z, const SortResult& r, long long n, const ColSet* cols, long long* perm_pre = nullptr) {
-    uint8_t* flags = (uint8_t*)salloc((size_t)(n > 0 ? n : 1));
-    long long* starts = (long long*)salloc((size_t)(n > 0 ? n : 1) * 8);
-    if (!flags || !starts) return E_DEVICE_OOM;
+    const long long ntiles = (n + GB_TILE - 1) / GB_TILE;
+    unsigned* bits = (unsigned*)salloc((size_t)(ntiles + 1) * (GB_TILE / 8));
+    unsigned* counts = (unsigned*)salloc((size_t)(ntiles + 1) * 4);
+    unsigned long long* offs = (unsigned long long*)salloc((size_t)(ntiles + 1) * 8);
+    if (!bits || !counts || !offs) return E_DEVICE_OOM;
+    unsigned long long G = 0;
     if (n > 0) {
-        if (cols) HG_LAUNCH("bound_cols", gcap(n), 256, 0, k_bound_cols, *cols, r.perm, n, flags);
-        else if (r.key64) HG_LAUNCH("bound_keys", gcap(n), 256, 0, k_bound_keys<unsigned long long>, (const unsigned long long*)r.keys, n, flags);
-        else HG_LAUNCH("bound_keys", gcap(n), 256, 0, k_bound_keys<unsigned>, (const unsigned*)r.keys, n, flags);
+        const unsigned g = (unsigned)ntiles;
+        if (cols) HG_LAUNCH("bound_bits", g, 256, 0, k_bound_bits<BoundCols>, (BoundCols{*cols, r.perm}), n, bits, counts);
+        else if (r.key64) HG_LAUNCH("bound_bits", g, 256, 0, k_bound_bits<BoundKeys<unsigned long long>>,
+                                    BoundKeys<unsigned long long>{(const unsigned long long*)r.keys}, n, bits, counts);
+        else HG_LAUNCH("bound_bits", g, 256, 0, k_bound_bits<BoundKeys<unsigned>>, BoundKeys<unsigned>{(const unsigned*)r.keys}, n,
+                       bits, counts);
+        HG_CHECK(scan_counts(counts, ntiles, offs));
+        HG_CHECK(rb_queue(&G, offs + ntiles, 8));
+        HG_CHECK(check_device_errors());  // synchronises
     }
-    long long G = 0;
-    HG_CHECK(compact_rows(flags, n, starts, &G));
-    {  // group starts stay in the output arena: aggregations over this dict reuse them
-        long long* keep = (long long*)dalloc((size_t)(G > 0 ? G : 1) * 8);
-        if (!keep) return E_DEVICE_OOM;
-        if (G > 0) HG_CU(cudaMemcpyAsync(keep, starts, (size_t)G * 8, cudaMemcpyDeviceToDevice, g_stream));
-        starts = keep;
-    }
+    // group starts stay in the output arena: aggregations over this dict reuse them
+    long long* starts = (long long*)dalloc((size_t)(G > 0 ? G : 1) * 8);
+    if (!starts) return E_DEVICE_OOM;
+    if (G > 0) HG_LAUNCH("bound_starts", (unsigned)ntiles, 256, 0, k_bound_starts, bits, offs, starts);
     // permutation as i64 (the rows of every group, concatenated)
     long long* perm = r.perm64 ? (long long*)r.perm64 : perm_pre;
     if (n > 0 && !r.perm64) {
@@ -1204,7 +1273,7 @@ static I group_dict(V z, const SortResult& r, long long n, const ColSet* cols, l
         if (!perm) return E_DEVICE_OOM;
         HG_LAUNCH("widen", gcap(n), 256, 0, k_widen, r.perm, n, perm, 0);
     }
-    return group_finish(z, starts, G, perm, n);
+    return group_finish(z, starts, (long long)G, perm, n);
 }
 
 // The dict of a grouping from its G group starts and its permutation (both
