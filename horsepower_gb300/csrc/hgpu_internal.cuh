@@ -48,6 +48,7 @@ extern unsigned* g_derr;   // device word
 enum {
     DW_CHAIN = 32,  // blocks of a fused reduction that have finished
     DW_STATS = 33,  // blocks of k_key_stats that have finished
+    DW_TRIE = 34,   // blocks of k_trie_present that have finished
 };
 I check_device_errors();   // syncs, reads and clears g_derr, maps to E_* codes
 // iteration limit for every device-side spin-wait

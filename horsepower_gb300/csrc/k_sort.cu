@@ -1375,21 +1375,56 @@ struct CodeInt {
     long long mn;
     __device__ __forceinline__ unsigned operator()(long long i) const { return (unsigned)((long long)p[i] - mn); }
 };
+// The codes present (bits, cleared before) and, from the block that finishes
+// last, the number of present codes below each word (wpre) and in all (*G):
+// the host reads one word, and no table goes back up.
+struct TrieRank { unsigned bits[2048]; unsigned short wpre[2048]; };
 template <typename Code>
-__global__ void k_trie_present(Code code_of, long long n, unsigned* __restrict__ bitmap) {
+__global__ void __launch_bounds__(256) k_trie_present(Code code_of, long long n, TrieRank* __restrict__ rk,
+                                                      unsigned* done, unsigned* __restrict__ G) {
     grid_entry();
-    __shared__ unsigned sb[2048];
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) sb[i] = 0;
+    __shared__ unsigned sb[2048], ws[8];
+    __shared__ bool last;
+    for (int i = threadIdx.x; i < 2048; i += 256) sb[i] = 0;
     __syncthreads();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned code = code_of(i);
-        atomicOr(&sb[code >> 5], 1u << (code & 31));
+    const long long step = (long long)gridDim.x * 256;
+    for (long long i0 = blockIdx.x * 256LL + threadIdx.x; i0 < n; i0 += 8 * step) {
+        unsigned c[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) c[k] = code_of(i0 + k * step < n ? i0 + k * step : i0);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const unsigned bit = 1u << (c[k] & 31);
+            if (!(sb[c[k] >> 5] & bit)) atomicOr(&sb[c[k] >> 5], bit);
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x)
-        if (sb[i]) atomicOr(&bitmap[i], sb[i]);
+    for (int i = threadIdx.x; i < 2048; i += 256)
+        if (sb[i]) atomicOr(&rk->bits[i], sb[i]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;  // back to 0 by the last
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    unsigned pc[8], sum = 0;  // eight adjacent words a thread
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        pc[k] = __popc(__ldcg(&rk->bits[threadIdx.x * 8 + k]));
+        sum += pc[k];
+    }
+    const unsigned incl = warp_incl_scan(sum);
+    if (lane_id() == 31) ws[threadIdx.x >> 5] = incl;
+    __syncthreads();
+    unsigned at = incl - sum;
+    for (unsigned q = 0; q < (threadIdx.x >> 5); q++) at += ws[q];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        rk->wpre[threadIdx.x * 8 + k] = (unsigned short)at;
+        at += pc[k];
+    }
+    if (threadIdx.x == 255) *G = at;
 }
-struct TrieRank { unsigned bits[2048]; unsigned short wpre[2048]; };
 __device__ __forceinline__ unsigned trie_bucket(const TrieRank& t, unsigned code) {
     const unsigned w = code >> 5;
     return t.wpre[w] + __popc(t.bits[w] & ((1u << (code & 31)) - 1u));
@@ -1422,8 +1457,10 @@ __global__ void __launch_bounds__(256) k_trie_count(Code code_of, long long n, c
 template <typename Code>
 __global__ void __launch_bounds__(256) k_trie_scatter(Code code_of, long long n, const TrieRank* __restrict__ rk, int G,
                                                       long long T, const unsigned long long* __restrict__ offs,
-                                                      long long* __restrict__ perm) {
+                                                      long long* __restrict__ perm, long long* __restrict__ starts) {
     grid_entry();
+    if (blockIdx.x == 0)
+        for (int b = threadIdx.x; b < G; b += blockDim.x) starts[b] = (long long)offs[(long long)b * T];
     __shared__ TrieRank r;
     __shared__ unsigned wcnt[8][TS_MAXG];  // per warp: rows of each bucket, then the warp's base
     __shared__ unsigned long long toff[TS_MAXG];  // the tile's first position in each bucket
@@ -1464,41 +1501,34 @@ __global__ void __launch_bounds__(256) k_trie_scatter(Code code_of, long long n,
     __syncthreads();
     }
 }
-__global__ void k_trie_starts(const unsigned long long* __restrict__ offs, int G, long long T, long long* __restrict__ starts) {
-    grid_entry();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < G) starts[b] = (long long)offs[(long long)b * T];
-}
-
 // *done = 1 with the dict in z; 0 when too many codes are present for the counting path
 template <typename Code>
 static I small_group(V z, Code code_of, long long n, int* done) {
     *done = 0;
-    unsigned* bitmap = (unsigned*)salloc(2048 * 4);
-    if (!bitmap) return E_DEVICE_OOM;
-    HG_CU(cudaMemsetAsync(bitmap, 0, 2048 * 4, g_stream));
-    unsigned grid = grid_for(n, 256);
+    TrieRank* drk = (TrieRank*)salloc(sizeof(TrieRank) + 16);
+    if (!drk) return E_DEVICE_OOM;
+    unsigned* dG = (unsigned*)(drk + 1);
+    HG_CU(cudaMemsetAsync(drk->bits, 0, sizeof(drk->bits), g_stream));
+    unsigned grid = grid_for(n, 256 * 8);
     if (grid > (unsigned)g_sms * 4) grid = g_sms * 4;
-    HG_LAUNCH("trie_present", grid, 256, 0, k_trie_present<Code>, code_of, n, bitmap);
-    TrieRank hr;
-    HG_CHECK(rb_queue(hr.bits, bitmap, 2048 * 4));
-    HG_CU(stream_sync());
+    unsigned* finished = g_derr + DW_TRIE;
+    HG_LAUNCH("trie_present", grid, 256, 0, k_trie_present<Code>, code_of, n, drk, finished, dG);
     unsigned G = 0;
-    for (int i = 0; i < 2048; i++) { hr.wpre[i] = (unsigned short)G; G += (unsigned)__builtin_popcount(hr.bits[i]); }
+    HG_CHECK(rb_queue(&G, dG, 4));
+    HG_CU(stream_sync());
     if (G == 0 || G > (unsigned)TS_MAXG) return 0;
-    TrieRank* drk = (TrieRank*)salloc(sizeof(TrieRank));
     const long long T = (n + TS_TILE - 1) / TS_TILE;
     unsigned* counts = (unsigned*)salloc((size_t)G * (size_t)T * 4);
     unsigned long long* offs = (unsigned long long*)salloc(((size_t)G * (size_t)T + 1) * 8);
     long long* perm = (long long*)dalloc((size_t)n * 8);
     long long* starts = (long long*)dalloc((size_t)G * 8);
-    if (!drk || !counts || !offs || !perm || !starts) return E_DEVICE_OOM;
-    HG_CU(cudaMemcpyAsync(drk, &hr, sizeof(TrieRank), cudaMemcpyHostToDevice, g_stream));
+    if (!counts || !offs || !perm || !starts) return E_DEVICE_OOM;
     const unsigned tg = (unsigned)(T < (long long)g_sms * 4 ? T : (long long)g_sms * 4);
     HG_LAUNCH("trie_count", (unsigned)T, 256, 0, k_trie_count<Code>, code_of, n, drk, (int)G, T, counts);
-    HG_CHECK(scan_exclusive(counts, (long long)G * T, offs, nullptr));
-    HG_LAUNCH("trie_scatter", tg, 256, 0, k_trie_scatter<Code>, code_of, n, drk, (int)G, T, offs, perm);
-    HG_LAUNCH("trie_starts", 1, 256, 0, k_trie_starts, offs, (int)G, T, starts);
+    // up to 8192 counts one block scans in one round, without status words to clear
+    if ((long long)G * T <= 8192) HG_CHECK(scan_counts(counts, (long long)G * T, offs));
+    else HG_CHECK(scan_exclusive(counts, (long long)G * T, offs, nullptr));
+    HG_LAUNCH("trie_scatter", tg, 256, 0, k_trie_scatter<Code>, code_of, n, drk, (int)G, T, offs, perm, starts);
     HG_CHECK(last_launch_error());
     *done = 1;
     return group_finish(z, starts, (long long)G, perm, n);

@@ -512,3 +512,25 @@ def test_shared_probe_keys(libs, ndim, span, repeat):
         for a, b in zip(r, P.join_group(gpu, ddim, dfact, lo, hi)):
             assert np.array_equal(a, gpu.to_py(b)), (lo, hi)
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("codes", [1, 2, 31, 255, 256, 257, 300])
+@pytest.mark.parametrize("n", [4096, 8191, 150_001])
+def test_group_few_codes(libs, codes, n):
+    """@group of i32 keys with few values in a narrow range (the counting path,
+    its rank table made on the device, one or several rounds of the scan) and
+    with one too many: keys and row lists of the stable order."""
+    gpu = libs[0]
+    rng = np.random.default_rng(codes)
+    vals = np.sort(rng.choice(60_000, codes, replace=False)).astype(np.int32)
+    key = rng.choice(vals, n)
+    key[:codes] = vals
+    g = gpu.call("pfnGroup", gpu.vec(key, H_I))
+    order = np.argsort(key, kind="stable")
+    starts = np.flatnonzero(np.r_[True, np.diff(key[order]) != 0])
+    assert np.array_equal(gpu.to_py(gpu.call("pfnKeys", g)), order[starts])
+    lists = gpu.to_py(gpu.call("pfnValues", g))
+    assert len(lists) == codes
+    for a, b in zip(lists, np.split(order, starts[1:])):
+        assert np.array_equal(a, b)
+    gpu.free_inputs()
