@@ -209,6 +209,14 @@ struct ChunkDesc {
     unsigned len;
     unsigned chunk;
 };
+// The value range of an integer column and the bits in which its values
+// (extended to 64 bits) differ; an empty column: [LLONG_MAX, LLONG_MIN], none.
+struct KeyStats {
+    long long mn, mx;
+    unsigned long long vary;
+};
+I key_stats(int nc, const void* const* p, const int* typ, long long n, KeyStats* st);  // in one wait
+I key_stats1(const void* p, I typ, long long n, KeyStats* st);
 struct ListInfo {
     const V0* nodes;          // host node array of the list
     long long ng;             // number of elements

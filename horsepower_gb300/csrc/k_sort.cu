@@ -1035,14 +1035,8 @@ static I sort_by_spec(const KeySpec& s, long long n, int total_bits, SortResult*
     return sort_keys_spec<unsigned>(s, n, vary_hint, ro, r);
 }
 
-// The value ranges of nc integer columns (at most KMAXC) and the bits in which
-// their values (extended to 64 bits) differ, in one round trip; an empty
-// column gives [LLONG_MAX, LLONG_MIN] and no bits.
-struct KeyStats {
-    long long mn, mx;
-    unsigned long long vary;
-};
-static I key_stats(int nc, const void* const* p, const int* typ, long long n, KeyStats* st) {
+// nc columns (at most KMAXC)
+I key_stats(int nc, const void* const* p, const int* typ, long long n, KeyStats* st) {
     for (int c = 0; c < nc; c++) st[c] = KeyStats{LLONG_MAX, LLONG_MIN, 0};
     if (n <= 0) return 0;
     unsigned long long* d = (unsigned long long*)salloc(32 * (KMAXC + KS_MAX_BLOCKS));
@@ -1071,7 +1065,7 @@ static I key_stats(int nc, const void* const* p, const int* typ, long long n, Ke
                          ~(h[4 * c + 2] | h[4 * c + 3])};
     return 0;
 }
-static I key_stats1(const void* p, I typ, long long n, KeyStats* st) {
+I key_stats1(const void* p, I typ, long long n, KeyStats* st) {
     const int t = (int)typ;
     return key_stats(1, &p, &t, n, st);
 }
