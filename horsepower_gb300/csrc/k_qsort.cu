@@ -590,7 +590,11 @@ __global__ void __launch_bounds__(256) k_qs_warps(QsLists lists, const unsigned 
 // The listed ranges of 33 to QS_BLOCK elements, one CTA each, in shared memory:
 // position w * 128 + 32 k + lane of the range belongs to item k of the thread,
 // so the prefixes are ballots.  Ranges that reach 32 elements wait in a list
-// for the CTA's warps.  What bounds a depth is its five barriers.
+// for the CTA's warps.  What bounds a depth is instruction issue, some 14K warp
+// instructions for 4096 rows (ncu), and its five barriers: so the warps' totals
+// are scanned with shuffles (one word a lane; each thread adding up all 32 of
+// them was a fifth of the instructions), and a warp without a live element
+// only passes the prefix on (ranges of a 114K-row sort: 0.108 -> 0.097 ms).
 struct QsBlockSmem {
     unsigned long long K[QS_BLOCK];
     unsigned P[QS_BLOCK];
@@ -639,29 +643,36 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, cons
         for (; __syncthreads_or((int)act); depths++) {
             unsigned pre[QB_ITEMS], run = 0;
             int c[QB_ITEMS];
+            // a warp without a live element only passes the prefix on
+            const bool live = __any_sync(0xffffffffu, act != 0);
 #pragma unroll
             for (int k = 0; k < QB_ITEMS; k++) {
-                const unsigned p = p0 + 32 * k;
-                const bool a = (act >> k) & 1u;
-                c[k] = a && p != lo[k] ? qs_cmp(key[k], sm.K[lo[k]]) : 2;  // 2: the pivot, or finished
-                const unsigned ble = __ballot_sync(0xffffffffu, c[k] <= 0), blt = __ballot_sync(0xffffffffu, c[k] < 0);
-                pre[k] = run + ((unsigned)__popc(ble & lanemask_lt()) | ((unsigned)__popc(blt & lanemask_lt()) << 16));
-                run += (unsigned)__popc(ble) | ((unsigned)__popc(blt) << 16);
+                pre[k] = 0;
+                c[k] = 2;
+            }
+            if (live) {
+#pragma unroll
+                for (int k = 0; k < QB_ITEMS; k++) {
+                    const unsigned p = p0 + 32 * k;
+                    const bool a = (act >> k) & 1u;
+                    c[k] = a && p != lo[k] ? qs_cmp(key[k], sm.K[lo[k]]) : 2;  // 2: the pivot, or finished
+                    const unsigned ble = __ballot_sync(0xffffffffu, c[k] <= 0), blt = __ballot_sync(0xffffffffu, c[k] < 0);
+                    pre[k] = run + ((unsigned)__popc(ble & lanemask_lt()) | ((unsigned)__popc(blt & lanemask_lt()) << 16));
+                    run += (unsigned)__popc(ble) | ((unsigned)__popc(blt) << 16);
+                }
             }
             if (lane == 0) sm.wt[w] = run;
             __syncthreads();
-            unsigned base = 0, all = 0;
-#pragma unroll
-            for (int q = 0; q < QB_WARPS; q++) {
-                const unsigned t = sm.wt[q];
-                if (q < (int)w) base += t;
-                all += t;
-            }
+            // every warp scans the warps' totals for itself
+            static_assert(QB_WARPS == 32, "one total a lane");
+            const unsigned wt = sm.wt[lane], wi = warp_incl_scan(wt);
+            const unsigned base = __shfl_sync(0xffffffffu, wi - wt, w), all = __shfl_sync(0xffffffffu, wi, 31);
 #pragma unroll
             for (int k = 0; k < QB_ITEMS; k++)
                 if (p0 + 32 * k < m) sm.S[p0 + 32 * k] = base + pre[k];
             if (threadIdx.x == 0) sm.S[m] = all;
             __syncthreads();
+            if (live)
 #pragma unroll
             for (int k = 0; k < QB_ITEMS; k++) {
                 if (!((act >> k) & 1u) || c[k] == 2) continue;
@@ -674,6 +685,7 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, cons
             __syncthreads();
             unsigned long long nkey[QB_ITEMS];
             unsigned nrow[QB_ITEMS];
+            if (live)
 #pragma unroll
             for (int k = 0; k < QB_ITEMS; k++) {
                 nkey[k] = key[k];
@@ -703,6 +715,7 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, cons
                 else { lo[k] = p == j ? j : j + 1; if (p == j) hi[k] = j; }  // an empty range for the pivot's place
             }
             __syncthreads();
+            if (live)
 #pragma unroll
             for (int k = 0; k < QB_ITEMS; k++) {
                 if (!((act >> k) & 1u)) continue;
@@ -922,7 +935,8 @@ static I qs_nan_check(const QsCounters& h) {
 // together.  @order of random f64 keys, us, with four launches a depth and
 // with this: 6000 rows 182 and 162, 20K 225 and 191, 114K 351 and 287, 300K 407
 // and 326, 600K 635 and 511; with 8 per thread (the registers spill) 600K 767,
-// 1.2M 1064 against 1045.
+// 1.2M 1064 against 1045.  (The CTA tier has since become 5 to 10 us faster on
+// either side.)
 static bool qs_depths_launch(long long n, QsDepths& q) {
     void* args[] = {&q};
     const long long most = (long long)(g_sms < QD_MAX_BLOCKS ? g_sms : QD_MAX_BLOCKS) * QD_THREADS;
