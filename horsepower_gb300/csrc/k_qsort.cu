@@ -116,16 +116,29 @@ __device__ __forceinline__ int qs_cmp(unsigned long long a, unsigned long long b
 
 // img[p] = image of col[perm[p]] (perm null: row p)
 __global__ void k_qs_image(const void* __restrict__ col, int typ, const unsigned* __restrict__ perm, long long n,
-                           unsigned long long flip, unsigned long long* __restrict__ img, unsigned* nanflag) {
+                           unsigned long long flip, unsigned long long* __restrict__ img, unsigned* nanflag,
+                           uint8_t* __restrict__ up, uint8_t* __restrict__ down) {
     grid_entry();
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
+    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         img[p] = qs_image(col, typ, perm ? (long long)perm[p] : p, nanflag) ^ flip;
+        if (up) up[p] = down[p] = 0;  // for k_qs_updown (a clear between kernels costs the chain 4 us)
+    }
 }
 
-__global__ void k_qs_iota(unsigned* __restrict__ v, long long n) {
+// rows in order; with `seg` also the one segment of a list's first column;
+// the sort's counters cleared
+__global__ void k_qs_iota(unsigned* __restrict__ v, long long n, unsigned* __restrict__ seg, long long* __restrict__ starts,
+                          QsCounters* cnt) {
     grid_entry();
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
+    const long long me = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long p = me; p < n; p += (long long)gridDim.x * blockDim.x) {
         v[p] = (unsigned)p;
+        if (seg) seg[p] = 0;
+    }
+    if (me == 0) {
+        *cnt = QsCounters{};
+        if (seg) starts[0] = 0;
+    }
 }
 
 // ---- one recursion depth over all ranges
@@ -754,8 +767,10 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, cons
 
 // ---- ranges (segments) of a list sort
 // seg[p] = index of the segment holding position p (starts ascending)
-__global__ void k_qs_segid(const long long* __restrict__ starts, long long ns, long long n, unsigned* __restrict__ seg) {
+__global__ void k_qs_segid(const long long* __restrict__ starts, long long ns, long long n, unsigned* __restrict__ seg,
+                           QsCounters* cnt) {
     grid_entry();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *cnt = QsCounters{};  // the next column's
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         long long a = 0, b = ns - 1;  // last start <= p
         while (a < b) {
@@ -844,8 +859,11 @@ __global__ void k_qs_reverse(const unsigned* __restrict__ perm, const unsigned* 
 // of segments that are not sorted keep their row.
 __global__ void k_qs_ranges(const unsigned* __restrict__ seg, const long long* __restrict__ starts, long long ns, long long n,
                             const uint8_t* __restrict__ mode, const unsigned* __restrict__ perm,
-                            unsigned* __restrict__ lo, unsigned* __restrict__ hi, unsigned* __restrict__ fin) {
+                            unsigned* __restrict__ lo, unsigned* __restrict__ hi, unsigned* __restrict__ fin,
+                            unsigned* __restrict__ act, int nact) {
     grid_entry();
+    if (act && blockIdx.x == 0)
+        for (int i = threadIdx.x; i < nact; i += blockDim.x) act[i] = 0;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned s = seg ? seg[p] : 0;
         const long long a = seg ? starts[s] : 0, b = seg ? (s + 1 < ns ? starts[s + 1] : n) : n;
@@ -966,7 +984,14 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
         hi = (unsigned*)salloc((size_t)n * 4);
         if (!lo || !hi) return E_DEVICE_OOM;
     }
-    HG_LAUNCH("qs_ranges", g, 256, 0, k_qs_ranges, seg, starts, ns, n, mode, perm, lo, hi, fin);
+    unsigned* act = nullptr;  // counts of a round's depths, then k_qs_depths' barrier and result
+    constexpr int nact = QD_ROUND + 3;
+    if (h->nbig) {
+        act = (unsigned*)salloc(nact * 4);
+        if (!act) return E_DEVICE_OOM;
+    }
+    bool act_clear = true;  // k_qs_ranges has cleared them
+    HG_LAUNCH("qs_ranges", g, 256, 0, k_qs_ranges, seg, starts, ns, n, mode, perm, lo, hi, fin, act, nact);
     if (h->nbig) {
         const long long nt = (n + QS_TILE - 1) / QS_TILE;
         unsigned* P2 = (unsigned*)salloc((size_t)n * 4);
@@ -975,10 +1000,9 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
         unsigned long long* ts = (unsigned long long*)salloc((size_t)(nt > QD_MAX_BLOCKS ? nt : QD_MAX_BLOCKS) * 8);
         unsigned* Lpos = (unsigned*)salloc((size_t)n * 4);
         unsigned* Rpos = (unsigned*)salloc((size_t)n * 4);
-        unsigned* act = (unsigned*)salloc((QD_ROUND + 3) * 4);  // counts, then k_qs_depths' barrier and result
         KL = (unsigned long long*)salloc((size_t)n * 8);
         PL = (unsigned*)salloc((size_t)n * 4);
-        if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos || !act || !KL || !PL) return E_DEVICE_OOM;
+        if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos || !KL || !PL) return E_DEVICE_OOM;
         // the ranges listed at the start are read from perm/img, which the
         // depths below reuse only at the positions of larger ranges
         unsigned* Pc = perm;
@@ -989,7 +1013,8 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
             if (level >= max_levels) return qs_too_deep(max_levels);
             if (resident) {
                 round = (int)(max_levels - level < QD_ROUND ? max_levels - level : QD_ROUND);
-                HG_CU(cudaMemsetAsync(act, 0, (QD_ROUND + 3) * 4, g_stream));
+                if (!act_clear) HG_CU(cudaMemsetAsync(act, 0, nact * 4, g_stream));
+                act_clear = false;
                 QsDepths q{lo, hi, {Kc, Kc == img ? K2 : img}, {Pc, Pc == perm ? P2 : perm}, S, ts, Lpos, Rpos, fin,
                            act, act + QD_ROUND, act + QD_ROUND + 1, KL, PL, lists, g_derr, (unsigned)n, (unsigned)level,
                            (unsigned)round};
@@ -1056,9 +1081,10 @@ static I qs_depth_check(long long n, const QsCounters& h) {
 }
 
 static I qs_image_of(const void* col, I typ, const unsigned* perm, long long n, bool desc, unsigned long long* img,
-                     unsigned* nanflag) {
+                     unsigned* nanflag, uint8_t* up = nullptr, uint8_t* down = nullptr) {
     if (n > 0)
-        HG_LAUNCH("qs_image", qs_grid(n), 256, 0, k_qs_image, col, (int)typ, perm, n, desc ? ~0ull : 0ull, img, nanflag);
+        HG_LAUNCH("qs_image", qs_grid(n), 256, 0, k_qs_image, col, (int)typ, perm, n, desc ? ~0ull : 0ull, img, nanflag, up,
+                  down);
     return last_launch_error();
 }
 
@@ -1074,8 +1100,7 @@ I qs_sort_vector(const void* col, I typ, long long n, bool asc, const unsigned**
     HG_CHECK(qs_lists_alloc(n, &lists));
     *perm_out = fin;
     if (n == 0) return 0;
-    HG_CU(cudaMemsetAsync(lists.cnt, 0, sizeof(QsCounters), g_stream));
-    HG_LAUNCH("qs_iota", qs_grid(n), 256, 0, k_qs_iota, perm, n);
+    HG_LAUNCH("qs_iota", qs_grid(n), 256, 0, k_qs_iota, perm, n, nullptr, nullptr, lists.cnt);
     HG_CHECK(qs_image_of(col, typ, nullptr, n, !asc, img, &lists.cnt->nan));
     HG_LAUNCH("qs_whole", 1, 1, 0, k_qs_whole, n, lists);
     QsCounters h;
@@ -1115,10 +1140,8 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
     uint8_t* mode = flags + 2 * nn;
     unsigned* nanflag = &lists.cnt->nan;
     const unsigned g = qs_grid(n);
-    HG_LAUNCH("qs_iota", g, 256, 0, k_qs_iota, perm, n);
+    HG_LAUNCH("qs_iota", g, 256, 0, k_qs_iota, perm, n, seg, starts, lists.cnt);
     long long ns = 1;  // segments: runs of rows equal on the columns sorted so far
-    HG_CU(cudaMemsetAsync(starts, 0, 8, g_stream));
-    HG_CU(cudaMemsetAsync(seg, 0, nn * 4, g_stream));
     for (int c = 0; c < nc; c++) {
         const I typ = typs[c];
         const bool desc = asc && !asc[c];
@@ -1126,10 +1149,8 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
             return set_error(E_NOT_IMPL, "descending char column in a list order (the reference indexes past the range)");
         const bool stable = typ == H_I || typ == H_L || typ == H_C;
         bool ran = false;  // a quicksort whose counters the next wait reads into h
-        HG_CU(cudaMemsetAsync(lists.cnt, 0, sizeof(QsCounters), g_stream));
-        HG_CHECK(qs_image_of(cols[c], typ, perm, n, desc, img, nanflag));
+        HG_CHECK(qs_image_of(cols[c], typ, perm, n, desc, img, nanflag, up, down));
         // lib_order_by_sorted
-        HG_CU(cudaMemsetAsync(flags, 0, 2 * nn, g_stream));
         HG_LAUNCH("qs_updown", g, 256, 0, k_qs_updown, img, seg, n, up, down);
         HG_LAUNCH("qs_mode", qs_grid(ns), 256, 0, k_qs_mode, up, down, starts, ns, n, desc ? 1 : 0, typ == H_C ? 10 : 2,
                   mode, lists);
@@ -1183,7 +1204,7 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
             HG_LAUNCH("qs_heads", g, 256, 0, k_qs_heads, img, seg, n, up);
             HG_CHECK(compact_rows(up, n, starts, &ns));  // waits, and reads the device errors
             if (ran) HG_CHECK(qs_depth_check(n, h));
-            HG_LAUNCH("qs_segid", g, 256, 0, k_qs_segid, starts, ns, n, seg);
+            HG_LAUNCH("qs_segid", g, 256, 0, k_qs_segid, starts, ns, n, seg, lists.cnt);
         } else if (ran) {
             HG_CHECK(check_device_errors());
             HG_CHECK(qs_depth_check(n, h));
