@@ -1008,13 +1008,13 @@ static I agg_typed(int ag, I xt, const T* src, const long long* rows, long long 
     using SA = typename std::conditional<isF, float, typename std::conditional<isE, double, long long>::type>::type;
     if (ag == AG_LEN) {
         *typ = H_L;
-        *out = salloc((size_t)(ng > 0 ? ng : 1) * 8);
+        if (!*out) *out = salloc((size_t)(ng > 0 ? ng : 1) * 8);
         if (!*out) return E_DEVICE_OOM;
         if (ng > 0) HG_LAUNCH("len_seg", gcap(ng), 256, 0, k_len_seg, starts, ng, total, (long long*)*out);
         return last_launch_error();
     }
     if (ag == AG_SUM || ag == AG_AVG) {
-        SA* s = (SA*)salloc((size_t)(ng > 0 ? ng : 1) * sizeof(SA));
+        SA* s = (SA*)(ag == AG_SUM && *out ? *out : salloc((size_t)(ng > 0 ? ng : 1) * sizeof(SA)));
         if (!s) return E_DEVICE_OOM;
         SegIO<T, SA> io{};
         io.src[0] = src;
@@ -1026,7 +1026,7 @@ static I agg_typed(int ag, I xt, const T* src, const long long* rows, long long 
             return 0;
         }
         *typ = isF ? H_F : H_E;
-        *out = salloc((size_t)(ng > 0 ? ng : 1) * 8);
+        if (!*out) *out = salloc((size_t)(ng > 0 ? ng : 1) * 8);
         if (!*out) return E_DEVICE_OOM;
         if (ng > 0) HG_LAUNCH("avg_seg", gcap(ng), 256, 0, k_avg_seg<SA>, s, starts, ng, total, *out);
         return last_launch_error();
@@ -1198,6 +1198,16 @@ __global__ void k_segment_nodes(const char* __restrict__ data, const long long* 
     }
 }
 
+// An output's memory before its node is touched (which may be an input's), and
+// the node once the output is computed: alloc_out in two steps.
+static void* out_memory(I typ, L len) { return len > 1 ? dalloc((size_t)len * esize(typ)) : salloc(16); }
+static void out_node(V z, I typ, L len, void* d) {
+    z->typ = typ;
+    z->len = len;
+    z->g = len > 1 ? (G)d : (G)&z->b;
+    if (len <= 1) z->i64 = 0;
+}
+
 static I group_agg(V z, V x, V y, int ag) {
     HG_CHECK(ensure_init());
     ScratchScope ss;
@@ -1210,13 +1220,23 @@ static I group_agg(V z, V x, V y, int ag) {
     HG_CHECK(list_segments(y, H_L, &starts, &total, &rows, &li));
     const void* px;
     HG_CHECK(in_ptr(x, &px));
-    void* res;
-    I typ;
+    // sums, averages and lengths, whose type is known before, are written where
+    // they stay; min and max of integers widen when a group is empty
+    void *res = nullptr, *dz = nullptr;
+    I typ = ag == AG_LEN ? H_L : x->typ == H_F ? H_F : (x->typ == H_E || ag == AG_AVG) ? H_E : H_L;
+    const L ng = y->len;
+    if (ag != AG_MIN && ag != AG_MAX) {
+        res = dz = out_memory(typ, ng);
+        if (!dz) return E_DEVICE_OOM;
+    }
     HG_CHECK(agg_dispatch<true>(ag, x->typ, px, (const long long*)rows, x->len, starts, y->len, total, &res, &typ, li));
     if (!(li && li->group_rows && x->len >= total)) HG_CHECK(check_device_errors());  // rows of @group are in range
-    void* dz;
-    HG_CHECK(alloc_out(z, typ, y->len, &dz));
-    if (y->len > 0) HG_CU(cudaMemcpyAsync(dz, res, (size_t)y->len * esize(typ), cudaMemcpyDeviceToDevice, g_stream));
+    if (!dz) {
+        dz = out_memory(typ, ng);
+        if (!dz) return E_DEVICE_OOM;
+        if (ng > 0) HG_CU(cudaMemcpyAsync(dz, res, (size_t)ng * esize(typ), cudaMemcpyDeviceToDevice, g_stream));
+    }
+    out_node(z, typ, ng, dz);
     return finish_out(z, dz);
 }
 
@@ -1260,12 +1280,16 @@ I hgpuGroupAggMany(V* z, V* x, V y, const I* aggs, L n) {
             const long long ng = y->len;
             const double* srcs[SEG_MANY];
             double* sums[SEG_MANY];
+            void* outs[SEG_MANY];
             long long nx = -1;
             for (int q = 0; q < nf; q++) {
                 const void* px;
                 HG_CHECK(in_ptr(x[fused[q]], &px));
                 srcs[q] = (const double*)px;
-                sums[q] = (double*)salloc((size_t)(ng > 0 ? ng : 1) * 8);
+                outs[q] = out_memory(H_E, ng);
+                if (!outs[q]) return E_DEVICE_OOM;
+                // a sum is reduced where it stays, an average's from scratch
+                sums[q] = (double*)(aggs[fused[q]] == AG_SUM ? outs[q] : salloc((size_t)(ng > 0 ? ng : 1) * 8));
                 if (!sums[q]) return E_DEVICE_OOM;
                 nx = nx < 0 ? x[fused[q]]->len : (x[fused[q]]->len < nx ? x[fused[q]]->len : nx);
             }
@@ -1274,15 +1298,12 @@ I hgpuGroupAggMany(V* z, V* x, V y, const I* aggs, L n) {
             if (!in_range) HG_CHECK(check_device_errors());
             for (int q = 0; q < nf; q++) {
                 const int k = fused[q];
-                void* dz;
-                HG_CHECK(alloc_out(z[k], H_E, ng, &dz));
                 if (aggs[k] == AG_AVG) {
-                    if (ng > 0) HG_LAUNCH("avg_seg", gcap(ng), 256, 0, k_avg_seg<double>, sums[q], starts, ng, total, dz);
+                    if (ng > 0) HG_LAUNCH("avg_seg", gcap(ng), 256, 0, k_avg_seg<double>, sums[q], starts, ng, total, outs[q]);
                     HG_CHECK(last_launch_error());
-                } else if (ng > 0) {
-                    HG_CU(cudaMemcpyAsync(dz, sums[q], (size_t)ng * 8, cudaMemcpyDeviceToDevice, g_stream));
                 }
-                HG_CHECK(finish_out(z[k], dz));
+                out_node(z[k], H_E, ng, outs[q]);
+                HG_CHECK(finish_out(z[k], outs[q]));
                 done[k] = true;
             }
         }
@@ -1356,7 +1377,7 @@ I pfnEach(V z, V x, I (*foo)(V, V)) {
             long long total;
             const void* vals;
             HG_CHECK(list_segments(x, t, &starts, &total, &vals));
-            void* res;
+            void* res = nullptr;
             I typ;
             ListInfo* lk = find_list(host_nodes(x), ng);
             HG_CHECK(agg_dispatch<false>(ag, t, vals, nullptr, 0, starts, ng, total, &res, &typ, lk));
