@@ -604,14 +604,13 @@ __device__ __forceinline__ bool key_stream(const void* p, int typ, long long i, 
 }
 
 // ------------------------------------------------------------------ member
-// A lane looks up eight keys at a time, all their reads in flight together;
-// with a direct table the presence bit is the answer (no row is read).  What
-// bounds it is the L2's rate of scattered sectors, 243 G/s (60M i32 keys
-// against 2.1M of a 15M range: 0.285 ms with one key at a time and the row
-// read behind its bit, 0.268 now, 0.247 at that rate).
+// Direct tables: the presence bit is the answer, and a lane has eight keys'
+// bits in flight.  What bounds it is the L2's rate of scattered sectors, 243
+// G/s (60M i32 keys against 2.1M of a 15M range: 0.285 ms with one key at a
+// time and the row read behind its bit, 0.268 now, 0.247 at that rate).
 template <typename K>
-__global__ void __launch_bounds__(256) k_member(Table<K> t, const void* __restrict__ y, int typ, long long n,
-                                                bool* __restrict__ z) {
+__global__ void __launch_bounds__(256) k_member_direct(Table<K> t, const void* __restrict__ y, int typ, long long n,
+                                                       bool* __restrict__ z) {
     grid_entry();
     constexpr int N = 8;
     const unsigned lane = lane_id();
@@ -619,30 +618,43 @@ __global__ void __launch_bounds__(256) k_member(Table<K> t, const void* __restri
     for (long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; w * (32 * N) < n; w += warps) {
         const long long i0 = w * (32 * N) + lane;
         K key[N];
-        bool valid[N], r[N];
+        bool valid[N];
+        long long fb[N];
+        unsigned fw[N];
 #pragma unroll
         for (int k = 0; k < N; k++) valid[k] = i0 + k * 32 < n && key_stream<K>(y, typ, i0 + k * 32, &key[k]);
-        if (t.direct) {
-            long long fb[N];
-            unsigned fw[N];
 #pragma unroll
-            for (int k = 0; k < N; k++) {
-                fb[k] = valid[k] ? filter_bit<K>(t, key[k]) : -1;
-                fw[k] = fb[k] >= 0 ? __ldg(t.filter + (fb[k] >> 5)) : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < N; k++) r[k] = (fw[k] >> (fb[k] & 31)) & 1u;
-        } else {
-            long long slot[N];
-            unsigned row[N];
-            table_find_n<K, N>(t, key, valid, slot, row);
-#pragma unroll
-            for (int k = 0; k < N; k++) r[k] = slot[k] != -1;
+        for (int k = 0; k < N; k++) {
+            fb[k] = valid[k] ? filter_bit<K>(t, key[k]) : -1;
+            fw[k] = fb[k] >= 0 ? __ldg(t.filter + (fb[k] >> 5)) : 0u;
         }
 #pragma unroll
         for (int k = 0; k < N; k++)
-            if (i0 + k * 32 < n) z[i0 + k * 32] = r[k];
+            if (i0 + k * 32 < n) z[i0 + k * 32] = (fw[k] >> (fb[k] & 31)) & 1u;
     }
+}
+// Hashed tables: one key at a time.  A walk along the slots is as long as the
+// longest of the warp's, and with eight keys a lane their state takes the
+// registers that hide it (40M f64 keys against 200K: 0.73 ms with eight a lane,
+// 0.37 now; 40M sparse i32 keys 0.50 and 0.35).
+template <typename K>
+__global__ void k_member_hash(Table<K> t, const void* __restrict__ y, int typ, long long n, bool* __restrict__ z) {
+    grid_entry();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        K k;
+        bool r = false;
+        long long row;
+        if (key_at<K>(y, typ, i, &k)) r = table_find<K>(t, k, &row) != -1;
+        z[i] = r;
+    }
+}
+template <typename K>
+static I member_of(const Table<K>& t, const void* y, int typ, long long n, void* z) {
+    if (n > 0 && t.direct)
+        HG_LAUNCH("member", grid_cap((n + 7) / 8), 256, 0, k_member_direct<K>, t, y, typ, n, (bool*)z);
+    else if (n > 0)
+        HG_LAUNCH("member_hash", grid_cap(n), 256, 0, k_member_hash<K>, t, y, typ, n, (bool*)z);
+    return last_launch_error();
 }
 
 // sets of one or two elements: direct == compares (lib_member_fast1/2, h_libs.cc:900-945)
@@ -1625,11 +1637,11 @@ I pfnMember(V z, V y, V x) {
         } else if (key64(typ)) {
             Table<unsigned long long> t;
             HG_CHECK(table_build<unsigned long long>(&t, px, typ, nx, false));
-            if (n > 0) HG_LAUNCH("member", grid_cap((n + 7) / 8), 256, 0, k_member<unsigned long long>, t, py, (int)typ, n, (bool*)dz);
+            HG_CHECK(member_of(t, py, (int)typ, n, dz));
         } else {
             Table<unsigned> t;
             HG_CHECK(table_build<unsigned>(&t, px, typ, nx, false));
-            if (n > 0) HG_LAUNCH("member", grid_cap((n + 7) / 8), 256, 0, k_member<unsigned>, t, py, (int)typ, n, (bool*)dz);
+            HG_CHECK(member_of(t, py, (int)typ, n, dz));
         }
         HG_CHECK(last_launch_error());
         HG_CHECK(check_device_errors());
@@ -1642,7 +1654,7 @@ I pfnMember(V z, V y, V x) {
         HG_CHECK(alloc_out(z, H_B, n, &dz));
         Table<unsigned> t;
         HG_CHECK(table_build<unsigned>(&t, px, H_J, nx, false));
-        if (n > 0) HG_LAUNCH("member", grid_cap((n + 7) / 8), 256, 0, k_member<unsigned>, t, py, (int)H_J, n, (bool*)dz);
+        HG_CHECK(member_of(t, py, (int)H_J, n, dz));
         HG_CHECK(last_launch_error());
         HG_CHECK(check_device_errors());
         return finish_out(z, dz);
