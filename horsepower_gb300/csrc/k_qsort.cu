@@ -77,15 +77,22 @@ static long long qs_max_levels(long long n) {
     const long long m = (1LL << 36) / (n > 0 ? n : 1);
     return ((m > 8192 ? m : 8192) + 7) / 8 * 8;
 }
-// Depths issued before the host reads the active count: a random range of n
-// rows needs about 2 log2(n / QS_BLOCK) of them to come down to QS_BLOCK at
-// its worst place; after these the count is read every QS_ROUND depths.
-constexpr int QS_ROUND = 4, QS_MAX_ROUND = 64;
-static int qs_first_round(long long n) {
+// Depths issued between two reads of the active count: a random range of n rows
+// needs about 2 log2(n / QS_BLOCK) of them to come down to QS_BLOCK at its
+// worst place, keys of few values a handful.  So the first round is short and
+// the second holds the rest of that estimate; a depth after the last one
+// (`prev` counts nothing left) writes nothing, and above QS_DIRECT tiles reads
+// nothing either.  A wait costs some 25 us, a depth 30 us at 1M rows and 1.1 ms
+// at 40M.  Keys of five values, with the whole estimate in one round and now:
+// 2M rows 0.68 and 0.38 ms, 10M 3.5 and 2.0, 60M 26.8 and 8.4; random keys 0.81
+// and 0.84 ms at 700K rows, even from 2M on.
+constexpr int QS_ROUND1 = 8, QS_ROUND = 4, QS_MAX_ROUND = 64;
+static int qs_second_round(long long n) {
     int d = 2;
     for (long long m = n; m > QS_BLOCK && d < QS_MAX_ROUND; m >>= 1) d += 2;
-    return d;
+    return d - QS_ROUND1 > QS_ROUND ? d - QS_ROUND1 : QS_ROUND;
 }
+__device__ __forceinline__ bool qs_idle(const unsigned* prev) { return prev && *prev == 0; }
 
 __device__ __forceinline__ long long qs_ival(const void* p, int typ, long long i) {
     switch (typ) {
@@ -154,8 +161,10 @@ __device__ __forceinline__ unsigned long long qs_flag(const unsigned* __restrict
 }
 
 __global__ void __launch_bounds__(QS_THREADS) k_qs_count(const unsigned* __restrict__ lo, const unsigned long long* __restrict__ K,
-                                                         long long n, unsigned long long* __restrict__ tile_sum) {
+                                                         long long n, unsigned long long* __restrict__ tile_sum,
+                                                         const unsigned* __restrict__ prev) {
     grid_entry();
+    if (qs_idle(prev)) return;
     __shared__ unsigned long long ws[QS_THREADS / 32];
     const long long base = (long long)blockIdx.x * QS_TILE + (long long)threadIdx.x * QS_ITEMS;
     unsigned long long s = 0;
@@ -172,12 +181,49 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_count(const unsigned* __restr
     }
 }
 
-// S[p] = exclusive prefix of the flag pairs; S[n] = total.  Each block sums
-// the tiles before its own.
+// The tile sums before each tile: up to QS_DIRECT tiles every block of
+// k_qs_prefix adds them up itself, beyond that they are scanned first, in place:
+// that adding up grows with the square of the tiles.  Random f64 keys, ms, added
+// up and scanned: 4M rows 3.45 and 3.52, 8M 7.19 and 7.24, 16M 16.37 and 16.27,
+// 60M 71.5 and 66.9, 150M 201 and 166.
+constexpr long long QS_DIRECT = 4096;
+__global__ void __launch_bounds__(1024) k_qs_scan_sums(unsigned long long* __restrict__ ts, long long nt,
+                                                       const unsigned* __restrict__ prev) {
+    grid_entry();
+    if (qs_idle(prev)) return;
+    constexpr int PER = 4;
+    __shared__ unsigned long long ws[32];
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (long long b = 0; b < nt; b += 1024 * PER) {
+        const long long at = b + (long long)threadIdx.x * PER;
+        unsigned long long v[PER], sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; k++) v[k] = at + k < nt ? ts[at + k] : 0ull;
+#pragma unroll
+        for (int k = 0; k < PER; k++) sum += v[k];
+        const unsigned long long incl = warp_incl_scan64(sum);
+        if (lane == 31) ws[w] = incl;
+        __syncthreads();
+        const unsigned long long x = ws[lane], xi = warp_incl_scan64(x);  // every warp scans the warps' totals
+        unsigned long long off = carry + __shfl_sync(0xffffffffu, xi - x, w) + incl - sum;
+        carry += __shfl_sync(0xffffffffu, xi, 31);
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            if (at + k < nt) ts[at + k] = off;
+            off += v[k];
+        }
+        __syncthreads();
+    }
+}
+
+// S[p] = exclusive prefix of the flag pairs; S[n] = total
 __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __restrict__ lo, const unsigned long long* __restrict__ K,
                                                           long long n, const unsigned long long* __restrict__ tile_sum,
-                                                          unsigned long long* __restrict__ S) {
+                                                          int scanned, unsigned long long* __restrict__ S,
+                                                          const unsigned* __restrict__ prev) {
     grid_entry();
+    const bool idle = qs_idle(prev);  // not looked at before the loads below are in flight
     __shared__ unsigned long long ws[QS_THREADS / 32], wb[QS_THREADS / 32];
     const long long base = (long long)blockIdx.x * QS_TILE + (long long)threadIdx.x * QS_ITEMS;
     unsigned long long v[QS_ITEMS], s = 0;
@@ -187,7 +233,9 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __rest
         s += v[k];
     }
     unsigned long long before = 0;
-    for (long long t = threadIdx.x; t < blockIdx.x; t += QS_THREADS) before += tile_sum[t];
+    if (scanned) before = threadIdx.x == 0 ? tile_sum[blockIdx.x] : 0ull;
+    else
+        for (long long t = threadIdx.x; t < blockIdx.x; t += QS_THREADS) before += tile_sum[t];
     before = warp_sum(before);
     const unsigned long long incl = warp_incl_scan64(s);
     if (lane_id() == 31) ws[threadIdx.x >> 5] = incl;
@@ -196,6 +244,7 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __rest
     unsigned long long off = incl - s;
 #pragma unroll
     for (unsigned w = 0; w < QS_THREADS / 32; w++) off += wb[w] + (w < (threadIdx.x >> 5) ? ws[w] : 0ull);
+    if (idle) return;
 #pragma unroll
     for (int k = 0; k < QS_ITEMS; k++) {
         if (base + k < n) S[base + k] = off;
@@ -213,8 +262,10 @@ __device__ __forceinline__ unsigned qs_lt(unsigned long long s) { return (unsign
 // it would mean inconsistent ranges and is recorded, not written.)
 __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __restrict__ hi,
                          const unsigned long long* __restrict__ K, const unsigned long long* __restrict__ S, long long n,
-                         unsigned* __restrict__ Lpos, unsigned* __restrict__ Rpos, unsigned* derr) {
+                         unsigned* __restrict__ Lpos, unsigned* __restrict__ Rpos, const unsigned* __restrict__ prev,
+                         unsigned* derr) {
     grid_entry();
+    if (qs_idle(prev)) return;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned l = lo[p];
         if (l == QS_DONE || (long long)l == p) continue;
@@ -240,9 +291,10 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
                           const unsigned* __restrict__ P, const unsigned long long* __restrict__ S, long long n,
                           const unsigned* __restrict__ Lpos, const unsigned* __restrict__ Rpos,
                           unsigned long long* __restrict__ K2, unsigned* __restrict__ P2, unsigned* __restrict__ fin,
-                          unsigned* __restrict__ active, unsigned depth, unsigned long long* __restrict__ KL,
+                          const unsigned* prev, unsigned* active, unsigned depth, unsigned long long* __restrict__ KL,
                           unsigned* __restrict__ PL, QsLists lists, unsigned* derr) {
     grid_entry();
+    if (qs_idle(prev)) return;
     unsigned still = 0;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const unsigned l = lo[p];
@@ -994,6 +1046,7 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
     HG_LAUNCH("qs_ranges", g, 256, 0, k_qs_ranges, seg, starts, ns, n, mode, perm, lo, hi, fin, act, nact);
     if (h->nbig) {
         const long long nt = (n + QS_TILE - 1) / QS_TILE;
+        const bool scan = nt > QS_DIRECT;
         unsigned* P2 = (unsigned*)salloc((size_t)n * 4);
         unsigned long long* K2 = (unsigned long long*)salloc((size_t)n * 8);
         unsigned long long* S = (unsigned long long*)salloc((size_t)(n + 1) * 8);
@@ -1007,9 +1060,9 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
         // depths below reuse only at the positions of larger ranges
         unsigned* Pc = perm;
         unsigned long long* Kc = img;
-        int round = qs_first_round(n);
+        int round = 0, rounds = 0;
         bool resident = true;  // k_qs_depths takes the depths, while the elements fit the chip's threads
-        for (long long level = 0;; level += round, round = QS_ROUND) {
+        for (long long level = 0;; level += round) {
             if (level >= max_levels) return qs_too_deep(max_levels);
             if (resident) {
                 round = (int)(max_levels - level < QD_ROUND ? max_levels - level : QD_ROUND);
@@ -1036,17 +1089,22 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                     round = (int)res[0];
                     continue;
                 }
-                round = level == 0 ? qs_first_round(n) : QS_ROUND;
             }
+            round = rounds == 0 ? QS_ROUND1 : rounds == 1 ? qs_second_round(n) : QS_ROUND;
+            rounds++;
             if (level + round > max_levels) round = (int)(max_levels - level);
             HG_CU(cudaMemsetAsync(act, 0, QS_MAX_ROUND * 4, g_stream));
             for (int d = 0; d < round; d++) {
-                HG_LAUNCH("qs_count", (unsigned)nt, QS_THREADS, 0, k_qs_count, lo, Kc, n, ts);
-                HG_LAUNCH("qs_prefix", (unsigned)nt, QS_THREADS, 0, k_qs_prefix, lo, Kc, n, ts, S);
-                HG_LAUNCH("qs_pos", g, 256, 0, k_qs_pos, lo, hi, Kc, S, n, Lpos, Rpos, g_derr);
+                // (a round begins with elements left; where a depth takes microseconds
+                // only the kernel that hides the look does it)
+                const unsigned *left = d ? act + d - 1 : nullptr, *prev = scan ? left : nullptr;
+                HG_LAUNCH("qs_count", (unsigned)nt, QS_THREADS, 0, k_qs_count, lo, Kc, n, ts, prev);
+                if (scan) HG_LAUNCH("qs_scan_sums", 1, 1024, 0, k_qs_scan_sums, ts, nt, prev);
+                HG_LAUNCH("qs_prefix", (unsigned)nt, QS_THREADS, 0, k_qs_prefix, lo, Kc, n, ts, scan ? 1 : 0, S, left);
+                HG_LAUNCH("qs_pos", g, 256, 0, k_qs_pos, lo, hi, Kc, S, n, Lpos, Rpos, prev, g_derr);
                 unsigned* Pn = Pc == perm ? P2 : perm;
                 unsigned long long* Kn = Kc == img ? K2 : img;
-                HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, Lpos, Rpos, Kn, Pn, fin, act + d,
+                HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, Lpos, Rpos, Kn, Pn, fin, prev, act + d,
                           (unsigned)(level + d), KL, PL, lists, g_derr);
                 Pc = Pn;
                 Kc = Kn;

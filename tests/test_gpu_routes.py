@@ -4,11 +4,13 @@ side of a rule's line, and that its result is the same on both.
 Bar: bit-exact.
 """
 import ctypes as C
+import os
+import subprocess
 
 import numpy as np
 import pytest
 
-from horsepower_gb300.abi import DTYPE, H_E, H_F, H_H, H_I, H_L
+from horsepower_gb300.abi import Builtins, DTYPE, H_B, H_E, H_F, H_H, H_I, H_L
 
 pytestmark = pytest.mark.gpu
 
@@ -19,6 +21,13 @@ def gpu():
     L = horsepower_gb300.load()
     L.lib.hgpuProfileRead.argtypes = [C.c_int32, C.POINTER(C.c_char_p), C.POINTER(C.c_double), C.POINTER(C.c_longlong)]
     return L
+
+
+@pytest.fixture(scope="module")
+def ora():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run(["make", "-s", "-C", os.path.join(root, "oracle"), "port"], check=True)
+    return Builtins(os.path.join(root, "oracle", "_build", "liboracle.so"), "oracle")
 
 
 def launches(L, fn):
@@ -55,3 +64,33 @@ def test_member_routes(gpu, typ, span, kernel, n):
     assert np.array_equal(gpu.to_py(z), np.isin(y, x))
     assert {k for k in got if k.startswith("member")} == {kernel}, got
     gpu.free_inputs()
+
+
+def order(L, x, asc=True):
+    return L.to_py(L.call("pfnOrderBy", L.vec(x, H_E), L.vec(np.array([asc]), H_B)))
+
+
+@pytest.mark.parametrize("n", [2048 * 4096, 2048 * 4096 + 1, 2048 * 4103 + 77])
+def test_quicksort_tile_sums(gpu, ora, n):
+    """Above 4096 tiles the tile sums of a quicksort depth are scanned by a
+    kernel of their own instead of added up by every block; keys with ties,
+    so that the permutation is the sequential quicksort's and no other."""
+    x = np.random.default_rng(n).integers(0, n // 2, n) * 0.5
+    got, k = launches(gpu, lambda: order(gpu, x))
+    assert ("qs_scan_sums" in k) == (n > 2048 * 4096), k
+    assert np.array_equal(got, order(ora, x))
+    gpu.free_inputs()
+    ora.free_inputs()
+
+
+@pytest.mark.parametrize("values", [1, 3, 5])
+def test_quicksort_few_values(gpu, ora, values):
+    """Keys of few values are sorted after a few depths: no more than the first
+    round of depths is issued for them."""
+    n = 700_001
+    x = np.random.default_rng(values).integers(0, values, n) * 0.5
+    got, k = launches(gpu, lambda: order(gpu, x))
+    assert 0 < k["qs_count"] <= 8, k
+    assert np.array_equal(got, order(ora, x))
+    gpu.free_inputs()
+    ora.free_inputs()
