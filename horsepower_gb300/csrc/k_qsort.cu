@@ -45,7 +45,12 @@ constexpr unsigned QS_DONE = 0xffffffffu;
 constexpr int QS_THREADS = 256, QS_ITEMS = 8, QS_TILE = QS_THREADS * QS_ITEMS;
 constexpr int QS_WARP = 32;         // largest range one warp sorts
 constexpr int QS_BLOCK = 4096;      // largest range one CTA sorts in shared memory
-constexpr int QB_THREADS = 1024, QB_ITEMS = QS_BLOCK / QB_THREADS, QB_WARPS = QB_THREADS / 32;
+// CTAs of QB_ITEMS elements a thread: of 32 threads for ranges of up to 128
+// elements, 128 for up to 512 and 1024 for up to QS_BLOCK
+constexpr int QB_ITEMS = 4, QB_CLASSES = 3;
+__host__ __device__ constexpr int qb_threads(int c) { return c == 0 ? 32 : c == 1 ? 128 : 1024; }
+__host__ __device__ constexpr int qb_rows(int c) { return qb_threads(c) * QB_ITEMS; }
+static_assert(qb_rows(QB_CLASSES - 1) == QS_BLOCK, "the largest CTA takes the largest listed range");
 // A range handed to a CTA or a warp: positions [lo, hi), the recursion depth
 // at which it was made, and whether its elements lie in the local buffers
 // (made by a partition) or in the sort's own (a range it started with).
@@ -54,20 +59,23 @@ struct QsRange {
 };
 // counters of one sort, in device memory
 struct QsCounters {
-    unsigned nblock, nwarp;  // ranges listed for CTAs and warps
+    unsigned nblock[QB_CLASSES], nwarp;  // ranges listed for CTAs of each size and for warps
     unsigned nbig;           // ranges the sort starts with that neither takes
     unsigned depth;          // recursion depth reached by the listed ranges
     unsigned nrev, nan;      // segments to reverse; a NaN key was seen
 };
 struct QsLists {
-    QsRange* block;
+    QsRange* block[QB_CLASSES];
     QsRange* warp;
     QsCounters* cnt;
 };
 __device__ __forceinline__ void qs_list(const QsLists& q, unsigned lo, unsigned hi, unsigned depth, unsigned local) {
     const unsigned m = hi - lo;
-    if (m > QS_WARP) q.block[atomicAdd(&q.cnt->nblock, 1u)] = QsRange{lo, hi, depth, local};
-    else q.warp[atomicAdd(&q.cnt->nwarp, 1u)] = QsRange{lo, hi, depth, local};
+    if (m > QS_WARP) {
+        const int c = m <= qb_rows(0) ? 0 : m <= qb_rows(1) ? 1 : 2;
+        QsRange* list = c == 0 ? q.block[0] : c == 1 ? q.block[1] : q.block[2];
+        list[atomicAdd(&q.cnt->nblock[c], 1u)] = QsRange{lo, hi, depth, local};
+    } else q.warp[atomicAdd(&q.cnt->nwarp, 1u)] = QsRange{lo, hi, depth, local};
 }
 // A recursion deeper than max(8192, 2^36 / n) levels, rounded up to a multiple
 // of 8 (first-element pivots on nearly ordered keys, where the reference's own
@@ -660,31 +668,50 @@ __global__ void __launch_bounds__(256) k_qs_warps(QsLists lists, const unsigned 
 // are scanned with shuffles (one word a lane; each thread adding up all 32 of
 // them was a fifth of the instructions), and a warp without a live element
 // only passes the prefix on (ranges of a 114K-row sort: 0.108 -> 0.097 ms).
+// Short ranges take small CTAs, many to an SM: with 1024 threads for every
+// range a list order over 10M rows in segments of 40, 100 or 300 rows took 10.4,
+// 9.7 and 6.2 ms, and takes 2.0, 2.0 and 2.2.
+template <int C>
 struct QsBlockSmem {
-    unsigned long long K[QS_BLOCK];
-    unsigned P[QS_BLOCK];
-    unsigned S[QS_BLOCK + 1];         // exclusive prefix: (<= P) in the low half, (< P) in the high half
-    unsigned short L[QS_BLOCK], R[QS_BLOCK];
-    unsigned small[QS_BLOCK / 2];     // lo | (size - 1) << 12 | depth << 17
-    unsigned wt[QB_WARPS];
-    uint8_t slots[QB_WARPS][64];
+    static constexpr int ROWS = qb_rows(C), WARPS = qb_threads(C) / 32;
+    unsigned long long K[ROWS];
+    unsigned P[ROWS];
+    unsigned S[ROWS + 1];             // exclusive prefix: (<= P) in the low half, (< P) in the high half
+    unsigned short L[ROWS], R[ROWS];
+    unsigned small[ROWS / 2];         // lo | (size - 1) << 12 | depth << 17
+    unsigned wt[32];
+    uint8_t slots[WARPS][64];
     unsigned nsmall, depth;
 };
 static_assert(QS_BLOCK <= 4096 && QS_WARP <= 32, "packing of QsBlockSmem::small");
-__global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, const unsigned long long* __restrict__ K0,
-                                                             const unsigned* __restrict__ P0,
-                                                             const unsigned long long* __restrict__ KL,
-                                                             const unsigned* __restrict__ PL, unsigned* __restrict__ fin,
-                                                             unsigned* derr) {
+template <int C>
+__global__ void __launch_bounds__(qb_threads(C), C == 0 ? 24 : 1024 / qb_threads(C))
+k_qs_blocks(const __grid_constant__ QsLists lists, const unsigned long long* __restrict__ K0,
+            const unsigned* __restrict__ P0, const unsigned long long* __restrict__ KL, const unsigned* __restrict__ PL,
+            unsigned* __restrict__ fin, int low, unsigned* derr) {
     grid_entry();
     extern __shared__ __align__(16) unsigned char qb_smem[];
-    QsBlockSmem& sm = *reinterpret_cast<QsBlockSmem*>(qb_smem);
+    using Smem = QsBlockSmem<C>;
+    Smem& sm = *reinterpret_cast<Smem*>(qb_smem);
     const unsigned lane = lane_id(), w = threadIdx.x >> 5, p0 = w * (32 * QB_ITEMS) + lane;
     auto le = [](unsigned s) { return s & 0xffffu; };
     auto lt = [](unsigned s) { return s >> 16; };
-    const unsigned n = lists.cnt->nblock;
+    unsigned cnt[C + 1], n = 0;
+#pragma unroll
+    for (int c = 0; c <= C; c++) {
+        cnt[c] = lists.cnt->nblock[c];
+        if (c >= low) n += cnt[c];
+    }
     for (unsigned r = blockIdx.x; r < n; r += gridDim.x) {
-        const QsRange g = lists.block[r];
+        int c = C;  // the lists one after another, the longest ranges first
+        unsigned at = r;
+#pragma unroll
+        for (int q = C; q > 0; q--)
+            if (c == q && at >= cnt[q]) {
+                at -= cnt[q];
+                c = q - 1;
+            }
+        const QsRange g = lists.block[c][at];
         const unsigned m = g.hi - g.lo;
         if (threadIdx.x == 0) sm.nsmall = sm.depth = 0;
         unsigned long long key[QB_ITEMS];
@@ -729,8 +756,7 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, cons
             if (lane == 0) sm.wt[w] = run;
             __syncthreads();
             // every warp scans the warps' totals for itself
-            static_assert(QB_WARPS == 32, "one total a lane");
-            const unsigned wt = sm.wt[lane], wi = warp_incl_scan(wt);
+            const unsigned wt = lane < Smem::WARPS ? sm.wt[lane] : 0u, wi = warp_incl_scan(wt);
             const unsigned base = __shfl_sync(0xffffffffu, wi - wt, w), all = __shfl_sync(0xffffffffu, wi, 31);
 #pragma unroll
             for (int k = 0; k < QB_ITEMS; k++)
@@ -798,7 +824,7 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qs_blocks(QsLists lists, cons
         // every range of 2 to 32 elements left in the CTA
         unsigned deep = depths;
         const unsigned ns = sm.nsmall;
-        for (unsigned q = w; q < ns; q += QB_WARPS) {
+        for (unsigned q = w; q < ns; q += Smem::WARPS) {
             const unsigned v = sm.small[q], a = v & 4095u, mm = ((v >> 12) & 31u) + 1;
             unsigned long long k = 0;
             unsigned p = 0;
@@ -987,10 +1013,14 @@ static I qs_too_deep(long long levels) {
 }
 
 static I qs_lists_alloc(long long n, QsLists* q) {
-    q->block = (QsRange*)salloc((size_t)(n / QS_WARP + 1) * sizeof(QsRange));
+    bool ok = true;
+    for (int c = 0; c < QB_CLASSES; c++) {  // the class's shortest range: one more than the class below holds
+        q->block[c] = (QsRange*)salloc((size_t)(n / (c ? qb_rows(c - 1) : QS_WARP) + 1) * sizeof(QsRange));
+        ok = ok && q->block[c];
+    }
     q->warp = (QsRange*)salloc((size_t)(n / 2 + 1) * sizeof(QsRange));
     q->cnt = (QsCounters*)salloc(sizeof(QsCounters));
-    return q->block && q->warp && q->cnt ? 0 : E_DEVICE_OOM;
+    return ok && q->warp && q->cnt ? 0 : E_DEVICE_OOM;
 }
 
 // NaN keys, from counters already read back
@@ -1017,6 +1047,37 @@ static bool qs_depths_launch(long long n, QsDepths& q) {
     if (launch_cooperative_args(kern, grid_for(n, QD_THREADS * e), QD_THREADS, 0, args) == cudaSuccess) return true;
     cudaGetLastError();  // clears the refused launch's own error
     return false;
+}
+
+// the ranges of classes low to C, in CTAs of class C
+template <int C>
+static I qs_blocks(const QsLists& lists, const QsCounters& h, int low, const unsigned long long* img, const unsigned* perm,
+                   const unsigned long long* KL, const unsigned* PL, unsigned* fin) {
+    unsigned n = 0;
+    for (int c = low; c <= C; c++) n += h.nblock[c];
+    if (!n) return 0;
+    const int dsm = (int)sizeof(QsBlockSmem<C>);
+    // the attribute belongs to the current device's context: set it on every call (a host-side write)
+    HG_CU(cudaFuncSetAttribute(k_qs_blocks<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
+    const unsigned cap = (unsigned)g_sms * (2048 / qb_threads(C));
+    HG_LAUNCH(C == 0 ? "qs_blocks_128" : C == 1 ? "qs_blocks_512" : "qs_blocks", n < cap ? n : cap, qb_threads(C), (size_t)dsm,
+              k_qs_blocks<C>, lists, img, perm, KL, PL, fin, low, g_derr);
+    return last_launch_error();
+}
+// Short ranges have launches of their own, in small CTAs, when a class has more
+// than QB_OWN ranges a SM.  Fewer go with the class above: the launches follow
+// one another, each as long as its deepest range, while large CTAs that would
+// stand idle take them at once (100K random keys 0.27 ms, 0.33 with three
+// launches; 114K rows in segments of 300, some 2.5 a SM: 0.226 and 0.192).
+constexpr unsigned QB_OWN0 = 2, QB_OWN1 = 2;
+static I qs_all_blocks(const QsLists& lists, const QsCounters& h, const unsigned long long* img, const unsigned* perm,
+                       const unsigned long long* KL, const unsigned* PL, unsigned* fin) {
+    const bool own0 = h.nblock[0] > QB_OWN0 * g_sms;
+    const bool own1 = h.nblock[1] + (own0 ? 0 : h.nblock[0]) > QB_OWN1 * g_sms;
+    HG_CHECK(qs_blocks<2>(lists, h, own1 ? 2 : own0 ? 1 : 0, img, perm, KL, PL, fin));
+    if (own1) HG_CHECK(qs_blocks<1>(lists, h, own0 ? 1 : 0, img, perm, KL, PL, fin));
+    if (own0) HG_CHECK(qs_blocks<0>(lists, h, 0, img, perm, KL, PL, fin));
+    return 0;
 }
 
 // The quicksort of every sorted range at once.  perm/img: the elements in
@@ -1117,14 +1178,7 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
             if (left == 0) break;
         }
     }
-    if (h->nblock) {
-        const int dsm = (int)sizeof(QsBlockSmem);
-        // the attribute belongs to the current device's context: set it on every call (a host-side write)
-        HG_CU(cudaFuncSetAttribute(k_qs_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
-        const unsigned cap = 2u * (unsigned)g_sms;
-        HG_LAUNCH("qs_blocks", h->nblock < cap ? h->nblock : cap, QB_THREADS, (size_t)dsm, k_qs_blocks, lists, img, perm, KL,
-                  PL, fin, g_derr);
-    }
+    HG_CHECK(qs_all_blocks(lists, *h, img, perm, KL, PL, fin));
     if (h->nwarp) {
         const unsigned cap = 16u * (unsigned)g_sms, want = grid_for(h->nwarp, 8);
         HG_LAUNCH("qs_warps", want < cap ? want : cap, 256, 0, k_qs_warps, lists, img, perm, KL, PL, fin);
@@ -1221,7 +1275,7 @@ I qs_sort_list(int nc, const void* const* cols, const I* typs, const B* asc, lon
             unsigned* t = perm; perm = tmp; tmp = t;
             HG_CHECK(qs_image_of(cols[c], typ, perm, n, desc, img, nanflag));
         }
-        if (!h.nbig && !h.nblock && (!h.nwarp || stable)) {
+        if (!h.nbig && !h.nblock[0] && !h.nblock[1] && !h.nblock[2] && (!h.nwarp || stable)) {
             // nothing is left to sort, or only short segments in stable order
             if (h.nwarp) {
                 const unsigned cap = 16u * (unsigned)g_sms, want = grid_for(h.nwarp, 8);

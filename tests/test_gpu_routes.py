@@ -94,3 +94,30 @@ def test_quicksort_few_values(gpu, ora, values):
     assert np.array_equal(got, order(ora, x))
     gpu.free_inputs()
     ora.free_inputs()
+
+
+@pytest.mark.parametrize("copies,kernels", [(7, {"qs_blocks"}), (200, {"qs_blocks", "qs_blocks_128", "qs_blocks_512"})])
+def test_quicksort_classes(gpu, ora, copies, kernels):
+    """Segments of a list order on either side of what a CTA of 32, 128 and
+    1024 threads holds: many of a size have a launch of their own, few go with
+    the larger ones.  Keys with ties, some segments of one value or ordered."""
+    sizes = np.tile([32, 33, 64, 127, 128, 129, 200, 511, 512, 513, 1024, 4095, 4096], copies)
+    rng = np.random.default_rng(copies)
+    rng.shuffle(sizes)
+    seg = np.repeat(np.arange(sizes.size, dtype=np.int32), sizes)
+    key = rng.integers(0, 60, seg.size) * 0.5
+    key[np.isin(seg, np.arange(0, sizes.size, 11))] = 2.0
+    rising = np.isin(seg, np.arange(3, sizes.size, 13))
+    key[rising] = np.arange(rising.sum())
+    mix = rng.permutation(seg.size)
+    seg, key = seg[mix], key[mix]
+
+    def run(L, up=(True, True)):
+        return L.to_py(L.call("pfnOrderBy", L.list([L.vec(seg, H_I), L.vec(key, H_E)]), L.vec(np.array(up), H_B)))
+
+    got, k = launches(gpu, lambda: run(gpu))
+    assert {x for x in k if x.startswith("qs_blocks")} == kernels, k
+    assert np.array_equal(got, run(ora))
+    assert np.array_equal(run(gpu, (True, False)), run(ora, (True, False)))
+    gpu.free_inputs()
+    ora.free_inputs()
