@@ -49,6 +49,13 @@ int get_radix_digit_bits() { return g_digit_bits; }
 static int g_radix_pass = 2;
 void set_radix_pass_mode(int m) { g_radix_pass = m < 0 ? 0 : (m > 2 ? 2 : m); }
 int get_radix_pass_mode() { return g_radix_pass; }
+static bool counted_passes(long long n) { return g_radix_pass != 0 && n <= RX_MAX_ROWS; }
+// Row ids are 32 bits wide on either path: checked before a sort's memory is
+// taken, so that no result is left half written.
+static I radix_rows(long long n) {
+    if (n <= RX_MAX_ROWS + 1) return 0;
+    return set_error(E_NOT_IMPL, "radix order or grouping of more than 2^32 rows");
+}
 
 template <typename SRC>
 __global__ void k_key_bits(SRC src, long long n, unsigned long long* orv, unsigned long long* andv) {
@@ -348,6 +355,7 @@ template <typename SRC, typename KR>
 static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, const unsigned* init_vals,
                  unsigned long long vary_hint, const RadixOut* out) {
     using K = typename SRC::key_t;
+    if (n > RX_MAX_ROWS) return set_error(E_NOT_IMPL, "counted radix passes over more than 2^32 - 1 rows");
     unsigned long long vary = vary_hint;
     if (!vary_hint && n > 1) HG_CHECK(varying_bits(src, n, &vary));
     if (vary == 0 || n <= 1) return identity_order<SRC, KR>(src, n, kres, vres, init_vals, out);
@@ -530,7 +538,8 @@ static I lookback_sort(const K* keys, long long n, const K** kres, const unsigne
 
 template <typename K>
 I radix_sort(const K* keys, long long n, const K** kres, const unsigned** vres, const unsigned* init_vals = nullptr) {
-    if (g_radix_pass == 0) return lookback_sort<K>(keys, n, kres, vres, init_vals, 0, nullptr, nullptr);
+    HG_CHECK(radix_rows(n));
+    if (!counted_passes(n)) return lookback_sort<K>(keys, n, kres, vres, init_vals, 0, nullptr, nullptr);
     return rx_sort<RxKeys<K>, K>(RxKeys<K>{keys}, n, kres, vres, init_vals, 0, nullptr);
 }
 
@@ -971,10 +980,11 @@ struct SortResult {
 template <typename K>
 static I sort_keys_spec(const KeySpec& s, long long n, unsigned long long vary_hint, const RadixOut* ro,
                         SortResult* r) {
+    HG_CHECK(radix_rows(n));
     const K* ks = nullptr;
     const unsigned long long hint0 = n > 1 ? vary_hint : 0;
     r->perm64 = ro ? ro->perm64 : nullptr;
-    if (g_radix_pass != 0) {
+    if (counted_passes(n)) {
         // the first counted pass reads the columns themselves where the key
         // is one integer column's bits or two range-compressed ones packed
         // (150M rows: writing and reading a key array took 0.5 - 1 ms)
@@ -1004,7 +1014,7 @@ static I sort_keys_spec(const KeySpec& s, long long n, unsigned long long vary_h
     }
     K* k = (K*)salloc((size_t)(n > 0 ? n : 1) * sizeof(K));
     if (!k) return E_DEVICE_OOM;
-    if (g_radix_pass != 0) {
+    if (counted_passes(n)) {
         if (n > 0) HG_LAUNCH("make_keys", gcap(n), 256, 0, k_make_keys<K>, s, n, k);
         HG_CHECK((rx_sort<RxKeys<K>, K>(RxKeys<K>{k}, n, &ks, &r->perm, nullptr, hint0, ro)));
         r->keys = ks;
@@ -1194,6 +1204,7 @@ static I final_order(const KeySpec& s, long long n, const uint8_t* dirbit, SortR
 }
 
 static I order_columns_exact(int nc, V* cols, const void** ptrs, const B* asc, long long n, SortResult* r) {
+    HG_CHECK(radix_rows(n));
     uint8_t* dirbit = (uint8_t*)salloc((size_t)(n > 0 ? n : 1));
     unsigned* flags = (unsigned*)salloc((size_t)(n > 0 ? n : 1) * 4 + 16);
     if (!dirbit || !flags) return E_DEVICE_OOM;
@@ -1305,6 +1316,7 @@ static I group_finish(V z, long long* starts, long long G, long long* perm, long
 static I order_prealloc(V z, long long n, bool reverse, RadixOut* ro, void** d) {
     *d = nullptr;
     if (n <= 1) return 0;
+    HG_CHECK(radix_rows(n));
     HG_CHECK(alloc_out(z, H_L, n, d));
     ro->perm64 = (long long*)*d;
     ro->reverse = reverse;
@@ -1577,6 +1589,7 @@ I pfnGroupBasic(V z, V x) {
             }
         }
         // the permutation is allocated first, so that the last radix pass writes it
+        HG_CHECK(radix_rows(x->len));
         long long* pre = x->len > 1 ? (long long*)dalloc((size_t)x->len * 8) : nullptr;
         if (x->len > 1 && !pre) return E_DEVICE_OOM;
         RadixOut ro;
@@ -1614,6 +1627,7 @@ I pfnGroupBasic(V z, V x) {
             s.ncol = 2;
             s.col[0] = ptrs[0]; s.typ[0] = H_I; s.xf[0] = XF_CASE1;
             s.col[1] = ptrs[1]; s.typ[1] = H_I;
+            HG_CHECK(radix_rows(n));
             // 32 or 64 bits as lib_radixsort_long decides on the packed keys
             unsigned long long* k = (unsigned long long*)salloc((size_t)(n > 0 ? n : 1) * 8);
             if (!k) return E_DEVICE_OOM;
@@ -1719,6 +1733,7 @@ I pfnOrderBy(V z, V x, V y) {
             const void *p0, *p1;
             HG_CHECK(in_ptr(&c[0], &p0));
             HG_CHECK(in_ptr(&c[1], &p1));
+            HG_CHECK(radix_rows(n));
             KeySpec s{};
             s.ncol = 2;
             s.col[0] = p0; s.typ[0] = H_I; s.xf[0] = XF_CASE1;

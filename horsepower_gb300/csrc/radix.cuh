@@ -110,6 +110,7 @@ __device__ __forceinline__ unsigned rx_match(unsigned d) {
 // records, ms, 8 and 9 bits:  3 x 16 0.585 and 0.84;  3 x 12 0.63, 1.01;
 // 2 x 20 0.61, 0.71;  2 x 24 0.60, 0.676;  2 x 28 0.61, 0.71;  2 x 32 0.67,
 // 0.75;  4 x 10 0.73, 1.2.
+constexpr long long RX_MAX_ROWS = 0xffffffffll;  // counts, positions and row ids are 32 bits wide
 constexpr int RX_THREADS = 256, RX_WARPS = RX_THREADS / 32, RX_MAX_PER_SM = 3, RX_MAX_DIGITS = 512;
 template <int BITS>
 struct RxShape {

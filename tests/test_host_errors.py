@@ -1,0 +1,75 @@
+"""Host code around launches, on a CUDA runtime without a device
+(tests/fake_cudart.c): what is refused before memory is taken or a kernel
+runs, and what becomes of a launch that fails.  No GPU is used: each test is a
+child process with the stand-in preloaded, in which kernels do nothing.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+CUDA = next((d for d in (os.environ.get("CUDA_HOME"), "/usr/local/cuda") if d and os.path.isdir(d)), "/usr/local/cuda")
+
+PRELUDE = r"""
+import ctypes as C, sys
+sys.path.insert(0, sys.argv[1])
+import horsepower_gb300
+from horsepower_gb300.abi import V0, H_B, H_C, H_E, H_I, H_L
+import numpy as np
+fake = C.CDLL(None)
+L = horsepower_gb300.load(build_if_missing=False)
+fake.cudaMalloc.argtypes = [C.c_void_p, C.c_size_t]
+
+def column(typ, n, width):
+    p = C.c_void_p()
+    assert fake.cudaMalloc(C.byref(p), n * width) == 0
+    v = V0()
+    v.typ, v.len, v.g = typ, n, p.value
+    return v
+
+def count(*names):
+    return [fake.fake_count(k.encode()) for k in names]
+
+up, down = (L.vec(np.array([a]), H_B) for a in (True, False))
+"""
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    if not os.path.exists(os.path.join(ROOT, "horsepower_gb300", "libhgpu.so")):
+        pytest.skip("libhgpu.so is not built")
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    r = subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-w", "-I" + os.path.join(CUDA, "include"), "-o", so,
+                        os.path.join(HERE, "fake_cudart.c")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def run(body, **env):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + body, ROOT], capture_output=True, text=True, timeout=300,
+                           env=dict(os.environ, LD_PRELOAD=so, **env))
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_rows_beyond_the_row_ids(child):
+    """@order and @group by radix passes refuse more than 2^32 rows, whose row
+    ids do not fit 32 bits, before a pass runs; 2^32 rows, one more than the
+    counted passes' positions hold, take the look-back passes.  (The stand-in's
+    key statistics read as if every bit varied.)"""
+    child(r"""
+one, two = (lambda x: x), (lambda x: L.list([x, x]))
+for n, rc, passes in ((2**32 - 1, 0, "k_rx_scatter"), (2**32, 0, "k_onesweep"), (2**32 + 1, 99, None)):
+    for typ, width, shape in ((H_I, 4, one), (H_L, 8, one), (H_I, 4, two)):
+        x = shape(column(typ, n, width))
+        dirs = [L.vec(np.array([a] * (2 if shape is two else 1)), H_B) for a in (True, False)]
+        for call in (lambda: L.rc("pfnOrderBy", x, dirs[0]), lambda: L.rc("pfnOrderBy", x, dirs[1]), lambda: L.rc("pfnGroup", x)):
+            fake.fake_reset()
+            L.lib.setHeapOffset(0)
+            assert call() == rc, (n, typ, L.lib.hgpuLastError())
+            ran = [k for k in ("k_rx_scatter", "k_onesweep") if count(k)[0]]
+            assert ran == ([passes] if passes else []), (n, typ, ran)
+x = column(H_C, 2**32 + 1, 1)
+assert L.rc("pfnOrderBy", x, up) == 99 and L.rc("pfnGroup", x) == 99
+""")
