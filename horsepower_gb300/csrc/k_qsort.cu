@@ -1031,22 +1031,28 @@ static I qs_nan_check(const QsCounters& h) {
 }
 
 // Launches k_qs_depths when n elements fit one block per SM of at most 4 per
-// thread; false when they do not, or the device does not take the blocks
+// thread; *took = false when they do not, or the device does not take the blocks
 // together.  @order of random f64 keys, us, with four launches a depth and
 // with this: 6000 rows 182 and 162, 20K 225 and 191, 114K 351 and 287, 300K 407
 // and 326, 600K 635 and 511; with 8 per thread (the registers spill) 600K 767,
 // 1.2M 1064 against 1045.  (The CTA tier has since become 5 to 10 us faster on
 // either side.)
-static bool qs_depths_launch(long long n, QsDepths& q) {
+static I qs_depths_launch(long long n, QsDepths& q, bool* took) {
     void* args[] = {&q};
+    *took = false;
     const long long most = (long long)(g_sms < QD_MAX_BLOCKS ? g_sms : QD_MAX_BLOCKS) * QD_THREADS;
     const int e = n <= 2 * most ? 2 : 4;
-    if (n > e * most) return false;
+    if (n > e * most) return 0;
+    HG_CHECK(last_launch_error());  // of the launches before, while the error is theirs
     const void* kern = e == 2 ? (const void*)k_qs_depths<2> : (const void*)k_qs_depths<4>;
     LaunchScope ls("qs_depths");
-    if (launch_cooperative_args(kern, grid_for(n, QD_THREADS * e), QD_THREADS, 0, args) == cudaSuccess) return true;
-    cudaGetLastError();  // clears the refused launch's own error
-    return false;
+    const cudaError_t rc = launch_cooperative_args(kern, grid_for(n, QD_THREADS * e), QD_THREADS, 0, args);
+    *took = rc == cudaSuccess;
+    if (*took) return 0;
+    cudaGetLastError();  // the refused launch's own
+    if (rc == cudaErrorCooperativeLaunchTooLarge || rc == cudaErrorNotSupported) return 0;
+    HG_CU(rc);
+    return 0;
 }
 
 // the ranges of classes low to C, in CTAs of class C
@@ -1132,7 +1138,7 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                 QsDepths q{lo, hi, {Kc, Kc == img ? K2 : img}, {Pc, Pc == perm ? P2 : perm}, S, ts, Lpos, Rpos, fin,
                            act, act + QD_ROUND, act + QD_ROUND + 1, KL, PL, lists, g_derr, (unsigned)n, (unsigned)level,
                            (unsigned)round};
-                resident = qs_depths_launch(n, q);
+                HG_CHECK(qs_depths_launch(n, q, &resident));
                 if (resident) {
                     unsigned res[2];
                     HG_CHECK(rb_queue(res, q.done, 8));

@@ -73,3 +73,31 @@ for n, rc, passes in ((2**32 - 1, 0, "k_rx_scatter"), (2**32, 0, "k_onesweep"), 
 x = column(H_C, 2**32 + 1, 1)
 assert L.rc("pfnOrderBy", x, up) == 99 and L.rc("pfnGroup", x) == 99
 """)
+
+
+@pytest.mark.parametrize("kernel,err,rc,passes", [
+    ("", 0, 100, True),                # nothing fails: the stand-in's barrier result reads as one that gave up
+    ("k_qs_depths", 720, 0, True),     # cudaErrorCooperativeLaunchTooLarge: the depths take launches of their own
+    ("k_qs_depths", 801, 0, True),     # cudaErrorNotSupported: the same
+    ("k_qs_depths", 1, 100, False),    # any other refusal is the call's error
+    ("k_qs_depths", 719, 100, False),
+    ("k_qs_ranges", 1, 100, False),    # a failed launch before it is not taken for its refusal
+])
+def test_quicksort_launch_errors(child, kernel, err, rc, passes):
+    """The quicksort's resident kernel may be refused, which has a path of its
+    own; every other failed launch of the sort is reported."""
+    child(r"""
+kernel, err, rc, passes = %r, %d, %d, %r
+x = column(H_E, 10_000, 8)
+fake.fake_reset()
+if kernel:
+    fake.fake_fail(kernel.encode(), err)
+fake.fake_poke(b"k_qs_whole", 1, 32, 4, 1)  # QsCounters::nbig: one range for the depths
+got = L.rc("pfnOrderBy", x, up)
+assert got == rc, (got, L.lib.hgpuLastError())
+took, own = count("k_qs_depths", "k_qs_count")
+if not kernel:
+    assert took == 1 and b"barrier" in L.lib.hgpuLastError()
+else:
+    assert took == 0 and (own > 0) == passes, own
+""" % (kernel, err, rc, passes))
