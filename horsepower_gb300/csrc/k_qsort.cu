@@ -52,10 +52,20 @@ __host__ __device__ constexpr int qb_threads(int c) { return c == 0 ? 32 : c == 
 __host__ __device__ constexpr int qb_rows(int c) { return qb_threads(c) * QB_ITEMS; }
 static_assert(qb_rows(QB_CLASSES - 1) == QS_BLOCK, "the largest CTA takes the largest listed range");
 // A range handed to a CTA or a warp: positions [lo, hi), the recursion depth
-// at which it was made, and whether its elements lie in the local buffers
-// (made by a partition) or in the sort's own (a range it started with).
+// at which it was made, and which of the sort's two buffers holds its elements.
+// Both buffers are free for them: a depth reads one and writes the other, and
+// later depths touch neither at the positions of a listed range.
 struct QsRange {
-    unsigned lo, hi, depth, local;
+    unsigned lo, hi, depth, buf;
+};
+// ... of up to QS_WARP elements, of which a sort may list one for every two
+// rows, in half the space.  The depth fits: no more than the rows of a small
+// sort, or 2^36 by the rows of a large one, either way below 2^19.
+struct QsShort {
+    unsigned lo, rest;  // size - 1, buffer << 5, depth << 6
+    __device__ __forceinline__ QsRange range() const {
+        return QsRange{lo, lo + (rest & 31u) + 1, rest >> 6, (rest >> 5) & 1u};
+    }
 };
 // counters of one sort, in device memory
 struct QsCounters {
@@ -66,16 +76,18 @@ struct QsCounters {
 };
 struct QsLists {
     QsRange* block[QB_CLASSES];
-    QsRange* warp;
+    QsShort* warp;
     QsCounters* cnt;
 };
-__device__ __forceinline__ void qs_list(const QsLists& q, unsigned lo, unsigned hi, unsigned depth, unsigned local) {
+__device__ __forceinline__ void qs_list(const QsLists& q, unsigned lo, unsigned hi, unsigned depth, unsigned buf) {
     const unsigned m = hi - lo;
     if (m > QS_WARP) {
         const int c = m <= qb_rows(0) ? 0 : m <= qb_rows(1) ? 1 : 2;
         QsRange* list = c == 0 ? q.block[0] : c == 1 ? q.block[1] : q.block[2];
-        list[atomicAdd(&q.cnt->nblock[c], 1u)] = QsRange{lo, hi, depth, local};
-    } else q.warp[atomicAdd(&q.cnt->nwarp, 1u)] = QsRange{lo, hi, depth, local};
+        list[atomicAdd(&q.cnt->nblock[c], 1u)] = QsRange{lo, hi, depth, buf};
+    } else {
+        q.warp[atomicAdd(&q.cnt->nwarp, 1u)] = QsShort{lo, (m - 1) | (buf << 5) | (depth << 6)};
+    }
 }
 // A recursion deeper than max(8192, 2^36 / n) levels, rounded up to a multiple
 // of 8 (first-element pivots on nearly ordered keys, where the reference's own
@@ -293,14 +305,14 @@ __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __rest
 
 // Moves every element of the partitioned ranges to its place, records the
 // next depth's range of every element (or its final place; ranges of up to
-// QS_BLOCK elements go to the local buffers and lists) and counts the elements
-// still in a larger range.
+// QS_BLOCK elements go to the lists) and counts the elements still in a larger
+// range.  buf: which buffer K2 and P2 are.
 __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, const unsigned long long* __restrict__ K,
                           const unsigned* __restrict__ P, const unsigned long long* __restrict__ S, long long n,
                           const unsigned* __restrict__ Lpos, const unsigned* __restrict__ Rpos,
                           unsigned long long* __restrict__ K2, unsigned* __restrict__ P2, unsigned* __restrict__ fin,
-                          const unsigned* prev, unsigned* active, unsigned depth, unsigned long long* __restrict__ KL,
-                          unsigned* __restrict__ PL, QsLists lists, unsigned* derr) {
+                          const unsigned* prev, unsigned* active, unsigned depth, unsigned buf, QsLists lists,
+                          unsigned* derr) {
     grid_entry();
     if (qs_idle(prev)) return;
     unsigned still = 0;
@@ -344,10 +356,10 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
             fin[p] = P[q];
             lo[p] = QS_DONE;
         } else if (nh - nl <= QS_BLOCK) {
-            PL[p] = P[q];
-            KL[p] = K[q];
+            P2[p] = P[q];
+            K2[p] = K[q];
             lo[p] = QS_DONE;
-            if (p == nl) qs_list(lists, (unsigned)nl, (unsigned)nh, depth + 1, 1);
+            if (p == nl) qs_list(lists, (unsigned)nl, (unsigned)nh, depth + 1, buf);
         } else {
             P2[p] = P[q];
             K2[p] = K[q];
@@ -379,11 +391,9 @@ struct QsDepths {
     unsigned *Lpos, *Rpos, *fin;
     unsigned *act, *bar;  // elements left after each depth of this launch; the barrier's arrivals (all zero)
     unsigned* done;       // depths run, then elements left
-    unsigned long long* KL;
-    unsigned* PL;
     QsLists lists;
     unsigned* derr;
-    unsigned n, level, maxd;
+    unsigned n, level, maxd, buf;  // buf: which buffer K[0] and P[0] are
 };
 __device__ __forceinline__ bool qd_barrier(unsigned* bar, unsigned& target, unsigned* derr) {
     __shared__ bool ok;
@@ -558,17 +568,17 @@ __global__ void __launch_bounds__(QD_THREADS, 1) k_qs_depths(const __grid_consta
             if (p == j || nh - nl < 2) {
                 a.fin[p] = row[k];
                 lo[k] = QS_DONE;
-            } else if (nh - nl <= (unsigned)QS_BLOCK) {
-                a.PL[p] = row[k];
-                a.KL[p] = key[k];
-                lo[k] = QS_DONE;
-                if (p == nl) qs_list(a.lists, nl, nh, a.level + d + 1, 1);
             } else {
                 a.P[(d & 1) ^ 1][p] = row[k];
                 a.K[(d & 1) ^ 1][p] = key[k];
-                lo[k] = nl;
-                hi[k] = nh;
-                still++;
+                if (nh - nl <= (unsigned)QS_BLOCK) {
+                    lo[k] = QS_DONE;
+                    if (p == nl) qs_list(a.lists, nl, nh, a.level + d + 1, a.buf ^ (d & 1) ^ 1);
+                } else {
+                    lo[k] = nl;
+                    hi[k] = nh;
+                    still++;
+                }
             }
         }
         still = warp_sum(still);
@@ -638,20 +648,20 @@ __device__ __forceinline__ unsigned qs_warp_range(unsigned long long k, unsigned
 // the listed ranges of 2 to 32 elements, one warp each
 __global__ void __launch_bounds__(256) k_qs_warps(QsLists lists, const unsigned long long* __restrict__ K0,
                                                   const unsigned* __restrict__ P0,
-                                                  const unsigned long long* __restrict__ KL,
-                                                  const unsigned* __restrict__ PL, unsigned* __restrict__ fin) {
+                                                  const unsigned long long* __restrict__ K1,
+                                                  const unsigned* __restrict__ P1, unsigned* __restrict__ fin) {
     grid_entry();
     __shared__ uint8_t slots[8][64];
     const unsigned lane = lane_id(), w = threadIdx.x >> 5, n = lists.cnt->nwarp;
     unsigned deep = 0;
     for (unsigned r = blockIdx.x * 8 + w; r < n; r += gridDim.x * 8) {
-        const QsRange g = lists.warp[r];
+        const QsRange g = lists.warp[r].range();
         const unsigned m = g.hi - g.lo;
         unsigned long long k = 0;
         unsigned p = 0;
         if (lane < m) {
-            k = (g.local ? KL : K0)[g.lo + lane];
-            p = (g.local ? PL : P0)[g.lo + lane];
+            k = (g.buf ? K1 : K0)[g.lo + lane];
+            p = (g.buf ? P1 : P0)[g.lo + lane];
         }
         const unsigned d = g.depth + qs_warp_range(k, p, m, slots[w], slots[w] + 32);
         deep = d > deep ? d : deep;
@@ -687,7 +697,7 @@ static_assert(QS_BLOCK <= 4096 && QS_WARP <= 32, "packing of QsBlockSmem::small"
 template <int C>
 __global__ void __launch_bounds__(qb_threads(C), C == 0 ? 24 : 1024 / qb_threads(C))
 k_qs_blocks(const __grid_constant__ QsLists lists, const unsigned long long* __restrict__ K0,
-            const unsigned* __restrict__ P0, const unsigned long long* __restrict__ KL, const unsigned* __restrict__ PL,
+            const unsigned* __restrict__ P0, const unsigned long long* __restrict__ K1, const unsigned* __restrict__ P1,
             unsigned* __restrict__ fin, int low, unsigned* derr) {
     grid_entry();
     extern __shared__ __align__(16) unsigned char qb_smem[];
@@ -722,8 +732,8 @@ k_qs_blocks(const __grid_constant__ QsLists lists, const unsigned long long* __r
             key[k] = 0;
             row[k] = lo[k] = hi[k] = 0;
             if (p < m) {
-                key[k] = (g.local ? KL : K0)[g.lo + p];
-                row[k] = (g.local ? PL : P0)[g.lo + p];
+                key[k] = (g.buf ? K1 : K0)[g.lo + p];
+                row[k] = (g.buf ? P1 : P0)[g.lo + p];
                 hi[k] = m;
                 act |= 1u << k;
                 sm.K[p] = key[k];
@@ -905,7 +915,7 @@ __global__ void __launch_bounds__(256) k_qs_stable_small(QsLists lists, const un
     grid_entry();
     const unsigned lane = lane_id(), n = lists.cnt->nwarp;
     for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
-        const QsRange g = lists.warp[r];
+        const QsRange g = lists.warp[r].range();
         const unsigned m = g.hi - g.lo;
         const unsigned long long k = lane < m ? img[g.lo + lane] : ~0ull;
         const unsigned row = lane < m ? perm[g.lo + lane] : 0u;
@@ -1018,7 +1028,7 @@ static I qs_lists_alloc(long long n, QsLists* q) {
         q->block[c] = (QsRange*)salloc((size_t)(n / (c ? qb_rows(c - 1) : QS_WARP) + 1) * sizeof(QsRange));
         ok = ok && q->block[c];
     }
-    q->warp = (QsRange*)salloc((size_t)(n / 2 + 1) * sizeof(QsRange));
+    q->warp = (QsShort*)salloc((size_t)(n / 2 + 1) * sizeof(QsShort));
     q->cnt = (QsCounters*)salloc(sizeof(QsCounters));
     return ok && q->warp && q->cnt ? 0 : E_DEVICE_OOM;
 }
@@ -1058,7 +1068,7 @@ static I qs_depths_launch(long long n, QsDepths& q, bool* took) {
 // the ranges of classes low to C, in CTAs of class C
 template <int C>
 static I qs_blocks(const QsLists& lists, const QsCounters& h, int low, const unsigned long long* img, const unsigned* perm,
-                   const unsigned long long* KL, const unsigned* PL, unsigned* fin) {
+                   const unsigned long long* K2, const unsigned* P2, unsigned* fin) {
     unsigned n = 0;
     for (int c = low; c <= C; c++) n += h.nblock[c];
     if (!n) return 0;
@@ -1067,7 +1077,7 @@ static I qs_blocks(const QsLists& lists, const QsCounters& h, int low, const uns
     HG_CU(cudaFuncSetAttribute(k_qs_blocks<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
     const unsigned cap = (unsigned)g_sms * (2048 / qb_threads(C));
     HG_LAUNCH(C == 0 ? "qs_blocks_128" : C == 1 ? "qs_blocks_512" : "qs_blocks", n < cap ? n : cap, qb_threads(C), (size_t)dsm,
-              k_qs_blocks<C>, lists, img, perm, KL, PL, fin, low, g_derr);
+              k_qs_blocks<C>, lists, img, perm, K2, P2, fin, low, g_derr);
     return last_launch_error();
 }
 // Short ranges have launches of their own, in small CTAs, when a class has more
@@ -1077,12 +1087,12 @@ static I qs_blocks(const QsLists& lists, const QsCounters& h, int low, const uns
 // launches; 114K rows in segments of 300, some 2.5 a SM: 0.226 and 0.192).
 constexpr unsigned QB_OWN0 = 2, QB_OWN1 = 2;
 static I qs_all_blocks(const QsLists& lists, const QsCounters& h, const unsigned long long* img, const unsigned* perm,
-                       const unsigned long long* KL, const unsigned* PL, unsigned* fin) {
+                       const unsigned long long* K2, const unsigned* P2, unsigned* fin) {
     const bool own0 = h.nblock[0] > QB_OWN0 * g_sms;
     const bool own1 = h.nblock[1] + (own0 ? 0 : h.nblock[0]) > QB_OWN1 * g_sms;
-    HG_CHECK(qs_blocks<2>(lists, h, own1 ? 2 : own0 ? 1 : 0, img, perm, KL, PL, fin));
-    if (own1) HG_CHECK(qs_blocks<1>(lists, h, own0 ? 1 : 0, img, perm, KL, PL, fin));
-    if (own0) HG_CHECK(qs_blocks<0>(lists, h, 0, img, perm, KL, PL, fin));
+    HG_CHECK(qs_blocks<2>(lists, h, own1 ? 2 : own0 ? 1 : 0, img, perm, K2, P2, fin));
+    if (own1) HG_CHECK(qs_blocks<1>(lists, h, own0 ? 1 : 0, img, perm, K2, P2, fin));
+    if (own0) HG_CHECK(qs_blocks<0>(lists, h, 0, img, perm, K2, P2, fin));
     return 0;
 }
 
@@ -1095,8 +1105,8 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                 long long ns, const uint8_t* mode, const QsLists& lists, QsCounters* h, unsigned* fin) {
     const unsigned g = qs_grid(n);
     const long long max_levels = qs_max_levels(n);
-    unsigned long long* KL = nullptr;  // the elements of listed ranges that a partition has made
-    unsigned* PL = nullptr;
+    unsigned long long* K2 = nullptr;  // the second buffer (img and perm are the first)
+    unsigned* P2 = nullptr;
     unsigned *lo = nullptr, *hi = nullptr;
     if (h->nbig) {
         lo = (unsigned*)salloc((size_t)n * 4);
@@ -1114,15 +1124,13 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
     if (h->nbig) {
         const long long nt = (n + QS_TILE - 1) / QS_TILE;
         const bool scan = nt > QS_DIRECT;
-        unsigned* P2 = (unsigned*)salloc((size_t)n * 4);
-        unsigned long long* K2 = (unsigned long long*)salloc((size_t)n * 8);
+        P2 = (unsigned*)salloc((size_t)n * 4);
+        K2 = (unsigned long long*)salloc((size_t)n * 8);
         unsigned long long* S = (unsigned long long*)salloc((size_t)(n + 1) * 8);
         unsigned long long* ts = (unsigned long long*)salloc((size_t)(nt > QD_MAX_BLOCKS ? nt : QD_MAX_BLOCKS) * 8);
         unsigned* Lpos = (unsigned*)salloc((size_t)n * 4);
         unsigned* Rpos = (unsigned*)salloc((size_t)n * 4);
-        KL = (unsigned long long*)salloc((size_t)n * 8);
-        PL = (unsigned*)salloc((size_t)n * 4);
-        if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos || !KL || !PL) return E_DEVICE_OOM;
+        if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos) return E_DEVICE_OOM;
         // the ranges listed at the start are read from perm/img, which the
         // depths below reuse only at the positions of larger ranges
         unsigned* Pc = perm;
@@ -1136,8 +1144,8 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                 if (!act_clear) HG_CU(cudaMemsetAsync(act, 0, nact * 4, g_stream));
                 act_clear = false;
                 QsDepths q{lo, hi, {Kc, Kc == img ? K2 : img}, {Pc, Pc == perm ? P2 : perm}, S, ts, Lpos, Rpos, fin,
-                           act, act + QD_ROUND, act + QD_ROUND + 1, KL, PL, lists, g_derr, (unsigned)n, (unsigned)level,
-                           (unsigned)round};
+                           act, act + QD_ROUND, act + QD_ROUND + 1, lists, g_derr, (unsigned)n, (unsigned)level,
+                           (unsigned)round, Kc == img ? 0u : 1u};
                 HG_CHECK(qs_depths_launch(n, q, &resident));
                 if (resident) {
                     unsigned res[2];
@@ -1172,7 +1180,7 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                 unsigned* Pn = Pc == perm ? P2 : perm;
                 unsigned long long* Kn = Kc == img ? K2 : img;
                 HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, Lpos, Rpos, Kn, Pn, fin, prev, act + d,
-                          (unsigned)(level + d), KL, PL, lists, g_derr);
+                          (unsigned)(level + d), Kn == img ? 0u : 1u, lists, g_derr);
                 Pc = Pn;
                 Kc = Kn;
             }
@@ -1184,10 +1192,10 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
             if (left == 0) break;
         }
     }
-    HG_CHECK(qs_all_blocks(lists, *h, img, perm, KL, PL, fin));
+    HG_CHECK(qs_all_blocks(lists, *h, img, perm, K2, P2, fin));
     if (h->nwarp) {
         const unsigned cap = 16u * (unsigned)g_sms, want = grid_for(h->nwarp, 8);
-        HG_LAUNCH("qs_warps", want < cap ? want : cap, 256, 0, k_qs_warps, lists, img, perm, KL, PL, fin);
+        HG_LAUNCH("qs_warps", want < cap ? want : cap, 256, 0, k_qs_warps, lists, img, perm, K2, P2, fin);
     }
     HG_CHECK(last_launch_error());
     // read again with the caller's next wait, for qs_depth_check

@@ -101,3 +101,16 @@ if not kernel:
 else:
     assert took == 0 and (own > 0) == passes, own
 """ % (kernel, err, rc, passes))
+
+
+def test_quicksort_scratch(child):
+    """A quicksort of n rows takes less than 60 bytes of scratch a row: its two
+    buffers hold the elements of the ranges listed on the way as well."""
+    child(r"""
+n = 4_000_000
+x = column(H_E, n, 8)
+fake.fake_reset()
+fake.fake_poke(b"k_qs_whole", 1, 32, 4, 1)  # QsCounters::nbig: one range for the depths
+assert L.rc("pfnOrderBy", x, up) == 0, L.lib.hgpuLastError()
+assert count("k_qs_move")[0] > 0
+""", HGPU_SCRATCH_LIMIT_MB=str(4_000_000 * 60 >> 20))
