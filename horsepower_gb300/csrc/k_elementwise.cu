@@ -69,11 +69,12 @@ struct Lane16 {
     }
 };
 __device__ __forceinline__ bool ew_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-// the warps' chunks of n elements
-#define EW_CHUNKS(c, n)                                                                                           \
-    for (long long c = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, nc_ = ((n) + EW_CHUNK - 1) / EW_CHUNK, \
-                   st_ = ((long long)gridDim.x * blockDim.x) >> 5;                                                \
+// the warps' chunks of n elements, from the warp's first one
+#define EW_CHUNKS_FROM(c, first, n)                                                                      \
+    for (long long c = (first), nc_ = ((n) + EW_CHUNK - 1) / EW_CHUNK,                                   \
+                   st_ = ((long long)gridDim.x * blockDim.x) >> 5;                                       \
          c < nc_; c += st_)
+#define EW_CHUNKS(c, n) EW_CHUNKS_FROM(c, (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, n)
 
 // compareFloat(x,y) (h_primitive.cc:1061), or the exact order of integers: -1, 0, 1
 template <typename T>
@@ -169,14 +170,17 @@ __global__ void __launch_bounds__(256, 3) k_compare(const T* __restrict__ x, con
     }
 }
 
+// spread: consecutive chunks go to different blocks, so that what is left over
+// after the warps' equal shares is shared by all SMs
 template <typename T>
 __global__ void __launch_bounds__(256) k_arith(const T* __restrict__ x, const T* __restrict__ y,
                                                T* __restrict__ z, long long n, int op, int mode, T sx, T sy,
-                                               unsigned* derr) {
+                                               int spread, unsigned* derr) {
     grid_entry();
     const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
     bool dz = false;
-    EW_CHUNKS(c, n) {
+    EW_CHUNKS_FROM(c, spread ? (threadIdx.x >> 5) * (long long)gridDim.x + blockIdx.x
+                             : (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, n) {
         const Lane16<T> at(c);
         const bool fast = al && (c + 1) * EW_CHUNK <= n;
         T a[16], b[16];
@@ -394,8 +398,15 @@ static I run_arith(V z, V x, V y, I typ, int op) {
     long long mark = out_mark();
     void* dz;
     HG_CHECK(alloc_out(z, typ, n, &dz));
+    // f64 columns take 103 registers, two blocks an SM, and their division is
+    // bound by the FP64 unit: with one block for each 4096 rows the SMs that get
+    // one more set the time (1.6M divisions 58 us a call with 16 consecutive rows
+    // a thread, 63 with the warps' chunks in such blocks, 48 spread over the SMs)
+    unsigned grid = ew_grid(n);
+    const int spread = std::is_same<T, double>::value && op == 3 && grid > 2u * (unsigned)g_sms;
+    if (spread) grid = 2u * (unsigned)g_sms;
     if (n > 0)
-        HG_LAUNCH("arith", ew_grid(n), 256, 0, k_arith<T>, px, py, (T*)dz, (long long)n, op, mode, sx, sy, g_derr);
+        HG_LAUNCH(spread ? "arith_spread" : "arith", grid, 256, 0, k_arith<T>, px, py, (T*)dz, (long long)n, op, mode, sx, sy, spread, g_derr);
     HG_CHECK(last_launch_error());
     if (op == 3) {  // checkZero (h_system.cc:254-267) runs before the division in the reference
         I e = check_device_errors();

@@ -121,3 +121,24 @@ def test_quicksort_classes(gpu, ora, copies, kernels):
     assert np.array_equal(run(gpu, (True, False)), run(ora, (True, False)))
     gpu.free_inputs()
     ora.free_inputs()
+
+
+@pytest.mark.parametrize("n", [304 * 4096, 304 * 4096 + 1, 1_600_003, 2 * 304 * 4096 + 511])
+@pytest.mark.parametrize("form", ["vv", "vs", "sv"])
+def test_arith_spread(gpu, n, form):
+    """f64 division over more blocks than the SMs hold at once: the chunks are
+    spread over them, the last one ragged; a zero divisor in it is found."""
+    rng = np.random.default_rng(n)
+    a, b = rng.standard_normal(n), rng.standard_normal(n)
+    b[b == 0] = 1.0
+    x = gpu.vec(a, H_E) if form[0] == "v" else gpu.scalar(a[0], H_E)
+    y = gpu.vec(b, H_E) if form[1] == "v" else gpu.scalar(b[0], H_E)
+    ha, hb = (a if form[0] == "v" else a[0]), (b if form[1] == "v" else b[0])
+    for f, want in (("pfnPlus", ha + hb), ("pfnMinus", ha - hb), ("pfnMul", ha * hb), ("pfnDiv", ha / hb)):
+        z, k = launches(gpu, lambda: gpu.call(f, x, y))
+        assert np.array_equal(gpu.to_py(z), want), f
+        assert ("arith_spread" in k) == (f == "pfnDiv" and n > 304 * 4096), k
+    if form[1] == "v":
+        b[n - 1] = 0.0
+        assert gpu.rc("pfnDiv", x, gpu.vec(b, H_E)) == 4  # E_DIV_ZERO
+    gpu.free_inputs()
