@@ -142,3 +142,64 @@ def test_arith_spread(gpu, n, form):
         b[n - 1] = 0.0
         assert gpu.rc("pfnDiv", x, gpu.vec(b, H_E)) == 4  # E_DIV_ZERO
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("n", [1, 4097, 70_001])
+def test_chain_many_columns(gpu, n):
+    """A chain of more than 1024 columns takes its pointers from device memory
+    instead of the kernel's parameters: each kind of sink against numpy."""
+    from horsepower_gb300 import plans as P
+    rng = np.random.default_rng(n)
+    a, b = rng.standard_normal(n), rng.integers(-9, 10, n).astype(np.int32)
+    cols = [gpu.vec(a, H_E)] + [gpu.vec(b, H_I)] * 1028 + [gpu.vec(2 * a, H_E)]
+    assert len(cols) == 1030
+
+    def run(text, many=0):
+        ch = P.Chain(gpu, text)
+        return [gpu.to_py(z) for z in (ch.run_many(cols, many) if many else [ch.run(cols)])]
+
+    keep = b > 2
+    got = run("(map (plus x0 x1029) (plus x1028 1:i32))", 2)
+    assert np.array_equal(got[0], a + 2 * a) and np.array_equal(got[1], b + 1)
+    got = run("(compress (gt x1000 2:i32) (mul x1029 x0) x7)", 2)
+    assert np.array_equal(got[0], (2 * a * a)[keep]) and np.array_equal(got[1], b[keep])
+    assert run("(count (gt x1000 2:i32))")[0] == keep.sum()
+    assert run("(sum (mul x1 x1028) (gt x1000 2:i32))")[0] == (b.astype(np.int64) ** 2)[keep].sum()
+    if keep.any():
+        assert run("(max x1029 (gt x1000 2:i32))")[0] == (2 * a)[keep].max()
+    gpu.free_inputs()
+
+
+@pytest.mark.parametrize("n", [2, 3071, 3072, 3073, 9216 + 5, 200_003])
+@pytest.mark.parametrize("shape", ["both signs", "one positive", "a constant bit"])
+def test_radix_signed_keys(gpu, n, shape):
+    """@order and @group of i64 keys in which 63 or 64 bits vary, the sign among
+    them: key and row id never fit one record, so these take the passes over two
+    arrays.  With a value of 2^32 or more the order is that of the unsigned
+    words, negatives behind the others; either direction, every digit, whole
+    and ragged tiles."""
+    rng = np.random.default_rng(n + len(shape))
+    key = rng.integers(-2 ** 63, 2 ** 63, n, dtype=np.int64)
+    key[rng.random(n) < 0.3] = key[0]
+    if shape == "one positive":
+        key = (key.view(np.uint64) | np.uint64(2 ** 63)).view(np.int64)
+        key[n // 2] = 2 ** 63 - 1
+    elif shape == "a constant bit":
+        key &= ~np.int64(32)
+        key[:2] = [-2 ** 63, 2 ** 63 - 1 - 32]
+    else:
+        key[:2] = [-2 ** 63, 2 ** 63 - 1]
+    rng.shuffle(key)
+    want = np.argsort(key.view(np.uint64), kind="stable")
+    k = gpu.vec(key, H_L)
+    up, names = launches(gpu, lambda: gpu.to_py(gpu.call("pfnOrderBy", k, gpu.vec(np.array([1], bool), H_B))))
+    assert np.array_equal(up, want)
+    assert n == 2 or names["radix_scatter"] == 8, names  # (of two keys fewer bits may vary)
+    down = gpu.to_py(gpu.call("pfnOrderBy", k, gpu.vec(np.array([0], bool), H_B)))
+    assert np.array_equal(down, want[::-1])
+    if n < 20_000:
+        g = gpu.to_py(gpu.call("pfnGroup", k))
+        heads = np.flatnonzero(np.r_[True, key[want][1:] != key[want][:-1]])
+        assert np.array_equal(g[1], want[heads])
+        assert np.array_equal(np.concatenate(g[2]), want)
+    gpu.free_inputs()
