@@ -571,7 +571,7 @@ static I run_chain(hgpu_chain_s* c, V z, V* zs_many, V* x) {
         *arg = dev;
         return 0;
     };
-    void *acols, *aouts;
+    void *acols = nullptr, *aouts = nullptr;
     HG_CHECK(pass(ptrs.data(), nin, &dcols, &acols));
     if (cm->sink == "map") {
         // the values go straight into the outputs; with no operation that

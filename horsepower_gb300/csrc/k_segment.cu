@@ -106,19 +106,6 @@ __device__ __forceinline__ A sblock8(A acc, A* sh) {
     return r;
 }
 
-// element j of segment [s, e): x[rows[s+j]] (gather) or vals[s+j]
-template <typename T, bool GATHER>
-__device__ __forceinline__ T seg_elem(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
-                                      long long k, bool& bad) {
-    if constexpr (GATHER) {
-        long long r = rows[k];
-        if (r < 0 || r >= nx) { bad = true; return T(0); }
-        return src[r];
-    } else {
-        return src[k];
-    }
-}
-
 // 16 elements of one lane, STRIDE apart: positions first + k * STRIDE, k =
 // 0..15, those below `end` loaded (row numbers first, then the values, so all
 // 16 gathers are in flight together).
@@ -931,24 +918,17 @@ static I seg_reduce(const SegIO<T, A>& io, int ncol, const long long* rows, long
     return last_launch_error();
 }
 
-// f64 sums of ncol columns over the segments of one grouping, any number of
-// columns, in sets of SEG_MANY; sums[q] receives column q's ng sums.
+// f64 sums of ncol columns, at most SEG_MANY, over the segments of one
+// grouping; sums[q] receives column q's ng sums.
 template <bool GATHER>
 static I seg_sum_cols(const double* const* srcs, int ncol, const long long* rows, long long nx, const long long* starts,
                       long long ng, long long total, double* const* sums, ListInfo* li) {
-    ListInfo local{};
-    local.scratch = 1;
-    if (!li) li = &local;
-    for (int c0 = 0; c0 < ncol; c0 += SEG_MANY) {
-        SegIO<double, double> io{};
-        const int nc = ncol - c0 < SEG_MANY ? ncol - c0 : SEG_MANY;
-        for (int q = 0; q < nc; q++) {
-            io.src[q] = srcs[c0 + q];
-            io.out[q] = sums[c0 + q];
-        }
-        HG_CHECK((seg_reduce<double, double, OP_SUM, GATHER>(io, nc, rows, nx, starts, ng, total, 0.0, li)));
+    SegIO<double, double> io{};
+    for (int q = 0; q < ncol; q++) {
+        io.src[q] = srcs[q];
+        io.out[q] = sums[q];
     }
-    return 0;
+    return seg_reduce<double, double, OP_SUM, GATHER>(io, ncol, rows, nx, starts, ng, total, 0.0, li);
 }
 
 // f64 sums of several columns over segments gathered through row ids (the
