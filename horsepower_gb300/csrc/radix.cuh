@@ -84,9 +84,10 @@ __device__ __forceinline__ void rx_forget(unsigned long long& v) { asm volatile(
 // The lanes whose BITS-bit digit equals this lane's (every lane takes part).
 // Each ballot comes from a predicate set straight from the bit, and the same
 // predicate turns the ballot round for a lane whose bit is clear: 3.5
-// instructions a bit.  With an all-ones word per bit as the mask of both, as
-// the compiler makes of the C++ form, a bit takes 5 (150M rows, 8-bit pass:
-// 0.69 ms against 0.585).
+// instructions a bit.  These four instructions are those of CUB's MatchAny
+// (util_ptx.cuh, BSD-3-Clause).  With an all-ones word per bit as the mask of
+// both, as the compiler makes of the C++ form, a bit takes 5 (150M rows, 8-bit
+// pass: 0.69 ms against 0.585).
 template <int BITS>
 __device__ __forceinline__ unsigned rx_match(unsigned d) {
     unsigned same[BITS], peers = 0xffffffffu;
