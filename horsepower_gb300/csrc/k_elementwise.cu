@@ -16,9 +16,9 @@
 // an f64 load touched 32, and the L1's one line a cycle bound the kernels at
 // 4.1-4.5 TB/s.  60M rows, kernel time: @compare f64 with a scalar 0.132 ->
 // 0.082 ms (6.6 TB/s), i64 0.227 -> 0.092, i32 0.055 -> 0.046; @mul f64 0.322
-// -> 0.226 ms (6.4 TB/s); @and 0.034 -> 0.0185 ms.  Operands of different types are first converted to
-// the common type (the reference's promoteValue), then the same-type kernel
-// runs.
+// -> 0.226 ms (6.4 TB/s); @and 0.034 -> 0.027 ms.  Operands of different types
+// are first converted to the common type (the reference's promoteValue), then
+// the same-type kernel runs.
 #include <climits>
 #include <cstring>
 

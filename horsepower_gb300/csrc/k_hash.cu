@@ -607,7 +607,7 @@ __device__ __forceinline__ bool key_stream(const void* p, int typ, long long i, 
 // Direct tables: the presence bit is the answer, and a lane has eight keys'
 // bits in flight.  What bounds it is the L2's rate of scattered sectors, 243
 // G/s (60M i32 keys against 2.1M of a 15M range: 0.285 ms with one key at a
-// time and the row read behind its bit, 0.268 now, 0.247 at that rate).
+// time and the row read behind its bit, 0.246 now, which is that rate).
 template <typename K>
 __global__ void __launch_bounds__(256) k_member_direct(Table<K> t, const void* __restrict__ y, int typ, long long n,
                                                        bool* __restrict__ z) {

@@ -45,7 +45,7 @@ __device__ __forceinline__ A sop(A a, A b) {
 // each step; here the first three steps give the freed half another warp's
 // values instead (lane bit 16 picks warps 0-3 or 4-7, bit 8 then bit 4 halve
 // again), so 8 warps cost 4 + 2 + 1 + 1 + 1 operations and 3 for the tile
-// instead of 40 and 7.  GB300 issues an FP64 instruction every 16 cycles per
+// instead of 40 and 7.  GB300 issues an FP64 instruction every 19 cycles per
 // SM, which is what bounds these folds.  Every operand pair, and its order in
 // lane 0's tree, is that of the separate butterflies.
 template <typename A, int OP>
@@ -216,7 +216,7 @@ __global__ void k_seg_class_ids(const long long* __restrict__ starts, long long 
 // of up to 4, eight of up to 32): the butterfly's first two steps are its own
 // and the rest go over L lanes.  What bounds the kernel is latency (segment
 // id, start, row id and value are loads one behind the other) and the FP64
-// unit, which takes a warp's instruction every 16 cycles however few lanes
+// unit, which takes a warp's instruction every 19 cycles however few lanes
 // matter: four loads in flight per lane, and 1.5 additions a segment of 17 to
 // 32 rows against 6 with one place per lane.  5.8M groups of 1 to 32 rows (18M
 // rows) of a 150M-row Zipf grouping: 0.65-0.77 ms with one place per lane,

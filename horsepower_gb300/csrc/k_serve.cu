@@ -40,7 +40,7 @@ constexpr int SQ_MAXW = 256;  // request windows per shared-scan launch
 // its rows in the tile-tree order (lane t: rows t, t+256, ..., t+3840; xor
 // butterfly; pairwise warp combine).  Rows outside a window add nothing,
 // exactly as in the fused chain's full-range reduction.  GB300 issues an FP64
-// instruction every 16 cycles per SM, which bounds the kernel, so a warp folds
+// instruction every 19 cycles per SM, which bounds the kernel, so a warp folds
 // the butterflies of eight windows together (9 additions instead of 40: the
 // first three steps give the lanes that would hold copies another window's
 // sum); every pair added is that of the separate butterflies.
