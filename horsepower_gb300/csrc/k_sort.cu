@@ -1549,8 +1549,11 @@ extern "C" {
 I pfnGroupTrie(V z, V x) {
     HG_CHECK(ensure_init());
     ScratchScope ss;
+    // both columns are read as bytes over the first one's length
+    if (x->typ != H_G || x->len < 2) return set_error(E_DOMAIN, "group_trie takes a list of two char columns");
     V0* c = host_nodes(x);
     long long n = c[0].len;
+    if (c[1].len < n) return set_error(E_LENGTH, "group_trie: columns of %lld and %lld rows", n, (long long)c[1].len);
     const void *p0, *p1;
     HG_CHECK(in_ptr(&c[0], &p0));
     HG_CHECK(in_ptr(&c[1], &p1));

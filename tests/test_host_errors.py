@@ -114,3 +114,18 @@ fake.fake_poke(b"k_qs_whole", 1, 32, 4, 1)  # QsCounters::nbig: one range for th
 assert L.rc("pfnOrderBy", x, up) == 0, L.lib.hgpuLastError()
 assert count("k_qs_move")[0] > 0
 """, HGPU_SCRATCH_LIMIT_MB=str(4_000_000 * 60 >> 20))
+
+
+def test_group_trie_columns(child):
+    """@group_trie reads its second column over the first one's length: a list
+    without one, or with a shorter one, and a plain vector are refused before
+    anything is read."""
+    child(r"""
+a, b, c = (column(H_C, n, 1) for n in (5000, 4999, 5000))
+# (a node behind the one-column list, which a reader of two columns would take)
+one = L.list([a, c]); one.len = 1
+for x, rc in ((one, 1), (L.list([]), 1), (a, 1), (L.list([a, b]), 5), (L.list([a, c]), 0), (L.list([b, a]), 0)):
+    fake.fake_reset()
+    assert L.rc("pfnGroupTrie", x) == rc, (x.len, L.lib.hgpuLastError())
+    assert (count("k_trie_present")[0] > 0) == (rc == 0)
+""")
