@@ -16,9 +16,7 @@
 // an f64 load touched 32, and the L1's one line a cycle bound the kernels at
 // 4.1-4.5 TB/s.  60M rows, kernel time: @compare f64 with a scalar 0.132 ->
 // 0.082 ms (6.6 TB/s), i64 0.227 -> 0.092, i32 0.055 -> 0.046; @mul f64 0.322
-// -> 0.226 ms (6.4 TB/s); @and 0.034 -> 0.027 ms.  A column that does not
-// begin on 16 bytes is read element by element, and the others and the result
-// still 16 bytes at a time.  Operands of different types
+// -> 0.226 ms (6.4 TB/s); @and 0.034 -> 0.027 ms.  Operands of different types
 // are first converted to the common type (the reference's promoteValue), then
 // the same-type kernel runs.
 #include <climits>
@@ -39,7 +37,7 @@ struct Lane16 {
     long long at;  // the lane's first element
     __device__ __forceinline__ Lane16(long long chunk) : at(chunk * EW_CHUNK + (long long)lane_id() * VW) {}
     __device__ __forceinline__ long long elem(int k) const { return at + (k / VW) * (32 * VW) + k % VW; }
-    // `fast`: the chunk is complete and p (z) is 16-byte aligned
+    // `fast`: the chunk is complete and p is 16-byte aligned
     __device__ __forceinline__ void load(const T* __restrict__ p, long long n, bool fast, T (&v)[16]) const {
         if (fast) {
             uint4 tmp[NJ];
@@ -152,23 +150,23 @@ template <typename T>
 __global__ void __launch_bounds__(256, 3) k_compare(const T* __restrict__ x, const T* __restrict__ y,
                                                  bool* __restrict__ z, long long n, unsigned mask, int mode, T sx, T sy) {
     grid_entry();
-    const bool alx = ew_aligned(x), aly = ew_aligned(y), alz = ew_aligned(z);
+    const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
     EW_CHUNKS(c, n) {
         const Lane16<T> at(c);
-        const bool full = (c + 1) * EW_CHUNK <= n;
+        const bool fast = al && (c + 1) * EW_CHUNK <= n;
         T a[16], b[16];
         if (mode == MODE_SV) {
 #pragma unroll
             for (int k = 0; k < 16; k++) a[k] = sx;
-        } else at.load(x, n, full && alx, a);
+        } else at.load(x, n, fast, a);
         if (mode == MODE_VS) {
 #pragma unroll
             for (int k = 0; k < 16; k++) b[k] = sy;
-        } else at.load(y, n, full && aly, b);
+        } else at.load(y, n, fast, b);
         alignas(16) bool r[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) r[k] = (mask >> (cmp3<T>(a[k], b[k]) + 1)) & 1u;
-        at.store(z, n, full && alz, r);
+        at.store(z, n, fast, r);
     }
 }
 
@@ -179,29 +177,29 @@ __global__ void __launch_bounds__(256) k_arith(const T* __restrict__ x, const T*
                                                T* __restrict__ z, long long n, int op, int mode, T sx, T sy,
                                                int spread, unsigned* derr) {
     grid_entry();
-    const bool alx = ew_aligned(x), aly = ew_aligned(y), alz = ew_aligned(z);
+    const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
     bool dz = false;
     EW_CHUNKS_FROM(c, spread ? (threadIdx.x >> 5) * (long long)gridDim.x + blockIdx.x
                              : (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, n) {
         const Lane16<T> at(c);
-        const bool full = (c + 1) * EW_CHUNK <= n;
+        const bool fast = al && (c + 1) * EW_CHUNK <= n;
         T a[16], b[16];
         alignas(16) T r[16];
         if (mode == MODE_SV) {
 #pragma unroll
             for (int k = 0; k < 16; k++) a[k] = sx;
-        } else at.load(x, n, full && alx, a);
+        } else at.load(x, n, fast, a);
         if (mode == MODE_VS) {
 #pragma unroll
             for (int k = 0; k < 16; k++) b[k] = sy;
-        } else at.load(y, n, full && aly, b);
+        } else at.load(y, n, fast, b);
 #pragma unroll
         for (int k = 0; k < 16; k++) {
             bool d = false;
             r[k] = arith_op<T>(op, a[k], b[k], d);
             if (d && at.elem(k) < n) dz = true;
         }
-        at.store(z, n, full && alz, r);
+        at.store(z, n, fast, r);
     }
     if (dz) flag_error(derr, DERR_DIVZERO);
 }
@@ -216,33 +214,26 @@ __device__ __forceinline__ unsigned logic_word(int op, unsigned a, unsigned b) {
     default: return 0x01010101u;     // nand / nor: ~(.) as bool is always true
     }
 }
-__global__ void __launch_bounds__(256, 8) k_logic(const uint8_t* __restrict__ x, const uint8_t* __restrict__ y,
+__global__ void __launch_bounds__(256) k_logic(const uint8_t* __restrict__ x, const uint8_t* __restrict__ y,
                                                uint8_t* __restrict__ z, long long n, int op, int mode,
                                                uint8_t sx, uint8_t sy) {
     grid_entry();
-    const bool alx = ew_aligned(x), aly = ew_aligned(y), alz = ew_aligned(z);
+    const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
     EW_CHUNKS(c, n) {
-        const long long i0 = Lane16<uint8_t>(c).at;
-        const bool full = (c + 1) * EW_CHUNK <= n;
-        auto load = [&](const uint8_t* p, bool al) {
-            if (full && al) return __ldcs(reinterpret_cast<const uint4*>(p + i0));
-            unsigned w[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-            for (int k = 0; k < 16; k++) w[k / 4] |= (unsigned)(i0 + k < n ? p[i0 + k] : 0) << (8 * (k % 4));
-            return make_uint4(w[0], w[1], w[2], w[3]);
-        };
-        const unsigned ax = sx * 0x01010101u, by = sy * 0x01010101u;
-        const uint4 a = mode == MODE_SV ? make_uint4(ax, ax, ax, ax) : load(x, alx);
-        const uint4 b = mode == MODE_VS ? make_uint4(by, by, by, by) : load(y, aly);
-        const uint4 r = make_uint4(logic_word(op, a.x, b.x), logic_word(op, a.y, b.y), logic_word(op, a.z, b.z),
-                                   logic_word(op, a.w, b.w));
-        if (full && alz) {
-            *reinterpret_cast<uint4*>(z + i0) = r;
+        const Lane16<uint8_t> at(c);
+        if (al && (c + 1) * EW_CHUNK <= n) {
+            const unsigned ax = sx * 0x01010101u, by = sy * 0x01010101u;
+            uint4 a = make_uint4(ax, ax, ax, ax), b = make_uint4(by, by, by, by);
+            if (mode != MODE_SV) a = __ldcs(reinterpret_cast<const uint4*>(x + at.at));
+            if (mode != MODE_VS) b = __ldcs(reinterpret_cast<const uint4*>(y + at.at));
+            *reinterpret_cast<uint4*>(z + at.at) = make_uint4(logic_word(op, a.x, b.x), logic_word(op, a.y, b.y),
+                                                              logic_word(op, a.z, b.z), logic_word(op, a.w, b.w));
         } else {
-            const unsigned w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-            for (int k = 0; k < 16; k++)
-                if (i0 + k < n) z[i0 + k] = (uint8_t)(w[k / 4] >> (8 * (k % 4)));
+            for (int k = 0; k < 16; k++) {
+                const long long i = at.elem(k);
+                if (i < n)
+                    z[i] = (uint8_t)logic_word(op, mode == MODE_SV ? sx : x[i], mode == MODE_VS ? sy : y[i]);
+            }
         }
     }
 }
@@ -357,16 +348,16 @@ F64Range f64_cmp_range(double s, bool scalar_first, int op) {
 __global__ void __launch_bounds__(256) k_compare_f64_fixed(const double* __restrict__ x, bool* __restrict__ z,
                                                            long long n, F64Range range) {
     grid_entry();
-    const bool alx = ew_aligned(x), alz = ew_aligned(z);
+    const bool al = ew_aligned(x) && ew_aligned(z);
     EW_CHUNKS(c, n) {
         const Lane16<double> at(c);
-        const bool full = (c + 1) * EW_CHUNK <= n;
+        const bool fast = al && (c + 1) * EW_CHUNK <= n;
         double a[16];
-        at.load(x, n, full && alx, a);
+        at.load(x, n, fast, a);
         alignas(16) bool r[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) r[k] = f64_in_range(a[k], range);
-        at.store(z, n, full && alz, r);
+        at.store(z, n, fast, r);
     }
 }
 
