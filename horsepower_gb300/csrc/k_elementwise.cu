@@ -37,7 +37,7 @@ struct Lane16 {
     long long at;  // the lane's first element
     __device__ __forceinline__ Lane16(long long chunk) : at(chunk * EW_CHUNK + (long long)lane_id() * VW) {}
     __device__ __forceinline__ long long elem(int k) const { return at + (k / VW) * (32 * VW) + k % VW; }
-    // `fast`: the chunk is complete and p is 16-byte aligned
+    // `fast`: the chunk is complete and p (z) is 16-byte aligned
     __device__ __forceinline__ void load(const T* __restrict__ p, long long n, bool fast, T (&v)[16]) const {
         if (fast) {
             uint4 tmp[NJ];
@@ -68,7 +68,22 @@ struct Lane16 {
         }
     }
 };
-__device__ __forceinline__ bool ew_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+__host__ __device__ __forceinline__ bool ew_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+// The operands of a call all begin on 16 bytes (AL of the kernels below).  When
+// one does not, it is read element by element and the others and the result
+// still 16 bytes at a time; that is an instance of its own, as both in one take
+// the logic kernel from 32 to 39 registers and a fourth of its warps (@and 60M
+// rows 33 us a call, 37).  20M rows, one column a byte off, us a call: @and 68
+// with every access by element and 24 now, @lt i8 57 and 33, @mul i16 57 and 34.
+static bool ew_all_aligned(const void* x, const void* y, const void* z, int mode) {
+    return (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
+}
+// Launches KERN<..., true> or KERN<..., false> by that.
+#define EW_LAUNCH(name, grid, KT, KF, al, ...)                          \
+    do {                                                                \
+        if (al) HG_LAUNCH(name, grid, 256, 0, KT, __VA_ARGS__);         \
+        else HG_LAUNCH(name, grid, 256, 0, KF, __VA_ARGS__);            \
+    } while (0)
 // the warps' chunks of n elements, from the warp's first one
 #define EW_CHUNKS_FROM(c, first, n)                                                                      \
     for (long long c = (first), nc_ = ((n) + EW_CHUNK - 1) / EW_CHUNK,                                   \
@@ -146,60 +161,60 @@ __device__ __forceinline__ T arith_op(int op, T a, T b, bool& divzero) {
 
 // (three blocks an SM: at the 84 registers the compiler would take, f64 columns
 // leave two, whose last wave costs 3 to 13% at 1.5M to 8M rows)
-template <typename T>
+template <typename T, bool AL>
 __global__ void __launch_bounds__(256, 3) k_compare(const T* __restrict__ x, const T* __restrict__ y,
                                                  bool* __restrict__ z, long long n, unsigned mask, int mode, T sx, T sy) {
     grid_entry();
-    const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
+    const bool alx = AL || ew_aligned(x), aly = AL || ew_aligned(y), alz = AL || ew_aligned(z);
     EW_CHUNKS(c, n) {
         const Lane16<T> at(c);
-        const bool fast = al && (c + 1) * EW_CHUNK <= n;
+        const bool full = (c + 1) * EW_CHUNK <= n;
         T a[16], b[16];
         if (mode == MODE_SV) {
 #pragma unroll
             for (int k = 0; k < 16; k++) a[k] = sx;
-        } else at.load(x, n, fast, a);
+        } else at.load(x, n, full && alx, a);
         if (mode == MODE_VS) {
 #pragma unroll
             for (int k = 0; k < 16; k++) b[k] = sy;
-        } else at.load(y, n, fast, b);
+        } else at.load(y, n, full && aly, b);
         alignas(16) bool r[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) r[k] = (mask >> (cmp3<T>(a[k], b[k]) + 1)) & 1u;
-        at.store(z, n, fast, r);
+        at.store(z, n, full && alz, r);
     }
 }
 
 // spread: consecutive chunks go to different blocks, so that what is left over
 // after the warps' equal shares is shared by all SMs
-template <typename T>
+template <typename T, bool AL>
 __global__ void __launch_bounds__(256) k_arith(const T* __restrict__ x, const T* __restrict__ y,
                                                T* __restrict__ z, long long n, int op, int mode, T sx, T sy,
                                                int spread, unsigned* derr) {
     grid_entry();
-    const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
+    const bool alx = AL || ew_aligned(x), aly = AL || ew_aligned(y), alz = AL || ew_aligned(z);
     bool dz = false;
     EW_CHUNKS_FROM(c, spread ? (threadIdx.x >> 5) * (long long)gridDim.x + blockIdx.x
                              : (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, n) {
         const Lane16<T> at(c);
-        const bool fast = al && (c + 1) * EW_CHUNK <= n;
+        const bool full = (c + 1) * EW_CHUNK <= n;
         T a[16], b[16];
         alignas(16) T r[16];
         if (mode == MODE_SV) {
 #pragma unroll
             for (int k = 0; k < 16; k++) a[k] = sx;
-        } else at.load(x, n, fast, a);
+        } else at.load(x, n, full && alx, a);
         if (mode == MODE_VS) {
 #pragma unroll
             for (int k = 0; k < 16; k++) b[k] = sy;
-        } else at.load(y, n, fast, b);
+        } else at.load(y, n, full && aly, b);
 #pragma unroll
         for (int k = 0; k < 16; k++) {
             bool d = false;
             r[k] = arith_op<T>(op, a[k], b[k], d);
             if (d && at.elem(k) < n) dz = true;
         }
-        at.store(z, n, fast, r);
+        at.store(z, n, full && alz, r);
     }
     if (dz) flag_error(derr, DERR_DIVZERO);
 }
@@ -214,27 +229,34 @@ __device__ __forceinline__ unsigned logic_word(int op, unsigned a, unsigned b) {
     default: return 0x01010101u;     // nand / nor: ~(.) as bool is always true
     }
 }
+template <bool AL>
 __global__ void __launch_bounds__(256) k_logic(const uint8_t* __restrict__ x, const uint8_t* __restrict__ y,
                                                uint8_t* __restrict__ z, long long n, int op, int mode,
                                                uint8_t sx, uint8_t sy) {
     grid_entry();
-    const bool al = (mode == MODE_SV || ew_aligned(x)) && (mode == MODE_VS || ew_aligned(y)) && ew_aligned(z);
+    const bool alx = AL || ew_aligned(x), aly = AL || ew_aligned(y);  // z begins a result's memory
     EW_CHUNKS(c, n) {
-        const Lane16<uint8_t> at(c);
-        if (al && (c + 1) * EW_CHUNK <= n) {
-            const unsigned ax = sx * 0x01010101u, by = sy * 0x01010101u;
-            uint4 a = make_uint4(ax, ax, ax, ax), b = make_uint4(by, by, by, by);
-            if (mode != MODE_SV) a = __ldcs(reinterpret_cast<const uint4*>(x + at.at));
-            if (mode != MODE_VS) b = __ldcs(reinterpret_cast<const uint4*>(y + at.at));
-            *reinterpret_cast<uint4*>(z + at.at) = make_uint4(logic_word(op, a.x, b.x), logic_word(op, a.y, b.y),
-                                                              logic_word(op, a.z, b.z), logic_word(op, a.w, b.w));
-        } else {
-            for (int k = 0; k < 16; k++) {
-                const long long i = at.elem(k);
-                if (i < n)
-                    z[i] = (uint8_t)logic_word(op, mode == MODE_SV ? sx : x[i], mode == MODE_VS ? sy : y[i]);
-            }
+        const long long i0 = Lane16<uint8_t>(c).at;
+        const bool full = (c + 1) * EW_CHUNK <= n;
+        const unsigned ax = sx * 0x01010101u, by = sy * 0x01010101u;
+        if (!full) {
+            for (int k = 0; k < 16; k++)
+                if (i0 + k < n)
+                    z[i0 + k] = (uint8_t)logic_word(op, mode == MODE_SV ? sx : x[i0 + k], mode == MODE_VS ? sy : y[i0 + k]);
+            continue;
         }
+        auto load = [&](const uint8_t* p, bool al) {
+            if (al) return __ldcs(reinterpret_cast<const uint4*>(p + i0));
+            unsigned w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int k = 0; k < 16; k++) w[k / 4] |= (unsigned)p[i0 + k] << (8 * (k % 4));
+            return make_uint4(w[0], w[1], w[2], w[3]);
+        };
+        uint4 a = make_uint4(ax, ax, ax, ax), b = make_uint4(by, by, by, by);
+        if (mode != MODE_SV) a = load(x, alx);
+        if (mode != MODE_VS) b = load(y, aly);
+        *reinterpret_cast<uint4*>(z + i0) = make_uint4(logic_word(op, a.x, b.x), logic_word(op, a.y, b.y),
+                                                       logic_word(op, a.z, b.z), logic_word(op, a.w, b.w));
     }
 }
 
@@ -348,16 +370,16 @@ F64Range f64_cmp_range(double s, bool scalar_first, int op) {
 __global__ void __launch_bounds__(256) k_compare_f64_fixed(const double* __restrict__ x, bool* __restrict__ z,
                                                            long long n, F64Range range) {
     grid_entry();
-    const bool al = ew_aligned(x) && ew_aligned(z);
+    const bool alx = ew_aligned(x), alz = ew_aligned(z);
     EW_CHUNKS(c, n) {
         const Lane16<double> at(c);
-        const bool fast = al && (c + 1) * EW_CHUNK <= n;
+        const bool full = (c + 1) * EW_CHUNK <= n;
         double a[16];
-        at.load(x, n, fast, a);
+        at.load(x, n, full && alx, a);
         alignas(16) bool r[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) r[k] = f64_in_range(a[k], range);
-        at.store(z, n, fast, r);
+        at.store(z, n, full && alz, r);
     }
 }
 
@@ -380,8 +402,9 @@ static I run_compare(V z, V x, V y, I typX, int op) {
             return finish_out(z, dz);
         }
     }
-    if (n > 0) HG_LAUNCH("compare", ew_grid(n), 256, 0, k_compare<T>, px, py, (bool*)dz, (long long)n,
-                         cmp_mask(op), mode, sx, sy);
+    if (n > 0)
+        EW_LAUNCH("compare", ew_grid(n), (k_compare<T, true>), (k_compare<T, false>), ew_all_aligned(px, py, dz, mode), px,
+                  py, (bool*)dz, (long long)n, cmp_mask(op), mode, sx, sy);
     HG_CHECK(last_launch_error());
     return finish_out(z, dz);
 }
@@ -406,7 +429,8 @@ static I run_arith(V z, V x, V y, I typ, int op) {
     const int spread = std::is_same<T, double>::value && op == 3 && grid > 2u * (unsigned)g_sms;
     if (spread) grid = 2u * (unsigned)g_sms;
     if (n > 0)
-        HG_LAUNCH(spread ? "arith_spread" : "arith", grid, 256, 0, k_arith<T>, px, py, (T*)dz, (long long)n, op, mode, sx, sy, spread, g_derr);
+        EW_LAUNCH(spread ? "arith_spread" : "arith", grid, (k_arith<T, true>), (k_arith<T, false>),
+                  ew_all_aligned(px, py, dz, mode), px, py, (T*)dz, (long long)n, op, mode, sx, sy, spread, g_derr);
     HG_CHECK(last_launch_error());
     if (op == 3) {  // checkZero (h_system.cc:254-267) runs before the division in the reference
         I e = check_device_errors();
@@ -514,8 +538,8 @@ static I logic(V z, V x, V y, int op) {
     void* dz;
     HG_CHECK(alloc_out(z, H_B, n, &dz));
     if (n > 0)
-        HG_LAUNCH("logic", ew_grid(n), 256, 0, k_logic, (const uint8_t*)px, (const uint8_t*)py, (uint8_t*)dz,
-                  (long long)n, op, mode, (uint8_t)(bx & 1), (uint8_t)(by & 1));
+        EW_LAUNCH("logic", ew_grid(n), k_logic<true>, k_logic<false>, ew_all_aligned(px, py, dz, mode), (const uint8_t*)px,
+                  (const uint8_t*)py, (uint8_t*)dz, (long long)n, op, mode, (uint8_t)(bx & 1), (uint8_t)(by & 1));
     HG_CHECK(last_launch_error());
     return finish_out(z, dz);
 }
@@ -535,8 +559,8 @@ I pfnNot(V z, V x) {
     void* dz;
     HG_CHECK(alloc_out(z, H_B, x->len, &dz));
     if (x->len > 0)
-        HG_LAUNCH("not", ew_grid(x->len), 256, 0, k_logic, (const uint8_t*)px, (const uint8_t*)px, (uint8_t*)dz,
-                  (long long)x->len, 5, MODE_VV, (uint8_t)0, (uint8_t)0);
+        EW_LAUNCH("not", ew_grid(x->len), k_logic<true>, k_logic<false>, ew_all_aligned(px, px, dz, MODE_VV), (const uint8_t*)px,
+                  (const uint8_t*)px, (uint8_t*)dz, (long long)x->len, 5, MODE_VV, (uint8_t)0, (uint8_t)0);
     HG_CHECK(last_launch_error());
     return finish_out(z, dz);
 }

@@ -10,7 +10,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from horsepower_gb300.abi import Builtins, DTYPE, H_B, H_E, H_F, H_H, H_I, H_L
+from horsepower_gb300.abi import Builtins, DTYPE, H_B, H_E, H_F, H_H, H_I, H_J, H_L
 
 pytestmark = pytest.mark.gpu
 
@@ -202,4 +202,30 @@ def test_radix_signed_keys(gpu, n, shape):
         heads = np.flatnonzero(np.r_[True, key[want][1:] != key[want][:-1]])
         assert np.array_equal(g[1], want[heads])
         assert np.array_equal(np.concatenate(g[2]), want)
+    gpu.free_inputs()
+
+
+@pytest.mark.parametrize("n", [2, 511, 512, 513, 4096 + 7, 70_001])
+@pytest.mark.parametrize("typ", [H_B, H_J, H_H, H_I, H_L, H_F, H_E])
+def test_one_unaligned_operand(gpu, typ, n):
+    """An operand that does not begin on 16 bytes is read element by element
+    beside one that is read 16 bytes at a time: the results of every
+    combination are those of two aligned columns."""
+    from horsepower_gb300 import batch as B
+    rng = np.random.default_rng(n + typ)
+    a, b = (rng.integers(0, 2 if typ == H_B else 100, n).astype(DTYPE[typ]) for _ in range(2))
+
+    def column(c, skip):
+        d = B.to_device(gpu, np.concatenate([c[:1]] * skip + [c]), typ)
+        d.g, d.len = d.g + skip * c.itemsize, n
+        return d
+
+    names = ["pfnLt", "pfnEq", "pfnPlus", "pfnMul"] + (["pfnAnd", "pfnXor"] if typ == H_B else [])
+    s = gpu.scalar(1, typ)
+    for f in names:
+        def run(da, db):
+            return [gpu.to_py(gpu.call(f, x, y)).tobytes() for x, y in ((da, db), (da, s), (s, db))]
+        want = run(column(a, 0), column(b, 0))
+        for sa, sb in ((1, 0), (0, 1), (1, 3), (5, 5)):
+            assert run(column(a, sa), column(b, sb)) == want, (f, sa, sb)
     gpu.free_inputs()
