@@ -58,15 +58,15 @@ static_assert(qb_rows(QB_CLASSES - 1) == QS_BLOCK, "the largest CTA takes the la
 struct QsRange {
     unsigned lo, hi, depth, buf;
 };
-// ... of up to QS_WARP elements, of which a sort may list one for every two
-// rows, in half the space.  The depth fits: no more than the rows of a small
-// sort, or 2^36 by the rows of a large one, either way below 2^19.
-struct QsShort {
-    unsigned lo, rest;  // size - 1, buffer << 5, depth << 6
+// ... as it is listed.  The depth fits: no more than the rows of a small sort,
+// or 2^36 by the rows of a large one, either way below 2^19.
+struct QsEntry {
+    unsigned lo, rest;  // size - 1, buffer << 12, depth << 13
     __device__ __forceinline__ QsRange range() const {
-        return QsRange{lo, lo + (rest & 31u) + 1, rest >> 6, (rest >> 5) & 1u};
+        return QsRange{lo, lo + (rest & 4095u) + 1, rest >> 13, (rest >> 12) & 1u};
     }
 };
+static_assert(QS_BLOCK <= 4096, "packing of QsEntry::rest");
 // counters of one sort, in device memory
 struct QsCounters {
     unsigned nblock[QB_CLASSES], nwarp;  // ranges listed for CTAs of each size and for warps
@@ -74,19 +74,25 @@ struct QsCounters {
     unsigned depth;          // recursion depth reached by the listed ranges
     unsigned nrev, nan;      // segments to reverse; a NaN key was seen
 };
+// Ranges for warps are listed from the front of `ends` and those for the
+// smallest CTAs from its back: they hold at least 2 and 33 of the n rows each
+// and share none, so n / 2 + 1 entries are enough for both.
 struct QsLists {
-    QsRange* block[QB_CLASSES];
-    QsShort* warp;
+    QsEntry *ends, *block[QB_CLASSES];  // block[0]: the last entry of `ends`
     QsCounters* cnt;
+    __device__ __forceinline__ QsEntry& warp_entry(unsigned i) const { return ends[i]; }
+    __device__ __forceinline__ QsEntry& block_entry(int c, unsigned i) const {
+        return c == 0 ? *(block[0] - i) : c == 1 ? block[1][i] : block[2][i];
+    }
 };
 __device__ __forceinline__ void qs_list(const QsLists& q, unsigned lo, unsigned hi, unsigned depth, unsigned buf) {
     const unsigned m = hi - lo;
+    const QsEntry e{lo, (m - 1) | (buf << 12) | (depth << 13)};
     if (m > QS_WARP) {
         const int c = m <= qb_rows(0) ? 0 : m <= qb_rows(1) ? 1 : 2;
-        QsRange* list = c == 0 ? q.block[0] : c == 1 ? q.block[1] : q.block[2];
-        list[atomicAdd(&q.cnt->nblock[c], 1u)] = QsRange{lo, hi, depth, buf};
+        q.block_entry(c, atomicAdd(&q.cnt->nblock[c], 1u)) = e;
     } else {
-        q.warp[atomicAdd(&q.cnt->nwarp, 1u)] = QsShort{lo, (m - 1) | (buf << 5) | (depth << 6)};
+        q.warp_entry(atomicAdd(&q.cnt->nwarp, 1u)) = e;
     }
 }
 // A recursion deeper than max(8192, 2^36 / n) levels, rounded up to a multiple
@@ -276,14 +282,14 @@ __global__ void __launch_bounds__(QS_THREADS) k_qs_prefix(const unsigned* __rest
 __device__ __forceinline__ unsigned qs_le(unsigned long long s) { return (unsigned)s; }
 __device__ __forceinline__ unsigned qs_lt(unsigned long long s) { return (unsigned)(s >> 32); }
 
-// Lpos[lo + k] = the k-th element > P inside (lo, j] from the left;
-// Rpos[lo + k] = the k-th element <= P inside (j, hi) from the right
-// (Every slot index lies in [lo, hi) by the counting above; a slot outside
-// it would mean inconsistent ranges and is recorded, not written.)
+// trade[lo + k] = the k-th element > P inside (lo, j] from the left;
+// trade[hi - 1 - k] = the k-th element <= P inside (j, hi) from the right
+// (They are equally many, at most half of (lo, hi), so neither side's slots
+// reach the other's.  A slot outside [lo, hi) would mean inconsistent ranges and
+// is recorded, not written.)
 __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __restrict__ hi,
                          const unsigned long long* __restrict__ K, const unsigned long long* __restrict__ S, long long n,
-                         unsigned* __restrict__ Lpos, unsigned* __restrict__ Rpos, const unsigned* __restrict__ prev,
-                         unsigned* derr) {
+                         unsigned* __restrict__ trade, const unsigned* __restrict__ prev, unsigned* derr) {
     grid_entry();
     if (qs_idle(prev)) return;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
@@ -293,12 +299,11 @@ __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __rest
         const unsigned le_lo = qs_le(S[l]), le_hi = qs_le(S[h]), le_p = qs_le(S[p]);
         const long long j = (long long)l + (le_hi - le_lo);
         const int c = qs_cmp(K[p], K[l]);
-        long long slot = -1;
-        unsigned* dst = nullptr;
-        if (p <= j && c > 0) { slot = (long long)l + (long long)(p - l - 1) - (long long)(le_p - le_lo); dst = Lpos; }
-        else if (p > j && c <= 0) { slot = (long long)l + (long long)le_hi - (long long)le_p - 1; dst = Rpos; }
-        if (!dst) continue;
-        if (slot >= (long long)l && slot < (long long)h) dst[slot] = (unsigned)p;
+        long long slot;
+        if (p <= j && c > 0) slot = (long long)l + (long long)(p - l - 1) - (long long)(le_p - le_lo);
+        else if (p > j && c <= 0) slot = (long long)h - (long long)le_hi + (long long)le_p;
+        else continue;
+        if (slot >= (long long)l && slot < (long long)h) trade[slot] = (unsigned)p;
         else flag_error(derr, DERR_INDEX);
     }
 }
@@ -309,9 +314,8 @@ __global__ void k_qs_pos(const unsigned* __restrict__ lo, const unsigned* __rest
 // range.  buf: which buffer K2 and P2 are.
 __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, const unsigned long long* __restrict__ K,
                           const unsigned* __restrict__ P, const unsigned long long* __restrict__ S, long long n,
-                          const unsigned* __restrict__ Lpos, const unsigned* __restrict__ Rpos,
-                          unsigned long long* __restrict__ K2, unsigned* __restrict__ P2, unsigned* __restrict__ fin,
-                          const unsigned* prev, unsigned* active, unsigned depth, unsigned buf, QsLists lists,
+                          const unsigned* __restrict__ trade, unsigned long long* __restrict__ K2,
+                          unsigned* __restrict__ P2, unsigned* __restrict__ fin, const unsigned* prev, unsigned* active, unsigned depth, unsigned buf, QsLists lists,
                           unsigned* derr) {
     grid_entry();
     if (qs_idle(prev)) return;
@@ -329,24 +333,24 @@ __global__ void k_qs_move(unsigned* __restrict__ lo, unsigned* __restrict__ hi, 
             continue;
         }
         const unsigned long long kp = K[l];
-        // slot of the k-th element > P in (l, j] counted from the left, or of
-        // the k-th element <= P in (j, h) counted from the right
-        auto left_slot = [&](long long x) { return (long long)l + (x - l - 1) - (long long)(qs_le(S[x]) - qs_le(sl)); };
-        auto right_slot = [&](long long x) { return (long long)l + (long long)qs_le(sh) - (long long)qs_le(S[x]) - 1; };
+        // the partner's slot of the k-th element > P in (l, j] counted from the
+        // left, or of the k-th element <= P in (j, h) counted from the right
+        auto left = [&](long long x) { return (long long)h - 1 - (x - l - 1) + (long long)(qs_le(S[x]) - qs_le(sl)); };
+        auto right = [&](long long x) { return (long long)l + (long long)qs_le(sh) - (long long)qs_le(S[x]) - 1; };
         long long q = p, slot = -1;
-        const unsigned* from = nullptr;
+        bool trades = false;
         if (p == (long long)l) {
             q = j;
-            if (j > (long long)l && qs_cmp(K[j], kp) > 0) { slot = left_slot(j); from = Rpos; }
+            if (j > (long long)l && qs_cmp(K[j], kp) > 0) { slot = left(j); trades = true; }
         } else if (p == j) {
             q = l;
         } else {
             const int c = qs_cmp(K[p], kp);
-            if (p < j && c > 0) { slot = left_slot(p); from = Rpos; }
-            else if (p > j && c <= 0) { slot = right_slot(p); from = Lpos; }
+            if (p < j && c > 0) { slot = left(p); trades = true; }
+            else if (p > j && c <= 0) { slot = right(p); trades = true; }
         }
-        if (from) {
-            if (slot >= (long long)l && slot < (long long)h) q = from[slot];
+        if (trades) {
+            if (slot >= (long long)l && slot < (long long)h) q = trade[slot];
             else { flag_error(derr, DERR_INDEX); q = p; }
         }
         if (q < (long long)l || q >= (long long)h) { flag_error(derr, DERR_INDEX); q = p; }
@@ -388,7 +392,7 @@ struct QsDepths {
     unsigned long long* K[2];  // images and rows by position, of even and odd depths of this launch
     unsigned* P[2];
     unsigned long long *S, *ts;  // block-relative prefixes, the blocks' totals
-    unsigned *Lpos, *Rpos, *fin;
+    unsigned *trade, *fin;
     unsigned *act, *bar;  // elements left after each depth of this launch; the barrier's arrivals (all zero)
     unsigned* done;       // depths run, then elements left
     QsLists lists;
@@ -515,12 +519,11 @@ __global__ void __launch_bounds__(QD_THREADS, 1) k_qs_depths(const __grid_consta
             if (l == QS_DONE || l == p) continue;
             const unsigned le_p = qs_le(rel[k]);
             const long long j = (long long)l + (qs_le(sh[k]) - qs_le(sl[k]));
-            long long slot = -1;
-            unsigned* dst = nullptr;
-            if (p <= j && c[k] > 0) { slot = (long long)l + (long long)(p - l - 1) - (long long)(le_p - qs_le(sl[k])); dst = a.Lpos; }
-            else if (p > j && c[k] <= 0) { slot = (long long)l + (long long)qs_le(sh[k]) - (long long)le_p - 1; dst = a.Rpos; }
-            if (!dst) continue;
-            if (slot >= (long long)l && slot < (long long)hi[k]) dst[slot] = p;
+            long long slot;
+            if (p <= j && c[k] > 0) slot = (long long)l + (long long)(p - l - 1) - (long long)(le_p - qs_le(sl[k]));
+            else if (p > j && c[k] <= 0) slot = (long long)hi[k] - (long long)qs_le(sh[k]) + (long long)le_p;
+            else continue;
+            if (slot >= (long long)l && slot < (long long)hi[k]) a.trade[slot] = p;
             else flag_error(a.derr, DERR_INDEX);
         }
         if (!qd_barrier(a.bar, target, a.derr)) return;
@@ -536,26 +539,26 @@ __global__ void __launch_bounds__(QD_THREADS, 1) k_qs_depths(const __grid_consta
                 lo[k] = QS_DONE;
                 continue;
             }
-            auto left_slot = [&](long long x, unsigned le_x) { return (long long)l + (x - l - 1) - (long long)(le_x - qs_le(sl[k])); };
+            auto left = [&](long long x, unsigned le_x) { return (long long)h - 1 - (x - l - 1) + (long long)(le_x - qs_le(sl[k])); };
             long long q = p, slot = -1;
-            const unsigned* from = nullptr;
+            bool trades = false;
             if (p == l) {
                 q = j;
                 if (j > (long long)l && qs_cmp(__ldcg(K + j), kp[k]) > 0) {
-                    slot = left_slot(j, qs_le(prefix((unsigned)j)));
-                    from = a.Rpos;
+                    slot = left(j, qs_le(prefix((unsigned)j)));
+                    trades = true;
                 }
             } else if (p == j) {
                 q = l;
             } else if (p < j && c[k] > 0) {
-                slot = left_slot(p, qs_le(rel[k]));
-                from = a.Rpos;
+                slot = left(p, qs_le(rel[k]));
+                trades = true;
             } else if (p > j && c[k] <= 0) {
                 slot = (long long)l + (long long)qs_le(sh[k]) - (long long)qs_le(rel[k]) - 1;
-                from = a.Lpos;
+                trades = true;
             }
-            if (from) {
-                if (slot >= (long long)l && slot < (long long)h) q = __ldcg(from + slot);
+            if (trades) {
+                if (slot >= (long long)l && slot < (long long)h) q = __ldcg(a.trade + slot);
                 else { flag_error(a.derr, DERR_INDEX); q = p; }
             }
             if (q < (long long)l || q >= (long long)h) { flag_error(a.derr, DERR_INDEX); q = p; }
@@ -655,7 +658,7 @@ __global__ void __launch_bounds__(256) k_qs_warps(QsLists lists, const unsigned 
     const unsigned lane = lane_id(), w = threadIdx.x >> 5, n = lists.cnt->nwarp;
     unsigned deep = 0;
     for (unsigned r = blockIdx.x * 8 + w; r < n; r += gridDim.x * 8) {
-        const QsRange g = lists.warp[r].range();
+        const QsRange g = lists.warp_entry(r).range();
         const unsigned m = g.hi - g.lo;
         unsigned long long k = 0;
         unsigned p = 0;
@@ -721,7 +724,7 @@ k_qs_blocks(const __grid_constant__ QsLists lists, const unsigned long long* __r
                 at -= cnt[q];
                 c = q - 1;
             }
-        const QsRange g = lists.block[c][at];
+        const QsRange g = lists.block_entry(c, at).range();
         const unsigned m = g.hi - g.lo;
         if (threadIdx.x == 0) sm.nsmall = sm.depth = 0;
         unsigned long long key[QB_ITEMS];
@@ -915,7 +918,7 @@ __global__ void __launch_bounds__(256) k_qs_stable_small(QsLists lists, const un
     grid_entry();
     const unsigned lane = lane_id(), n = lists.cnt->nwarp;
     for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
-        const QsRange g = lists.warp[r].range();
+        const QsRange g = lists.warp_entry(r).range();
         const unsigned m = g.hi - g.lo;
         const unsigned long long k = lane < m ? img[g.lo + lane] : ~0ull;
         const unsigned row = lane < m ? perm[g.lo + lane] : 0u;
@@ -1024,13 +1027,16 @@ static I qs_too_deep(long long levels) {
 
 static I qs_lists_alloc(long long n, QsLists* q) {
     bool ok = true;
-    for (int c = 0; c < QB_CLASSES; c++) {  // the class's shortest range: one more than the class below holds
-        q->block[c] = (QsRange*)salloc((size_t)(n / (c ? qb_rows(c - 1) : QS_WARP) + 1) * sizeof(QsRange));
+    const size_t ends = (size_t)(n / 2 + 1);
+    q->ends = (QsEntry*)salloc(ends * sizeof(QsEntry));
+    ok = ok && q->ends;
+    q->block[0] = q->ends + (ends - 1);
+    for (int c = 1; c < QB_CLASSES; c++) {  // the class's shortest range: one more than the class below holds
+        q->block[c] = (QsEntry*)salloc((size_t)(n / qb_rows(c - 1) + 1) * sizeof(QsEntry));
         ok = ok && q->block[c];
     }
-    q->warp = (QsShort*)salloc((size_t)(n / 2 + 1) * sizeof(QsShort));
     q->cnt = (QsCounters*)salloc(sizeof(QsCounters));
-    return ok && q->warp && q->cnt ? 0 : E_DEVICE_OOM;
+    return ok && q->cnt ? 0 : E_DEVICE_OOM;
 }
 
 // NaN keys, from counters already read back
@@ -1103,6 +1109,7 @@ static I qs_all_blocks(const QsLists& lists, const QsCounters& h, const unsigned
 // position's row.
 static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsigned* seg, const long long* starts,
                 long long ns, const uint8_t* mode, const QsLists& lists, QsCounters* h, unsigned* fin) {
+    ScratchScope ss;  // the next column of a list takes the same memory
     const unsigned g = qs_grid(n);
     const long long max_levels = qs_max_levels(n);
     unsigned long long* K2 = nullptr;  // the second buffer (img and perm are the first)
@@ -1128,9 +1135,8 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
         K2 = (unsigned long long*)salloc((size_t)n * 8);
         unsigned long long* S = (unsigned long long*)salloc((size_t)(n + 1) * 8);
         unsigned long long* ts = (unsigned long long*)salloc((size_t)(nt > QD_MAX_BLOCKS ? nt : QD_MAX_BLOCKS) * 8);
-        unsigned* Lpos = (unsigned*)salloc((size_t)n * 4);
-        unsigned* Rpos = (unsigned*)salloc((size_t)n * 4);
-        if (!P2 || !K2 || !S || !ts || !Lpos || !Rpos) return E_DEVICE_OOM;
+        unsigned* trade = (unsigned*)salloc((size_t)n * 4);
+        if (!P2 || !K2 || !S || !ts || !trade) return E_DEVICE_OOM;
         // the ranges listed at the start are read from perm/img, which the
         // depths below reuse only at the positions of larger ranges
         unsigned* Pc = perm;
@@ -1143,7 +1149,7 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                 round = (int)(max_levels - level < QD_ROUND ? max_levels - level : QD_ROUND);
                 if (!act_clear) HG_CU(cudaMemsetAsync(act, 0, nact * 4, g_stream));
                 act_clear = false;
-                QsDepths q{lo, hi, {Kc, Kc == img ? K2 : img}, {Pc, Pc == perm ? P2 : perm}, S, ts, Lpos, Rpos, fin,
+                QsDepths q{lo, hi, {Kc, Kc == img ? K2 : img}, {Pc, Pc == perm ? P2 : perm}, S, ts, trade, fin,
                            act, act + QD_ROUND, act + QD_ROUND + 1, lists, g_derr, (unsigned)n, (unsigned)level,
                            (unsigned)round, Kc == img ? 0u : 1u};
                 HG_CHECK(qs_depths_launch(n, q, &resident));
@@ -1176,10 +1182,10 @@ static I qs_run(long long n, unsigned* perm, unsigned long long* img, const unsi
                 HG_LAUNCH("qs_count", (unsigned)nt, QS_THREADS, 0, k_qs_count, lo, Kc, n, ts, prev);
                 if (scan) HG_LAUNCH("qs_scan_sums", 1, 1024, 0, k_qs_scan_sums, ts, nt, prev);
                 HG_LAUNCH("qs_prefix", (unsigned)nt, QS_THREADS, 0, k_qs_prefix, lo, Kc, n, ts, scan ? 1 : 0, S, left);
-                HG_LAUNCH("qs_pos", g, 256, 0, k_qs_pos, lo, hi, Kc, S, n, Lpos, Rpos, prev, g_derr);
+                HG_LAUNCH("qs_pos", g, 256, 0, k_qs_pos, lo, hi, Kc, S, n, trade, prev, g_derr);
                 unsigned* Pn = Pc == perm ? P2 : perm;
                 unsigned long long* Kn = Kc == img ? K2 : img;
-                HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, Lpos, Rpos, Kn, Pn, fin, prev, act + d,
+                HG_LAUNCH("qs_move", g, 256, 0, k_qs_move, lo, hi, Kc, Pc, S, n, trade, Kn, Pn, fin, prev, act + d,
                           (unsigned)(level + d), Kn == img ? 0u : 1u, lists, g_derr);
                 Pc = Pn;
                 Kc = Kn;

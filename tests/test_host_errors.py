@@ -129,3 +129,18 @@ for x, rc in ((one, 1), (L.list([]), 1), (a, 1), (L.list([a, b]), 5), (L.list([a
     assert L.rc("pfnGroupTrie", x) == rc, (x.len, L.lib.hgpuLastError())
     assert (count("k_trie_present")[0] > 0) == (rc == 0)
 """)
+
+
+@pytest.mark.parametrize("cols,kernel,arg,row", [(1, "k_qs_whole", 1, 53), (2, "k_qs_mode", 8, 68)])
+def test_quicksort_scratch_of_listed_ranges(child, cols, kernel, arg, row):
+    """The lists of ranges and the trades add little to what the quicksort's
+    buffers take: 52 bytes of scratch a row for a vector, 67 for a list of
+    columns."""
+    child(r"""
+n, cols, row = 4_000_000, %d, %d
+x = column(H_E, n, 8)
+fake.fake_reset()
+fake.fake_poke(%r, %d, 32, 4, 1)  # QsCounters::nbig: one range for the depths
+assert L.rc("pfnOrderBy", *((x, up) if cols == 1 else (L.list([x] * cols), L.vec(np.array([True] * cols), H_B)))) == 0
+assert count("k_qs_move")[0] > 0
+""" % (cols, row, kernel.encode(), arg), HGPU_SCRATCH_LIMIT_MB=str(4_000_000 * row >> 20))
