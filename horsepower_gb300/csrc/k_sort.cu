@@ -387,7 +387,8 @@ static I rx_sort(SRC src, long long n, const KR** kres, const unsigned** vres, c
         pl.bits = pl.bits > 8 ? 8 : pl.bits;
         pl.npass = (total + pl.bits - 1) / pl.bits;
     }
-    unsigned* counts = (unsigned*)salloc((size_t)RX_MAX_PER_SM * g_sms * RX_MAX_DIGITS * 4);
+    // (the smallest tile makes the most chunks)
+    unsigned* counts = (unsigned*)salloc(((size_t)rx_chunks((n + RX_KV_TILE - 1) / RX_KV_TILE, RX_MAX_PER_SM) << pl.bits) * 4);
     unsigned* tot = (unsigned*)salloc((size_t)pl.npass * RX_MAX_DIGITS * 4);
     // key or record buffers, and u32 row ids where they are a result or
     // travel beside the keys; the last pass of a permutation alone writes neither

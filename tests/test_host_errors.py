@@ -144,3 +144,16 @@ fake.fake_poke(%r, %d, 32, 4, 1)  # QsCounters::nbig: one range for the depths
 assert L.rc("pfnOrderBy", *((x, up) if cols == 1 else (L.list([x] * cols), L.vec(np.array([True] * cols), H_B)))) == 0
 assert count("k_qs_move")[0] > 0
 """ % (cols, row, kernel.encode(), arg), HGPU_SCRATCH_LIMIT_MB=str(4_000_000 * row >> 20))
+
+
+def test_radix_scratch_of_small_orders(child):
+    """The digit counts of a radix pass are sized by its chunks: an order of
+    20,000 rows takes less than a megabyte of scratch."""
+    child(r"""
+for typ, width in ((H_I, 4), (H_L, 8)):
+    x = column(typ, 20_000, width)
+    for d in (up, down):
+        fake.fake_reset()
+        assert L.rc("pfnOrderBy", x, d) == 0, L.lib.hgpuLastError()
+        assert count("k_rx_scatter")[0] > 0
+""", HGPU_SCRATCH_LIMIT_MB="1")
