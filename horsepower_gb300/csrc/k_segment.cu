@@ -143,6 +143,8 @@ __device__ __forceinline__ void seg_load16(const T* __restrict__ src, const long
 
 // The columns one launch reduces over the same segments: block row blockIdx.y
 // takes column blockIdx.y.
+// (a __grid_constant__ parameter where that saves the stack frame that an index
+// into a copy takes; k_seg_mid, which has no register left, is faster without)
 constexpr int SEG_MANY = 4;
 template <typename T, typename A>
 struct SegIO {
@@ -227,8 +229,8 @@ __global__ void k_seg_class_ids(const long long* __restrict__ starts, long long 
 constexpr int SEG_LANE_ITEMS = 4;
 __host__ __device__ constexpr int seg_lanes(int c) { return c <= 2 ? 1 : (1 << c) / SEG_LANE_ITEMS; }  // L of class c
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256) k_seg_warps(SegIO<T, A> io, const long long* __restrict__ rows,
-                                                   long long nx, const long long* __restrict__ starts, long long ng,
+__global__ void __launch_bounds__(256) k_seg_warps(const __grid_constant__ SegIO<T, A> io,
+                                                   const long long* __restrict__ rows, long long nx, const long long* __restrict__ starts, long long ng,
                                                    long long total, const unsigned* __restrict__ ids,
                                                    const unsigned* __restrict__ cnt, A ident,
                                                    unsigned* derr) {
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long l
 template <typename A, int OP>
 __global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ parts, const long long* __restrict__ pstarts,
                                                       const long long* __restrict__ big, long long nbig,
-                                                      long long nchunks, A ident, SegIO<A, A> io) {
+                                                      long long nchunks, A ident, const __grid_constant__ SegIO<A, A> io) {
     grid_entry();
     __shared__ A ws[256];
     const long long g = blockIdx.x;
@@ -409,8 +411,8 @@ __global__ void __launch_bounds__(256) k_seg_partials(const A* __restrict__ part
 // descriptor (one 16-byte load; finding the chunk by a binary search over the
 // segments instead put seven dependent loads before its first row)
 template <typename T, typename A, int OP, bool GATHER>
-__global__ void __launch_bounds__(256, 4) k_seg_chunk(SegIO<T, A> io, const long long* __restrict__ rows,
-                                                      long long nx, const ChunkDesc* __restrict__ order, A ident,
+__global__ void __launch_bounds__(256, 4) k_seg_chunk(const __grid_constant__ SegIO<T, A> io,
+                                                      const long long* __restrict__ rows, long long nx, const ChunkDesc* __restrict__ order, A ident,
                                                       A* __restrict__ part, unsigned* derr) {
     grid_entry();
     const T* __restrict__ src = io.src[blockIdx.y];
@@ -797,7 +799,8 @@ void seg_plan_adopt(ListInfo& li, const SmallPlan& p) {
 // bit-identical to k_seg_chunk's for that column.
 struct SegCols { const double* src[SEG_MANY]; };
 template <int NCOL>
-__global__ void __launch_bounds__(256, 4) k_seg_chunk_many(SegCols cols, const long long* __restrict__ rows, long long nx,
+__global__ void __launch_bounds__(256, 4) k_seg_chunk_many(const __grid_constant__ SegCols cols,
+                                                           const long long* __restrict__ rows, long long nx,
                                                            unsigned long long nchunks,
                                                            const ChunkDesc* __restrict__ order,
                                                            double* __restrict__ part, unsigned* derr) {
