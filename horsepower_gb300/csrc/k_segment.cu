@@ -106,21 +106,21 @@ __device__ __forceinline__ A sblock8(A acc, A* sh) {
     return r;
 }
 
-// 16 elements of one lane, STRIDE apart: positions first + k * STRIDE, k =
-// 0..15, those below `end` loaded (row numbers first, then the values, so all
-// 16 gathers are in flight together).
-template <typename T, bool GATHER, int STRIDE>
-__device__ __forceinline__ void seg_load16s(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
-                                            long long first, long long end, T v[16], bool& bad) {
+// N elements of one lane, STRIDE apart: positions first + k * STRIDE, k = 0 ..
+// N - 1, those below `end` loaded (row numbers first, then the values, so all N
+// gathers are in flight together).
+template <typename T, bool GATHER, int STRIDE, int N>
+__device__ __forceinline__ void seg_load(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
+                                         long long first, long long end, T (&v)[N], bool& bad) {
     if constexpr (GATHER) {
-        long long r[16];
+        long long r[N];
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
+        for (int k = 0; k < N; k++) {
             const long long j = first + (long long)k * STRIDE;
             r[k] = j < end ? rows[j] : 0;
         }
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
+        for (int k = 0; k < N; k++) {
             const bool in = first + (long long)k * STRIDE < end;
             const bool ok = r[k] >= 0 && r[k] < nx;
             bad |= in && !ok;
@@ -128,7 +128,7 @@ __device__ __forceinline__ void seg_load16s(const T* __restrict__ src, const lon
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
+        for (int k = 0; k < N; k++) {
             const long long j = first + (long long)k * STRIDE;
             v[k] = j < end ? src[j] : T(0);
         }
@@ -137,8 +137,8 @@ __device__ __forceinline__ void seg_load16s(const T* __restrict__ src, const lon
 // the 16 elements of one lane of a 256-lane tile
 template <typename T, bool GATHER>
 __device__ __forceinline__ void seg_load16(const T* __restrict__ src, const long long* __restrict__ rows, long long nx,
-                                           long long first, long long end, T v[16], bool& bad) {
-    seg_load16s<T, GATHER, 256>(src, rows, nx, first, end, v, bad);
+                                           long long first, long long end, T (&v)[16], bool& bad) {
+    seg_load<T, GATHER, 256>(src, rows, nx, first, end, v, bad);
 }
 
 // The columns one launch reduces over the same segments: block row blockIdx.y
@@ -308,13 +308,14 @@ __global__ void __launch_bounds__(256) k_seg_warps(const __grid_constant__ SegIO
 // all 8 virtual warps at once; the block's longer segments are taken one after
 // another by all 8 warps, warp v as virtual warp v.  (One warp walking the 8
 // virtual warps in turn, for every size: 0.98 ms against 0.61 ms for the
-// 157K mid-size groups of a 150M-row Zipf grouping.)
+// 157K mid-size groups of a 150M-row Zipf grouping.)  `walk`: rounds of eight
+// such segments are k_seg_walk's.
 template <typename T, typename A, int OP, bool GATHER>
 __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long long* __restrict__ rows,
                                                  long long nx, const long long* __restrict__ starts, long long ng,
                                                  long long total, const unsigned* __restrict__ ids,
                                                  const unsigned* __restrict__ cnt, A ident,
-                                                 unsigned* derr) {
+                                                 int walk, unsigned* derr) {
     grid_entry();
     const T* __restrict__ src = io.src[blockIdx.y];
     A* __restrict__ out = io.out[blockIdx.y];
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long l
         if (lane == 0) sbig[warp] = m > 512 ? g : -1;
         if (g >= 0 && m <= 512) {
             T x[16];  // x[v + 8 k]: element k of lane `lane` of virtual warp v
-            seg_load16s<T, GATHER, 32>(src, rows, nx, s + lane, e, x, bad);
+            seg_load<T, GATHER, 32>(src, rows, nx, s + lane, e, x, bad);
             A acc[8], r;
 #pragma unroll
             for (int v = 0; v < 8; v++) {
@@ -362,7 +363,10 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long l
             if (lane == 0) out[g] = r;
         }
         __syncthreads();
-        for (int q = 0; q < 8; q++) {
+        int nq = walk ? 0 : 8;  // 0: all eight are k_seg_walk's
+        for (int q = 0; q < 8; q++)
+            if (sbig[q] < 0) nq = 8;
+        for (int q = 0; q < nq; q++) {
             const long long gb = sbig[q];  // the same in every warp
             if (gb < 0) continue;
             const long long sb = starts[gb], eb = (gb + 1 < ng) ? starts[gb + 1] : total;
@@ -377,6 +381,59 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long l
             __syncthreads();
         }
         __syncthreads();  // sbig is rewritten by the next round
+    }
+    if (bad) flag_error(derr, DERR_INDEX);
+}
+
+// The rounds of k_seg_mid whose eight segments are all longer than 512, when
+// there are several rounds to a block and the class can average more than 512
+// rows (seg_reduce): each warp walks a segment of its own, 256 elements (a lane's
+// element of each of the 8 virtual warps) at a time.  A grouping's row lists
+// are ascending, so the warps of the chip walk through the column side by side
+// and meet in its sectors, where a segment read at once takes them from all of
+// the column.  Groups of 1000 rows, f64 sums: 60M rows 1.25 ms by k_seg_mid
+// alone and 1.15 so, 150M rows 3.25 and 3.03; of 3000, 150M rows 3.24 and 2.93.
+// With one round to a block it is the other way round (20M rows in groups of
+// 1000: 0.42 and 0.71 ms).  Five blocks an SM spill (3.25 ms at 150M rows).
+template <typename T, typename A, int OP, bool GATHER>
+__global__ void __launch_bounds__(256, 4) k_seg_walk(const __grid_constant__ SegIO<T, A> io,
+                                                     const long long* __restrict__ rows, long long nx,
+                                                     const long long* __restrict__ starts, long long ng,
+                                                     long long total, const unsigned* __restrict__ ids,
+                                                     const unsigned* __restrict__ cnt, A ident, unsigned* derr) {
+    grid_entry();
+    const T* __restrict__ src = io.src[blockIdx.y];
+    A* __restrict__ out = io.out[blockIdx.y];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    unsigned first = 0;
+    for (int c = 0; c < 6; c++) first += cnt[c];
+    const long long n6 = cnt[6];
+    bool bad = false;
+    for (long long w0 = blockIdx.x; w0 < n6; w0 += (long long)gridDim.x * 8) {
+        const long long w = w0 + (long long)gridDim.x * (lane & 7);  // lane q looks at warp q's segment
+        long long g = 0, s = 0, e = 0;
+        if (w < n6) {
+            g = ids[first + w];
+            s = starts[g];
+            e = (g + 1 < ng) ? starts[g + 1] : total;
+        }
+        if (!__all_sync(0xffffffffu, e - s > 512)) continue;
+        g = __shfl_sync(0xffffffffu, g, warp);
+        s = __shfl_sync(0xffffffffu, s, warp);
+        e = __shfl_sync(0xffffffffu, e, warp);
+        A acc[8];
+#pragma unroll
+        for (int v = 0; v < 8; v++) acc[v] = ident;
+#pragma unroll 1
+        for (long long b = s; b < e; b += 256) {
+            T x[8];
+            seg_load<T, GATHER, 32>(src, rows, nx, b + lane, e, x, bad);
+#pragma unroll
+            for (int v = 0; v < 8; v++)
+                if (b + v * 32 + (int)lane < e) acc[v] = sop<A, OP>(acc[v], (A)x[v]);
+        }
+        const A r = stile8<A, OP>(acc);
+        if (lane == 0) out[g] = r;
     }
     if (bad) flag_error(derr, DERR_INDEX);
 }
@@ -880,9 +937,16 @@ static I seg_reduce(const SegIO<T, A>& io, int ncol, const long long* rows, long
     if (small_w)
         HG_LAUNCH("seg_warps", dim3(gcap(small_w * 32), nc), 256, 0, (k_seg_warps<T, A, OP, GATHER>), io, rows, nx,
                   starts, ng, total, ids, ccnt, ident, g_derr);
-    if (mid_w)
-        HG_LAUNCH("seg_mid", dim3(gcap(mid_w * 32), nc), 256, 0, (k_seg_mid<T, A, OP, GATHER>), io, rows, nx, starts,
-                  ng, total, ids, ccnt, ident, g_derr);
+    if (mid_w) {
+        const unsigned g = gcap(mid_w * 32);
+        const long long rest = total - (long long)(li->nchunks - li->nbig) * TILE_SUM;  // no fewer than class 6 holds
+        const int walk = mid_w > (long long)g * 8 && rest > 512 * mid_w;
+        HG_LAUNCH("seg_mid", dim3(g, nc), 256, 0, (k_seg_mid<T, A, OP, GATHER>), io, rows, nx, starts, ng, total, ids,
+                  ccnt, ident, walk, g_derr);
+        if (walk)
+            HG_LAUNCH("seg_walk", dim3(g, nc), 256, 0, (k_seg_walk<T, A, OP, GATHER>), io, rows, nx, starts, ng, total,
+                      ids, ccnt, ident, g_derr);
+    }
     const long long nbig = li->nbig;
     const unsigned long long nchunks = li->nchunks;
     if (nbig == 0) return last_launch_error();

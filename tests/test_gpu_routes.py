@@ -229,3 +229,43 @@ def test_one_unaligned_operand(gpu, typ, n):
         for sa, sb in ((1, 0), (0, 1), (1, 3), (5, 5)):
             assert run(column(a, sa), column(b, sb)) == want, (f, sa, sb)
     gpu.free_inputs()
+
+
+@pytest.mark.parametrize("length,every,short,walks", [
+    (513, 0, 0, True),          # every round's eight segments are long
+    (640, 97, 40, True),        # most rounds'
+    (1100, 3, 512, True),       # none: a third of the segments is not
+    (513, 2, 33, False),        # the class averages fewer than 512 rows
+])
+def test_long_mid_segments_walk(gpu, ora, length, every, short, walks):
+    """More mid-size segments than one round of the grid takes, long on
+    average: rounds of eight segments above 512 rows go to a kernel in which
+    each warp walks one.  i64 sums and maxima equal numpy's, f64 sums the fixed
+    tile tree of their rows, in rounds of either kind."""
+    ora.lib.hgoTreeSumF64.restype = C.c_double
+    ora.lib.hgoTreeSumF64.argtypes = [C.c_void_p, C.c_longlong]
+    groups = 32 * 8 * 152 + 1003
+    sizes = np.full(groups, length)
+    if every:
+        sizes[::every] = short
+    rng = np.random.default_rng(length)
+    key = np.repeat(np.arange(groups, dtype=np.int32), sizes)
+    key = np.roll(key, 12_345)          # groups are found by value, not by place
+    n = key.size
+    pay = rng.standard_normal(n) * 10.0 ** rng.integers(-6, 6, n)
+    ipay = rng.integers(-2 ** 62, 2 ** 62, n)
+    vals = gpu.call("pfnValues", gpu.call("pfnGroup", gpu.vec(key, H_I)))
+    dpay, dipay = gpu.vec(pay, H_E), gpu.vec(ipay, H_L)
+    sums, ran = launches(gpu, lambda: gpu.to_py(gpu.call("hgpuGroupSum", dpay, vals)))
+    assert ("seg_walk" in ran) == walks, ran
+    isums = gpu.to_py(gpu.call("hgpuGroupSum", dipay, vals))
+    imax = gpu.to_py(gpu.call("hgpuGroupMax", dipay, vals))
+    order = np.argsort(key, kind="stable")
+    starts = np.r_[0, np.cumsum(sizes)[:-1]]
+    assert np.array_equal(isums, np.add.reduceat(ipay[order], starts))
+    assert np.array_equal(imax, np.maximum.reduceat(ipay[order], starts))
+    for g in np.r_[:20, rng.integers(0, groups, 400), groups - 20:groups]:
+        x = np.ascontiguousarray(pay[order[starts[g]:starts[g] + sizes[g]]])
+        want = ora.lib.hgoTreeSumF64(x.ctypes.data, x.size)
+        assert sums[g].tobytes() == np.float64(want).tobytes(), (g, sizes[g])
+    gpu.free_inputs()
