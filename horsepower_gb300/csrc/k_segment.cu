@@ -308,14 +308,15 @@ __global__ void __launch_bounds__(256) k_seg_warps(const __grid_constant__ SegIO
 // all 8 virtual warps at once; the block's longer segments are taken one after
 // another by all 8 warps, warp v as virtual warp v.  (One warp walking the 8
 // virtual warps in turn, for every size: 0.98 ms against 0.61 ms for the
-// 157K mid-size groups of a 150M-row Zipf grouping.)  `walk`: rounds of eight
-// such segments are k_seg_walk's.
-template <typename T, typename A, int OP, bool GATHER>
+// 157K mid-size groups of a 150M-row Zipf grouping.)  WALK: rounds of eight such
+// segments are k_seg_walk's (an instance of its own: looking for them costs
+// groups of 50 rows 2%).
+template <typename T, typename A, int OP, bool GATHER, bool WALK>
 __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long long* __restrict__ rows,
                                                  long long nx, const long long* __restrict__ starts, long long ng,
                                                  long long total, const unsigned* __restrict__ ids,
                                                  const unsigned* __restrict__ cnt, A ident,
-                                                 int walk, unsigned* derr) {
+                                                 unsigned* derr) {
     grid_entry();
     const T* __restrict__ src = io.src[blockIdx.y];
     A* __restrict__ out = io.out[blockIdx.y];
@@ -363,9 +364,12 @@ __global__ void __launch_bounds__(256, 4) k_seg_mid(SegIO<T, A> io, const long l
             if (lane == 0) out[g] = r;
         }
         __syncthreads();
-        int nq = walk ? 0 : 8;  // 0: all eight are k_seg_walk's
-        for (int q = 0; q < 8; q++)
-            if (sbig[q] < 0) nq = 8;
+        int nq = 8;
+        if constexpr (WALK) {
+            nq = 0;  // all eight are k_seg_walk's
+            for (int q = 0; q < 8; q++)
+                if (sbig[q] < 0) nq = 8;
+        }
         for (int q = 0; q < nq; q++) {
             const long long gb = sbig[q];  // the same in every warp
             if (gb < 0) continue;
@@ -940,12 +944,12 @@ static I seg_reduce(const SegIO<T, A>& io, int ncol, const long long* rows, long
     if (mid_w) {
         const unsigned g = gcap(mid_w * 32);
         const long long rest = total - (long long)(li->nchunks - li->nbig) * TILE_SUM;  // no fewer than class 6 holds
-        const int walk = mid_w > (long long)g * 8 && rest > 512 * mid_w;
-        HG_LAUNCH("seg_mid", dim3(g, nc), 256, 0, (k_seg_mid<T, A, OP, GATHER>), io, rows, nx, starts, ng, total, ids,
-                  ccnt, ident, walk, g_derr);
-        if (walk)
-            HG_LAUNCH("seg_walk", dim3(g, nc), 256, 0, (k_seg_walk<T, A, OP, GATHER>), io, rows, nx, starts, ng, total,
-                      ids, ccnt, ident, g_derr);
+        const bool walk = mid_w > (long long)g * 8 && rest > 512 * mid_w;
+        auto launch = [&](const char* name, auto kern) {
+            HG_LAUNCH(name, dim3(g, nc), 256, 0, kern, io, rows, nx, starts, ng, total, ids, ccnt, ident, g_derr);
+        };
+        launch("seg_mid", walk ? k_seg_mid<T, A, OP, GATHER, true> : k_seg_mid<T, A, OP, GATHER, false>);
+        if (walk) launch("seg_walk", k_seg_walk<T, A, OP, GATHER>);
     }
     const long long nbig = li->nbig;
     const unsigned long long nchunks = li->nchunks;
